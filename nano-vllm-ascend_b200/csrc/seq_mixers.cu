@@ -12,6 +12,7 @@
 //                      computed per token from a projected dt (the selective state-space form of Mamba-2), or a
 //                      forget gate per key channel that also decides what is written (k = 1 - f: the tied form
 //                      of HGRN2), S_t = diag(f_t) S_(t-1) + (1 - f_t) v_t^T.
+#include "attn_tiled.cuh"
 #include "seq_common.cuh"
 
 namespace b200 {
@@ -676,6 +677,14 @@ extern "C" int b200_attn_generic(void* out, const void* q, int64_t q_stride, con
   B200_RETURN_IF(window < 0 || keep_first < 0 || chunk < 0 || (window > 0 && chunk > 0) || (!v && vdim > dim), B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(!block_tables && !cu_q, B200_ERR_NULL_POINTER);       // decode rows read the paged cache
   const int rep = num_heads / num_kv_heads;
+  if (cu_q && attn_tiled_fits(max_q, rep, dim, vdim)) {              // prompt portions: 64 rows share every key tile
+    AttnTiledParams A;
+    A.out = out, A.q = q, A.k = k, A.v = v, A.q_stride = q_stride, A.k_stride = k_stride, A.v_stride = v_stride;
+    A.block_tables = block_tables, A.bt_stride = bt_stride, A.block_size = block_size, A.cu_q = cu_q, A.cu_k = cu_k;
+    A.H = num_heads, A.G = num_kv_heads, A.dim = dim, A.vdim = vdim, A.scale = scale, A.window = window;
+    A.keep_first = keep_first, A.chunk = chunk, A.softcap = softcap, A.sink = sink, A.gate = gate, A.gate_stride = gate_stride;
+    return attn_tiled_launch(A, num_seqs, max_q, dtype, (cudaStream_t)stream);
+  }
   const dim3 grid((max_q * rep + kAttnRows - 1) / kAttnRows, num_kv_heads, num_seqs);
   const size_t smem = (size_t)(kAttnRows * dim + kAttnKeys * (dim + 1) + (v ? kAttnKeys * vdim : 0)) * sizeof(float);
   B200_RETURN_IF(smem > 200 * 1024, B200_ERR_UNSUPPORTED);
