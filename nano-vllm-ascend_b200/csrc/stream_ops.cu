@@ -297,6 +297,62 @@ delta_prep_kernel(float* __restrict__ qk, float* __restrict__ decay, float* __re
   if (lane == 0) beta[(int64_t)t * H + h] = sigmoid_f(to_f32<T>(b[(int64_t)t * b_stride + h]));
 }
 
+// The same with 8 elements per lane: gl adjacent lanes (a power of two, 8 gl >= dim) share a unit, 32 / gl units per warp. dim,
+// the strides and the bases in multiples of 16 bytes. What bounds it is HBM (reads 2, writes 4 bytes per q, k and decay
+// element); the element-wise form moves 64 bytes per warp load. 14,459 tokens of 8 heads over 4 of 128: 76 us -> 56 us, where the
+// exponentials and logarithms of the decays bind it.
+template <typename T>
+__global__ void __launch_bounds__(256)
+delta_prep_vec_kernel(float* __restrict__ qk, float* __restrict__ decay, float* __restrict__ beta,
+                      const T* __restrict__ qk_in, int64_t qk_stride, const T* __restrict__ a, int64_t a_stride,
+                      const T* __restrict__ b, int64_t b_stride, const float* __restrict__ dt_bias,
+                      const float* __restrict__ a_log, int tokens, int H, int G, int dim, float unit_eps, float q_scale,
+                      int per_head, int gl) {
+  pdl_wait();
+  const int lane = threadIdx.x & 31, sub = lane % gl;
+  const int64_t unit = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 / gl) + lane / gl;
+  const int per_tok = 2 * G + (per_head ? 1 : H);
+  const bool live = unit < (int64_t)tokens * per_tok;
+  const int t = live ? (int)(unit / per_tok) : 0, u = live ? (int)(unit % per_tok) : 0;
+  const int i = sub * 8;
+  const bool mine = live && i < dim, is_qk = u < 2 * G;
+  float x[8];
+  float ss = 0.f;
+  if (mine && is_qk) {
+    load8<T>(qk_in + (int64_t)t * qk_stride + (int64_t)u * dim + i, x);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += x[j] * x[j];
+  }
+  for (int o = 1; o < gl; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (!live) return;
+  if (is_qk) {
+    if (!mine) return;
+    const float mul = (u < G ? q_scale : 1.0f) / sqrtf(ss + unit_eps);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] *= mul;
+    store8<float>(qk + (int64_t)t * (2 * G * dim) + (int64_t)u * dim + i, x);
+    return;
+  }
+  if (per_head) {
+    for (int h = sub; h < H; h += gl) {
+      decay[(int64_t)t * H + h] = expf(-expf(a_log[h]) * softplus_f(to_f32<T>(a[(int64_t)t * a_stride + h]) + dt_bias[h]));
+      beta[(int64_t)t * H + h] = sigmoid_f(to_f32<T>(b[(int64_t)t * b_stride + h]));
+    }
+    return;
+  }
+  const int h = u - 2 * G;
+  if (mine) {
+    const float rate = expf(a_log[h]);
+    float bias[8];
+    load8<T>(a + (int64_t)t * a_stride + (int64_t)h * dim + i, x);
+    load8<float>(dt_bias + (int64_t)h * dim + i, bias);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = expf(-rate * softplus_f(x[j] + bias[j]));
+    store8<float>(decay + (int64_t)t * ((int64_t)H * dim) + (int64_t)h * dim + i, x);
+  }
+  if (sub == 0) beta[(int64_t)t * H + h] = sigmoid_f(to_f32<T>(b[(int64_t)t * b_stride + h]));
+}
+
 // ------------------------------------------------------------------ inputs of a wkv recurrence
 // Per (token, head): r and k to fp32, decay = exp(-exp(z + w0)) per key channel, bonus = sum_i r_i u_i k_i. gl = 1 .. 32
 // adjacent lanes per head (the smallest power of two that covers it with 8 elements per lane, VEC; a full warp element by
@@ -726,6 +782,19 @@ extern "C" int b200_delta_prep(float* qk, float* decay, float* beta, const void*
   if (tokens == 0) return B200_OK;
   B200_RETURN_IF(!qk || !decay || !beta || !qk_in || !a || !b || !dt_bias || !a_log, B200_ERR_NULL_POINTER);
   const int64_t units = (int64_t)tokens * (2 * groups + (per_head ? 1 : num_heads));
+  const int64_t lanes16 = dtype == B200_DTYPE_F32 ? 4 : 8;           // elements of 16 bytes
+  const bool vec = dim % 8 == 0 && dim <= 256 && qk_stride % lanes16 == 0 && aligned16(qk_in) && aligned16(qk) &&
+                   (per_head || (a_stride % lanes16 == 0 && aligned16(a) && aligned16(decay) && aligned16(dt_bias)));
+  if (vec) {
+    int gl = 1;
+    while (gl * 8 < dim) gl <<= 1;
+    const int64_t per_cta = 8 * (32 / gl);
+    B200_DISPATCH_3(dtype, T, launch_pdl(delta_prep_vec_kernel<T>, dim3((unsigned)((units + per_cta - 1) / per_cta)), dim3(256),
+                                         0, (cudaStream_t)stream, qk, decay, beta, (const T*)qk_in, qk_stride, (const T*)a,
+                                         a_stride, (const T*)b, b_stride, dt_bias, a_log, tokens, num_heads, groups, dim,
+                                         unit_eps, q_scale, per_head, gl));
+    return finish_launch();
+  }
   const dim3 grid((unsigned)((units + 7) / 8));
   B200_DISPATCH_3(dtype, T, launch_pdl(delta_prep_kernel<T>, grid, dim3(256), 0, (cudaStream_t)stream, qk, decay, beta,
                                        (const T*)qk_in, qk_stride, (const T*)a, a_stride, (const T*)b, b_stride,
