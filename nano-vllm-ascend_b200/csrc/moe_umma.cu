@@ -210,6 +210,237 @@ moe_umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   if (warp == 1) umma::tmem_dealloc(tb, 128);
 }
 
+// ------------------------------------------------------------------------------------ 256-column tiles, persistent
+// The same grouped GEMM for batches that fill the chip. The kernel above is bound by two things: a 1-CTA SS-mode MMA with N =
+// 128 spends 107 cycles on 64 cycles of mathematics (43 to read the 4 KB A tile, measured, tools/umma_probe.cu), and every CTA
+// pays its prologue, its epilogue's scattered 16-byte stores and a cold ring for 12 to 32 K blocks. Here a tile is 128 rows of
+// one expert x 256 weight rows (gate_up: 128 gate + the 128 matching up rows), so that an MMA is M128 N256 K16: 171 cycles for
+// 128 of mathematics; one CTA per SM walks tiles blockIdx.x, + gridDim.x, ..; the accumulators are double-buffered in TMEM
+// (2 x 256 columns), so the ring (4 stages of 16 KB A + 32 KB W) never drains and a tile's epilogue runs under the next
+// tile's products. Row tiles of one expert and one column band are neighbours in the tile order: they run at the same time
+// and their weights come from HBM once. The epilogue passes 32 rows x 64 columns at a time through shared memory, so that
+// global stores are whole 128-byte segments.
+// Measured (4096 tokens, top 8 of 128 experts, hidden 2048, inter 768): gate_up 332 -> 215 us (960 TFLOP/s), down 312 -> 121
+// us (850 TFLOP/s).
+// Waits are bounded: a wait that gives up sets a flag on which every role leaves its loop (g_wait_gave_up counts it).
+__device__ unsigned int g_wait_gave_up;
+
+constexpr int kMwStages = 4;
+constexpr int kMwStageBytes = 3 * kMuPanel;                 // 128 rows of A, 256 rows of W, 64 columns each
+constexpr int kMwOut = 4 * 32 * 128;                        // epilogue: 32 rows x 128 bytes per warp
+constexpr int kMwMaxExperts = 256;
+constexpr int kMwSmem = 1024 + kMwStages * kMwStageBytes + kMwOut + 128 + (kMwMaxExperts + 4) * 4;
+
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
+  for (int n = 0; n < (1 << 24); ++n) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (*gave_up) return false;
+  }
+  *gave_up = 1;
+  atomicAdd(&g_wait_gave_up, 1u);
+  return false;
+}
+
+template <typename T, bool kGateUp>
+__global__ void __launch_bounds__(kMuThreads, 1)
+moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const MoeUmmaParams p) {
+  extern __shared__ __align__(1024) uint8_t mu_smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(mu_smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* s_out = smem + kMwStages * kMwStageBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_out + kMwOut);
+  uint64_t *full = bars, *empty = bars + kMwStages, *acc_full = bars + 2 * kMwStages, *acc_empty = acc_full + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* first = reinterpret_cast<int*>(s_out + kMwOut + 128);      // [num_local + 1] row tiles of the experts before
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  pdl_wait();
+  if (warp == 0) {                                                // prefix sum of the experts' row tiles
+    int before = 0;
+    for (int e0 = 0; e0 < p.num_local; e0 += 32) {
+      const int e = e0 + lane;
+      int n = e < p.num_local ? (p.offsets[e + 1] - p.offsets[e] + 127) >> 7 : 0;
+      const int own = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, n, o);
+        if (lane >= o) n += up;
+      }
+      if (e < p.num_local) first[e] = before + n - own;
+      before += __shfl_sync(0xffffffffu, n, 31);
+    }
+    if (lane == 0) first[p.num_local] = before;
+  }
+  if (threadIdx.x == 32) {
+    for (int s = 0; s < kMwStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 128);
+    }
+    mbar_fence_init();
+    *gave_up = 0;
+  }
+  if (warp == 1) umma::tmem_alloc(tmem_slot, 512);
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tb = *tmem_slot;
+  const int bands = p.n_out / (kGateUp ? 128 : 256), KB = p.K / 64;
+  const int tiles = first[p.num_local] * bands;
+
+  // tile -> expert, first row of the tile inside the expert, column band: experts in order, then bands, then row tiles
+  struct Tile {
+    int e, m0, band;
+  };
+  auto tile_of = [&](int t) {
+    const int rt = t / bands;                                     // an expert's tiles are first[e] * bands ..
+    int lo = 0, hi = p.num_local;                                 // last e with first[e] <= rt
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (first[mid] <= rt) lo = mid;
+      else hi = mid;
+    }
+    const int n = first[lo + 1] - first[lo], in = t - first[lo] * bands;
+    return Tile{lo, (in % n) * 128, in / n};
+  };
+
+  if (warp == 0) {
+    // =========================== TMA producer ===========================
+    if (lane == 0) {
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmW);
+      uint64_t keep;
+      asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
+      const uint64_t stream = l2_policy_evict_first();
+      int it = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+        const Tile tl = tile_of(t);
+        const int row = p.offsets[tl.e] + tl.m0;
+        const int w0 = kGateUp ? tl.e * 2 * p.n_out + tl.band * 128 : tl.e * p.n_out + tl.band * 256;
+        const int w1 = w0 + (kGateUp ? p.n_out : 128);
+        for (int kb = 0; kb < KB; ++kb, ++it) {
+          const int s = it % kMwStages;
+          ok = mbar_wait_bounded(&empty[s], ((it / kMwStages) & 1) ^ 1, gave_up);
+          if (!ok) break;
+          uint8_t* sa = smem + s * kMwStageBytes;
+          mbar_expect_tx(&full[s], kMwStageBytes);
+          tma_load_3d(sa, &tmA, &full[s], 0, row, kb, keep);
+          tma_load_3d(sa + kMuPanel, &tmW, &full[s], 0, w0, kb, stream);
+          tma_load_3d(sa + 2 * kMuPanel, &tmW, &full[s], 0, w1, kb, stream);
+        }
+      }
+      // copies in flight land before the CTA's shared memory is given back (on the ordinary way out they are consumed)
+      if (!ok)
+        for (int s = 0; s < kMwStages; ++s)
+          for (int n = 0; n < (1 << 16); ++n)
+            if (mbar_try_wait(&full[s], 0) && mbar_try_wait(&full[s], 1)) break;
+    }
+  } else if (warp == 1) {
+    // =========================== MMA issuer ===========================
+    const uint32_t idesc = umma::make_idesc<T>(128, 256, 0, 0);
+    const uint64_t ad0 = umma::desc_kmajor(smem_u32(smem)), bd0 = umma::desc_kmajor(smem_u32(smem + kMuPanel));
+    const bool leader = umma::elect_one();
+    int it = 0, n = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++n) {
+      const int buf = n & 1;
+      ok = mbar_wait_bounded(&acc_empty[buf], ((n >> 1) & 1) ^ 1, gave_up);
+      umma::fence_after_sync();
+      for (int kb = 0; kb < KB && ok; ++kb, ++it) {
+        const int s = it % kMwStages;
+        ok = mbar_wait_bounded(&full[s], (it / kMwStages) & 1, gave_up);
+        if (!ok) break;
+        umma::fence_after_sync();
+        if (leader) {
+          const uint64_t ad = umma::desc_advance(ad0, s * kMwStageBytes), bd = umma::desc_advance(bd0, s * kMwStageBytes);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma::mma_ss(tb + buf * 256, umma::desc_advance(ad, ks * 32), umma::desc_advance(bd, ks * 32), idesc,
+                         (kb > 0 || ks > 0) ? 1u : 0u);
+          umma::commit(&empty[s]);
+          if (kb == KB - 1) umma::commit(&acc_full[buf]);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    // =========================== epilogue warps (2..5) ===========================
+    const int quarter = warp & 3;                    // the TMEM lane quarter this warp may access
+    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    uint8_t* stage = s_out + quarter * 32 * 128;
+    T* out = reinterpret_cast<T*>(p.out);
+    int n = 0;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
+      const Tile tl = tile_of(t);
+      const int begin = p.offsets[tl.e], cnt = p.offsets[tl.e + 1] - begin;
+      const int row0 = tl.m0 + quarter * 32;         // this warp's 32 rows inside the expert
+      const bool valid = row0 + lane < cnt;
+      const int64_t pos = begin + row0 + (valid ? lane : 0);
+      const int buf = n & 1;
+      float sc = 1.f;                                // gate_up: weight on the expert's input; down: on its output
+      if (kGateUp) {
+        if (p.in_scale != nullptr && valid) sc = p.in_scale[p.sorted_pair[pos]];
+      } else if (p.pair_scale != nullptr && valid) {
+        sc = to_f32<T>(reinterpret_cast<const T*>(p.pair_scale)[p.sorted_pair[pos]]);
+      }
+      if (!mbar_wait_bounded(&acc_full[buf], (n >> 1) & 1, gave_up)) break;
+      umma::fence_after_sync();
+      const uint32_t acc = tb + lane_base + buf * 256;
+      if (row0 < cnt) {
+        for (int c0 = 0; c0 < (kGateUp ? 128 : 256); c0 += 64) {        // 64 output columns: one 128-byte row per lane
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t a[32], u[32], w[16];
+            umma::ld32(acc + c0 + half * 32, a);
+            if (kGateUp) umma::ld32(acc + 128 + c0 + half * 32, u);
+            umma::wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if (kGateUp) {
+                // gate_up in the model dtype, silu in fp32 -> dtype, dtype multiply (activation.py:11-13)
+                const float g0 = to_f32<T>(from_f32<T>(sc * __uint_as_float(a[2 * j])));
+                const float g1 = to_f32<T>(from_f32<T>(sc * __uint_as_float(a[2 * j + 1])));
+                const float u0 = to_f32<T>(from_f32<T>(sc * __uint_as_float(u[2 * j])));
+                const float u1 = to_f32<T>(from_f32<T>(sc * __uint_as_float(u[2 * j + 1])));
+                const float s0 = to_f32<T>(from_f32<T>(__fdividef(g0, 1.0f + __expf(-g0))));
+                const float s1 = to_f32<T>(from_f32<T>(__fdividef(g1, 1.0f + __expf(-g1))));
+                w[j] = pack2<T>(__fmul_rn(s0, u0), __fmul_rn(s1, u1));
+              } else {
+                // expert output in the model dtype, then a dtype multiply with the routing weight (1 without one)
+                const float y0 = to_f32<T>(from_f32<T>(__uint_as_float(a[2 * j])));
+                const float y1 = to_f32<T>(from_f32<T>(__uint_as_float(a[2 * j + 1])));
+                w[j] = pack2<T>(__fmul_rn(y0, sc), __fmul_rn(y1, sc));
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              *reinterpret_cast<uint4*>(stage + umma::sw128(lane, half * 4 + c)) =
+                  make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+          }
+          __syncwarp();
+          T* to = out + (int64_t)(begin + row0) * p.n_out + tl.band * (kGateUp ? 128 : 256) + c0;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {              // 8 lanes write one row's 128 bytes
+            const int r = 4 * i + (lane >> 3), c = lane & 7;
+            if (row0 + r < cnt)
+              *reinterpret_cast<uint4*>(to + (int64_t)r * p.n_out + c * 8) = *reinterpret_cast<const uint4*>(stage + umma::sw128(r, c));
+          }
+          __syncwarp();
+        }
+      }
+      umma::fence_before_sync();
+      mbar_arrive(&acc_empty[buf]);
+    }
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) umma::tmem_dealloc(tb, 512);
+}
+
 // XS[pos] = X[sorted_pair[pos] / top_k] for the positions the plan holds; one warp per row
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -228,6 +459,20 @@ moe_gather_rows_kernel(T* __restrict__ xs, const T* __restrict__ x, const int32_
   }
 }
 
+static int moe_sm_count() {
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+// The persistent kernel where its 256-column bands divide the output and full row tiles alone give every SM a tile; fewer
+// tiles than SMs leave it with idle SMs and one cold ring per tile, where the 128-column kernels (two CTAs per SM or a deep
+// ring) are the better ones. fp32 outputs (attention scores) stay there as well.
+static bool moe_umma_wide(bool gate_up, int pairs, int n_out, int out_f32) {
+  const int band = gate_up ? 128 : 256;
+  return !out_f32 && n_out % band == 0 && (long long)(pairs / 128) * (n_out / band) >= moe_sm_count();
+}
+
 template <typename T, bool kGateUp, int kStages>
 static int moe_umma_launch_s(const CUtensorMap& ma, const CUtensorMap& mw, const MoeUmmaParams& p,
                              dim3 grid, cudaStream_t stream) {
@@ -243,14 +488,21 @@ static int moe_umma_launch_s(const CUtensorMap& ma, const CUtensorMap& mw, const
   return finish_launch();
 }
 
+template <typename T, bool kGateUp>
+static int moe_umma_wide_launch(const CUtensorMap& ma, const CUtensorMap& mw, const MoeUmmaParams& p, cudaStream_t stream) {
+  auto kern = moe_umma_wide_kernel<T, kGateUp>;
+  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMwSmem);
+  if (configured != cudaSuccess) return (int)configured;
+  launch_pdl(kern, dim3(moe_sm_count()), dim3(kMuThreads), (size_t)kMwSmem, stream, ma, mw, p);
+  return finish_launch();
+}
+
 template <typename T>
 static int moe_umma_launch(bool gate_up, const CUtensorMap& ma, const CUtensorMap& mw,
                            const MoeUmmaParams& p, int pairs, cudaStream_t stream) {
   const int row_tiles = (pairs + 127) / 128 + p.num_local;      // upper bound; surplus CTAs exit at once
   const dim3 grid(p.n_out / (gate_up ? 64 : 128), row_tiles);
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const bool deep = (long long)grid.x * ((pairs + 127) / 128) <= 2ll * sms;   // few live CTAs: latency-bound
+  const bool deep = (long long)grid.x * ((pairs + 127) / 128) <= 2ll * moe_sm_count();   // few live CTAs: latency-bound
   if (gate_up)
     return deep ? moe_umma_launch_s<T, true, 6>(ma, mw, p, grid, stream)
                 : moe_umma_launch_s<T, true, 3>(ma, mw, p, grid, stream);
@@ -299,9 +551,17 @@ static int moe_umma_common(bool gate_up, void* out, const void* a, const void* w
   int rc = get_panel_map(a, pairs, (int64_t)K * 2, K / 64, 128, 1, dtype, &ma);
   if (rc != B200_OK) return rc;
   const int64_t w_rows = (int64_t)num_local * (gate_up ? 2 : 1) * n_out;
-  rc = get_panel_map(w, w_rows, (int64_t)K * 2, K / 64, 64, 1, dtype, &mw);
+  const bool wide = moe_umma_wide(gate_up, pairs, n_out, out_f32);
+  rc = get_panel_map(w, w_rows, (int64_t)K * 2, K / 64, wide ? 128 : 64, 1, dtype, &mw);
   if (rc != B200_OK) return rc;
   MoeUmmaParams p{offsets, sorted_pair, pair_scale, out, num_local, K, n_out, out_f32, in_scale};
+  if (wide) {
+    if (dtype == B200_DTYPE_BF16)
+      return gate_up ? moe_umma_wide_launch<__nv_bfloat16, true>(ma, mw, p, (cudaStream_t)stream)
+                     : moe_umma_wide_launch<__nv_bfloat16, false>(ma, mw, p, (cudaStream_t)stream);
+    return gate_up ? moe_umma_wide_launch<__half, true>(ma, mw, p, (cudaStream_t)stream)
+                   : moe_umma_wide_launch<__half, false>(ma, mw, p, (cudaStream_t)stream);
+  }
   return dtype == B200_DTYPE_BF16 ? moe_umma_launch<__nv_bfloat16>(gate_up, ma, mw, p, pairs, (cudaStream_t)stream)
                                   : moe_umma_launch<__half>(gate_up, ma, mw, p, pairs, (cudaStream_t)stream);
 }

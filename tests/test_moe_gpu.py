@@ -241,3 +241,29 @@ def test_dense_layers_on_the_grouped_tcgen05_kernel(M, K, inter):
     _close(ops.gate_up_silu_umma(x, w), ops.silu_and_mul(torch.nn.functional.linear(x, w)), ("gate_up", M, K, inter))
     if (2 * inter) % 128 == 0:
         _close(ops.linear_umma(x, w), torch.nn.functional.linear(x, w), ("linear", M, K, inter))
+
+
+@pytest.mark.parametrize("dtype,k,hidden,inter,weigh_input", [
+    (torch.bfloat16, 1, 256, 128, False), (torch.float16, 2, 512, 256, True), (torch.bfloat16, 1, 768, 384, False)])
+def test_persistent_256_column_tiles(monkeypatch, dtype, k, hidden, inter, weigh_input):
+    """moe_umma_wide_kernel at its edges: an empty expert, experts of 1, 127, 128, 129 and many rows, fewer K blocks than
+    ring stages, one column band and several, weights on the input or the output; against the weight-streaming kernels."""
+    from nanovllm import ops
+    g = torch.Generator().manual_seed(hidden + k)
+    counts = [0, 1, 127, 128, 129, 640, 0, 18975 // k]
+    E, T = len(counts), max(sum(counts), 19000 // k)
+    first = torch.repeat_interleave(torch.arange(E), torch.tensor(counts[:-1] + [T - sum(counts[:-1])]))
+    ids = first[torch.randperm(T, generator=g)].view(T, 1)
+    if k == 2:
+        ids = torch.cat([ids, (ids + 1 + torch.randint(0, E - 1, (T, 1), generator=g)) % E], 1)
+    ids = ids.to(torch.int32).cuda()
+    x = torch.randn(T, hidden, generator=g).to(dtype).cuda()
+    w13 = (hidden ** -0.5 * torch.randn(E, 2 * inter, hidden, generator=g)).to(dtype).cuda()
+    w2 = (inter ** -0.5 * torch.randn(E, hidden, inter, generator=g)).to(dtype).cuda()
+    w = torch.rand(T, k, generator=g).to(torch.float32 if weigh_input else dtype).cuda()
+    plan = ops.moe_align(ids, 0, E)
+    monkeypatch.setattr(ops, "_MOE_BIG_GEMM", "stream")
+    a = ops.moe_experts(x, w13, w2, ids, w, plan, weigh_input=weigh_input)
+    monkeypatch.setattr(ops, "_MOE_BIG_GEMM", "umma")
+    b = ops.moe_experts(x, w13, w2, ids, w, plan, weigh_input=weigh_input)
+    _close(b, a, f"hidden {hidden}, inter {inter}")
