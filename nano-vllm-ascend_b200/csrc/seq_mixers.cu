@@ -346,20 +346,20 @@ static void recurrence_launch_as(const RecParams& P, int num_seqs, cudaStream_t 
 // keeps rows 16w .. 16w+15 of S^T [vdim x kdim] as accumulator fragments, which are at the same time the A
 // fragments of S^T q (the layout identity that flash attention uses for P V). Sizes are zero-padded to
 // kdim <= D (template, 32 / 64 / 128) and vdim <= 128 in shared memory.
-__device__ __forceinline__ void split3(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const __nv_bfloat16 h = __float2bfloat16_rn(x);
-  const float r1 = x - __bfloat162float(h);
-  const __nv_bfloat16 m = __float2bfloat16_rn(r1);
-  const __nv_bfloat16 l = __float2bfloat16_rn(r1 - __bfloat162float(m));
-  hi = __bfloat16_as_ushort(h), mid = __bfloat16_as_ushort(m), lo = __bfloat16_as_ushort(l);
-}
-// two fp32 -> three packed bf16 pairs (first value in the low half)
+// Bound: latency and issue of a warp's chain per chunk (2 CTAs of 4 to 8 warps per SM by their 255 registers), so what
+// counts is instructions: fragments come by ldmatrix (the A fragment of Q is also the B fragment of Q^T), the splits
+// by packed conversions, every warp keeps the decays in its lanes (one CTA barrier per chunk) and stores its outputs
+// straight from the accumulators. 16 x 1024 tokens, 32 heads of 128 x 64, selective: 673 -> 419 us, 1950 -> 1420
+// instructions per warp and chunk.
+// two fp32 -> three packed bf16 pairs hi, mid, lo (first value in the low half), each term the rounding of what the ones
+// before it leave. The packed conversion runs at half of the fp32 rate, the scalar one on the special-function unit at
+// an eighth (it was 41 % busy with the splits).
 __device__ __forceinline__ void split3x2(float x, float y, uint32_t (&w)[3]) {
-  uint32_t a[3], b[3];
-  split3(x, a[0], a[1], a[2]);
-  split3(y, b[0], b[1], b[2]);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) w[i] = a[i] | (b[i] << 16);
+  for (int i = 0; i < 3; ++i) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(y), "f"(x));
+    if (i < 2) x -= __uint_as_float(w[i] << 16), y -= __uint_as_float(w[i] & 0xffff0000u);
+  }
 }
 __device__ __forceinline__ uint32_t bf16_bits(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float bits_f32(uint32_t b16) { return __uint_as_float(b16 << 16); }
@@ -376,8 +376,6 @@ chunk_recurrence_kernel(const RecParams P) {
   constexpr int VS = 128 + 8;
   constexpr int NB = VEC ? 2 : 1;
   __shared__ __align__(16) unsigned short sQb[NB][kChunk * QS], sKb[NB][kChunk * QS], sVb[NB][kChunk * VS];
-  __shared__ float sCum[kChunk], sDt[kChunk];
-  __shared__ float sO[kChunk * 129];
   pdl_wait();
   const int s = blockIdx.z, h = blockIdx.y;
   const SeqSpan sp = seq_span(P.cu_q, P.cu_k, P.ctx_lens, s);
@@ -429,12 +427,15 @@ chunk_recurrence_kernel(const RecParams P) {
     }
     cp_async_commit();
   };
-  float dt_next = 0.f;                                // this thread's token of the next chunk (threads < 16)
+  float dt_next = 0.f;                                // lane j: token j of the next chunk (every warp keeps its own copy)
   auto fetch_dt = [&](int c0) {
     dt_next = 0.f;
-    if (P.mode == 1 && threadIdx.x < kChunk && c0 + (int)threadIdx.x < sp.q_len)
-      dt_next = __bfloat162float(dt[(sp.q_start + c0 + threadIdx.x) * P.dt_stride + h]);
+    if (P.mode == 1 && lane < kChunk && c0 + lane < sp.q_len)
+      dt_next = __bfloat162float(dt[(sp.q_start + c0 + lane) * P.dt_stride + h]);
   };
+  // ldmatrix addresses inside a 16-row tile: rows in order of the lanes, the second 16 lanes 8 columns on (A operand from
+  // [row][k], B operand from [k][n] transposed), or the second 8 lanes 8 columns on (B operand from [n][k], A from [k][m])
+  const int r_a = lane & 15, c_a = (lane >> 4) * 8, r_b = (lane & 7) + (lane >> 4) * 8, c_b = ((lane >> 3) & 1) * 8;
   if (VEC) copy_async(0, 0);
   fetch_dt(0);
 
@@ -484,62 +485,68 @@ chunk_recurrence_kernel(const RecParams P) {
         sV[j * VS + i] = (unsigned short)bf16_bits(x);
       }
     }
-    if (warp == 0) {                                  // log-decay of every token and its prefix sum; step sizes
-      float la = 0.f, step = 1.f;                     // a padded token neither decays nor adds
-      if (lane < nt) {
-        la = log_a_const;
-        if (P.mode == 1) {
-          step = softplus_f(dt_next + dt_b);
-          la = -rate * step;
-        }
-      }
-#pragma unroll
-      for (int off = 1; off < kChunk; off <<= 1) {
-        const float up = __shfl_up_sync(0xffffffffu, la, off);
-        if (lane >= off) la += up;
-      }
-      if (lane < kChunk) {
-        sCum[lane] = la;
-        sDt[lane] = step;
+    // log-decay of every token and its prefix sum, step sizes: lane j holds token j. A padded token neither decays nor adds
+    float cum = 0.f, step = 1.f;
+    if (lane < nt) {
+      cum = log_a_const;
+      if (P.mode == 1) {
+        step = softplus_f(dt_next + dt_b);
+        cum = -rate * step;
       }
     }
+#pragma unroll
+    for (int off = 1; off < kChunk; off <<= 1) {
+      const float up = __shfl_up_sync(0xffffffffu, cum, off);
+      if (lane >= off) cum += up;
+    }
     fetch_dt(c0 + kChunk);
-    __syncthreads();
+    if (!VEC || P.act_silu) __syncthreads();          // tiles written by the CTA's threads themselves
     if (r0 < vdim) {                                  // (every warp of the CTA, by the launch's block size)
-      // ---- 1. scores q_i . k_j : rows i = g, g+8; columns j = 8*nj + 2t, +1
+      // ---- 1. scores q_i . k_j (rows i = g, g+8; columns j = 8*nj + 2t, +1) and the carried part S^T q_i: the A fragment of
+      //         Q is the B fragment of Q^T. One accumulator per term of S keeps the chains of dependent products short
       float qk[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      float oi[3][2][4];
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni) oi[p][ni][0] = oi[p][ni][1] = oi[p][ni][2] = oi[p][ni][3] = 0.f;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
-        const int kk = 16 * ks + 2 * t;
-        const uint32_t a0 = *reinterpret_cast<const uint32_t*>(sQ + g * QS + kk);
-        const uint32_t a1 = *reinterpret_cast<const uint32_t*>(sQ + (g + 8) * QS + kk);
-        const uint32_t a2 = *reinterpret_cast<const uint32_t*>(sQ + g * QS + kk + 8);
-        const uint32_t a3 = *reinterpret_cast<const uint32_t*>(sQ + (g + 8) * QS + kk + 8);
+        uint32_t qa[4], kb[4], a0[3], a1[3], a2[3], a3[3];
+        ldsm_x4(smem_u32(sQ + r_a * QS + 16 * ks + c_a), qa[0], qa[1], qa[2], qa[3]);
+        ldsm_x4(smem_u32(sK + r_b * QS + 16 * ks + c_b), kb[0], kb[1], kb[2], kb[3]);
+        mma_16816<T>(qk[0], qa[0], qa[1], qa[2], qa[3], kb[0], kb[1]);
+        mma_16816<T>(qk[1], qa[0], qa[1], qa[2], qa[3], kb[2], kb[3]);
+        split3x2(S[2 * ks][0], S[2 * ks][1], a0);
+        split3x2(S[2 * ks][2], S[2 * ks][3], a1);
+        split3x2(S[2 * ks + 1][0], S[2 * ks + 1][1], a2);
+        split3x2(S[2 * ks + 1][2], S[2 * ks + 1][3], a3);
 #pragma unroll
-        for (int nj = 0; nj < 2; ++nj) {
-          const uint32_t b0 = *reinterpret_cast<const uint32_t*>(sK + (8 * nj + g) * QS + kk);
-          const uint32_t b1 = *reinterpret_cast<const uint32_t*>(sK + (8 * nj + g) * QS + kk + 8);
-          mma_16816<T>(qk[nj], a0, a1, a2, a3, b0, b1);
+        for (int p = 0; p < 3; ++p) {
+          mma_16816<T>(oi[p][0], a0[p], a1[p], a2[p], a3[p], qa[0], qa[2]);
+          mma_16816<T>(oi[p][1], a0[p], a1[p], a2[p], a3[p], qa[1], qa[3]);
         }
       }
       // ---- 2. decayed, causal: p_ij = (j <= i) e^{c_i - c_j} b_j (q_i . k_j)
-      const float ci[2] = {sCum[g], sCum[g + 8]};
+      float ci[2], cj[4], bj[4];                      // j = 2t, 2t+1, 2t+8, 2t+9
+#pragma unroll
+      for (int u = 0; u < 2; ++u) ci[u] = __shfl_sync(0xffffffffu, cum, g + 8 * u);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        cj[u] = __shfl_sync(0xffffffffu, cum, 2 * t + (u & 1) + 8 * (u >> 1));
+        bj[u] = __shfl_sync(0xffffffffu, step, 2 * t + (u & 1) + 8 * (u >> 1));
+      }
+      const float c_end = __shfl_sync(0xffffffffu, cum, kChunk - 1);
 #pragma unroll
       for (int nj = 0; nj < 2; ++nj)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const int i = g + (c >> 1) * 8, j = 8 * nj + 2 * t + (c & 1);
-          qk[nj][c] = j <= i ? qk[nj][c] * expf(ci[c >> 1] - sCum[j]) * sDt[j] : 0.f;
+          const int i = g + (c >> 1) * 8, u = 2 * nj + (c & 1), j = 8 * nj + 2 * t + (c & 1);
+          qk[nj][c] = j <= i ? qk[nj][c] * expf(ci[c >> 1] - cj[u]) * bj[u] : 0.f;
         }
       // ---- 3. o^T (rows: value channels, columns: tokens i) = V^T P^T
       uint32_t va[4];                                 // V^T fragment: rows r0+g / +8, k = tokens 2t,2t+1 / 2t+8,2t+9
-      {
-        const unsigned short* vp = sV + r0 + g;
-        va[0] = vp[(2 * t) * VS] | ((uint32_t)vp[(2 * t + 1) * VS] << 16);
-        va[1] = vp[(2 * t) * VS + 8] | ((uint32_t)vp[(2 * t + 1) * VS + 8] << 16);
-        va[2] = vp[(2 * t + 8) * VS] | ((uint32_t)vp[(2 * t + 9) * VS] << 16);
-        va[3] = vp[(2 * t + 8) * VS + 8] | ((uint32_t)vp[(2 * t + 9) * VS + 8] << 16);
-      }
+      ldsm_x4_trans(smem_u32(sV + r_b * VS + r0 + c_b), va[0], va[1], va[2], va[3]);
       float o[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
       for (int ni = 0; ni < 2; ++ni) {                // token columns i = 8*ni + g  (B[k = j][n = i] = p_ij)
@@ -549,65 +556,42 @@ chunk_recurrence_kernel(const RecParams P) {
 #pragma unroll
         for (int p = 0; p < 3; ++p) mma_16816<T>(o[ni], va[0], va[1], va[2], va[3], b0[p], b1[p]);
       }
-      // ---- 4. carried part: o^T += (S^T Q^T) scaled per token column by e^{c_i}
-      float oi[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) {
-        uint32_t a0[3], a1[3], a2[3], a3[3];
-        split3x2(S[2 * ks][0], S[2 * ks][1], a0);
-        split3x2(S[2 * ks][2], S[2 * ks][3], a1);
-        split3x2(S[2 * ks + 1][0], S[2 * ks + 1][1], a2);
-        split3x2(S[2 * ks + 1][2], S[2 * ks + 1][3], a3);
-        const int kk = 16 * ks + 2 * t;
-#pragma unroll
-        for (int ni = 0; ni < 2; ++ni) {
-          const uint32_t b0 = *reinterpret_cast<const uint32_t*>(sQ + (8 * ni + g) * QS + kk);
-          const uint32_t b1 = *reinterpret_cast<const uint32_t*>(sQ + (8 * ni + g) * QS + kk + 8);
-#pragma unroll
-          for (int p = 0; p < 3; ++p) mma_16816<T>(oi[ni], a0[p], a1[p], a2[p], a3[p], b0, b1);
-        }
-      }
-#pragma unroll
-      for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int i = 8 * ni + 2 * t + (c & 1), row = r0 + g + (c >> 1) * 8;
-          float val = o[ni][c] + oi[ni][c] * expf(sCum[i]);
-          if (P.mode == 1) val += d_skip * bits_f32(sV[i * VS + row]);
-          sO[i * 129 + row] = val;
-        }
-      // ---- 5. S^T <- e^{c_15} S^T + V'^T K,  v'_j = e^{c_15 - c_j} b_j v_j
-      const float c_end = sCum[kChunk - 1];
+      // ---- 4. S^T <- e^{c_15} S^T + V'^T K,  v'_j = e^{c_15 - c_j} b_j v_j
       const float grow = expf(c_end);
-#pragma unroll
-      for (int n = 0; n < D / 8; ++n)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) S[n][c] *= grow;
       uint32_t wa[4][3];
       {
-        const int js[4] = {2 * t, 2 * t + 1, 2 * t + 8, 2 * t + 9};
         float f[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) f[u] = expf(c_end - sCum[js[u]]) * sDt[js[u]];
+        for (int u = 0; u < 4; ++u) f[u] = expf(c_end - cj[u]) * bj[u];
         split3x2(bits_f32(va[0] & 0xffffu) * f[0], bits_f32(va[0] >> 16) * f[1], wa[0]);
         split3x2(bits_f32(va[1] & 0xffffu) * f[0], bits_f32(va[1] >> 16) * f[1], wa[1]);
         split3x2(bits_f32(va[2] & 0xffffu) * f[2], bits_f32(va[2] >> 16) * f[3], wa[2]);
         split3x2(bits_f32(va[3] & 0xffffu) * f[2], bits_f32(va[3] >> 16) * f[3], wa[3]);
       }
 #pragma unroll
-      for (int n = 0; n < D / 8; ++n) {               // B[k = token j][n = key column 8n + g] = k_j
-        const unsigned short* kp = sK + 8 * n + g;
-        const uint32_t b0 = kp[(2 * t) * QS] | ((uint32_t)kp[(2 * t + 1) * QS] << 16);
-        const uint32_t b1 = kp[(2 * t + 8) * QS] | ((uint32_t)kp[(2 * t + 9) * QS] << 16);
+      for (int n = 0; n < D / 8; n += 2) {            // B[k = token j][n = key column 8n + g] = k_j
+        uint32_t kb[4];
+        ldsm_x4_trans(smem_u32(sK + r_a * QS + 8 * n + c_a), kb[0], kb[1], kb[2], kb[3]);
 #pragma unroll
-        for (int p = 0; p < 3; ++p) mma_16816<T>(S[n], wa[0][p], wa[1][p], wa[2][p], wa[3][p], b0, b1);
+        for (int m = 0; m < 2; ++m) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) S[n + m][c] *= grow;
+#pragma unroll
+          for (int p = 0; p < 3; ++p) mma_16816<T>(S[n + m], wa[0][p], wa[1][p], wa[2][p], wa[3][p], kb[2 * m], kb[2 * m + 1]);
+        }
       }
-    }
-    __syncthreads();
-    float* outp = P.out + tok0 * ((int64_t)P.H * vdim) + (int64_t)h * vdim;
-    for (int e = threadIdx.x; e < nt * vdim; e += nthreads) {
-      const int i = e / vdim, c = e - i * vdim;
-      outp[(int64_t)i * ((int64_t)P.H * vdim) + c] = sO[i * 129 + c];
+      // ---- 5. the chunk's output, straight from the fragments: 8 lanes write 8 neighbouring channels of a token (32 bytes)
+      float* outp = P.out + tok0 * ((int64_t)P.H * vdim) + (int64_t)h * vdim;
+      const float e_i = expf(cum);                    // lane i: e^{c_i}
+#pragma unroll
+      for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int i = 8 * ni + 2 * t + (c & 1), row = r0 + g + (c >> 1) * 8;
+          float val = o[ni][c] + (oi[0][ni][c] + (oi[1][ni][c] + oi[2][ni][c])) * __shfl_sync(0xffffffffu, e_i, i);
+          if (P.mode == 1) val += d_skip * bits_f32(sV[i * VS + row]);
+          if (i < nt && row < vdim) outp[(int64_t)i * ((int64_t)P.H * vdim) + row] = val;
+        }
     }
   }
   if (slot != nullptr && r0 < vdim) {
