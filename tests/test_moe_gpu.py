@@ -267,3 +267,27 @@ def test_persistent_256_column_tiles(monkeypatch, dtype, k, hidden, inter, weigh
     monkeypatch.setattr(ops, "_MOE_BIG_GEMM", "umma")
     b = ops.moe_experts(x, w13, w2, ids, w, plan, weigh_input=weigh_input)
     _close(b, a, f"hidden {hidden}, inter {inter}")
+
+
+@pytest.mark.parametrize("T,k,E,begin,n,shift", [(1, 1, 1, 0, 1, 0), (16, 8, 128, 0, 128, 0), (127, 1, 8, 2, 5, 1),
+                                                 (513, 8, 128, 96, 32, 3), (5000, 4, 256, 0, 256, 0), (9001, 1, 3, 1, 2, 2)])
+def test_plan_is_a_stable_sort_by_expert(T, k, E, begin, n, shift):
+    """b200_moe_align on short and long pair lists, at the edges of the 128-pair vectors, with ids that do not start on a
+    16-byte boundary and experts that live elsewhere: exactly numpy's stable sort."""
+    import numpy as np
+    from nanovllm import ops
+    g = torch.Generator().manual_seed(T)
+    ids = torch.randint(0, E, (T, k), generator=g, dtype=torch.int32)
+    store = torch.zeros(T * k + 4, dtype=torch.int32, device="cuda")
+    dev = store[shift:shift + T * k].view(T, k)
+    dev.copy_(ids)
+    plan = ops.moe_align(dev, begin, n)
+    flat = ids.flatten().numpy()
+    local = np.flatnonzero((flat >= begin) & (flat < begin + n))
+    order = local[np.argsort(flat[local], kind="stable")]
+    pos = np.full(T * k, -1)
+    pos[order] = np.arange(len(order))
+    assert (plan.sorted_pair.cpu().numpy()[:len(order)] == order).all()
+    assert (plan.pos_of_pair.cpu().numpy() == pos).all()
+    counts = np.bincount(flat[local] - begin, minlength=n)
+    assert (plan.offsets.cpu().numpy() == np.concatenate([[0], np.cumsum(counts)])).all()

@@ -1,7 +1,7 @@
 """Thread-level emulation (numpy, CPU) of the index arithmetic in nano-vllm-ascend_b200/csrc/moe.cu.
 
 It transcribes, formula by formula,
-  * moe_count_kernel / moe_place_kernel (per-warp chunks, ballot ranks) and checks the result
+  * moe_plan_kernel (per-warp chunks, ballot ranks) and checks the result
     against oracle/moe_ref.py::dispatch_plan,
   * moe_gemm_pass<gate_up / down, MI = 1 / 2>: the cp.async placement of every thread into the
     128-byte-swizzled stage, the ldmatrix.x4 row addresses of every lane, mma.sync.m16n8k16
@@ -28,44 +28,39 @@ from oracle import moe_ref  # noqa: E402
 
 
 # ------------------------------------------------------------------ dispatch plan
-def emulate_align(ids_flat: np.ndarray, expert_begin: int, num_local: int):
+def emulate_align(ids_flat: np.ndarray, expert_begin: int, num_local: int, warps: int = 8):
+    """moe_plan_kernel: CTA e counts its pairs and those of the local experts before it, warp by warp, then ranks its own
+    by ballots over vectors of four pairs per lane."""
     P = len(ids_flat)
     counts = np.zeros(num_local, np.int64)
-    pos_of_pair = np.full(P, 12345, np.int64)              # garbage: the count kernel must reset it
-    grid = num_local
-    for e in range(grid):                                  # moe_count_kernel
-        per = (P + grid - 1) // grid
-        hi = min(P, (e + 1) * per)
-        for tid in range(256):
-            for i in range(e * per + tid, hi, 256):
-                pos_of_pair[i] = -1
-        counts[e] = sum(int(ids_flat[i] == expert_begin + e) for i in range(P))
     offsets = np.zeros(num_local + 1, np.int64)
     sorted_pair = np.full(P, -7, np.int64)
-    for e in range(grid):                                  # moe_place_kernel
+    pos_of_pair = np.full(P, 12345, np.int64)              # garbage: every entry must be written
+    chunk = (P + warps * 128 - 1) // (warps * 128) * 128
+    for e in range(num_local):
         target = expert_begin + e
-        s_base = int(counts[:e].sum())
-        chunk = (((P + 7) // 8) + 31) // 32 * 32
-        warp_cnt = []
-        for warp in range(8):
-            lo = min(P, warp * chunk)
-            hi = min(P, lo + chunk)
-            warp_cnt.append(sum(int(ids_flat[i] == target) for i in range(lo, hi)))
-        for warp in range(8):
-            lo = min(P, warp * chunk)
-            hi = min(P, lo + chunk)
-            before = s_base + sum(warp_cnt[:warp])
-            for i0 in range(lo, hi, 32):
-                ballot = [(i0 + lane < hi) and ids_flat[i0 + lane] == target for lane in range(32)]
-                for lane in range(32):
-                    if ballot[lane]:
-                        pos = before + sum(ballot[:lane])
-                        sorted_pair[pos] = i0 + lane
-                        pos_of_pair[i0 + lane] = pos
-                before += sum(ballot)
-        offsets[e] = s_base
+        spans = [(min(P, w * chunk), min(P, min(P, w * chunk) + chunk)) for w in range(warps)]
+        mine = [int((ids_flat[lo:hi] == target).sum()) for lo, hi in spans]
+        base = sum(int(((ids_flat[lo:hi] >= expert_begin) & (ids_flat[lo:hi] < target)).sum()) for lo, hi in spans)
+        counts[e], offsets[e] = sum(mine), base
         if e == num_local - 1:
-            offsets[num_local] = s_base + sum(warp_cnt)
+            offsets[num_local] = base + sum(mine)
+        for w, (lo, hi) in enumerate(spans):
+            before = base + sum(mine[:w])
+            for i0 in range(lo, hi, 128):
+                m = [[i0 + 4 * lane + c < hi and ids_flat[i0 + 4 * lane + c] == target for c in range(4)] for lane in range(32)]
+                for lane in range(32):
+                    at = before + sum(m[below][c] for below in range(lane) for c in range(4))
+                    for c in range(4):
+                        if m[lane][c]:
+                            sorted_pair[at] = i0 + 4 * lane + c
+                            pos_of_pair[i0 + 4 * lane + c] = at
+                            at += 1
+                before += sum(map(sum, m))
+        per = (P + num_local - 1) // num_local
+        for i in range(min(P, e * per), min(P, (e + 1) * per)):
+            if ids_flat[i] < expert_begin or ids_flat[i] >= expert_begin + num_local:
+                pos_of_pair[i] = -1
     return offsets, sorted_pair, pos_of_pair
 
 
