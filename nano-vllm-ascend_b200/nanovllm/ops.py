@@ -31,7 +31,16 @@ def _need_cuda(*tensors: torch.Tensor) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device, without the Stream object that torch.cuda.current_stream() builds."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+def _stream_of(device) -> int:
+    """The current stream of `device` (a tensor's device, or whatever torch.cuda.current_stream takes)."""
+    index = getattr(device, "index", None)
+    if index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(index)
 
 
 def _ptr(t):
@@ -42,9 +51,12 @@ def _cache_dims(cache: torch.Tensor, row_elems: int) -> tuple[int, int]:
     """(num_blocks, block_size) of a cache given as [nb, bs, Hkv*D] or [nb, bs, Hkv, D]."""
     if cache.dim() not in (3, 4) or not cache.is_contiguous():
         raise ValueError("KV cache must be a contiguous [nb, bs, Hkv*D] (or [nb, bs, Hkv, D]) tensor")
-    if cache[0, 0].numel() != row_elems:
-        raise ValueError(f"KV cache row has {cache[0, 0].numel()} elements, expected {row_elems}")
-    return cache.shape[0], cache.shape[1]
+    nb, bs, row = cache.shape[0], cache.shape[1], cache.shape[2] * (cache.shape[3] if cache.dim() == 4 else 1)
+    if nb == 0 or bs == 0:
+        raise IndexError("KV cache without blocks")
+    if row != row_elems:
+        raise ValueError(f"KV cache row has {row} elements, expected {row_elems}")
+    return nb, bs
 
 
 def launch_count() -> int:
@@ -107,14 +119,20 @@ def reshape_and_cache_fp8(key, value, k_cache, v_cache, slot_mapping, k_scale=1.
 
 
 _decode_ws: dict = {}
+_decode_need: dict = {}      # bytes that a launch of these sizes needs: a pure function of them
 
 
 def decode_workspace(batch, num_heads, num_kv_heads, head_dim, device) -> torch.Tensor:
-    need = _C.load().b200_paged_decode_attn_workspace_size(batch, num_heads, num_kv_heads, head_dim)
+    sizes = (batch, num_heads, num_kv_heads, head_dim)
+    need = _decode_need.get(sizes)
+    if need is None:
+        if len(_decode_need) > 4096:
+            _decode_need.clear()
+        need = _decode_need[sizes] = _C.load().b200_paged_decode_attn_workspace_size(batch, num_heads, num_kv_heads, head_dim)
     if need == 0:
         raise _C.B200Error("b200_paged_decode_attn: unsupported head configuration "
                            f"(H={num_heads}, Hkv={num_kv_heads}, D={head_dim})")
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
+    key = (device, _stream_of(device))
     ws = _decode_ws.get(key)
     if ws is None or ws.numel() < need:
         ws = torch.zeros(need, dtype=torch.uint8, device=device)   # arrival counters start at 0
@@ -214,7 +232,7 @@ _prefill_ws: dict = {}
 def prefill_workspace(device, head_dim: int) -> torch.Tensor:
     """The split-KV workspace of the prefill kernel (b200_prefill_workspace_size bytes, a few MB),
     one per device and stream, allocated on first use -- outside CUDA-graph capture; prefill runs eagerly."""
-    key = (device, head_dim, torch.cuda.current_stream(device).cuda_stream)   # concurrent launches must not share it
+    key = (device, head_dim, _stream_of(device))   # concurrent launches must not share it
     ws = _prefill_ws.get(key)
     if ws is None:
         n = int(_C.load().b200_prefill_workspace_size(int(head_dim)))
