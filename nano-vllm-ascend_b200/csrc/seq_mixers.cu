@@ -239,7 +239,7 @@ linear_recurrence_kernel(const RecParams P) {
     for (int n = 0; n < NQ; ++n) {
       const int e = threadIdx.x + n * 128;
       float qv = to_f32<T>(pq[n]), kv = to_f32<T>(pk[n]);
-      // the activation's result is an activation of the model's element type (as in the 16-token form, whose
+      // the activation's result is an activation of the model's element type (as in the chunked form, whose
       // tensor-core operands are bf16 values); silu(0) = 0: the padding stays zero
       if (P.act_silu) {
         qv = sizeof(T) == 2 ? silu_fast(qv) : silu_f(qv);
@@ -336,9 +336,9 @@ static void recurrence_launch_as(const RecParams& P, int num_seqs, cudaStream_t 
   launch_pdl(linear_recurrence_kernel<T, TV, KPT, NS>, grid, dim3(128), smem, stream, P);
 }
 
-// ------------------------------------------------------------------ the same recurrence, 16 tokens at a time
-// Prompt portions of bf16 models. With c_i = sum_{s<=i} log a_s inside a chunk of 16 tokens (S0 = state before it):
-//   o_i = e^{c_i} S0^T q_i + sum_{j<=i} e^{c_i - c_j} b_j (q_i . k_j) v_j          S16 = e^{c_15} S0 + sum_j e^{c_15 - c_j} b_j k_j v_j^T
+// ------------------------------------------------------------------ the same recurrence, 32 tokens at a time
+// Prompt portions of bf16 models. With c_i = sum_{s<=i} log a_s inside a chunk of 32 tokens (S0 = state before it):
+//   o_i = e^{c_i} S0^T q_i + sum_{j<=i} e^{c_i - c_j} b_j (q_i . k_j) v_j          S32 = e^{c_31} S0 + sum_j e^{c_31 - c_j} b_j k_j v_j^T
 // -- three small matrix products per chunk on the tensor cores (mma.sync m16n8k16, fp32 accumulation). The
 // 32-bit rule of the recurrence is kept: q, k, v are bf16 values already (exact operands), and every fp32 operand
 // (the decayed scores, the state, the decayed values) enters the tensor core as the sum of three bf16 terms
@@ -349,8 +349,11 @@ static void recurrence_launch_as(const RecParams& P, int num_seqs, cudaStream_t 
 // Bound: latency and issue of a warp's chain per chunk (2 CTAs of 4 to 8 warps per SM by their 255 registers), so what
 // counts is instructions: fragments come by ldmatrix (the A fragment of Q is also the B fragment of Q^T), the splits
 // by packed conversions, every warp keeps the decays in its lanes (one CTA barrier per chunk) and stores its outputs
-// straight from the accumulators. 16 x 1024 tokens, 32 heads of 128 x 64, selective: 673 -> 419 us, 1950 -> 1420
-// instructions per warp and chunk.
+// straight from the accumulators; and the split and the scaling of the state are paid once per 32 tokens, not per 16.
+// 16 x 1024 tokens, 32 heads of 128 x 64, selective: 673 us at first (1950 instructions per warp and 16 tokens), 419 us with
+// chunks of 16 (1420), 328 us with chunks of 32. Chunks of 64 would need 10 more score tiles per warp than there are registers.
+// The decays of a chunk are exponentials of sums over at most 16 tokens: across the two blocks they are multiplied, since a
+// prefix sum over 32 loses a bit (error of the outputs against 64 bits 4.2e-7 with it, 2.5e-7 so).
 // two fp32 -> three packed bf16 pairs hi, mid, lo (first value in the low half), each term the rounding of what the ones
 // before it leave. The packed conversion runs at half of the fp32 rate, the scalar one on the special-function unit at
 // an eighth (it was 41 % busy with the splits).
@@ -364,18 +367,26 @@ __device__ __forceinline__ void split3x2(float x, float y, uint32_t (&w)[3]) {
 __device__ __forceinline__ uint32_t bf16_bits(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float bits_f32(uint32_t b16) { return __uint_as_float(b16 << 16); }
 
-constexpr int kChunk = 16;
+constexpr int kChunk = 32;             // two 16-token blocks
 
 // VEC: q, k, v rows start on 16-byte boundaries (strides, sizes and slice offsets % 8 == 0): the tiles of the next
 // chunk are copied global -> shared with cp.async while the current chunk is computed (two sets of tiles).
-template <int D, bool VEC>
-__global__ void __launch_bounds__(256)
+// NW: warps that the shared-memory rows of V are sized for (vdim <= 16 NW); MODE, SILU: P.mode, P.act_silu.
+template <int D, int NW>
+constexpr int chunk_recurrence_smem(bool vec) {
+  return (vec ? 2 : 1) * kChunk * (2 * (D + 8) + 16 * NW + 8) * 2;
+}
+template <int D, int NW, bool VEC, int MODE, bool SILU>
+__global__ void __launch_bounds__(32 * NW, 8 / NW)
 chunk_recurrence_kernel(const RecParams P) {
   using T = __nv_bfloat16;
   constexpr int QS = D + 8;                           // row stride (elements) of the q / k tiles: conflict-free
-  constexpr int VS = 128 + 8;
+  constexpr int VS = 16 * NW + 8;
   constexpr int NB = VEC ? 2 : 1;
-  __shared__ __align__(16) unsigned short sQb[NB][kChunk * QS], sKb[NB][kChunk * QS], sVb[NB][kChunk * VS];
+  extern __shared__ __align__(16) unsigned short s_tiles[];
+  unsigned short* sQb = s_tiles;                      // [NB][kChunk][QS]
+  unsigned short* sKb = sQb + NB * kChunk * QS;
+  unsigned short* sVb = sKb + NB * kChunk * QS;       // [NB][kChunk][VS]
   pdl_wait();
   const int s = blockIdx.z, h = blockIdx.y;
   const SeqSpan sp = seq_span(P.cu_q, P.cu_k, P.ctx_lens, s);
@@ -389,10 +400,10 @@ chunk_recurrence_kernel(const RecParams P) {
   const T* k = (const T*)P.k + (int64_t)grp * kdim;
   const T* v = (const T*)P.v + (int64_t)h * vdim;
   const T* dt = (const T*)P.dt;
-  const float log_a_const = P.mode == 0 ? fmaxf(logf(P.decay[h]), -60.f) : 0.f;   // e^-60: nothing survives a step
-  const float rate = P.mode == 1 ? expf(P.a_log[h]) : 0.f;
-  const float dt_b = P.mode == 1 ? P.dt_bias[h] : 0.f;
-  const float d_skip = P.mode == 1 ? P.d_skip[h] : 0.f;
+  const float log_a_const = MODE == 0 ? fmaxf(logf(P.decay[h]), -60.f) : 0.f;   // e^-60: nothing survives a step
+  const float rate = MODE == 1 ? expf(P.a_log[h]) : 0.f;
+  const float dt_b = MODE == 1 ? P.dt_bias[h] : 0.f;
+  const float d_skip = MODE == 1 ? P.d_skip[h] : 0.f;
 
   // S^T slab: n-tile n = key columns 8n .. 8n+7; [0],[1]: row r0+g, cols 8n+2t, +1; [2],[3]: row r0+g+8
   float S[D / 8][4];
@@ -416,21 +427,21 @@ chunk_recurrence_kernel(const RecParams P) {
       const int j = e / (D / 8), i = (e % (D / 8)) * 8;
       const bool ok = j < nt && i < kdim;
       const int64_t tok = ok ? tok0 + j : sp.q_start;
-      cp_async_16(smem_u32(&sQb[buf][j * QS + i]), q + tok * P.q_stride + (ok ? i : 0), ok);
-      cp_async_16(smem_u32(&sKb[buf][j * QS + i]), k + tok * P.k_stride + (ok ? i : 0), ok);
+      cp_async_16(smem_u32(&sQb[(buf * kChunk + j) * QS + i]), q + tok * P.q_stride + (ok ? i : 0), ok);
+      cp_async_16(smem_u32(&sKb[(buf * kChunk + j) * QS + i]), k + tok * P.k_stride + (ok ? i : 0), ok);
     }
-    for (int e = threadIdx.x; e < kChunk * 16; e += nthreads) {
-      const int j = e >> 4, i = (e & 15) * 8;
+    for (int e = threadIdx.x; e < kChunk * 2 * NW; e += nthreads) {
+      const int j = e / (2 * NW), i = (e % (2 * NW)) * 8;
       const bool ok = j < nt && i < vdim;
       const int64_t tok = ok ? tok0 + j : sp.q_start;
-      cp_async_16(smem_u32(&sVb[buf][j * VS + i]), v + tok * P.v_stride + (ok ? i : 0), ok);
+      cp_async_16(smem_u32(&sVb[(buf * kChunk + j) * VS + i]), v + tok * P.v_stride + (ok ? i : 0), ok);
     }
     cp_async_commit();
   };
   float dt_next = 0.f;                                // lane j: token j of the next chunk (every warp keeps its own copy)
   auto fetch_dt = [&](int c0) {
     dt_next = 0.f;
-    if (P.mode == 1 && lane < kChunk && c0 + lane < sp.q_len)
+    if (MODE == 1 && c0 + lane < sp.q_len)
       dt_next = __bfloat162float(dt[(sp.q_start + c0 + lane) * P.dt_stride + h]);
   };
   // ldmatrix addresses inside a 16-row tile: rows in order of the lanes, the second 16 lanes 8 columns on (A operand from
@@ -443,19 +454,19 @@ chunk_recurrence_kernel(const RecParams P) {
     const int nt = min(kChunk, sp.q_len - c0);
     const int64_t tok0 = sp.q_start + c0;
     const int buf = VEC ? (it & 1) : 0;
-    unsigned short* sQ = sQb[buf];
-    unsigned short* sK = sKb[buf];
-    unsigned short* sV = sVb[buf];
+    unsigned short* sQ = sQb + buf * kChunk * QS;
+    unsigned short* sK = sKb + buf * kChunk * QS;
+    unsigned short* sV = sVb + buf * kChunk * VS;
     if (VEC) cp_async_wait<0>();
     __syncthreads();                                  // this chunk's tiles have landed; the previous chunk is consumed
     if (VEC) {
       if (c0 + kChunk < sp.q_len) copy_async(c0 + kChunk, buf ^ 1);
-      if (P.act_silu) {                               // activation in place, 8 values per step
-        for (int e = threadIdx.x; e < kChunk * (D / 8) * 2 + kChunk * 16; e += nthreads) {
+      if (SILU) {                                     // activation in place, 8 values per step
+        constexpr int NQ = kChunk * (D / 8);
+        for (int e = threadIdx.x; e < 2 * NQ + kChunk * 2 * NW; e += nthreads) {
           unsigned short* p;
-          if (e < kChunk * (D / 8)) p = sQ + (e / (D / 8)) * QS + (e % (D / 8)) * 8;
-          else if (e < 2 * kChunk * (D / 8)) p = sK + ((e - kChunk * (D / 8)) / (D / 8)) * QS + ((e - kChunk * (D / 8)) % (D / 8)) * 8;
-          else p = sV + ((e - 2 * kChunk * (D / 8)) >> 4) * VS + ((e - 2 * kChunk * (D / 8)) & 15) * 8;
+          if (e < 2 * NQ) p = (e < NQ ? sQ : sK) + ((e % NQ) / (D / 8)) * QS + (e % (D / 8)) * 8;
+          else p = sV + ((e - 2 * NQ) / (2 * NW)) * VS + ((e - 2 * NQ) % (2 * NW)) * 8;
           float f[8];
           load8<T>(reinterpret_cast<const T*>(p), f);
 #pragma unroll
@@ -470,129 +481,169 @@ chunk_recurrence_kernel(const RecParams P) {
         if (j < nt && i < kdim) {
           qv = __bfloat162float(q[(tok0 + j) * P.q_stride + i]);
           kv = __bfloat162float(k[(tok0 + j) * P.k_stride + i]);
-          if (P.act_silu) qv = silu_fast(qv), kv = silu_fast(kv);
+          if (SILU) qv = silu_fast(qv), kv = silu_fast(kv);
         }
         sQ[j * QS + i] = (unsigned short)bf16_bits(qv);
         sK[j * QS + i] = (unsigned short)bf16_bits(kv);
       }
-      for (int e = threadIdx.x; e < kChunk * 128; e += nthreads) {
-        const int j = e >> 7, i = e & 127;
+      for (int e = threadIdx.x; e < kChunk * 16 * NW; e += nthreads) {
+        const int j = e / (16 * NW), i = e % (16 * NW);
         float x = 0.f;
         if (j < nt && i < vdim) {
           x = __bfloat162float(v[(tok0 + j) * P.v_stride + i]);
-          if (P.act_silu) x = silu_fast(x);
+          if (SILU) x = silu_fast(x);
         }
         sV[j * VS + i] = (unsigned short)bf16_bits(x);
       }
     }
-    // log-decay of every token and its prefix sum, step sizes: lane j holds token j. A padded token neither decays nor adds
+    // log-decay of every token, its prefix sum inside each block of 16 (sums over 32 would lose a bit of the decays), step
+    // sizes: lane j holds token j. A padded token neither decays nor adds
     float cum = 0.f, step = 1.f;
     if (lane < nt) {
       cum = log_a_const;
-      if (P.mode == 1) {
+      if (MODE == 1) {
         step = softplus_f(dt_next + dt_b);
         cum = -rate * step;
       }
     }
 #pragma unroll
-    for (int off = 1; off < kChunk; off <<= 1) {
-      const float up = __shfl_up_sync(0xffffffffu, cum, off);
-      if (lane >= off) cum += up;
+    for (int off = 1; off < 16; off <<= 1) {
+      const float up = __shfl_up_sync(0xffffffffu, cum, off, 16);
+      if ((lane & 15) >= off) cum += up;
     }
+    const float block_end = __shfl_sync(0xffffffffu, cum, 15, 16);
+    const float e_blk = expf(cum);                    // decay from the block's start to and with the token
+    const float f_blk = expf(block_end - cum) * step; // b_j times the decay from the token to its block's end
+    const float through = expf(block_end);            // of the whole block
+    const float through0 = __shfl_sync(0xffffffffu, through, 0), through1 = __shfl_sync(0xffffffffu, through, 16);
     fetch_dt(c0 + kChunk);
-    if (!VEC || P.act_silu) __syncthreads();          // tiles written by the CTA's threads themselves
-    if (r0 < vdim) {                                  // (every warp of the CTA, by the launch's block size)
-      // ---- 1. scores q_i . k_j (rows i = g, g+8; columns j = 8*nj + 2t, +1) and the carried part S^T q_i: the A fragment of
-      //         Q is the B fragment of Q^T. One accumulator per term of S keeps the chains of dependent products short
-      float qk[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      float oi[3][2][4];
+    if (!VEC || SILU) __syncthreads();                // tiles written by the CTA's threads themselves
+    if (r0 >= vdim) continue;                         // (no warp of the CTA, by the launch's block size)
+    // ---- 1. scores q_i . k_j (block m of 16 queries, tile n of 8 keys; rows 16 m + g, + 8; columns 8 n + 2 t, + 1; tiles
+    //         above the diagonal left out) and the carried part S^T q_i: the A fragment of Q is the B fragment of Q^T
+    float qk0[2][4], qk1[4][4], o[4][4];              // o: n-tile ni = tokens 8 ni .., rows r0 + g, + 8
 #pragma unroll
-      for (int p = 0; p < 3; ++p)
+    for (int c = 0; c < 4; ++c) {
+      qk0[0][c] = qk0[1][c] = 0.f;
 #pragma unroll
-        for (int ni = 0; ni < 2; ++ni) oi[p][ni][0] = oi[p][ni][1] = oi[p][ni][2] = oi[p][ni][3] = 0.f;
+      for (int n = 0; n < 4; ++n) qk1[n][c] = o[n][c] = 0.f;
+    }
 #pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) {
-        uint32_t qa[4], kb[4], a0[3], a1[3], a2[3], a3[3];
-        ldsm_x4(smem_u32(sQ + r_a * QS + 16 * ks + c_a), qa[0], qa[1], qa[2], qa[3]);
-        ldsm_x4(smem_u32(sK + r_b * QS + 16 * ks + c_b), kb[0], kb[1], kb[2], kb[3]);
-        mma_16816<T>(qk[0], qa[0], qa[1], qa[2], qa[3], kb[0], kb[1]);
-        mma_16816<T>(qk[1], qa[0], qa[1], qa[2], qa[3], kb[2], kb[3]);
-        split3x2(S[2 * ks][0], S[2 * ks][1], a0);
-        split3x2(S[2 * ks][2], S[2 * ks][3], a1);
-        split3x2(S[2 * ks + 1][0], S[2 * ks + 1][1], a2);
-        split3x2(S[2 * ks + 1][2], S[2 * ks + 1][3], a3);
+    for (int ks = 0; ks < D / 16; ++ks) {
+      uint32_t qa[2][4], kb[2][4], a0[3], a1[3], a2[3], a3[3];
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
-          mma_16816<T>(oi[p][0], a0[p], a1[p], a2[p], a3[p], qa[0], qa[2]);
-          mma_16816<T>(oi[p][1], a0[p], a1[p], a2[p], a3[p], qa[1], qa[3]);
-        }
-      }
-      // ---- 2. decayed, causal: p_ij = (j <= i) e^{c_i - c_j} b_j (q_i . k_j)
-      float ci[2], cj[4], bj[4];                      // j = 2t, 2t+1, 2t+8, 2t+9
-#pragma unroll
-      for (int u = 0; u < 2; ++u) ci[u] = __shfl_sync(0xffffffffu, cum, g + 8 * u);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        cj[u] = __shfl_sync(0xffffffffu, cum, 2 * t + (u & 1) + 8 * (u >> 1));
-        bj[u] = __shfl_sync(0xffffffffu, step, 2 * t + (u & 1) + 8 * (u >> 1));
-      }
-      const float c_end = __shfl_sync(0xffffffffu, cum, kChunk - 1);
-#pragma unroll
-      for (int nj = 0; nj < 2; ++nj)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int i = g + (c >> 1) * 8, u = 2 * nj + (c & 1), j = 8 * nj + 2 * t + (c & 1);
-          qk[nj][c] = j <= i ? qk[nj][c] * expf(ci[c >> 1] - cj[u]) * bj[u] : 0.f;
-        }
-      // ---- 3. o^T (rows: value channels, columns: tokens i) = V^T P^T
-      uint32_t va[4];                                 // V^T fragment: rows r0+g / +8, k = tokens 2t,2t+1 / 2t+8,2t+9
-      ldsm_x4_trans(smem_u32(sV + r_b * VS + r0 + c_b), va[0], va[1], va[2], va[3]);
-      float o[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-      for (int ni = 0; ni < 2; ++ni) {                // token columns i = 8*ni + g  (B[k = j][n = i] = p_ij)
-        uint32_t b0[3], b1[3];
-        split3x2(qk[0][2 * ni], qk[0][2 * ni + 1], b0);          // j = 2t, 2t+1
-        split3x2(qk[1][2 * ni], qk[1][2 * ni + 1], b1);          // j = 2t+8, 2t+9
-#pragma unroll
-        for (int p = 0; p < 3; ++p) mma_16816<T>(o[ni], va[0], va[1], va[2], va[3], b0[p], b1[p]);
-      }
-      // ---- 4. S^T <- e^{c_15} S^T + V'^T K,  v'_j = e^{c_15 - c_j} b_j v_j
-      const float grow = expf(c_end);
-      uint32_t wa[4][3];
-      {
-        float f[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) f[u] = expf(c_end - cj[u]) * bj[u];
-        split3x2(bits_f32(va[0] & 0xffffu) * f[0], bits_f32(va[0] >> 16) * f[1], wa[0]);
-        split3x2(bits_f32(va[1] & 0xffffu) * f[0], bits_f32(va[1] >> 16) * f[1], wa[1]);
-        split3x2(bits_f32(va[2] & 0xffffu) * f[2], bits_f32(va[2] >> 16) * f[3], wa[2]);
-        split3x2(bits_f32(va[3] & 0xffffu) * f[2], bits_f32(va[3] >> 16) * f[3], wa[3]);
+      for (int m = 0; m < 2; ++m) {
+        ldsm_x4(smem_u32(sQ + (16 * m + r_a) * QS + 16 * ks + c_a), qa[m][0], qa[m][1], qa[m][2], qa[m][3]);
+        ldsm_x4(smem_u32(sK + (16 * m + r_b) * QS + 16 * ks + c_b), kb[m][0], kb[m][1], kb[m][2], kb[m][3]);
       }
 #pragma unroll
-      for (int n = 0; n < D / 8; n += 2) {            // B[k = token j][n = key column 8n + g] = k_j
-        uint32_t kb[4];
-        ldsm_x4_trans(smem_u32(sK + r_a * QS + 8 * n + c_a), kb[0], kb[1], kb[2], kb[3]);
+      for (int n = 0; n < 4; ++n) {
+        const uint32_t b0 = kb[n >> 1][2 * (n & 1)], b1 = kb[n >> 1][2 * (n & 1) + 1];
+        if (n < 2) mma_16816<T>(qk0[n], qa[0][0], qa[0][1], qa[0][2], qa[0][3], b0, b1);
+        mma_16816<T>(qk1[n], qa[1][0], qa[1][1], qa[1][2], qa[1][3], b0, b1);
+      }
+      split3x2(S[2 * ks][0], S[2 * ks][1], a0);
+      split3x2(S[2 * ks][2], S[2 * ks][3], a1);
+      split3x2(S[2 * ks + 1][0], S[2 * ks + 1][1], a2);
+      split3x2(S[2 * ks + 1][2], S[2 * ks + 1][3], a3);
+#pragma unroll
+      for (int p = 2; p >= 0; --p)                    // the small terms first
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) S[n + m][c] *= grow;
-#pragma unroll
-          for (int p = 0; p < 3; ++p) mma_16816<T>(S[n + m], wa[0][p], wa[1][p], wa[2][p], wa[3][p], kb[2 * m], kb[2 * m + 1]);
-        }
-      }
-      // ---- 5. the chunk's output, straight from the fragments: 8 lanes write 8 neighbouring channels of a token (32 bytes)
-      float* outp = P.out + tok0 * ((int64_t)P.H * vdim) + (int64_t)h * vdim;
-      const float e_i = expf(cum);                    // lane i: e^{c_i}
-#pragma unroll
-      for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int i = 8 * ni + 2 * t + (c & 1), row = r0 + g + (c >> 1) * 8;
-          float val = o[ni][c] + (oi[0][ni][c] + (oi[1][ni][c] + oi[2][ni][c])) * __shfl_sync(0xffffffffu, e_i, i);
-          if (P.mode == 1) val += d_skip * bits_f32(sV[i * VS + row]);
-          if (i < nt && row < vdim) outp[(int64_t)i * ((int64_t)P.H * vdim) + row] = val;
+          mma_16816<T>(o[2 * m], a0[p], a1[p], a2[p], a3[p], qa[m][0], qa[m][2]);
+          mma_16816<T>(o[2 * m + 1], a0[p], a1[p], a2[p], a3[p], qa[m][1], qa[m][3]);
         }
     }
+    // ---- 2. decayed, causal: p_ij = (j <= i) (decay from j to i) b_j (q_i . k_j)
+    float cj[8], bj[8];                               // j = 8 n + 2 t, + 1
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      cj[u] = __shfl_sync(0xffffffffu, cum, 8 * (u >> 1) + 2 * t + (u & 1));
+      bj[u] = __shfl_sync(0xffffffffu, step, 8 * (u >> 1) + 2 * t + (u & 1));
+    }
+    float f[8];                                       // f_blk of the tokens of this thread's columns
+#pragma unroll
+    for (int u = 0; u < 8; ++u) f[u] = __shfl_sync(0xffffffffu, f_blk, 8 * (u >> 1) + 2 * t + (u & 1));
+    float ci[4], e1[2];                               // i = g, g + 8, g + 16, g + 24
+#pragma unroll
+    for (int u = 0; u < 4; ++u) ci[u] = __shfl_sync(0xffffffffu, cum, g + 8 * u);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) e1[u] = __shfl_sync(0xffffffffu, e_blk, g + 16 + 8 * u);
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int u = 2 * n + (c & 1), i = g + (c >> 1) * 8, j = 8 * n + 2 * t + (c & 1);
+        qk0[n][c] = j <= i ? qk0[n][c] * expf(ci[c >> 1] - cj[u]) * bj[u] : 0.f;
+        qk1[n][c] *= e1[c >> 1] * f[u];               // keys of the first block, queries of the second
+        qk1[2 + n][c] = j <= i ? qk1[2 + n][c] * expf(ci[2 + (c >> 1)] - cj[4 + u]) * bj[4 + u] : 0.f;
+      }
+    // ---- 3. o^T (rows: value channels, columns: tokens i) = e^{c_i} (S^T Q^T) + V^T P^T
+    uint32_t va[2][4];                                // V^T fragment: rows r0+g / +8, k = tokens 16 b + 2t,2t+1 / 2t+8,2t+9
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+      ldsm_x4_trans(smem_u32(sV + (16 * b + r_b) * VS + r0 + c_b), va[b][0], va[b][1], va[b][2], va[b][3]);
+    const float e_i = lane < 16 ? e_blk : e_blk * through0;   // lane i: e^{c_i}
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) {                  // token columns i = 8*ni + g  (B[k = j][n = i] = p_ij)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float e = __shfl_sync(0xffffffffu, e_i, 8 * ni + 2 * t + c);
+        o[ni][c] *= e, o[ni][c + 2] *= e;
+      }
+      const int r = 2 * (ni & 1);
+#pragma unroll
+      for (int b = 0; b <= (ni >> 1); ++b) {
+        uint32_t b0[3], b1[3];
+        const float* x0 = ni < 2 ? qk0[2 * b] : qk1[2 * b];
+        const float* x1 = ni < 2 ? qk0[(2 * b + 1) & 1] : qk1[2 * b + 1];
+        split3x2(x0[r], x0[r + 1], b0);               // j = 16 b + 2t, 2t+1
+        split3x2(x1[r], x1[r + 1], b1);               // j = 16 b + 2t+8, 2t+9
+#pragma unroll
+        for (int p = 2; p >= 0; --p) mma_16816<T>(o[ni], va[b][0], va[b][1], va[b][2], va[b][3], b0[p], b1[p]);
+      }
+    }
+    // ---- 4. S^T <- e^{c_31} S^T + V'^T K,  v'_j = e^{c_31 - c_j} b_j v_j
+    const float grow = through0 * through1;
+    uint32_t wa[2][4][3];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      float fb[4];                                    // j = 16 b + 2t, 2t+1, 2t+8, 2t+9
+#pragma unroll
+      for (int u = 0; u < 4; ++u) fb[u] = b == 0 ? f[u] * through1 : f[4 + u];
+      split3x2(bits_f32(va[b][0] & 0xffffu) * fb[0], bits_f32(va[b][0] >> 16) * fb[1], wa[b][0]);
+      split3x2(bits_f32(va[b][1] & 0xffffu) * fb[0], bits_f32(va[b][1] >> 16) * fb[1], wa[b][1]);
+      split3x2(bits_f32(va[b][2] & 0xffffu) * fb[2], bits_f32(va[b][2] >> 16) * fb[3], wa[b][2]);
+      split3x2(bits_f32(va[b][3] & 0xffffu) * fb[2], bits_f32(va[b][3] >> 16) * fb[3], wa[b][3]);
+    }
+#pragma unroll
+    for (int n = 0; n < D / 8; n += 2) {              // B[k = token j][n = key column 8n + g] = k_j
+      uint32_t kb[2][4];
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+        ldsm_x4_trans(smem_u32(sK + (16 * b + r_a) * QS + 8 * n + c_a), kb[b][0], kb[b][1], kb[b][2], kb[b][3]);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) S[n + m][c] *= grow;
+#pragma unroll
+        for (int p = 2; p >= 0; --p)
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+            mma_16816<T>(S[n + m], wa[b][0][p], wa[b][1][p], wa[b][2][p], wa[b][3][p], kb[b][2 * m], kb[b][2 * m + 1]);
+      }
+    }
+    // ---- 5. the chunk's output, straight from the fragments: 8 lanes write 8 neighbouring channels of a token (32 bytes)
+    float* outp = P.out + tok0 * ((int64_t)P.H * vdim) + (int64_t)h * vdim;
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int i = 8 * ni + 2 * t + (c & 1), row = r0 + g + (c >> 1) * 8;
+        float val = o[ni][c];
+        if (MODE == 1) val += d_skip * bits_f32(sV[i * VS + row]);
+        if (i < nt && row < vdim) outp[(int64_t)i * ((int64_t)P.H * vdim) + row] = val;
+      }
   }
   if (slot != nullptr && r0 < vdim) {
 #pragma unroll
@@ -610,7 +661,7 @@ static bool chunk_recurrence_ok(const RecParams& P, int dtype, int max_q) {
     const char* e = getenv("B200_CHUNK_RECURRENCE");
     return e != nullptr && e[0] == '0';
   }();
-  return !off && P.mode != 2 && dtype == B200_DTYPE_BF16 && P.cu_q != nullptr && max_q >= kChunk && P.kdim <= 128 && P.vdim <= 128;
+  return !off && P.mode != 2 && dtype == B200_DTYPE_BF16 && P.cu_q != nullptr && max_q >= 16 && P.kdim <= 128 && P.vdim <= 128;
 }
 
 static int chunk_recurrence_launch(const RecParams& P, int num_seqs, cudaStream_t stream) {
@@ -618,15 +669,36 @@ static int chunk_recurrence_launch(const RecParams& P, int num_seqs, cudaStream_
   const dim3 block(32 * ((P.vdim + 15) / 16));
   const bool vec = P.kdim % 8 == 0 && P.vdim % 8 == 0 && P.q_stride % 8 == 0 && P.k_stride % 8 == 0 &&
                    P.v_stride % 8 == 0 && aligned16(P.q) && aligned16(P.k) && aligned16(P.v);
-#define B200_CHUNK_REC(DV)                                                                       \
-  do {                                                                                           \
-    if (vec) launch_pdl(chunk_recurrence_kernel<DV, true>, grid, block, 0, stream, P);           \
-    else launch_pdl(chunk_recurrence_kernel<DV, false>, grid, block, 0, stream, P);              \
+  // rows of V for 4 warps where the value size allows: less shared memory, and a register budget for two CTAs per SM
+#define B200_CHUNK_REC_AS(DV, NW, VEC, M, SILU)                                                                     \
+  do {                                                                                                              \
+    auto kern = chunk_recurrence_kernel<DV, NW, VEC, M, SILU>;                                                      \
+    constexpr int smem = chunk_recurrence_smem<DV, NW>(VEC);                                                        \
+    static const cudaError_t configured =                                                                           \
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);                              \
+    if (configured != cudaSuccess) return (int)configured;                                                          \
+    launch_pdl(kern, grid, block, (size_t)smem, stream, P);                                                         \
+  } while (0)
+#define B200_CHUNK_REC_V(DV, M, SILU)                                           \
+  do {                                                                          \
+    if (P.vdim <= 64 && vec) B200_CHUNK_REC_AS(DV, 4, true, M, SILU);           \
+    else if (P.vdim <= 64) B200_CHUNK_REC_AS(DV, 4, false, M, SILU);            \
+    else if (vec) B200_CHUNK_REC_AS(DV, 8, true, M, SILU);                      \
+    else B200_CHUNK_REC_AS(DV, 8, false, M, SILU);                              \
+  } while (0)
+#define B200_CHUNK_REC(DV)                                             \
+  do {                                                                 \
+    if (P.mode == 1 && P.act_silu) B200_CHUNK_REC_V(DV, 1, true);      \
+    else if (P.mode == 1) B200_CHUNK_REC_V(DV, 1, false);              \
+    else if (P.act_silu) B200_CHUNK_REC_V(DV, 0, true);                \
+    else B200_CHUNK_REC_V(DV, 0, false);                               \
   } while (0)
   if (P.kdim <= 32) B200_CHUNK_REC(32);
   else if (P.kdim <= 64) B200_CHUNK_REC(64);
   else B200_CHUNK_REC(128);
 #undef B200_CHUNK_REC
+#undef B200_CHUNK_REC_V
+#undef B200_CHUNK_REC_AS
   return finish_launch();
 }
 
