@@ -101,7 +101,8 @@ int b200_reshape_and_cache_2d(const void* key, const void* value, void* k_cache,
  * `out` is written as zeros and nothing else is touched (padded graph rows,
  * engine/model_runner.py:303-311).
  * workspace: >= b200_paged_decode_attn_workspace_size(...) bytes, 16-byte aligned.
- * num_ctas: 0 = auto (one persistent CTA per SM), otherwise the persistent grid size.
+ * num_ctas: 0 = auto (by batch, head sizes and table width, at most one persistent CTA per SM), otherwise the persistent
+ * grid size.
  * Supported (anything else returns B200_ERR_UNSUPPORTED, and the workspace-size query returns 0):
  *   head_dim 64 or 128; num_kv_heads 1, 2, 4 or a multiple of 8; GQA group num_heads/num_kv_heads <= 8
  *   (the group is the M dimension of one m16n8k16 tile; every BASELINE model fits -- the reference's

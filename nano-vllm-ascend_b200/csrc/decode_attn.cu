@@ -629,7 +629,17 @@ extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const v
                      p.rows_box, hkv_cta * value_dim / 64, dtype, &mv);
   if (rc != B200_OK) return rc;
 
+  // num_ctas 0: the library's choice (us at 64 / 112 / 148 CTAs; contexts a third to all of the length named).
+  // * A CTA's tiles of 8 heads of 128 (64 KB per stage) in batches of 16 and more: three quarters of the SMs, each with
+  //   192 KB under way, keep HBM busier than all of them: 256 x 1074 tokens 152 / 114 / 119, 64 x 1074 46 / 37.6 / 38.7, 256 x
+  //   50 21 / 16.9 / 18.3, 16 x 1024 17 / 14.8 / 15.3. Smaller tiles need every SM: 8 heads of 64 105 / 73 / 68.
+  // * One or two sequences of up to 8192 tokens in all (by the width of the block table): what counts is the number of
+  //   partial results to merge: 1 x 300 6.9 / 7.4 / 7.7, 1 x 1500 8.7 / 9.3 / 9.4, 1 x 8000 12.8 / 13.1 / 13.0, 2 x 700 8.5 / 9.8 / 10.5.
   int grid = num_ctas > 0 ? num_ctas : num_sms();
+  if (num_ctas <= 0) {
+    if (batch <= 2 && (int64_t)batch * block_table_stride * block_size <= 8192) grid = min(grid, 64);
+    else if (batch >= 16 && hkv_cta * (head_dim + value_dim) >= 2048) grid = (grid * 3 / 4 + 7) / 8 * 8;
+  }
   if (grid > kMaxCtas) grid = kMaxCtas;
 #define B200_DECODE_DISPATCH(T)                                                              \
   (head_dim == 128 ? (value_dim == 128 ? decode_launch_d<T, 128, 128>(hkv_cta, mk, mv, p, grid, stream)  \
