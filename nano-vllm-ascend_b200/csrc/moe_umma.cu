@@ -212,7 +212,7 @@ moe_umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
 // ------------------------------------------------------------------------------------ 256-column tiles, persistent
 // The same grouped GEMM for batches that fill the chip. The kernel above is bound by two things: a 1-CTA SS-mode MMA with N =
-// 128 spends 107 cycles on 64 cycles of mathematics (43 to read the 4 KB A tile, measured, tools/umma_probe.cu), and every CTA
+// 128 spends 107 cycles on 64 cycles of mathematics (43 to read the 4 KB A tile, measured), and every CTA
 // pays its prologue, its epilogue's scattered 16-byte stores and a cold ring for 12 to 32 K blocks. Here a tile is 128 rows of
 // one expert x 256 weight rows (gate_up: 128 gate + the 128 matching up rows), so that an MMA is M128 N256 K16: 171 cycles for
 // 128 of mathematics; one CTA per SM walks tiles blockIdx.x, + gridDim.x, ..; the accumulators are double-buffered in TMEM

@@ -5,7 +5,7 @@
 // layers/attention_ori.py:63-70). Same semantics: bottom-right causal mask, packed K/V or paged K/V
 // through block_tables.
 //
-// Shape of the kernel ("FA4 shape"; measured instruction costs on this part, profiles/r01_umma_probe.log: SS M128 N64 K16 75
+// Shape of the kernel ("FA4 shape"; measured instruction costs on this part: SS M128 N64 K16 75
 // cycles, SS N128 107, TS N128 74).
 // Template parameter QT = 128-row query tiles per CTA, chosen per launch (prefill_query_tiles).
 // QT = 2: two query tiles t = 0, 1 that ping-pong and share every K / V tile: 128 rows of two heads of one kv head, or (heads

@@ -85,8 +85,8 @@ __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_
       : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem desc]: the ".ts" form (A is K-major by construction; a 16-bit A
-// operand packs two consecutive K elements per 32-bit column, lane = M row). Probed by
-// tools/umma_probe.cu modes 2/3; not used by the product kernels yet.
+// operand packs two consecutive K elements per 32-bit column, lane = M row). The P V
+// products of prefill_umma.cu.
 __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
                                        uint32_t idesc, uint32_t accumulate) {
   asm volatile(

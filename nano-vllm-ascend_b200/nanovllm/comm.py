@@ -9,13 +9,13 @@ of the rows and pushes the sums into every rank's gather buffer) for larger ones
 torch.distributed only to exchange the 64-byte IPC handles.
 
 Form selection (``mode``): one-shot while (world-1) x message <= 4 MB, two-shot beyond (both validated on
-hardware inside the engine, eager and CUDA-graph decode, r02), NCCL for shapes neither takes.
+hardware inside the engine, eager and CUDA-graph decode), NCCL for shapes neither takes.
 ``B200_ALLREDUCE`` forces one form for every shape it can take -- a measurement aid for A/B runs:
 ``nccl`` | ``oneshot`` | ``twoshot`` | ``nvls`` | ``nvls_fused`` | ``nvls_one``. The NVLS values make the region a
 torch symmetric-memory allocation (plumbing: cuMemCreate + handle exchange + cuMulticastBindMem done by
 ``torch.distributed._symmetric_memory``), which yields the same per-rank peer pointers PLUS one multicast
 address for the whole region; messages then go through b200_allreduce_add_rmsnorm_nvls[_fused]
-(in-switch reduce + in-switch broadcast). NVLS status (r02): the kernels pass their 2-GPU tests and the
+(in-switch reduce + in-switch broadcast). NVLS status: the kernels pass their 2-GPU tests and the
 eager TP=2 engine test; the CUDA-graph TP=2 engine test timed out, so it is never selected by default.
 """
 from __future__ import annotations

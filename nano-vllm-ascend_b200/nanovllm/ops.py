@@ -421,7 +421,7 @@ def _dense_plan(rows: int, device) -> torch.Tensor:
 def gate_up_silu_umma(x: torch.Tensor, w_gate_up: torch.Tensor) -> torch.Tensor:
     """SiluAndMul(x @ w_gate_up.T) in ONE kernel: the gate|up GEMM of a dense MLP on the grouped tcgen05
     kernel (one group) with the activation as its TMEM epilogue. Not on the decode path: at M = 256
-    it measured 41.87 k tok/s against 41.93 k for cuBLAS + silu_and_mul (no gain, r02).
+    it measured 41.87 k tok/s against 41.93 k for cuBLAS + silu_and_mul (no gain).
     x [M, K] contiguous; w_gate_up [2*I, K] (gate rows, then up rows); K % 64 == 0, I % 64 == 0."""
     _need_cuda(x, w_gate_up)
     M, K = x.shape

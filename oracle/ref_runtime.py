@@ -8,9 +8,9 @@ runner metadata (prepare_prefill / prepare_decode, engine/model_runner.py:238-36
 restated in oracle/model_ref.py.
 
 Two locations serve as the reference tree:
-  /root/reference        the build container (oracle/gen_golden.py writes tests/golden/ from it)
+  /root/reference        where that tree is mounted (oracle/gen_golden.py writes tests/golden/ from it)
   oracle/_ref/           reference_path.zip: the handful of modules this path needs, packed by
-                         oracle/stage_ref.py; git-ignored, travels to the GPU box with the snapshot
+                         oracle/stage_ref.py; git-ignored, copied with the tree
                          so that `bench.py --impl reference` and the `cpu_baseline` leg time the
                          reference's own code there (cpu_baseline.kind = "reference").
 Only tests/, __graft_entry__.smoke()/build() and bench.py's CPU legs may import this module.

@@ -1,5 +1,5 @@
-"""Pack the reference modules of the hot path into oracle/_ref/reference_path.zip (git-ignored; NOT
-gpurun-ignored, so the archive travels to the GPU box with the snapshot like a built .so does).
+"""Pack the reference modules of the hot path into oracle/_ref/reference_path.zip (git-ignored: the
+archive goes where the tree is copied to, as a built .so does).
 
 Why: the reference is pure Python, there is nothing to compile -- "building" it for the oracle
 means making the unmodified modules importable where /root/reference does not exist. With the
@@ -8,7 +8,7 @@ models/qwen3.py + layers/attention_torch_native.py (cpu_baseline.kind = "referen
 they fall back to the oracle port (kind = "port"). Nothing here enters git history, and nothing
 under nano-vllm-ascend_b200/ imports it.
 
-  python -m oracle.stage_ref            # build container only; called by __graft_entry__.build()
+  python -m oracle.stage_ref            # needs the reference tree; called by __graft_entry__.build()
 """
 from __future__ import annotations
 

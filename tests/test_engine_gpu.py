@@ -113,7 +113,7 @@ def test_qwen3_0_6b_config1_greedy_matches_reference(golden_models):
     """BASELINE config 1 on the GPU: random-init Qwen3-0.6B (N(0, 0.02)), 1 prompt, block 16, 32 tokens.
     Greedy ids against the unmodified reference's run; fp32 logits against the exact oracle -- the
     north_star's "logits within 1e-3" in the only form two bf16 pipelines can meet.
-    Measured on a B200 (r02, profiles/r02_parity_measured.log); bounds are <= 2x the measured values."""
+    Measured on a B200; bounds are <= 2x the measured values."""
     g = golden_models["qwen3_0_6b_config1"]
     got, mine, got32, forced = _config1_run(g)
     decided, err = _ids_on_decided_steps(got, mine, g)
@@ -125,7 +125,7 @@ def test_qwen3_0_6b_config1_greedy_matches_reference(golden_models):
     print(f"config 1 (N(0,0.02) init) fp32 logits vs oracle(exact): max-abs {d.max():.3e} rms "
           f"{d.pow(2).mean().sqrt():.3e} max|logit| {want32.abs().max():.2f}; bf16 logits vs reference run at "
           f"its top-8: max-abs {err:.3e}; decided steps {int(decided.sum())}/{len(mine)}")
-    # measured r02: max-abs 4.9e-2, rms 9.0e-3 at max|logit| 3.16 -- two bf16 pipelines (cuBLAS / tcgen05 on
+    # measured: max-abs 4.9e-2, rms 9.0e-3 at max|logit| 3.16 -- two bf16 pipelines (cuBLAS / tcgen05 on
     # the GPU, torch CPU kernels in the oracle) that round every activation of 28 layers to bf16 agree to
     # about 1.5 % of the logit range, not to 1e-3; bounds = 2x measured
     assert d.max() < 0.1 and d.pow(2).mean().sqrt() < 0.018, (d.max(), d.pow(2).mean().sqrt())
@@ -148,8 +148,8 @@ def test_qwen3_0_6b_config1_varied_ids(golden_models):
     print(f"config 1 (varied init) ids vs reference run: decided steps {int(decided.sum())}/{len(mine)}, distinct "
           f"ids compared {len(ids)}; bf16 logits vs reference run at its top-8: max-abs {err:.3e}; fp32 logits "
           f"vs oracle(exact): max-abs {d.max():.3e} rms {d.pow(2).mean().sqrt():.3e} max|logit| {want32.abs().max():.2f}")
-    assert len(ids) >= 20, (len(ids), int(decided.sum()))         # measured r02: 32 distinct ids on 35 decided steps
-    # measured r02: 0.156 / 0.255 / 0.0437 at max|logit| 6.8; bounds = 2x measured
+    assert len(ids) >= 20, (len(ids), int(decided.sum()))         # measured: 32 distinct ids on 35 decided steps
+    # measured: 0.156 / 0.255 / 0.0437 at max|logit| 6.8; bounds = 2x measured
     assert err < 0.32 and d.max() < 0.51 and d.pow(2).mean().sqrt() < 0.088
 
 

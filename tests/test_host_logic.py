@@ -750,7 +750,7 @@ def test_decode_step_form_selection():
 
 
 def test_overlap_summary_tool_on_a_synthetic_trace(tmp_path):
-    """tools/overlap_summary.py (the script behind profiles/r02b_timeline_decode_*.txt): attention-resident
+    """tools/overlap_summary.py: attention-resident
     time is the UNION of the attention kernels' intervals, whatever the streams."""
     import json
     import subprocess

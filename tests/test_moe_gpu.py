@@ -1,6 +1,5 @@
 """-m gpu: the sparse-MoE kernels (csrc/moe.cu, csrc/moe_umma.cu) and the Qwen3-MoE engine against
 the reference-generated goldens (tests/golden/moe.pt) and the CPU oracle (oracle/moe_ref.py).
-First hardware run: r02, 29 cases green (profiles/r02_validation_summary.log).
 
 Tolerances. Routing: expert ids must equal the reference's wherever the reference's own
 probabilities are not tied at the top-k boundary; weights within one rounding of the model dtype.

@@ -181,7 +181,7 @@ def test_moe_kernel_rounding_chain_reproduces_reference(golden_moe):
 
 def test_reference_archive_is_the_unmodified_reference_and_runs():
     """oracle/_ref/reference_path.zip (packed by oracle/stage_ref.py at build time; what the CPU arm of
-    bench.py imports on the GPU box): every file's SHA-256 equals the manifest's and, where the reference
+    bench.py imports): every file's SHA-256 equals the manifest's and, where the reference
     tree is present, the tree's; the reference's own Qwen3ForCausalLM decodes a step straight from it."""
     import hashlib
     import json

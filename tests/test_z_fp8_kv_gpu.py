@@ -211,7 +211,7 @@ def test_fp8_gather_dequant_bit_exact(fp8_alive, G, D, bs, dtype, scales):
 
 
 def test_fp8_chunked_and_prefix_hit_prefill(fp8_alive):
-    """kv_cache_dtype="fp8" with chunked prefill / true prefix-hit prefill (r01 rejected the combination):
+    """kv_cache_dtype="fp8" with chunked prefill / true prefix-hit prefill (once rejected):
     later windows read the earlier ones back from the e4m3 cache through gather + de-quantise. Same
     workload as the 16-bit chunked-prefill test; tokens may only drift from the un-chunked fp8 run where
     logits nearly tie (the un-chunked prefill attends over un-quantised K/V of its own step)."""

@@ -1,12 +1,11 @@
-"""First-run diagnostics + kernel-only timing for the sparse-MoE kernels (csrc/moe.cu, csrc/moe_umma.cu).
+"""Diagnostics + kernel-only timing for the sparse-MoE kernels (csrc/moe.cu, csrc/moe_umma.cu).
 
   python tools/moe_diag.py check            # every stage against an fp32 torch evaluation on the GPU,
                                             # with an error MAP (which row / column blocks are wrong)
   python tools/moe_diag.py bench            # CUDA-event timing: decode shape (HBM GB/s of expert weights)
                                             # and prefill shape (TFLOP/s), streaming vs umma vs library
-  ncu --set full -k regex:moe_ -c 6 python tools/moe_diag.py bench --once     # capture for profiles/
 
-`check` is written for the FIRST hardware run of these kernels: instead of a bare assert it prints, per
+`check` is written for a kernel that does not work yet: instead of a bare assert it prints, per
 stage, the max/mean error and the fraction of wrong elements per 16-row and per 64-column block, so that
 an indexing mistake (a swapped fragment, a wrong tile offset, a missing row mask) is recognisable from a
 single run.

@@ -1,7 +1,7 @@
-"""Summarise a chrome trace written by tools/overlap_timeline.py (one replayed decode step): per-kernel
+"""Summarise a chrome trace of one replayed decode step (torch.profiler): per-kernel
 launch counts and device times, the fraction of the step during which a paged-decode attention kernel is
 resident (the HBM-bound part), and the kernels of one layer in start order with their streams.
-Usage: python tools/overlap_summary.py gpurun_out/trace_<variant>.json [--window 2500 2720]"""
+Usage: python tools/overlap_summary.py trace.json [--window 2500 2720]"""
 import argparse
 import collections
 import json

@@ -1,5 +1,5 @@
 """A/B of the all-reduce forms on the tensor-parallel decode step in ONE torchrun
-launch (8-GPU box time is charged 8x: no repeated interpreter / NCCL start-up). One JSON line per form.
+launch (no repeated interpreter / NCCL start-up). One JSON line per form.
 
   python -m torch.distributed.run --nproc-per-node 8 --master-addr 127.0.0.1 --master-port 29621 \
       tools/tp_forms_bench.py --forms auto,nvls_fused,nccl,nvls [--model qwen3-32b] [--steps 24]
