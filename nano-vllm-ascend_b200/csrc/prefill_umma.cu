@@ -505,6 +505,8 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     auto look_up = [&](int slot) -> bool {
       Item x;
       const bool found = next_item(cur, x);
+      __syncwarp();                                  // every lane has read what this slot held (an item with no key tiles
+                                                     // for this warp has no other meeting point of its lanes)
       if (lane == 0) slots[slot] = x;
       __syncwarp();
       return found;
