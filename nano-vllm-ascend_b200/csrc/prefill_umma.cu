@@ -217,12 +217,14 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
   }
+  // The kernel before this one may still have CTAs on the SM that have yet to allocate their columns (it lets its dependents
+  // in at its start): taking all 512 before it has finished could leave both waiting.
+  pdl_wait();
   if (warp == kMmaWarp) umma::tmem_alloc(tmem_slot, kTmemCols);
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tb = *tmem_slot;
-  pdl_wait();
 
   // Work items: (row tile, sequence, head, key split) in order of falling row tile, so that the longest come first and a
   // CTA's items have about the same number of key tiles as any other's; inside a row tile key
