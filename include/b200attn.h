@@ -50,6 +50,7 @@ enum {
   B200_ERR_WORKSPACE = -5,       /* workspace too small */
   B200_ERR_DRIVER = -6,          /* cuTensorMapEncodeTiled unavailable / failed */
   B200_ERR_BAD_DTYPE = -7,
+  B200_ERR_WAIT = -8,            /* a wait inside a kernel of an EARLIER call ran out: that call's output is not valid */
 };
 
 /* Version of the loaded library (== B200ATTN_VERSION it was built with). */
@@ -60,6 +61,12 @@ const char* b200_error_string(int code);
  * (host-side counter; lets bench.py report `gpu_launches`). */
 int64_t b200_launch_count(void);
 void b200_reset_launch_count(void);
+/* Waits of the persistent grouped GEMM (b200_moe_gemm_*_umma on prompt-sized batches) are bounded. When one runs out, the
+ * kernel returns without having written its output and sets a word of page-locked host memory. b200_take_wait_status asks
+ * and clears it: B200_ERR_WAIT or B200_OK, meaningful for kernels that the host has waited for. The same entry points ask it
+ * first of all, so that a call after the failed one returns B200_ERR_WAIT. b200_wait_status_word: the word itself. */
+int b200_take_wait_status(void);
+int32_t* b200_wait_status_word(void);
 
 /* ---------------------------------------------------------------------------------
  * K1  reshape_and_cache, flat slots.
@@ -386,6 +393,11 @@ int b200_moe_gemm_down_umma(void* y, const void* h, const void* w2, const int32_
                             const int32_t* sorted_pair, const void* topk_weights, int32_t pairs,
                             int32_t inter, int32_t hidden, int32_t num_local, int32_t dtype,
                             b200_stream_t stream);
+/* down_umma without weights and with its own limit on a single wait of the persistent kernel. 0: a wait whose phase is
+ * not complete at once gives up (how the way out is tested). */
+int b200_moe_gemm_down_umma_bounded(void* y, const void* h, const void* w2, const int32_t* offsets, int32_t pairs,
+                                    int32_t inter, int32_t hidden, int32_t num_local, int32_t dtype, int64_t wait_ns,
+                                    b200_stream_t stream);
 
 /* Grouped product with fp32 output on the same tcgen05 kernel, the accumulators stored as they are (attention
  * scores of 16-bit operands): rows offsets[g] .. offsets[g+1] of a [rows, K] are multiplied with w[g] ([groups,

@@ -19,6 +19,11 @@ extern long long g_launch_count;  // api.cu
     if (cond) return (code);       \
   } while (0)
 
+// The word that a kernel sets when one of its bounded waits runs out: page-locked, the same address on the host and every
+// device (nullptr: it could not be had). take_wait_status: was it set? It is cleared by the question (api.cu).
+int* wait_status();
+bool take_wait_status();
+
 inline int finish_launch(int kernels = 1) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;

@@ -32,6 +32,8 @@ struct MoeUmmaParams {
   int num_local, K, n_out;
   int out_f32;                 // plain epilogue only: the fp32 accumulators are stored as they are (out is float*)
   const float* in_scale = nullptr;   // gate_up: weight of every pair on the expert's INPUT (fp32), or nullptr
+  int64_t wait_ns = 0;               // moe_umma_wide_kernel: limit of one wait, and the word that a CTA sets when it runs out
+  int* wait_status = nullptr;
 };
 
 // Ring depth: 3 stages (97 KB, two CTAs per SM) for tensor-bound grouped GEMMs, where the second CTA's
@@ -222,22 +224,47 @@ moe_umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 // global stores are whole 128-byte segments.
 // Measured (4096 tokens, top 8 of 128 experts, hidden 2048, inter 768): gate_up 332 -> 215 us (960 TFLOP/s), down 312 -> 121
 // us (850 TFLOP/s).
-// Waits are bounded: a wait that gives up sets a flag on which every role leaves its loop (g_wait_gave_up counts it).
-__device__ unsigned int g_wait_gave_up;
-
+// Waits are bounded by time (p.wait_ns). A wait that runs out sets a flag of the CTA, on which every role leaves its loop, its
+// warps whole; the producer waits for the copies that are under way, the issuer for its products, and the CTA sets the
+// host's word (*p.wait_status): the output is not valid, and the library reports it (take_wait_status, api.cu).
 constexpr int kMwStages = 4;
 constexpr int kMwStageBytes = 3 * kMuPanel;                 // 128 rows of A, 256 rows of W, 64 columns each
 constexpr int kMwOut = 4 * 32 * 128;                        // epilogue: 32 rows x 128 bytes per warp
 constexpr int kMwMaxExperts = 256;
 constexpr int kMwSmem = 1024 + kMwStages * kMwStageBytes + kMwOut + 128 + (kMwMaxExperts + 4) * 4;
 
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
-  for (int n = 0; n < (1 << 24); ++n) {
+constexpr int64_t kMwWaitNs = 4000000000ll;                  // a launch takes milliseconds at most
+constexpr int64_t kMwDrainNs = 1000000000ll;
+
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {      // does not suspend
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ int64_t global_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return (int64_t)t;
+}
+// false: the phase did not complete within limit_ns, or another role of the CTA gave up first (gave_up, where given). One
+// thread's answer: warps vote on it
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* gave_up, int64_t limit_ns) {
+  if (mbar_test_wait(bar, parity)) return true;
+  if (limit_ns > 0) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (*gave_up) return false;
+    const int64_t t0 = global_ns();
+    do {
+      if (mbar_try_wait(bar, parity)) return true;
+      if (gave_up != nullptr && *gave_up) return false;
+    } while (global_ns() - t0 < limit_ns);
   }
-  *gave_up = 1;
-  atomicAdd(&g_wait_gave_up, 1u);
+  if (gave_up != nullptr) *gave_up = 1;
   return false;
 }
 
@@ -251,6 +278,7 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   uint64_t *full = bars, *empty = bars + kMwStages, *acc_full = bars + 2 * kMwStages, *acc_empty = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* drained = acc_empty + 3;                              // [1] the products that were under way when a wait ran out
   int* first = reinterpret_cast<int*>(s_out + kMwOut + 128);      // [num_local + 1] row tiles of the experts before
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -280,6 +308,7 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], 128);
     }
+    mbar_init(drained, 1);
     mbar_fence_init();
     *gave_up = 0;
   }
@@ -324,7 +353,7 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int w1 = w0 + (kGateUp ? p.n_out : 128);
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % kMwStages;
-          ok = mbar_wait_bounded(&empty[s], ((it / kMwStages) & 1) ^ 1, gave_up);
+          ok = mbar_wait_bounded(&empty[s], ((it / kMwStages) & 1) ^ 1, gave_up, p.wait_ns);
           if (!ok) break;
           uint8_t* sa = smem + s * kMwStageBytes;
           mbar_expect_tx(&full[s], kMwStageBytes);
@@ -333,11 +362,10 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           tma_load_3d(sa + 2 * kMuPanel, &tmW, &full[s], 0, w1, kb, stream);
         }
       }
-      // copies in flight land before the CTA's shared memory is given back (on the ordinary way out they are consumed)
-      if (!ok)
-        for (int s = 0; s < kMwStages; ++s)
-          for (int n = 0; n < (1 << 16); ++n)
-            if (mbar_try_wait(&full[s], 0) && mbar_try_wait(&full[s], 1)) break;
+      // copies under way land before the CTA's shared memory is given back, whichever role leaves early: the last ones of
+      // every stage, copies max(0, it - stages) .. it - 1
+      for (int j = max(0, it - kMwStages); j < it; ++j)
+        mbar_wait_bounded(&full[j % kMwStages], (j / kMwStages) & 1, nullptr, kMwDrainNs);
     }
   } else if (warp == 1) {
     // =========================== MMA issuer ===========================
@@ -348,11 +376,11 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++n) {
       const int buf = n & 1;
-      ok = mbar_wait_bounded(&acc_empty[buf], ((n >> 1) & 1) ^ 1, gave_up);
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&acc_empty[buf], ((n >> 1) & 1) ^ 1, gave_up, p.wait_ns));
       umma::fence_after_sync();
       for (int kb = 0; kb < KB && ok; ++kb, ++it) {
         const int s = it % kMwStages;
-        ok = mbar_wait_bounded(&full[s], (it / kMwStages) & 1, gave_up);
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], (it / kMwStages) & 1, gave_up, p.wait_ns));
         if (!ok) break;
         umma::fence_after_sync();
         if (leader) {
@@ -367,6 +395,11 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         __syncwarp();
       }
     }
+    // products under way finish before the columns and the operands go, whichever role leaves early
+    if (leader) umma::commit(drained);
+    __syncwarp();
+    mbar_wait_bounded(drained, 0, nullptr, kMwDrainNs);
+    __syncwarp();
   } else {
     // =========================== epilogue warps (2..5) ===========================
     const int quarter = warp & 3;                    // the TMEM lane quarter this warp may access
@@ -387,7 +420,7 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       } else if (p.pair_scale != nullptr && valid) {
         sc = to_f32<T>(reinterpret_cast<const T*>(p.pair_scale)[p.sorted_pair[pos]]);
       }
-      if (!mbar_wait_bounded(&acc_full[buf], (n >> 1) & 1, gave_up)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&acc_full[buf], (n >> 1) & 1, gave_up, p.wait_ns))) break;
       umma::fence_after_sync();
       const uint32_t acc = tb + lane_base + buf * 256;
       if (row0 < cnt) {
@@ -439,6 +472,10 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   umma::fence_before_sync();
   __syncthreads();
   if (warp == 1) umma::tmem_dealloc(tb, 512);
+  if (threadIdx.x == 0 && *gave_up) {
+    *reinterpret_cast<volatile int*>(p.wait_status) = 1;
+    __threadfence_system();
+  }
 }
 
 // XS[pos] = X[sorted_pair[pos] / top_k] for the positions the plan holds; one warp per row
@@ -539,7 +576,7 @@ extern "C" int b200_moe_gather_rows(void* xs, const void* x, const int32_t* offs
 static int moe_umma_common(bool gate_up, void* out, const void* a, const void* w, const int32_t* offsets,
                            const int32_t* sorted_pair, const void* pair_scale, int32_t pairs, int32_t K,
                            int32_t n_out, int32_t num_local, int32_t dtype, b200_stream_t stream,
-                           int out_f32 = 0, const float* in_scale = nullptr) {
+                           int out_f32 = 0, const float* in_scale = nullptr, int64_t wait_ns = kMwWaitNs) {
   B200_RETURN_IF(dtype != B200_DTYPE_BF16 && dtype != B200_DTYPE_F16, B200_ERR_BAD_DTYPE);
   B200_RETURN_IF(pairs < 0 || K <= 0 || n_out <= 0 || num_local <= 0, B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(K % 64 != 0 || n_out % (gate_up ? 64 : 128) != 0 || num_local > 256, B200_ERR_UNSUPPORTED);
@@ -547,6 +584,7 @@ static int moe_umma_common(bool gate_up, void* out, const void* a, const void* w
   B200_RETURN_IF(!out || !a || !w || !offsets, B200_ERR_NULL_POINTER);
   B200_RETURN_IF(!gate_up && ((sorted_pair == nullptr) != (pair_scale == nullptr)), B200_ERR_NULL_POINTER);
   B200_RETURN_IF(!aligned16(out) || !aligned16(a) || !aligned16(w), B200_ERR_MISALIGNED);
+  B200_RETURN_IF(take_wait_status(), B200_ERR_WAIT);             // of an earlier call
   CUtensorMap ma, mw;
   int rc = get_panel_map(a, pairs, (int64_t)K * 2, K / 64, 128, 1, dtype, &ma);
   if (rc != B200_OK) return rc;
@@ -554,8 +592,9 @@ static int moe_umma_common(bool gate_up, void* out, const void* a, const void* w
   const bool wide = moe_umma_wide(gate_up, pairs, n_out, out_f32);
   rc = get_panel_map(w, w_rows, (int64_t)K * 2, K / 64, wide ? 128 : 64, 1, dtype, &mw);
   if (rc != B200_OK) return rc;
-  MoeUmmaParams p{offsets, sorted_pair, pair_scale, out, num_local, K, n_out, out_f32, in_scale};
+  MoeUmmaParams p{offsets, sorted_pair, pair_scale, out, num_local, K, n_out, out_f32, in_scale, wait_ns, wait_status()};
   if (wide) {
+    B200_RETURN_IF(p.wait_status == nullptr, B200_ERR_DRIVER);
     if (dtype == B200_DTYPE_BF16)
       return gate_up ? moe_umma_wide_launch<__nv_bfloat16, true>(ma, mw, p, (cudaStream_t)stream)
                      : moe_umma_wide_launch<__nv_bfloat16, false>(ma, mw, p, (cudaStream_t)stream);
@@ -581,6 +620,14 @@ extern "C" int b200_moe_gemm_down_umma(void* y, const void* h, const void* w2, c
                                        b200_stream_t stream) {
   return moe_umma_common(false, y, h, w2, offsets, sorted_pair, topk_weights, pairs, inter, hidden, num_local,
                          dtype, stream);
+}
+
+extern "C" int b200_moe_gemm_down_umma_bounded(void* y, const void* h, const void* w2, const int32_t* offsets,
+                                               int32_t pairs, int32_t inter, int32_t hidden, int32_t num_local,
+                                               int32_t dtype, int64_t wait_ns, b200_stream_t stream) {
+  B200_RETURN_IF(wait_ns < 0, B200_ERR_BAD_SHAPE);
+  return moe_umma_common(false, y, h, w2, offsets, nullptr, nullptr, pairs, inter, hidden, num_local, dtype, stream, 0,
+                         nullptr, wait_ns);
 }
 
 extern "C" int b200_gemm_f32out_umma(float* out, const void* a, const void* w, const int32_t* offsets,

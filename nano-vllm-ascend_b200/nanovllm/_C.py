@@ -23,6 +23,8 @@ PROTOTYPES = {
     "b200_error_string": (c_char_p, [c_int32]),
     "b200_launch_count": (c_int64, []),
     "b200_reset_launch_count": (None, []),
+    "b200_take_wait_status": (c_int32, []),
+    "b200_wait_status_word": (c_void_p, []),
     "b200_reshape_and_cache": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                          c_int32, c_int32, c_int32, c_int64, c_int64, c_int32,
                                          c_int32, c_int32, c_void_p]),
@@ -100,6 +102,8 @@ PROTOTYPES = {
                                         c_int32, c_void_p]),
     "b200_moe_gemm_down_umma": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                           c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p]),
+    "b200_moe_gemm_down_umma_bounded": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
+                                                  c_int32, c_int32, c_int64, c_void_p]),
     "b200_moe_combine": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
                                    c_int64, c_int32, c_void_p]),
     "b200_allreduce_add_rmsnorm": (c_int32, [c_void_p, c_void_p, c_void_p, c_float, c_int32, c_int32,

@@ -24,6 +24,7 @@ import numpy as np
 import torch
 import torch.distributed as dist
 
+from .. import ops
 from ..config import Config, GraphMode
 from ..layers.sampler import Sampler
 from ..models.models_map import model_dict
@@ -593,6 +594,13 @@ class ModelRunner:
                 m.v_cache[-1].zero_()
 
     # ------------------------------------------------------------------ run
+    @staticmethod
+    def _tokens(out: torch.Tensor) -> list[int]:
+        """The sampled tokens of a prompt step on the host, where no kernel of the step gave up a wait."""
+        tokens = out.tolist()
+        ops.check_waits()
+        return tokens
+
     @torch.inference_mode()
     def run(self, seqs: list[Sequence], is_prefill: bool, logit_rows: list[int] | None = None):
         """One step. Returns the sampled token of every sequence -- or, with ``logit_rows`` (scoring and trace
@@ -606,6 +614,7 @@ class ModelRunner:
             if logit_rows:
                 rows = torch.tensor(logit_rows, dtype=torch.int64, pin_memory=True).to(self.device, non_blocking=True)
                 out = self.model.lm_head.logits_at(hidden, rows).float().cpu()
+                ops.check_waits()
             reset_context()
             return out
         if is_prefill:
@@ -619,7 +628,7 @@ class ModelRunner:
                 self.d_rng.add_(1)
                 self._sample_sharded(hidden, temps, torch.empty_like(out), out)
                 reset_context()
-                return out.tolist()
+                return self._tokens(out)
             logits = self.model.compute_logits(self.model(ids, pos))
             if self.rank == 0:
                 temps = torch.tensor([0.0 if s.greedy else s.temperature for s in seqs],
@@ -629,7 +638,7 @@ class ModelRunner:
             if self.world_size > 1:
                 dist.broadcast(out, 0)
             reset_context()
-            return out.tolist()
+            return self._tokens(out)
         use_graph = not self.enforce_eager and n <= self.config.max_num_seqs
         bs = next(b for b in self._buckets() if b >= n) if use_graph else n
         kv_tokens = self._stage_decode(seqs, bs)

@@ -290,3 +290,25 @@ def test_plan_is_a_stable_sort_by_expert(T, k, E, begin, n, shift):
     assert (plan.pos_of_pair.cpu().numpy() == pos).all()
     counts = np.bincount(flat[local] - begin, minlength=n)
     assert (plan.offsets.cpu().numpy() == np.concatenate([[0], np.cumsum(counts)])).all()
+
+
+def test_a_wait_that_runs_out_is_reported():
+    """The persistent grouped GEMM with no patience at all: it leaves with copies and products under way, the status word is
+    set, the next call raises, and the one after it is right."""
+    from nanovllm import _C, ops
+    lib = _C.load()
+    M, K, N = 20000, 768, 512
+    g = torch.Generator().manual_seed(3)
+    x, w = (torch.randn(r, K, generator=g).bfloat16().cuda() for r in (M, N))
+    want = (x.float() @ w.float().T).bfloat16()
+    offsets, out = torch.tensor([0, M], dtype=torch.int32, device="cuda"), torch.zeros(M, N, dtype=x.dtype, device="cuda")
+    torch.cuda.synchronize()
+    ops.check_waits()
+    _C.check(lib.b200_moe_gemm_down_umma_bounded(out.data_ptr(), x.data_ptr(), w.data_ptr(), offsets.data_ptr(), M, K, N, 1,
+                                                 _C.BF16, 0, torch.cuda.current_stream().cuda_stream), "bounded")
+    torch.cuda.synchronize()
+    with pytest.raises(_C.B200Error, match="ran out"):
+        ops.linear_umma(x, w)
+    _close(ops.linear_umma(x, w), want, "after it")
+    torch.cuda.synchronize()
+    ops.check_waits()
