@@ -37,10 +37,9 @@ def _stream() -> int:
 
 def _stream_of(device) -> int:
     """The current stream of `device` (a tensor's device, or whatever torch.cuda.current_stream takes)."""
-    index = getattr(device, "index", None)
-    if index is None:
-        return torch.cuda.current_stream(device).cuda_stream
-    return torch._C._cuda_getCurrentRawStream(index)
+    if isinstance(device, torch.device) and device.index is not None:
+        return torch._C._cuda_getCurrentRawStream(device.index)
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def _ptr(t):
