@@ -277,8 +277,9 @@ bool attn_tiled_fits(int max_q, int rep, int dim, int vdim) {
 template <typename T, int VC, bool VEC>
 static int attn_tiled_launch_as(const AttnTiledParams& P, dim3 grid, size_t smem, cudaStream_t stream) {
   auto kern = attn_tiled_kernel<T, VC, VEC>;
-  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-  if (configured != cudaSuccess) return (int)configured;
+  static std::atomic<uint64_t> devices{0};
+  const cudaError_t allowed = allow_smem(kern, 220 * 1024, devices);
+  if (allowed != cudaSuccess) return (int)allowed;
   launch_pdl(kern, grid, dim3(kTThreads), smem, stream, P);
   return finish_launch();
 }

@@ -7,6 +7,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "../../include/b200attn.h"
 
 namespace b200 {
@@ -63,6 +65,20 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Dynamic shared memory above 48 KB has to be asked for once per kernel and DEVICE: `devices` (a static of the launcher,
+// one per kernel) has a bit for each that was told. A failure is returned and asked for anew by the next call.
+template <typename Kernel>
+inline cudaError_t allow_smem(Kernel kernel, int bytes, std::atomic<uint64_t>& devices) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;
+  if (devices.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_relaxed);
+  return e;
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -528,8 +528,9 @@ static int moe_umma_launch_s(const CUtensorMap& ma, const CUtensorMap& mw, const
 template <typename T, bool kGateUp>
 static int moe_umma_wide_launch(const CUtensorMap& ma, const CUtensorMap& mw, const MoeUmmaParams& p, cudaStream_t stream) {
   auto kern = moe_umma_wide_kernel<T, kGateUp>;
-  static const cudaError_t configured = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMwSmem);
-  if (configured != cudaSuccess) return (int)configured;
+  static std::atomic<uint64_t> devices{0};
+  const cudaError_t allowed = allow_smem(kern, kMwSmem, devices);
+  if (allowed != cudaSuccess) return (int)allowed;
   launch_pdl(kern, dim3(moe_sm_count()), dim3(kMuThreads), (size_t)kMwSmem, stream, ma, mw, p);
   return finish_launch();
 }

@@ -674,9 +674,9 @@ static int chunk_recurrence_launch(const RecParams& P, int num_seqs, cudaStream_
   do {                                                                                                              \
     auto kern = chunk_recurrence_kernel<DV, NW, VEC, M, SILU>;                                                      \
     constexpr int smem = chunk_recurrence_smem<DV, NW>(VEC);                                                        \
-    static const cudaError_t configured =                                                                           \
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);                              \
-    if (configured != cudaSuccess) return (int)configured;                                                          \
+    static std::atomic<uint64_t> devices{0};                                                                        \
+    const cudaError_t allowed = allow_smem(kern, smem, devices);                                                    \
+    if (allowed != cudaSuccess) return (int)allowed;                                                                \
     launch_pdl(kern, grid, block, (size_t)smem, stream, P);                                                         \
   } while (0)
 #define B200_CHUNK_REC_V(DV, M, SILU)                                           \

@@ -19,3 +19,13 @@ def test_tensor_memory_is_allocated_after_the_kernel_before_has_finished():
             seen += 1
             at = text.find("umma::tmem_alloc(", at + 1)
     assert seen >= 3
+
+
+def test_shared_memory_is_asked_for_on_every_device():
+    """A kernel's attributes hold for one device: a launcher that remembers per process that it has asked refuses every call on
+    the second device. The launchers of these files serve calls that needed no such memory before, or asked each time."""
+    for name in ("attn_tiled.cu", "moe_umma.cu", "seq_mixers.cu"):
+        with open(os.path.join(CSRC, name)) as f:
+            text = f.read()
+        assert "static const cudaError_t" not in text, name
+        assert text.count("allow_smem(") >= 1, name
