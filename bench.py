@@ -459,7 +459,7 @@ def attention_roofline(runner, group, B, K, tpw, fp8, peak, peak_src):
 
     # launched the way the step launches it: the runner's grid size, and -- when the step runs as two
     # micro-batches at this batch / context -- two launches of half the rows each
-    ctas = runner._attn_ctas(B)
+    ctas = runner._grid(runner._attn_ctas(B))
     split = runner._overlap_split(B) if runner.use_split(B, int(runner.h_ctx[:B].sum())) else 0
     parts = [(0, split), (split, B)] if split else [(0, B)]
 

@@ -329,7 +329,8 @@ class Config:
                                             # resident attention kernel: measured, no overlap at all)
     decode_attn_ctas: int = -1         # persistent grid of the paged decode kernel in decode steps: 0 = one CTA
                                        # per SM; -1 = auto: 0.7 x #SMs (a multiple of 8) from 128 rows on -- the
-                                       # HBM-saturated regime, where 104 CTAs stream 6.7 TB/s and 148 CTAs 6.4
+                                       # HBM-saturated regime, where 104 CTAs stream 6.7 TB/s and 148 CTAs 6.4 --
+                                       # and the library's own choice below that and on tensor-parallel ranks
     device = "cuda"
 
     def __post_init__(self):

@@ -456,20 +456,25 @@ class ModelRunner:
         return int(lens.sum())
 
     def _attn_ctas(self, bs: int) -> int:
-        """Persistent grid of the paged decode kernel for a `bs`-row step (Config.decode_attn_ctas)."""
+        """Persistent grid of the paged decode kernel for a `bs`-row step (Config.decode_attn_ctas): 0 is the library's own
+        choice where Config leaves it to the runner (-1), and one CTA per SM where Config says 0 (_grid)."""
         n = self.config.decode_attn_ctas
         if n >= 0:
             return n
         if bs < 128 or self.shard_world > 1 or self._kv_token_bytes < 4096:
-            return 0                    # small launches are latency-bound: every SM helps
+            return 0                    # csrc/decode_attn.cu: by rows, head sizes and table width
         return max(8, int(self._num_sms * 0.7 + 4) // 8 * 8)
+
+    def _grid(self, ctas: int) -> int:
+        """What the kernels are told for `ctas` of _attn_ctas: their 0 is the library's choice, not one CTA per SM."""
+        return self._num_sms if ctas == 0 and self.config.decode_attn_ctas == 0 else ctas
 
     def _set_decode_context(self, bs: int, real_bs: int, lo: int = 0, own_gemm: bool = False, ctas: int | None = None):
         """Publish rows [lo, bs) of the static decode buffers as the step context."""
         set_context(False, slot_mapping=self.d_slots[lo:bs], context_lens=self.d_ctx[lo:bs],
                     block_tables=self.d_tables[lo:bs], is_enforce_eager=self.enforce_eager,
                     real_bs=real_bs, block_size=self.block_size,
-                    decode_attn_ctas=self._attn_ctas(bs) if ctas is None else ctas, own_gemm=own_gemm,
+                    decode_attn_ctas=self._grid(self._attn_ctas(bs) if ctas is None else ctas), own_gemm=own_gemm,
                     state_slots=self.d_state[lo:bs] if self.state_modules else None)
 
     # ------------------------------------------------------------------ the decode step

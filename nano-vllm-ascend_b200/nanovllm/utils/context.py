@@ -16,7 +16,7 @@ One addition: ``paged_prefill`` -- True when the prefill step feeds only the unc
 and attention must read K/V through block_tables (true prefix hit, attention_ori.py:65-66);
 the reference runner at this commit always recomputes, so it defaults to False.
 Second addition: ``decode_attn_ctas`` -- persistent grid size of the paged decode kernel for this step
-(0 = one CTA per SM); the runner's two-micro-batch decode step sets it so that the attention of one
+(0 = the library's own choice, csrc/decode_attn.cu); the runner's two-micro-batch decode step sets it so that the attention of one
 half leaves SMs to the GEMMs of the other (engine/model_runner.py). Third: ``own_gemm`` -- the
 linear layers of this step run on the library's single-CTA tcgen05 GEMM (ops.linear_umma) instead of
 cuBLAS, whose 2-CTA clustered kernels cannot be placed next to a resident attention kernel.
