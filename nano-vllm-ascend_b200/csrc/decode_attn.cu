@@ -633,11 +633,17 @@ extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const v
   // * A CTA's tiles of 8 heads of 128 (64 KB per stage) in batches of 16 and more: three quarters of the SMs, each with
   //   192 KB under way, keep HBM busier than all of them: 256 x 1074 tokens 152 / 114 / 119, 64 x 1074 46 / 37.6 / 38.7, 256 x
   //   50 21 / 16.9 / 18.3, 16 x 1024 17 / 14.8 / 15.3. Smaller tiles need every SM: 8 heads of 64 105 / 73 / 68.
-  // * One or two sequences of up to 8192 tokens in all (by the width of the block table): what counts is the number of
-  //   partial results to merge: 1 x 300 6.9 / 7.4 / 7.7, 1 x 1500 8.7 / 9.3 / 9.4, 1 x 8000 12.8 / 13.1 / 13.0, 2 x 700 8.5 / 9.8 / 10.5.
+  //   The line was drawn at 16 rows; 3 to 15 rows of 8 heads of 128 measure 0 to 6 % less with 112 as well (8 x 4000 21.5 / 22.4).
+  // * One or two (sequence, group of 8 kv heads) of up to 8192 tokens in all (by the width of the block table) whose query
+  //   heads have 2048 output columns and more: what counts is the partial results to merge, and there are as many as CTAs.
+  //   16 heads over 8 of 128: 1 x 300 7.0 / 7.5 / 8.1, 1 x 1000 8.4 / 8.7 / 9.2, 1 x 4000 11.2 / 11.6 / 12.5, 2 x 300 7.3 / 7.7 /
+  //   8.2, 2 x 1000 9.1 / 8.8 / 9.4, 2 x 4000 13.5 / 13.0 / 13.3; 32 over 8 of 64: 1 x 1000 8.2 / 9.6 / 10.7, 2 x 4000 11.5 / 12.1 /
+  //   13.6. Narrower ones and more groups want the SMs: 32 over 32 of 128 1 x 300 8.6 / 7.4 / 7.5, 2 x 4000 26.8 / 22.6 / 23.2; 16
+  //   over 16 of 64 1 x 4000 11.1 / 10.4 / 10.5; 8 over 2 of 128 2 x 4000 11.0 / 9.4 / 9.8; 4 over 4 of 128 2 x 4000 11.2 / 10.7 / 10.9.
   int grid = num_ctas > 0 ? num_ctas : num_sms();
   if (num_ctas <= 0) {
-    if (batch <= 2 && (int64_t)batch * block_table_stride * block_size <= 8192) grid = min(grid, 64);
+    if (batch * hg_count <= 2 && num_heads / hg_count * value_dim >= 2048 && (int64_t)batch * block_table_stride * block_size <= 8192)
+      grid = min(grid, 64);
     else if (batch >= 16 && hkv_cta * (head_dim + value_dim) >= 2048) grid = (grid * 3 / 4 + 7) / 8 * 8;
   }
   if (grid > kMaxCtas) grid = kMaxCtas;

@@ -31,3 +31,10 @@ def test_library_choice(B, H, G, D, most, width):
             p = torch.softmax(k[:, h * G // H] @ q[b, h].double() * D ** -0.5, 0)
             # probabilities and the result in fp16: 2^-12 each of values below ~4
             assert float((got[b, h * D:(h + 1) * D] - p @ v[:, h * G // H]).abs().max()) < 4e-3, (b, h)
+
+
+@pytest.mark.parametrize("B,H,G,D,most,width", [(1, 32, 32, 128, 500, 64), (1, 16, 16, 64, 900, 64), (2, 8, 2, 128, 700, 64),
+                                                (2, 32, 8, 64, 700, 64), (1, 32, 16, 128, 300, 32)])
+def test_groups_and_widths_of_the_small_rule(B, H, G, D, most, width):
+    """One or two rows: one, two and four groups of kv heads, query heads of 1024 and of 2048 output columns in a group."""
+    test_library_choice(B, H, G, D, most, width)
