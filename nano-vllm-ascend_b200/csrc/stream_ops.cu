@@ -785,10 +785,15 @@ extern "C" int b200_delta_prep(float* qk, float* decay, float* beta, const void*
   const int64_t lanes16 = dtype == B200_DTYPE_F32 ? 4 : 8;           // elements of 16 bytes
   const bool vec = dim % 8 == 0 && dim <= 256 && qk_stride % lanes16 == 0 && aligned16(qk_in) && aligned16(qk) &&
                    (per_head || (a_stride % lanes16 == 0 && aligned16(a) && aligned16(decay) && aligned16(dt_bias)));
-  if (vec) {
-    int gl = 1;
-    while (gl * 8 < dim) gl <<= 1;
-    const int64_t per_cta = 8 * (32 / gl);
+  int gl = 1;
+  while (gl * 8 < dim) gl <<= 1;
+  const int64_t per_cta = 8 * (32 / gl);
+  // The 16-byte form where its CTAs reach most SMs (it packs 32 / gl units into a warp), or, with a decay per head, where there
+  // is enough to hide a lane's walk over several heads. us, element form / this one, 8 heads over 4 of 128, 32 over 16 of 64,
+  // 32 over 16 of 128: per channel, 64 tokens 2.2 / 2.3, 2.6 / 2.6, 3.4 / 3.3; 128 tokens 2.6 / 2.5, 4.0 / 3.3, 4.6 / 4.1; 16
+  // tokens 2.1 / 2.3, 1.9 / 2.3, 2.2 / 2.4; per head, 256 tokens 2.0 / 2.2, 3.2 / 3.4, 3.0 / 3.2; 512 2.2 / 2.4, 4.9 / 3.7, 4.9 / 4.6;
+  // 1024 3.0 / 2.9, 8.7 / 5.5, 8.6 / 7.1.
+  if (vec && (per_head ? units >= 9216 : units >= 128 * per_cta)) {
     B200_DISPATCH_3(dtype, T, launch_pdl(delta_prep_vec_kernel<T>, dim3((unsigned)((units + per_cta - 1) / per_cta)), dim3(256),
                                          0, (cudaStream_t)stream, qk, decay, beta, (const T*)qk_in, qk_stride, (const T*)a,
                                          a_stride, (const T*)b, b_stride, dt_bias, a_log, tokens, num_heads, groups, dim,
