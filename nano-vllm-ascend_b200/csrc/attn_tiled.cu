@@ -15,7 +15,8 @@
 // Rows of Q, K and P are unpadded with their 16-byte chunks XOR-swizzled, so that 64 x 64 tiles of 128-wide heads take 112 KB
 // and two CTAs share an SM: one computes while the other waits at its barriers.
 // Measured (4 ragged prompts of 700-1024 tokens, 8 heads over 2 of 128, fp32, paged): 2427 us -> 352 us with the row tiles of one
-// sequence after the other (SMs idle 30 % of the time, FMA pipes 66 % busy otherwise), 298 us (21 TFLOP/s) with the longest tiles of all first.
+// sequence after the other, 298 us with the longest tiles of all first, 291 us (21.5 TFLOP/s) where warps whose rows lie past the
+// span only copy and the last tile ends at its last key.
 #include "seq_common.cuh"
 #include "attn_tiled.cuh"
 
@@ -60,6 +61,7 @@ attn_tiled_kernel(const AttnTiledParams P) {
   // ---- staging: nr rows of `width` columns as fp32, zero past them. Warp w copies rows 8 w .. 8 w + 7, a lane one 16-byte
   // chunk at a time; the eight row offsets (a division and a table look-up each) are found by eight lanes at once
   const int warp = tid >> 5, lane = tid & 31;
+  const bool live = r0 + 8 * warp < rows;                           // warp-uniform: some row of this warp exists
   auto stage = [&](float* dst, bool swizzled, int chunks, int width, int nr, const T* base, auto row_offset) {
     const int mine = 8 * warp + (lane & 7);
     const int64_t offset = mine < nr ? row_offset(mine) : 0;
@@ -146,19 +148,21 @@ attn_tiled_kernel(const AttnTiledParams P) {
     const int steps = (dim + 3) >> 2;
     const float4* kt = reinterpret_cast<const float4*>(sk) + tx * QC;
     const float4* qt = reinterpret_cast<const float4*>(sq) + 4 * ty * QC;
+    if (live) {                                       // (warps whose rows all lie past the span only copy)
 #pragma unroll 2
-    for (int c = 0; c < steps; ++c) {
-      float4 kk[4];
-      const int ck = c ^ (tx & 7), cq = c ^ (4 * (ty & 1));
+      for (int c = 0; c < steps; ++c) {
+        float4 kk[4];
+        const int ck = c ^ (tx & 7), cq = c ^ (4 * (ty & 1));
 #pragma unroll
-      for (int j = 0; j < 4; ++j) kk[j] = kt[16 * j * QC + ck];
+        for (int j = 0; j < 4; ++j) kk[j] = kt[16 * j * QC + ck];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 qq = qt[i * QC + (cq ^ i)];
+        for (int i = 0; i < 4; ++i) {
+          const float4 qq = qt[i * QC + (cq ^ i)];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          fma2(d[i][j], make_float2(qq.x, qq.y), make_float2(kk[j].x, kk[j].y));
-          fma2(d[i][j], make_float2(qq.z, qq.w), make_float2(kk[j].z, kk[j].w));
+          for (int j = 0; j < 4; ++j) {
+            fma2(d[i][j], make_float2(qq.x, qq.y), make_float2(kk[j].x, kk[j].y));
+            fma2(d[i][j], make_float2(qq.z, qq.w), make_float2(kk[j].z, kk[j].w));
+          }
         }
       }
     }
@@ -167,40 +171,42 @@ attn_tiled_kernel(const AttnTiledParams P) {
     else cp_async_commit();
     // ---- softmax. A masked pair's probability is stored as -0.0 (a visible one is never negative)
     const bool masked = j0 + nk - 1 > min_pos || nk < kTN || P.window > 0 || P.chunk > 0;
-    float p[4][4];
+    if (live) {
+      float p[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float mx = -INFINITY;
-      bool seen[4];
+      for (int i = 0; i < 4; ++i) {
+        float mx = -INFINITY;
+        bool seen[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int off = tx + 16 * j, key = j0 + off;
-        float sc = (d[i][j].x + d[i][j].y) * P.scale;
-        if (P.softcap > 0.f) sc = P.softcap * tanhf(sc / P.softcap);
-        seen[j] = !masked || (off < nk && key <= pos[i] && (key >= lo[i] || key < P.keep_first));
-        p[i][j] = seen[j] ? sc : -INFINITY;
-        mx = fmaxf(mx, p[i][j]);
+        for (int j = 0; j < 4; ++j) {
+          const int off = tx + 16 * j, key = j0 + off;
+          float sc = (d[i][j].x + d[i][j].y) * P.scale;
+          if (P.softcap > 0.f) sc = P.softcap * tanhf(sc / P.softcap);
+          seen[j] = !masked || (off < nk && key <= pos[i] && (key >= lo[i] || key < P.keep_first));
+          p[i][j] = seen[j] ? sc : -INFINITY;
+          mx = fmaxf(mx, p[i][j]);
+        }
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float m_new = fmaxf(m[i], mx);
+        const float corr = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);   // nothing visible so far: nothing to rescale
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float e = p[i][j] == -INFINITY ? 0.f : expf(p[i][j] - m_new);
+          sum += e;
+          p[i][j] = seen[j] ? e : -0.f;
+        }
+        l[i] = l[i] * corr + sum;
+        m[i] = m_new;
+#pragma unroll
+        for (int c = 0; c < 2 * VC; ++c) acc[i][c].x *= corr, acc[i][c].y *= corr;
       }
 #pragma unroll
-      for (int o = 1; o < 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float m_new = fmaxf(m[i], mx);
-      const float corr = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);   // nothing visible so far: nothing to rescale
-      float sum = 0.f;
-#pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float e = p[i][j] == -INFINITY ? 0.f : expf(p[i][j] - m_new);
-        sum += e;
-        p[i][j] = seen[j] ? e : -0.f;
+        const int key = tx + 16 * j;
+        *reinterpret_cast<float4*>(sp_ + (key * 16 + (ty ^ (key & 7))) * 4) = make_float4(p[0][j], p[1][j], p[2][j], p[3][j]);
       }
-      l[i] = l[i] * corr + sum;
-      m[i] = m_new;
-#pragma unroll
-      for (int c = 0; c < 2 * VC; ++c) acc[i][c].x *= corr, acc[i][c].y *= corr;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int key = tx + 16 * j;
-      *reinterpret_cast<float4*>(sp_ + (key * 16 + (ty ^ (key & 7))) * 4) = make_float4(p[0][j], p[1][j], p[2][j], p[3][j]);
     }
     cp_async_wait<1>();                               // V(j) has landed (K(j + 1) may be under way)
     // a value that is not finite must not reach rows that do not see its key (0 x inf): such tiles skip masked pairs
@@ -228,11 +234,12 @@ attn_tiled_kernel(const AttnTiledParams P) {
         }
       }
     };
-    if (wild) {
+    if (!live) {
+    } else if (wild) {
       for (int key = 0; key < nk; ++key) row_key(key, true);
     } else {
 #pragma unroll 4
-      for (int key = 0; key < kTN; ++key) row_key(key, false);      // rows past nk are zero, their probabilities too
+      for (int key = 0, end = (nk + 3) & ~3; key < end; ++key) row_key(key, false);   // rows past nk are zero, their p too
     }
     __syncthreads();                                  // V(j) and P(j) are consumed
     if (j_next <= max_pos) load_v(j_next);
@@ -269,9 +276,15 @@ static size_t attn_tiled_smem(int dim, int vdim) {
 // Spans of at least 16 rows (tokens x heads per group) somewhere in the step: below that most of a 64-row tile would be
 // padding (one token of 8 heads per group: 56 of 64 rows), and the 8-row kernel spreads over more CTAs. Values up to 256
 // columns (the accumulators of a thread), rows that fit shared memory; everything else stays on the 8-row kernel.
-// 16 rows of 8 heads over 2 of 128 against 2000 keys: 810 -> 378 us; 33 tokens of 4 heads of 32: 19.8 -> 18.8 us.
-bool attn_tiled_fits(int max_q, int rep, int dim, int vdim) {
-  return (int64_t)max_q * rep >= 16 && max_q > 1 && vdim <= 256 && attn_tiled_smem(dim, vdim) <= 220 * 1024;
+// Which spans a step mixes does not count: a span's single token takes one warp of its CTA, and its keys come 64 at a time. us,
+// 8-row kernel / this one, fp32, 8 heads of 128 over 8, 2 and 1 kv heads: a portion of 256 tokens and 200 single tokens on 1000
+// keys 2414 / 872, 1038 / 304, 1109 / 177; 512 and 64 on 2000 1993 / 610, 1790 / 337, 1848 / 335; 16 spans of 16 tokens on 500
+// keys 410 / 77, 287 / 101, 287 / 101; 64 of 16 on 16 32.8 / 26.4, 29.7 / 15.2, 28.9 / 15.0; one of 33, heads of 32, 10.1 / 10.6,
+// 10.0 / 10.6, 10.9 / 10.4.
+bool attn_tiled_fits(int max_q, int rep, int G, int num_seqs, int dim, int vdim) {
+  const int64_t tiles = ((int64_t)max_q * rep + kTM - 1) / kTM;
+  return (int64_t)max_q * rep >= 16 && max_q > 1 && vdim <= 256 && attn_tiled_smem(dim, vdim) <= 220 * 1024 &&
+         tiles * G <= 0x7fffffff / num_seqs;                         // one grid dimension holds them all
 }
 
 template <typename T, int VC, bool VEC>

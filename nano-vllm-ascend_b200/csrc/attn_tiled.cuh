@@ -22,7 +22,7 @@ struct AttnTiledParams {
   int64_t gate_stride;
 };
 
-bool attn_tiled_fits(int max_q, int rep, int dim, int vdim);
+bool attn_tiled_fits(int max_q, int rep, int G, int num_seqs, int dim, int vdim);
 int attn_tiled_launch(AttnTiledParams P, int num_seqs, int max_q, int dtype, cudaStream_t stream);
 
 }  // namespace b200

@@ -733,7 +733,7 @@ extern "C" int b200_attn_generic(void* out, const void* q, int64_t q_stride, con
   B200_RETURN_IF(window < 0 || keep_first < 0 || chunk < 0 || (window > 0 && chunk > 0) || (!v && vdim > dim), B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(!block_tables && !cu_q, B200_ERR_NULL_POINTER);       // decode rows read the paged cache
   const int rep = num_heads / num_kv_heads;
-  if (cu_q && attn_tiled_fits(max_q, rep, dim, vdim)) {              // prompt portions: 64 rows share every key tile
+  if (cu_q && attn_tiled_fits(max_q, rep, num_kv_heads, num_seqs, dim, vdim)) {              // prompt portions: 64 rows share every key tile
     AttnTiledParams A;
     A.out = out, A.q = q, A.k = k, A.v = v, A.q_stride = q_stride, A.k_stride = k_stride, A.v_stride = v_stride;
     A.block_tables = block_tables, A.bt_stride = bt_stride, A.block_size = block_size, A.cu_q = cu_q, A.cu_k = cu_k;
