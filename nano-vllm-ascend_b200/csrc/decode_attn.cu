@@ -274,7 +274,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK,
               if (key < hidden_hi && key >= p.keep_first) s[n][e] = -INFINITY;
             }
         }
-        // online softmax for row g (rows 8..15 are padding)
+        // online softmax for row g
         float mx = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
@@ -289,9 +289,15 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK,
         m_run = m_new;
         if (alpha != 1.f) {
 #pragma unroll
-          for (int n = 0; n < NT; ++n) o_acc[n][0] *= alpha, o_acc[n][1] *= alpha;
+          for (int n = 0; n < NT; ++n)
+            o_acc[n][0] *= alpha, o_acc[n][1] *= alpha, o_acc[n][2] *= alpha, o_acc[n][3] *= alpha;
         }
+        // the probabilities enter the product as two 16-bit terms: their roundings in rows 0..7 of the tile, what those leave
+        // in rows 8..15, which a group of at most 8 heads does not use. Otherwise their rounding is most of the result's
+        // error, and the more so the fewer CTAs share a sequence (a CTA's largest probability is exactly 1)
         const uint32_t pa0 = pack2<T>(p00, p01), pa2 = pack2<T>(p10, p11);
+        const float2 h0 = unpack2<T>(pa0), h1 = unpack2<T>(pa2);
+        const uint32_t pa1 = pack2<T>(p00 - h0.x, p01 - h0.y), pa3 = pack2<T>(p10 - h1.x, p11 - h1.y);
 
         mbar_wait(&full_v[stage], phase);
         uint8_t* vstage = vbuf + stage * V_BYTES + v_unit;
@@ -314,8 +320,8 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK,
           uint32_t r0_, r1_, r2_, r3_;
           ldsm_x4_trans(vb + (dt >> 3) * panel_bytes + v_tok * 128 + (((dt & 7) ^ (v_tok & 7)) << 4),
                         r0_, r1_, r2_, r3_);
-          mma_16816<T>(o_acc[2 * jp], pa0, 0u, pa2, 0u, r0_, r1_);
-          mma_16816<T>(o_acc[2 * jp + 1], pa0, 0u, pa2, 0u, r2_, r3_);
+          mma_16816<T>(o_acc[2 * jp], pa0, pa1, pa2, pa3, r0_, r1_);
+          mma_16816<T>(o_acc[2 * jp + 1], pa0, pa1, pa2, pa3, r2_, r3_);
         }
         if (valid < 16) fence_proxy_async_smem();
       } else {
@@ -326,7 +332,12 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmK,
       if (++stage == kStages) stage = 0, phase ^= 1;
     }
 
-    // ---- finalise this segment
+    // ---- finalise this segment. The second term is left out where an infinite value made it 0 x inf or inf - inf
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (fabsf(o_acc[n][2 + e]) < INFINITY) o_acc[n][e] += o_acc[n][2 + e];
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
     if (UNITS > 1) {
