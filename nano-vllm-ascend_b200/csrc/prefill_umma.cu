@@ -404,14 +404,21 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const uint64_t kd0 = umma::desc_kmajor(smem_u32(sK));
     const uint64_t vd0 = umma::desc_mnmajor(smem_u32(sV), KPANEL);
     const bool leader = umma::elect_one();
+    // Descriptors are made where they are used: kept across the loop, the 4 to 12 of every operand were more than this role's
+    // registers hold (keys of 192 columns, two query tiles: 652 bytes spilled, 104 so; 16 x 1024 tokens, 16 heads over 8 of 128,
+    // 92.6 -> 83.5 us in a window of 300, 16 heads of 192 152 -> 141). Two query tiles of 64-wide keys have the room, and making
+    // them again costs 2 %.
+    constexpr bool kRemake = DK > 64 || QT == 1;
     // S[t] against K ring tile jr: the caller has waited for k_full of stage jr % kUStages
     auto issue_s = [&](int t, int jr) {
       if (leader) {
+        uint64_t qd = qd0;
+        if (kRemake) asm volatile("" : "+l"(qd));   // see kRemake
         const uint64_t kd = umma::desc_advance(kd0, (jr % kUStages) * KTILE);
         const uint32_t d = tb + kSBase + t * 128;
 #pragma unroll
         for (int ks = 0; ks < DK / 16; ++ks) {
-          const uint64_t ad = umma::desc_advance(qd0, t * QTILE + (ks >> 2) * QPANEL + (ks & 3) * 32);
+          const uint64_t ad = umma::desc_advance(qd, t * QTILE + (ks >> 2) * QPANEL + (ks & 3) * 32);
           const uint64_t bd = umma::desc_advance(kd, (ks >> 2) * KPANEL + (ks & 3) * 32);
           umma::mma_ss(d, ad, bd, idesc_s, ks > 0);
         }
@@ -457,9 +464,11 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               mbar_wait(&p_full[2 * t + h], (done[t] + j) & 1);
               umma::fence_after_sync();
               if (leader) {
+                uint64_t vdh = vd;
+                if (kRemake) asm volatile("" : "+l"(vdh));
 #pragma unroll
                 for (int kk = h * 4; kk < h * 4 + 4; ++kk)
-                  umma::mma_ts(tb + t * 128, pa + kk * 8, umma::desc_advance(vd, kk * 16 * 128), idesc_o,
+                  umma::mma_ts(tb + t * 128, pa + kk * 8, umma::desc_advance(vdh, kk * 16 * 128), idesc_o,
                                (j > 0 || kk > 0) ? 1u : 0u);
               }
             }
