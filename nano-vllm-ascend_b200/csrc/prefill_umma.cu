@@ -64,6 +64,7 @@ struct PrefillUmmaParams {
   int k_split, v_split;   // 1: each TMA op carries a single 64-wide chunk (paged, rows_box < 128)
   int pair;          // QT = 2: the two query tiles are 128 rows of two heads that share K and V, not 256 rows of one head
   int m_tiles, num_seqs;   // row tiles of the longest sequence, sequences: the items are m_tiles x kv_splits x H x num_seqs
+  int ordered;       // the sequences are listed by length (several items per CTA), not in their own order
   int kv_splits;     // CTAs sharing one (sequence, head, 256 rows) along the keys; 1 = no split
   float* part_o;     // kv_splits > 1: [total_q][H][kv_splits][D] un-normalised O
   float* part_ml;    // kv_splits > 1: [total_q][H][kv_splits][2]  (row max in the exp2 domain, row sum)
@@ -230,8 +231,10 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // CTA's items have about the same number of key tiles as any other's; inside a row tile key
   // splits are neighbours, then the heads of a sequence (which share K and V in L2). The sequences that have a given row tile
   // are the first ones of the list sorted by length. Steps of more sequences than the list holds keep the sequences' own
-  // order and pass over the row tiles that a sequence does not have.
-  const bool sorted = p.num_seqs <= kOrderSeqs;
+  // order and pass over the row tiles that a sequence does not have; so do launches with a CTA for every item and those
+  // whose sequences are all one row tile, where the order is nothing and the list a round trip to L2, three barriers and a
+  // scan before the first load.
+  const bool sorted = p.ordered;
   const bool pair = QT == 2 && p.pair;
   const int item_rows = pair ? kUBM : QT * kUBM, row_step = pair ? 0 : kUBM, head_step = pair ? 1 : 0;   // of query tile t
   const int per_seq = p.kv_splits * (pair ? p.H / 2 : p.H);
@@ -243,13 +246,19 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const int s = threadIdx.x + u * blockDim.x;
       mine[u] = s < p.num_seqs ? min((p.cu_q[s + 1] - p.cu_q[s] + item_rows - 1) / item_rows, 65535) : 0;
       at[u] = 0;
-      if (s < p.num_seqs) s_tiles[s] = (uint16_t)mine[u];
+      if (s < kOrderSeqs) s_tiles[s] = (uint16_t)mine[u];             // 0 past the sequences: before nobody
     }
     __syncthreads();
-    for (int o = 0; o < p.num_seqs; ++o) {
-      const int other = s_tiles[o];
+    for (int o = 0; o < p.num_seqs; o += 8) {                         // 8 at a time: one by one it took 8 us of 256 sequences
+      const uint4 eight = *reinterpret_cast<const uint4*>(s_tiles + o);
+      const uint32_t w[4] = {eight.x, eight.y, eight.z, eight.w};
 #pragma unroll
-      for (int u = 0; u < kPer; ++u) at[u] += other > mine[u] || (other == mine[u] && o < (int)(threadIdx.x + u * blockDim.x));
+      for (int i = 0; i < 8; ++i) {
+        const int other = (int)((w[i >> 1] >> (16 * (i & 1))) & 0xffffu);
+#pragma unroll
+        for (int u = 0; u < kPer; ++u)
+          at[u] += other > mine[u] || (other == mine[u] && o + i < (int)(threadIdx.x + u * blockDim.x));
+      }
     }
     __syncthreads();
 #pragma unroll
@@ -773,6 +782,7 @@ static int prefill_umma_launch_c(const CUtensorMap& mq, const CUtensorMap& mk, c
   const int64_t items = (int64_t)p.m_tiles * p.kv_splits * (QT == 2 && p.pair ? p.H / 2 : p.H) * num_seqs;
   if (items > 0x7fffffff) return B200_ERR_UNSUPPORTED;
   const int slots = 148 * (DK > 128 ? 1 : 3 - QT);
+  p.ordered = num_seqs <= kOrderSeqs && p.m_tiles > 1 && items > slots;
   launch_pdl(kern, dim3((unsigned)(items < slots ? items : slots)), dim3(prefill_threads(QT)), smem, stream, mq, mk, mv, p);
   if (p.kv_splits > 1) {
     const int64_t rows = (int64_t)total_q * p.H;
