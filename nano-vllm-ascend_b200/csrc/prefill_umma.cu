@@ -827,11 +827,18 @@ int prefill_kv_splits(int num_seqs, int H, int max_seqlen_q, int max_seqlen_k, i
 // K and V wherever heads come in pairs; otherwise 256 rows of one head from 512 rows on (D 128) or 2048 (D 64, whose
 // tiles are cheaper), and where the grid is so small that keys are split across CTAs anyway.
 // b200_prefill_set_query_tiles(1|2) forces one layout (A/B runs, parity tests of both instantiations).
+// Launches whose 128-row tiles of one head find a CTA slot each (`slots`), with at most four key tiles, take QT = 1 in any
+// case: nothing is read often enough for sharing to count, and a CTA's start, two chains and end are shorter than those of a
+// pair (us, QT = 1 / pair, 16 heads over 8: D 128, 1 x 17 6.5 / 6.9, 1 x 300 10.0 / 11.3, 2 x 129 8.2 / 9.2; keys of 192, 1 x 300 9.1 / 11.1).
+static bool prefill_small(int num_seqs, int H, int max_seqlen_q, int max_seqlen_k, int slots) {
+  return (int64_t)((max_seqlen_q + kUBM - 1) / kUBM) * H * num_seqs <= slots && max_seqlen_k <= 4 * kUBN;
+}
 static int g_forced_query_tiles = 0;
 void prefill_force_query_tiles(int qt) { g_forced_query_tiles = qt; }
 
-int prefill_query_tiles(int num_seqs, int H, int rep, int max_seqlen_q, int D, int span) {
+int prefill_query_tiles(int num_seqs, int H, int rep, int max_seqlen_q, int max_seqlen_k, int D, int span) {
   if (g_forced_query_tiles) return g_forced_query_tiles;
+  if (prefill_small(num_seqs, H, max_seqlen_q, max_seqlen_k, 2 * 148)) return 1;
   if (rep % 2 == 0) return 2;
   const int64_t ctas2 = (int64_t)((max_seqlen_q + 2 * kUBM - 1) / (2 * kUBM)) * H * num_seqs;
   if (ctas2 * 2 <= 148) return 2;                 // key-split territory (prefill_kv_splits)
@@ -866,8 +873,9 @@ int prefill_umma_launch(void* out, const void* q, const void* k, const void* v,
   // keys that a 128-row query tile can see at most: what the choice of layout and of key splits is made on
   if (span > 0 && max_seqlen_k > span + p.keep_first + 3 * kUBM) max_seqlen_k = span + p.keep_first + 3 * kUBM;
   // one CTA per SM either way with keys of 192 columns: two ping-pong tiles wherever a sequence has them
-  const int qt = DK > 128 ? (max_seqlen_q > kUBM ? 2 : 1)
-                          : prefill_query_tiles(num_seqs, H, p.G, max_seqlen_q, DV, span > 0 ? max_seqlen_k : max_seqlen_q);
+  const int qt = DK > 128 ? (max_seqlen_q > kUBM && !prefill_small(num_seqs, H, max_seqlen_q, max_seqlen_k, 148) ? 2 : 1)
+                          : prefill_query_tiles(num_seqs, H, p.G, max_seqlen_q, max_seqlen_k, DV,
+                                                span > 0 ? max_seqlen_k : max_seqlen_q);
   p.pair = qt == 2 && p.G % 2 == 0;
   p.kv_splits = (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0)
                     ? prefill_kv_splits(num_seqs, H, max_seqlen_q, max_seqlen_k, total_q, DV, workspace_bytes, qt, p.pair)
