@@ -346,7 +346,8 @@ static void recurrence_launch_as(const RecParams& P, int num_seqs, cudaStream_t 
 // keeps rows 16w .. 16w+15 of S^T [vdim x kdim] as accumulator fragments, which are at the same time the A
 // fragments of S^T q (the layout identity that flash attention uses for P V). Sizes are zero-padded to
 // kdim <= D (template, 32 / 64 / 128) and vdim <= 128 in shared memory.
-// Bound: latency and issue of a warp's chain per chunk (2 CTAs of 4 to 8 warps per SM by their 255 registers), so what
+// Bound: latency and issue of a warp's chain per chunk (by their 255 registers an SM holds two CTAs of up to 4 warps for
+// vdim <= 64, one of up to 8 warps above), so what
 // counts is instructions: fragments come by ldmatrix (the A fragment of Q is also the B fragment of Q^T), the splits
 // by packed conversions, every warp keeps the decays in its lanes (one CTA barrier per chunk) and stores its outputs
 // straight from the accumulators; and the split and the scaling of the state are paid once per 32 tokens, not per 16.
@@ -371,13 +372,14 @@ constexpr int kChunk = 32;             // two 16-token blocks
 
 // VEC: q, k, v rows start on 16-byte boundaries (strides, sizes and slice offsets % 8 == 0): the tiles of the next
 // chunk are copied global -> shared with cp.async while the current chunk is computed (two sets of tiles).
-// NW: warps that the shared-memory rows of V are sized for (vdim <= 16 NW); MODE, SILU: P.mode, P.act_silu.
+// NW: warps that the shared-memory rows of V are sized for (vdim <= 16 NW); MODE, SILU: P.mode, P.act_silu; CTAS: how many of
+// 4 warps an SM is to hold (chunk_recurrence_launch).
 template <int D, int NW>
 constexpr int chunk_recurrence_smem(bool vec) {
   return (vec ? 2 : 1) * kChunk * (2 * (D + 8) + 16 * NW + 8) * 2;
 }
-template <int D, int NW, bool VEC, int MODE, bool SILU>
-__global__ void __launch_bounds__(32 * NW, 8 / NW)
+template <int D, int NW, bool VEC, int MODE, bool SILU, int CTAS>
+__global__ void __launch_bounds__(32 * NW, CTAS * 4 / NW)
 chunk_recurrence_kernel(const RecParams P) {
   using T = __nv_bfloat16;
   constexpr int QS = D + 8;                           // row stride (elements) of the q / k tiles: conflict-free
@@ -405,12 +407,58 @@ chunk_recurrence_kernel(const RecParams P) {
   const float dt_b = MODE == 1 ? P.dt_bias[h] : 0.f;
   const float d_skip = MODE == 1 ? P.d_skip[h] : 0.f;
 
-  // S^T slab: n-tile n = key columns 8n .. 8n+7; [0],[1]: row r0+g, cols 8n+2t, +1; [2],[3]: row r0+g+8
-  float S[D / 8][4];
   float* slot = P.state != nullptr
                     ? P.state + (((int64_t)P.state_slots[s] * P.H + h) * kdim) * (int64_t)vdim
                     : nullptr;
   const bool carried = slot != nullptr && sp.first_pos() > 0;
+  if (D <= 64 && sp.q_len == 1) {
+    // A single token (a decode row of a mixed step) of a small state is a rank-1 update: one pass over the state, in the order
+    // it lies in memory, and no fragments. Thread = value channel x half of the key rows; the block has at least 2 vdim threads.
+    // 200 of them beside a prompt of 256, 32 heads of 64 x 64: 134 us as chunks of 32, 98 as chunks of 16, 59 so; 16 heads of 64 x
+    // 128 138 / 96 / 61. States of 128 key channels are no slower as chunks (181 / 184), and their registers are all taken.
+    float* sq = reinterpret_cast<float*>(s_tiles);    // [D] q, [D] k, [vdim] partial outputs
+    float *sk = sq + D, *so = sk + D;
+    const int64_t tok = sp.q_start;
+    for (int i = threadIdx.x; i < kdim; i += nthreads) {
+      float qv = __bfloat162float(q[tok * P.q_stride + i]), kv = __bfloat162float(k[tok * P.k_stride + i]);
+      if (SILU) qv = bits_f32(bf16_bits(silu_fast(qv))), kv = bits_f32(bf16_bits(silu_fast(kv)));
+      sq[i] = qv, sk[i] = kv;
+    }
+    const int col = threadIdx.x % vdim, half = threadIdx.x / vdim;
+    float x = __bfloat162float(v[tok * P.v_stride + col]), a = MODE == 0 ? P.decay[h] : 0.f, step = 1.f;
+    if (SILU) x = bits_f32(bf16_bits(silu_fast(x)));
+    if (MODE == 1) {
+      step = softplus_f(__bfloat162float(dt[tok * P.dt_stride + h]) + dt_b);
+      a = expf(-rate * step);
+    }
+    __syncthreads();
+    const float bx = step * x;
+    const int k_lo = half == 0 ? 0 : (kdim + 1) / 2, k_hi = half == 0 ? (kdim + 1) / 2 : half == 1 ? kdim : 0;
+    float sum = 0.f;
+    for (int i0 = k_lo; i0 < k_hi; i0 += 16) {        // 16 rows on their way at a time
+      float row[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) row[i] = carried && i0 + i < k_hi ? slot[(int64_t)(i0 + i) * vdim + col] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (i0 + i >= k_hi) break;
+        row[i] = fmaf(sk[i0 + i], bx, a * row[i]);
+        if (slot != nullptr) slot[(int64_t)(i0 + i) * vdim + col] = row[i];
+        sum = fmaf(sq[i0 + i], row[i], sum);
+      }
+    }
+    if (half == 1) so[col] = sum;
+    __syncthreads();
+    if (half == 0) {
+      sum += so[col];
+      if (MODE == 1) sum = fmaf(d_skip, x, sum);
+      P.out[tok * ((int64_t)P.H * vdim) + (int64_t)h * vdim + col] = sum;
+    }
+    return;
+  }
+
+  // S^T slab: n-tile n = key columns 8n .. 8n+7; [0],[1]: row r0+g, cols 8n+2t, +1; [2],[3]: row r0+g+8
+  float S[D / 8][4];
 #pragma unroll
   for (int n = 0; n < D / 8; ++n)
 #pragma unroll
@@ -669,15 +717,24 @@ static int chunk_recurrence_launch(const RecParams& P, int num_seqs, cudaStream_
   const dim3 block(32 * ((P.vdim + 15) / 16));
   const bool vec = P.kdim % 8 == 0 && P.vdim % 8 == 0 && P.q_stride % 8 == 0 && P.k_stride % 8 == 0 &&
                    P.v_stride % 8 == 0 && aligned16(P.q) && aligned16(P.k) && aligned16(P.v);
-  // rows of V for 4 warps where the value size allows: less shared memory, and a register budget for two CTAs per SM
-#define B200_CHUNK_REC_AS(DV, NW, VEC, M, SILU)                                                                     \
+  // rows of V for 4 warps where the value size allows: less shared memory, and a register budget for two CTAs per SM (of 8
+  // warps: one). Twice as many (at 128 registers, with some spilled) where there are that many and the state is small: what
+  // counts then is how many states are on their way. 32 heads of 64 x 64, two / four: 256 prompts of 16 tokens 168 / 125 us, 16 of
+  // 1024 260 / 239, 64 of 40 73.6 / 59.9; 4 of 100 14.7 / 17.5, 1 of 700 69 / 84.
+  const bool many = (int64_t)P.H * num_seqs > (P.vdim <= 64 ? 2 : 1) * 148;
+#define B200_CHUNK_REC_AT(DV, NW, VEC, M, SILU, CTAS)                                                               \
   do {                                                                                                              \
-    auto kern = chunk_recurrence_kernel<DV, NW, VEC, M, SILU>;                                                      \
+    auto kern = chunk_recurrence_kernel<DV, NW, VEC, M, SILU, CTAS>;                                                \
     constexpr int smem = chunk_recurrence_smem<DV, NW>(VEC);                                                        \
     static std::atomic<uint64_t> devices{0};                                                                        \
     const cudaError_t allowed = allow_smem(kern, smem, devices);                                                    \
     if (allowed != cudaSuccess) return (int)allowed;                                                                \
     launch_pdl(kern, grid, block, (size_t)smem, stream, P);                                                         \
+  } while (0)
+#define B200_CHUNK_REC_AS(DV, NW, VEC, M, SILU)                                            \
+  do {                                                                                     \
+    if (DV <= 64 && many) B200_CHUNK_REC_AT(DV, NW, VEC, M, SILU, (DV <= 64 ? 4 : 2));     \
+    else B200_CHUNK_REC_AT(DV, NW, VEC, M, SILU, 2);                                       \
   } while (0)
 #define B200_CHUNK_REC_V(DV, M, SILU)                                           \
   do {                                                                          \
@@ -699,6 +756,7 @@ static int chunk_recurrence_launch(const RecParams& P, int num_seqs, cudaStream_
 #undef B200_CHUNK_REC
 #undef B200_CHUNK_REC_V
 #undef B200_CHUNK_REC_AS
+#undef B200_CHUNK_REC_AT
   return finish_launch();
 }
 
