@@ -18,7 +18,7 @@
 //    time, one lane each), warps 0-7 are consumers; a 3-stage mbarrier ring, separate
 //    K-full / V-full barriers so QK^T starts as soon as K lands.
 //  * Per consumer warp: one kv head x one 16-token unit per tile. The GQA group (<= 8 query
-//    heads) is the M dimension of mma.sync m16n8k16 (rows 8-15 are structurally zero), i.e.
+//    heads) is the M dimension of mma.sync m16n8k16 (in Q K rows 8-15 are zero), i.e.
 //    the whole group shares a single read of the KV bytes. fp32 online softmax in the exp2
 //    domain; running max/sum per thread, reduced with warp shuffles.
 //  * Optional sliding window with kept first tokens, or chunks (a row sees its own chunk, a window of its own length): the

@@ -1,9 +1,12 @@
-// moe_umma.cu -- grouped expert GEMMs for PREFILL-sized MoE batches on tcgen05 / TMEM (staged).
+// moe_umma.cu -- grouped expert GEMMs for PREFILL-sized MoE batches on tcgen05 / TMEM: moe_umma_gemm_kernel (128-column
+// tiles, one per CTA; described here) for launches that do not fill the chip, fp32 outputs and widths that 256 does not
+// divide, moe_umma_wide_kernel (persistent, 256-column tiles; described at the kernel) for the others. moe_umma_wide() has
+// the rule.
 //
 // moe.cu's expert GEMMs are weight-streaming kernels for decode (tens of rows per expert). A prefill
 // step routes ~1000 rows to every expert (16384 tokens x top-8 / 128 experts): 1.2 TFLOP per layer,
 // tensor-bound. Same contract as moe_gemm_kernel<gate_up/down> -- same plan (offsets/sorted_pair),
-// same rounding points, same outputs -- but:
+// same rounding points, same outputs -- but (moe_umma_gemm_kernel):
 //   * tiles are 128 rows of ONE expert x 128 weight rows, accumulated in TMEM (128 fp32 columns)
 //     by tcgen05.mma M128 N128 K16, both operands K-major SW128 panels (the QK^T configuration of
 //     prefill_umma.cu, descriptors and instruction forms identical);

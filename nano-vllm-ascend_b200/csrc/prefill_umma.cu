@@ -30,9 +30,10 @@
 //   TMEM columns (O at 0, S at 128), 105 KiB of shared memory -> two CTAs per SM.
 // A CTA walks several work items (Q of the next one is loaded, and its first S computed, under the epilogue of the one
 // before); a row's sizes live in shared memory, since 128 scores leave no registers for them. Sums and products of scores are
-// packed fp32 pairs, row maxima four chains. What bounds it (16 x 1024 tokens, D 128: 103 us = 670 TFLOP/s; 118-122 us with one
-// item per CTA and one head): the chain S -> softmax -> P V -> S of a tile, about 3300 cycles of which the tensor pipe works
-// 1448 for each of two tiles, plus the epilogue.
+// packed fp32 pairs, row maxima four chains. What bounds it (16 x 1024 tokens, 16 heads over 8 of 128, inputs that rotate: 107 us =
+// 643 TFLOP/s; 129 us with one item per CTA and one head): the chain S -> softmax -> P V -> S of a tile, 3300 to 3700 cycles of which
+// the tensor pipe works 1448 for each of two tiles, and what goes with an item -- first loads, drain, epilogue -- at about 7 us
+// (1024 items of 31 pair tiles per CTA against as many of 114).
 // Hazards: S[t](j+1) overwrites the columns PV[t](j) reads P from -- both are tcgen05.mma of the same
 // issuing thread and execute in issue order; softmax(j+1) of tile t starts only after S[t](j+1) has
 // completed, hence after PV[t](j) has.
@@ -817,19 +818,22 @@ int prefill_kv_splits(int num_seqs, int H, int max_seqlen_q, int max_seqlen_k, i
   return splits < 1 ? 1 : splits;
 }
 
-// Query tiles per CTA for a launch. Measured, us, QT = 1 / QT = 2 as 256 rows of a head / QT = 2 as 128 rows of two heads:
-//   D 128, 16 heads over 8:  16 x 1024  122 / 110 / 103;  32 x 512  88 / 83 / 78;  64 x 256  71 / 72 / 69;  64 x 128  35 / 39 / 35;
-//                            12 x 37-1483  78 / 80 / 70;  8 x 2048  178 / 159 / 153;  4 x 4096  306 / 269 / 270;
-//                            16 x 1024 in a window of 512  119 / 113 / 102
-//   D 64, 32 heads over 8:   16 x 1024  170 / 164 / 151;  1 x 8192  481 / 423 / 436;  12 x 37-1483 capped  175 / 192 / 162;  8 x 300  24 / 29.5 / 24
-// What decides is how often K and V cross from L2 (QT = 1 reads every tile for 128 rows of one head: 5.7 TB/s at 16 x 1024,
+// Query tiles per CTA for a launch. Measured, us, QT = 1 / QT = 2 as 128 rows of two heads:
+//   D 128, 16 heads over 8:  4 x 2000  83.5 / 75.5;  1 x 8192  256 / 233;  12 x 37-1483  68 / 65;  512 x 20  148 / 138;  256 x 16  77 / 72;
+//                            64 x 128  28.4 / 29.7;  16 x 1024 in a window of 300  96 / 84, in chunks of 200  87 / 77
+//   D 64, 32 heads over 8:   4 x 2000  129 / 121;  1 x 8192  419 / 389;  12 x 37-1483  102 / 97;  256 x 16  112 / 121;  64 x 128  34 / 36
+// and QT = 1 / QT = 2 as 256 rows of a head, where heads come alone:
+//   D 128, 8 heads over 8:   2 x 4096  77 / 67;  16 x 1024  60 / 58;  12 x 37-1483  45 / 46;  32 x 300  33 / 37;  64 x 100  17 / 21
+//          24 heads over 8:  2 x 4096  203 / 183;  16 x 1024  152 / 141;  12 x 37-1483  96 / 97;  32 x 300  72 / 82;  64 x 100  38 / 49
+//   D 64, 16 heads over 16:  2 x 4096  118 / 112;  16 x 1024  85 / 87;  12 x 37-1483  55 / 64;  32 x 300  44 / 49;  64 x 100  20 / 29
+// What decides is how often K and V cross from L2 (QT = 1 reads every tile for 128 rows of one head,
 // and its one-stage rings wait for them), then the rows that a 256-row tile computes for nothing. So: two heads that share
 // K and V wherever heads come in pairs; otherwise 256 rows of one head from 512 rows on (D 128) or 2048 (D 64, whose
 // tiles are cheaper), and where the grid is so small that keys are split across CTAs anyway.
 // b200_prefill_set_query_tiles(1|2) forces one layout (A/B runs, parity tests of both instantiations).
 // Launches whose 128-row tiles of one head find a CTA slot each (`slots`), with at most four key tiles, take QT = 1 in any
 // case: nothing is read often enough for sharing to count, and a CTA's start, two chains and end are shorter than those of a
-// pair (us, QT = 1 / pair, 16 heads over 8: D 128, 1 x 17 6.5 / 6.9, 1 x 300 10.0 / 11.3, 2 x 129 8.2 / 9.2; keys of 192, 1 x 300 9.1 / 11.1).
+// pair (us, QT = 1 / pair, 16 heads over 8: D 128, 1 x 17 6.6 / 7.1, 1 x 300 10.2 / 11.2, 2 x 129 8.2 / 9.2; keys of 192, 1 x 300 9.1 / 11.1).
 static bool prefill_small(int num_seqs, int H, int max_seqlen_q, int max_seqlen_k, int slots) {
   return (int64_t)((max_seqlen_q + kUBM - 1) / kUBM) * H * num_seqs <= slots && max_seqlen_k <= 4 * kUBN;
 }

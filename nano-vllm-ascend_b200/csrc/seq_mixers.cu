@@ -357,7 +357,7 @@ static void recurrence_launch_as(const RecParams& P, int num_seqs, cudaStream_t 
 // prefix sum over 32 loses a bit (error of the outputs against 64 bits 4.2e-7 with it, 2.5e-7 so).
 // two fp32 -> three packed bf16 pairs hi, mid, lo (first value in the low half), each term the rounding of what the ones
 // before it leave. The packed conversion runs at half of the fp32 rate, the scalar one on the special-function unit at
-// an eighth (it was 41 % busy with the splits).
+// an eighth (which is 3 % busy now).
 __device__ __forceinline__ void split3x2(float x, float y, uint32_t (&w)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {

@@ -560,9 +560,11 @@ def moe_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_ids: 
 
 
 # Prefill-sized batches (hundreds of rows per expert) are tensor-bound, not weight-streaming: from
-# _MOE_BIG_GEMM_ROWS average rows per local expert on they go through the tcgen05 grouped GEMM of
-# csrc/moe_umma.cu (measured on Qwen3-30B-A3B, 4096-token prefill layer: 721 us vs 1224 us for the
-# weight-streaming kernel; whole-model prefill 99.9 k vs 51.8 k tok/s). Module attributes, not
+# _MOE_BIG_GEMM_ROWS average rows per local expert on they go through the tcgen05 grouped GEMMs of
+# csrc/moe_umma.cu. The line dates from the 128-column kernel alone and is a safe one: with the kernels as they are,
+# a layer takes (us, weight-streaming / tcgen05, by rows per expert; hidden 2048, inter 768, 128 experts) 16: 213 / 359,
+# 32: 241 / 221, 48: 324 / 227, 64: 386 / 235, 96: 518 / 248, 192: 951 / 386; (hidden 1024, inter 512, 16 experts) 16: 23 / 25,
+# 32: 27 / 25, 64: 50 / 25, 96: 60 / 27; (2048, 1024, 16) 16: 46 / 56, 32: 60 / 57, 64: 90 / 60, 96: 110 / 61. Module attributes, not
 # environment switches: "stream" forces the weight-streaming kernel for every size, "library" routes
 # through torch._grouped_mm (comparator for tools/moe_diag.py and the tests).
 _MOE_BIG_GEMM = "umma"
