@@ -312,3 +312,17 @@ def test_a_wait_that_runs_out_is_reported():
     _close(ops.linear_umma(x, w), want, "after it")
     torch.cuda.synchronize()
     ops.check_waits()
+
+
+@pytest.mark.parametrize("dtype,M,K,inter", [(torch.bfloat16, 19000, 64, 128), (torch.float16, 9600, 320, 256), (torch.bfloat16, 18945, 256, 256)])
+def test_persistent_tiles_against_plain_products(dtype, M, K, inter):
+    """The persistent 256-column kernel as dense layers (one group; full row tiles give every SM one) against fp32 products:
+    one K block and more, M at and off a multiple of 128."""
+    from nanovllm import ops
+    g = torch.Generator().manual_seed(M)
+    x = torch.randn(M, K, generator=g).to(dtype).cuda()
+    w = (K ** -0.5 * torch.randn(2 * inter, K, generator=g)).to(dtype).cuda()
+    product = (x.float() @ w.float().T).to(dtype)
+    _close(ops.linear_umma(x, w), product, ("linear", M, K, inter))
+    gate, up = product.float().split(inter, 1)
+    _close(ops.gate_up_silu_umma(x, w), (torch.nn.functional.silu(gate).to(dtype).float() * up).to(dtype), ("gate_up", M, K, inter))
