@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Contract benchmark: decode tokens/s (+ p50 TTFT) of the paged-KV attention path.
 
-Workload (BASELINE.json configs[1]): Qwen3-0.6B (random-init, bf16), 256 sequences x 1024-token
+Workload: Qwen3-0.6B (random-init, bf16), 256 sequences x 1024-token
 prompts, kvcache_block_size 16, CUDA-graph decode, one engine per GPU.  A "step" is one decode
 step of the whole batch (one pass of the hot path: 28 x [K8 epilogue, paged decode attention,
 fused norms/activation] + cuBLAS GEMMs + sampling).
@@ -17,7 +17,7 @@ fused norms/activation] + cuBLAS GEMMs + sampling).
              attention) on the host cores, bounded sample of the same decode step
 
 N > 1 (torchrun): independent data-parallel replicas, no data-path collective ("weak" scaling) --
-the headline line -- plus a `tp` object: Qwen3-32B (BASELINE configs[3]) decode at the same batch /
+the headline line -- plus a `tp` object: Qwen3-32B decode at the same batch /
 context tensor-parallel over all N GPUs (fused NVLink all-reduce + residual add + RMSNorm), with
 the all-reduce form and its latency, and the same workload at TP=1 (rank 0) for the speed-up.
 `--tp` instead makes the tensor-parallel engine the whole line ("strong" scaling).
@@ -103,7 +103,7 @@ def parse_args():
     ap.add_argument("--block-size", type=int, default=16)
     ap.add_argument("--tp", action="store_true", help="tensor-parallel over --gpus instead of replicas")
     ap.add_argument("--tp-model", default="qwen3-32b",
-                    help="model of the `tp` object a multi-GPU replica run adds (BASELINE configs[3])")
+                    help="model of the `tp` object a multi-GPU replica run adds")
     ap.add_argument("--no-tp-block", action="store_true", help="multi-GPU replica run without the `tp` object")
     ap.add_argument("--tp-timeout", type=float, default=420.0, help="seconds before the `tp` object is abandoned")
     ap.add_argument("--no-cpu-baseline", action="store_true")
@@ -146,7 +146,7 @@ def tensor_peak():
 
 def prefill_roofline():
     """The tensor-bound kernel of the path (prefill_umma_kernel) timed alone with CUDA events on the
-    shapes BASELINE names: configs[1]'s prefill batch (16 x 1024 tokens, Qwen3-0.6B heads) and configs[2]
+    shapes of the serving workload's prefill batch (16 x 1024 tokens, Qwen3-0.6B heads) and of a long prompt
     (Llama-3.2-1B, 8192-token prompt: whole, and the prefix-cache-hit form -- 256 new tokens against
     7936 cached ones read through block tables). Flops = 4 * H * D * sum over rows of visible keys
     (causal); inputs rotate over copies totalling > L2."""
@@ -390,7 +390,7 @@ class Group:
 
 
 def decode_workload(llm, group, B, ctx, K, W, prompt_seed, rank):
-    """The workload of BASELINE configs[1] on one engine: submit B prompts of `ctx` tokens at t = 0,
+    """The serving workload on one engine: submit B prompts of `ctx` tokens at t = 0,
     prefill (TTFT), W warm-up decode steps, K decode steps through LLM.step() (e2e: pinned H2D of the
     step metadata + D2H of the sampled ids inside the timed region), then K replays of the captured
     step with its inputs resident (device). Times are CUDA events, max over the group's ranks."""
@@ -593,9 +593,9 @@ def tp_engine_measure(args, rank, world, K, W, peak, peak_src, kw):
 
 
 def tp_block(args, rank, world, K, W, peak, peak_src):
-    """BASELINE configs[3]: Qwen3-32B decode, batch 256, ctx 1024, tensor-parallel over ALL `world`
+    """Qwen3-32B decode, batch 256, ctx 1024, tensor-parallel over ALL `world`
     GPUs of this run, next to the same workload at TP=1 (rank 0 alone, the other ranks wait), so the
-    driver's scaling record carries the north_star's "TP=8 >= 6x TP=1" figure."""
+    line carries the "TP=8 >= 6x TP=1" figure."""
     import torch.distributed as dist
     from nanovllm import LLM
     B, ctx = args.batch, args.ctx
@@ -1646,7 +1646,7 @@ def main():
             line["prefill_roofline"] = {"error": f"{type(e).__name__}: {e}"[:300]}
     if world > 1 and not args.tp and not args.no_tp_block:
         # the replicas above say nothing about the collective design: the same run also measures the
-        # tensor-parallel path (BASELINE configs[3]) over all `world` GPUs, with its TP=1 comparison
+        # tensor-parallel path over all `world` GPUs, with its TP=1 comparison
         def bail():                       # a hung collective must not cost the replica line
             line["tp"] = {"error": f"tensor-parallel block did not finish within {args.tp_timeout} s"}
             if rank == 0:

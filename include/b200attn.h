@@ -2,7 +2,7 @@
  * b200attn.h -- C ABI of libb200attn.so: the paged-KV decode/attention hot path
  * of nano-vllm (reference: linzm1007/nano-vllm-ascend) as hand-written sm_100a CUDA.
  *
- * Boundary contract (SURVEY.md section 8b):
+ * Boundary contract:
  *   - plain C, raw device pointers + sizes, no torch types;
  *   - the caller owns every buffer (q/k/v, paged caches, tables, outputs, workspaces);
  *   - every entry point only ENQUEUES work on `stream` (a cudaStream_t): no allocation,
@@ -149,7 +149,7 @@ int b200_paged_decode_attn_windowed(void* out, const void* q, const void* k_cach
 
 
 /* ---------------------------------------------------------------------------------
- * K1/K2 + K6 over an FP8 (e4m3) KV cache -- SURVEY.md 8f row f3. An EXTENSION of the path: the
+ * K1/K2 + K6 over an FP8 (e4m3) KV cache. An EXTENSION of the path: the
  * reference keeps its caches in the model dtype (engine/model_runner.py:218-229); nothing in it is
  * replaced by these two entry points, they halve the bytes K6 streams.
  * Cache element = e4m3(x * (1/scale)), round-to-nearest-even, saturating at +-448; k_scale and
@@ -293,7 +293,7 @@ int b200_add_rmsnorm(void* x, void* residual, const void* weight, float eps, int
 int b200_silu_and_mul(void* out, const void* x, int32_t rows, int32_t inter, int32_t dtype,
                       b200_stream_t stream);
 
-/* f2 (SURVEY 8f "next"): greedy/temperature sampling tail without the fp32 logits
+/* Greedy/temperature sampling tail without the fp32 logits
  * round trip. Replaces layers/sampler.py:9-17 for the greedy parity path (argmax) and
  * for temperature sampling via the Gumbel-max trick with a counter-based RNG.
  * logits: [rows, vocab] in dtype (16-bit or fp32; row stride logits_stride elements);
@@ -320,7 +320,7 @@ int b200_sample_shard(int64_t* out_keys, const void* logits, const float* temper
                       uint64_t step, const int64_t* step_offset, int32_t dtype, b200_stream_t stream);
 
 /* ---------------------------------------------------------------------------------
- * MoE (SURVEY 8 f4)  sparse mixture-of-experts MLP: routing, dispatch plan, expert GEMMs, combine.
+ * MoE  sparse mixture-of-experts MLP: routing, dispatch plan, expert GEMMs, combine.
  * Replaces: Qwen3MoeSparseMoeBlock.forward                            models/qwen3_moe.py:146-186
  *           (softmax/top-k :150-158, per-expert gather + Qwen3MoeMLP :95-122 + index_add_ :160-186).
  * Expert parallelism: the caller owns experts [expert_begin, expert_begin + num_local) whole and

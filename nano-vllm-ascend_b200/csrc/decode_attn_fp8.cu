@@ -1,6 +1,6 @@
 // decode_attn_fp8.cu -- K6 over an FP8 (e4m3) paged KV cache, and the K1/K2 scatter that fills it.
 //
-// SURVEY.md section 8 row f3 ("FP8 KV-cache variant of K1/K6"): an extension of the path, not
+// An FP8 KV-cache variant of K1/K6: an extension of the path, not
 // something the reference has -- its caches are always the model dtype (engine/model_runner.py:
 // 218-229). Semantics: cache element = e4m3(x / scale) (round to nearest even, saturating at
 // +-448), one fp32 scale per tensor for K and one for V; attention runs over the de-quantised

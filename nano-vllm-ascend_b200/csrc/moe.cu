@@ -1,4 +1,4 @@
-// moe.cu -- sparse mixture-of-experts MLP (SURVEY 8 f4): routing, dispatch plan, expert GEMMs, combine.
+// moe.cu -- sparse mixture-of-experts MLP: routing, dispatch plan, expert GEMMs, combine.
 //
 // Replaces Qwen3MoeSparseMoeBlock.forward (models/qwen3_moe.py:146-186 of the reference): a Python
 // loop over the experts that were hit, each iteration gathering its tokens (torch.where + index),

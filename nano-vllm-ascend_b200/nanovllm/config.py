@@ -184,7 +184,7 @@ def ragilorn_preset(width: int, pattern: str, repeats: int, vocab: int = 32768, 
 
 
 def preset_hf_config(name: str):
-    """Architecture presets built offline from the public model cards (SURVEY.md section 8)."""
+    """Architecture presets built offline from the public model cards."""
     from transformers import LlamaConfig, Qwen3Config, Qwen3MoeConfig
     key = name.lower().rstrip("/").split("/")[-1]
     if key == "zegopel-1k":          # 28 layers at width 1024: the size class of qwen3-0.6b
@@ -301,7 +301,7 @@ class Config:
     prefix_hit_prefill: bool = False   # feed only uncached prompt tokens (attention_ori semantics)
     chunked_prefill: bool = False      # split prompts over several prefill steps when the token budget
                                        # (max_num_batched_tokens) runs out; later chunks attend to the
-                                       # earlier ones through the paged cache (SURVEY 8f f3)
+                                       # earlier ones through the paged cache
     graph_batch_sizes: tuple | None = None   # decode batch sizes to capture CUDA graphs for (None: the
                                        # default ladder 1, 2, 4, ..., max_num_seqs; max_num_seqs is always added)
     tp_shard_emulation: int = 0        # profiling aid: N > 1 builds rank 0's shard of an N-way tensor-parallel
@@ -315,7 +315,7 @@ class Config:
                                        # cached K/V blocks
     return_logits: bool = False        # keep every step's logits at the requested rows (scoring / trace replay)
     kv_cache_dtype: str = "auto"       # "auto": the model dtype (reference behaviour); "fp8" /
-                                       # "fp8_e4m3": e4m3 bytes, per-tensor scale 1.0 (SURVEY 8f f3)
+                                       # "fp8_e4m3": e4m3 bytes, per-tensor scale 1.0
     # Two-micro-batch decode (engine/model_runner.py::_forward_overlapped): a decode step whose attention
     # streams at least decode_overlap_min_kv_bytes of KV per layer (and at least 20x the layer's weight
     # bytes) runs as TWO half batches on two streams inside one CUDA graph, so that the HBM-bound attention

@@ -520,7 +520,7 @@ class ModelRunner:
         but the weights; what the split buys is overlap of two different bottlenecks -- the paged
         attention of one half streams KV at the HBM roofline while the other half runs its GEMM / norm /
         RoPE chain, ~8 launches of a few microseconds each that are latency-bound and would otherwise
-        leave HBM idle (DESIGN 3.8). Under CUDA-graph capture the second stream forks from and joins
+        leave HBM idle. Under CUDA-graph capture the second stream forks from and joins
         the capturing stream, so the step is still ONE graph with two parallel branches. Every kernel is
         row-wise (GEMMs included), so the result equals the one-batch step up to cuBLAS' choice of
         algorithm for M = bs / 2."""

@@ -103,7 +103,7 @@ class Sequence:
         self.num_prompt_tokens = self.num_tokens
 
     # state shipped to tensor-parallel workers each step. Unlike the reference
-    # (sequence.py:116-146, SURVEY appendix A) block_size and the sampling fields travel too,
+    # (sequence.py:116-146) block_size and the sampling fields travel too,
     # otherwise num_blocks raises on the worker side.
     # A decode step needs only the last token (the reference makes the same cut, sequence.py:116-125);
     # the prompt travels as packed int32 bytes, and only while the sequence is still being prefilled.

@@ -1,7 +1,7 @@
 """Tensor-parallel linear layers (reference: layers/linear.py).
 
 Same constructors and ``weight_loader(param, tensor[, shard_id])`` signatures. GEMMs stay on
-cuBLAS (``F.linear``; SURVEY G1). The one collective of a decoder layer is the SUM all-reduce
+cuBLAS (``F.linear``). The one collective of a decoder layer is the SUM all-reduce
 of the row-parallel output: NCCL over NVLink/NVSwitch through ``torch.distributed``, issued on
 the current stream so it is captured into the decode CUDA graph.
 """

@@ -1,7 +1,7 @@
 """Sampling tail (reference: layers/sampler.py:9-17).
 
 Reference semantics: trim padded graph rows, divide by temperature, softmax, multinomial.
-Here the whole tail is one kernel over the bf16 logits (SURVEY 8f row f2): Gumbel-max sampling
+Here the whole tail is one kernel over the bf16 logits: Gumbel-max sampling
 draws from exactly softmax(logits / T) without materialising fp32 logits or probabilities;
 ``greedy=True`` (temperature <= 0 is still rejected by SamplingParams, as in the reference)
 gives the argmax used by the parity tests.

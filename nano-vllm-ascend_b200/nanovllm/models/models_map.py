@@ -1,6 +1,6 @@
 """Which decoder class serves which HF ``architectures`` entry.
 
-The dense families of the hot-path scope and the Qwen3-MoE stack (SURVEY.md 8 f4) are registered;
+The dense families of the hot-path scope and the Qwen3-MoE stack are registered;
 the reference's registry (models/models_map.py) also lists its MiniCPM and vision-language stacks,
 which this build deliberately leaves out. Zegopel (a hybrid of softmax attention, lightning attention and
 Mamba-2 layers) and Nirelix (retention, gated delta rule and latent attention on a residual kept in several

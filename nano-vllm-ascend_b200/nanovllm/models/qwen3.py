@@ -12,7 +12,7 @@ def _rope_theta(config, default):
     """RoPE base. The reference reads ``getattr(config, "rope_theta", default)`` (qwen3.py:137,
     llama.py:133); transformers>=5 moved the value into ``config.rope_parameters``, where the
     reference no longer finds it and silently uses its default (right for Qwen3, wrong for
-    Llama-3.x -- SURVEY.md 8c). Here the checkpoint's real value is honoured in both layouts."""
+    Llama-3.x). Here the checkpoint's real value is honoured in both layouts."""
     theta = getattr(config, "rope_theta", None)
     if theta is None:
         params = getattr(config, "rope_parameters", None) or {}

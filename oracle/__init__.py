@@ -5,7 +5,7 @@ the path (``nanovllm/layers/attention_torch_native.py`` + the eager layers it si
 Only ``tests/``, ``__graft_entry__.smoke()`` and the ``cpu_baseline`` / ``--impl reference``
 legs of ``bench.py`` may import this package; nothing under ``nano-vllm-ascend_b200/`` does.
 
-Parity status: PINNED. The reference publishes no golden vectors for this path (SURVEY.md 8c),
+Parity status: PINNED. The reference publishes no golden vectors for this path,
 so the pin is made with outputs of the reference itself: ``oracle/gen_golden.py`` imports the
 unmodified reference modules from /root/reference (namespace stub), runs them on seeded inputs
 and stores the results in ``tests/golden/*.pt``; ``tests/test_oracle_golden.py`` asserts that

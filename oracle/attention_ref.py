@@ -144,7 +144,7 @@ def gather_paged_kv(k_cache, v_cache, block_tables, seq_lens):
 
 
 # ---------------------------------------------------------------------------------------------
-# FP8 (e4m3) KV cache -- SURVEY.md 8f row f3. NOT a restatement of reference code: the reference
+# FP8 (e4m3) KV cache. NOT a restatement of reference code: the reference
 # keeps its caches in the model dtype (engine/model_runner.py:218-229). This states the semantics
 # the fp8 kernels (csrc/decode_attn_fp8.cu) implement, with torch's own float8_e4m3fn cast as the
 # arithmetic authority, so the scatter can be checked bit for bit and attention against

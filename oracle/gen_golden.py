@@ -5,7 +5,7 @@ The reference package cannot be imported whole (torch_npu/torchair are absent), 
 namespace stub is registered and only its CPU-capable modules are imported: the torch-native
 attention (layers/attention_torch_native.py), the eager layers, and models/qwen3.py with the
 NPU attention module replaced by a constructor-adapting shim around the torch-native class
-(SURVEY.md 8c). The runner metadata (prepare_prefill / prepare_decode) is restated in
+The runner metadata (prepare_prefill / prepare_decode) is restated in
 oracle/model_ref.py because engine/model_runner.py is NPU-bound.
 
 Outputs are inputs + reference outputs for seeded cases; tests/test_oracle_golden.py replays

@@ -3,7 +3,7 @@
 The reference package cannot be imported whole (torch_npu / torchair are absent), so a namespace
 stub is registered and only its CPU-capable modules are imported: the torch-native attention
 (layers/attention_torch_native.py), the eager layers and models/qwen3.py with the NPU attention
-module replaced by a constructor-adapting shim around the torch-native class (SURVEY.md 8c). The
+module replaced by a constructor-adapting shim around the torch-native class. The
 runner metadata (prepare_prefill / prepare_decode, engine/model_runner.py:238-366, NPU-bound) is
 restated in oracle/model_ref.py.
 

@@ -21,7 +21,7 @@ SRC = os.environ.get("B200_REFERENCE_SRC", "/root/reference")
 DST = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_ref")
 ARCHIVE = os.path.join(DST, "reference_path.zip")
 
-# exactly the modules oracle/ref_runtime.py imports (SURVEY.md 8a/8c); the NPU-bound ones
+# exactly the modules oracle/ref_runtime.py imports; the NPU-bound ones
 # (layers/attention.py, engine/model_runner.py, engine/llm_engine.py) are deliberately absent
 FILES = [
     "nanovllm/layers/attention_torch_native.py",

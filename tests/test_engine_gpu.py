@@ -86,7 +86,7 @@ def _config1_run(g, **init):
 
 def _exact_fp32_logits(g, forced, **init):
     """The fp32-accumulating evaluation of the same graph (oracle attn_mode="exact", LM head kept in
-    fp32) under the same teacher forcing: the yardstick SURVEY 7 names for the logit bound."""
+    fp32) under the same teacher forcing: the yardstick for the logit bound."""
     cfg = M.ModelCfg.qwen3_0_6b()
     w = M.seeded_weights(cfg, seed=g["seed"], **init)
     tr = M.generate_greedy(w, cfg, g["prompts"], g["max_tokens"], g["block_size"], attn_mode="exact",
@@ -112,7 +112,7 @@ def _ids_on_decided_steps(got, mine, g):
 def test_qwen3_0_6b_config1_greedy_matches_reference(golden_models):
     """BASELINE config 1 on the GPU: random-init Qwen3-0.6B (N(0, 0.02)), 1 prompt, block 16, 32 tokens.
     Greedy ids against the unmodified reference's run; fp32 logits against the exact oracle -- the
-    north_star's "logits within 1e-3" in the only form two bf16 pipelines can meet.
+    "logits within 1e-3" in the only form two bf16 pipelines can meet.
     Measured on a B200; bounds are <= 2x the measured values."""
     g = golden_models["qwen3_0_6b_config1"]
     got, mine, got32, forced = _config1_run(g)

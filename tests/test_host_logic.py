@@ -145,7 +145,7 @@ def test_sequence_block_math_and_wire_state():
     assert (s.num_blocks, s.last_block_num_tokens, s.block(2)) == (3, 5, list(range(32, 37)))
     s.block_table = [4, 2, 9]
     t = pickle.loads(pickle.dumps(s))
-    # the reference drops block_size on the wire (SURVEY appendix A); workers need it
+    # the reference drops block_size on the wire; workers need it
     assert t.num_blocks == 3 and t.block_table == [4, 2, 9] and t.max_tokens == 9
 
 
@@ -214,7 +214,7 @@ def test_block_manager_prefix_sharing():
 
 
 def test_chunked_prefill_scheduling():
-    """chunked_prefill=True (extension): a prompt longer than the step's token budget is
+    """chunked_prefill=True (an extension): a prompt longer than the step's token budget is
     computed window by window; windows tile the prompt exactly, the budget is never exceeded, nothing is
     admitted behind a half-computed prompt, only the final window yields a token, and a prompt that
     leaves half-way takes the hashes of its never-computed blocks with it."""
@@ -364,7 +364,7 @@ def test_decode_wire_message_is_small_and_complete():
 
 def test_sampler_noise_key_is_the_device_counter_alone():
     """With a device step counter the host step passed to the kernel is 0 for every launch, so the
-    value baked into a CUDA graph at capture cannot alias another bucket's (ADVICE r1)."""
+    value baked into a CUDA graph at capture cannot alias another bucket's."""
     from nanovllm.layers.sampler import Sampler
     s = Sampler(seed=3)
     assert [s._next_step(object()) for _ in range(4)] == [0, 0, 0, 0] and s.step == 0
@@ -483,7 +483,7 @@ def test_seeded_init_matches_oracle_weights():
     assert model.lm_head.weight.data_ptr() == model.model.embed_tokens.weight.data_ptr()
 
 
-# ------------------------------------------------------------------ Qwen3-MoE (SURVEY 8 f4): host side
+# ------------------------------------------------------------------ Qwen3-MoE: host side
 def _build_tiny_moe(tp=None, seed=None):
     """Tiny Qwen3-MoE on CPU, optionally as rank tp[0] of tp[1], optionally seeded-initialised
     (the initialiser needs the same tensor-parallel view as the constructor)."""
@@ -705,7 +705,7 @@ def test_sharded_sampling_key_packing_arithmetic():
 
 
 def test_decode_step_form_selection():
-    """ModelRunner's host-side choices for a decode step (DESIGN 3.8, 3.1): one batch or two micro-batches,
+    """ModelRunner's host-side choices for a decode step: one batch or two micro-batches,
     and the attention grid -- pure arithmetic on the step's context lengths, checked on a stub runner."""
     import types
     from nanovllm.config import Config

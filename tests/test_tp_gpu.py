@@ -41,7 +41,7 @@ def test_tp2_matches_tp1():
     """TP=2 engine == TP=1 token ids, eager and CUDA-graph decode, with the default collectives (one-shot
     fused all-reduce at this size, vocab-sharded sampling), with every all-reduce forced through the
     two-shot kernel, and with plain NCCL + logits gather (the reference's structure). One test function
-    (six engine runs) so that a single-GPU box reports one skip, not six."""
+    (six engine runs) so that a machine with one GPU reports one skip, not six."""
     _need_gpus(2)
     rnd = random.Random(8)
     prompts = [[rnd.randint(0, 511) for _ in range(n)] for n in (9, 40, 17)]

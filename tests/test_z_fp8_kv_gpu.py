@@ -1,5 +1,5 @@
 """-m gpu: FP8 (e4m3) KV-cache variant of the scatter (K1/K2) and of paged decode attention (K6),
-SURVEY.md 8f row f3, through the C ABI, against the oracle's statement of the same semantics
+through the C ABI, against the oracle's statement of the same semantics
 (oracle/attention_ref.py: quantize_e4m3 / decode_attention_fp8).
 
 Tolerances: the quantising scatter is bit-exact (same fp32 product, same round-to-nearest-even

@@ -3,7 +3,7 @@ usage: python tools/kbench.py [decode|prefill|fa2|all]
 
 `fa2` times the reference's CUDA attention variant (layers/attention_ori.py:63-74: flash_attn 2.8.3
 flash_attn_with_kvcache / flash_attn_varlen_func, library code) on the same shapes -- the
-"kernel to beat" of SURVEY.md 8(d). FA2's paged path needs page_block_size % 256 == 0, so it runs
+"kernel to beat". FA2's paged path needs page_block_size % 256 == 0, so it runs
 at block 256 (the reference default); ours is timed at block 16 and 256."""
 import argparse
 import json
