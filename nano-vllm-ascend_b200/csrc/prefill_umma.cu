@@ -219,14 +219,23 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
   }
+  // One query tile per CTA is the form of the smallest launches: its producer needs no columns and does not wait for them
+  // before its first loads (us, 16 heads over 8 of 128: 1 x 17 tokens 6.6 -> 6.3, 1 x 300 10.2 -> 9.6). With two it made no difference, and the compiler spilled more.
+  constexpr bool kEarly = QT == 1;
+  if (kEarly) __syncthreads();                       // the barriers are initialised
   // The kernel before this one may still have CTAs on the SM that have yet to allocate their columns (it lets its dependents
   // in at its start): taking all 512 before it has finished could leave both waiting.
   pdl_wait();
   if (warp == kMmaWarp) umma::tmem_alloc(tmem_slot, kTmemCols);
-  umma::fence_before_sync();
-  __syncthreads();
-  umma::fence_after_sync();
-  const uint32_t tb = *tmem_slot;
+  if (kEarly && warp == kTmaWarp) {
+    named_bar_arrive(1, prefill_threads(QT));
+  } else {
+    umma::fence_before_sync();
+    if (kEarly) named_bar_sync(1, prefill_threads(QT));
+    else __syncthreads();
+    umma::fence_after_sync();
+  }
+  const uint32_t tb = *tmem_slot;                    // (the early producer has no use for it)
 
   // Work items: (row tile, sequence, head, key split) in order of falling row tile, so that the longest come first and a
   // CTA's items have about the same number of key tiles as any other's; inside a row tile key
@@ -833,7 +842,7 @@ int prefill_kv_splits(int num_seqs, int H, int max_seqlen_q, int max_seqlen_k, i
 // b200_prefill_set_query_tiles(1|2) forces one layout (A/B runs, parity tests of both instantiations).
 // Launches whose 128-row tiles of one head find a CTA slot each (`slots`), with at most four key tiles, take QT = 1 in any
 // case: nothing is read often enough for sharing to count, and a CTA's start, two chains and end are shorter than those of a
-// pair (us, QT = 1 / pair, 16 heads over 8: D 128, 1 x 17 6.6 / 7.1, 1 x 300 10.2 / 11.2, 2 x 129 8.2 / 9.2; keys of 192, 1 x 300 9.1 / 11.1).
+// pair (us, QT = 1 / pair, 16 heads over 8: D 128, 1 x 17 6.3 / 7.1, 1 x 300 9.6 / 11.2, 2 x 129 8.1 / 9.2; keys of 192, 1 x 300 8.9 / 11.1).
 static bool prefill_small(int num_seqs, int H, int max_seqlen_q, int max_seqlen_k, int slots) {
   return (int64_t)((max_seqlen_q + kUBM - 1) / kUBM) * H * num_seqs <= slots && max_seqlen_k <= 4 * kUBN;
 }
