@@ -623,6 +623,16 @@ int b200_linear_recurrence(float* out, const void* q, int64_t q_stride, const vo
                            int32_t mode, int32_t act_silu, const float* decay, const void* dt,
                            int64_t dt_stride, const float* dt_bias, const float* a_log, const float* d_skip,
                            int32_t qk_f32, int32_t dtype, b200_stream_t stream);
+/* The same where the caller knows the tokens of the step (0: unknown): spans that are long on average, bf16, key rows and values on
+ * 16-byte boundaries, vdim 128, or 64 with an even number of heads per group, run 64 tokens at a time on the 5th-generation tensor cores. */
+int b200_linear_recurrence_step(float* out, const void* q, int64_t q_stride, const void* k, int64_t k_stride,
+                           const void* v, int64_t v_stride, float* state, const int32_t* state_slots,
+                           const int32_t* cu_q, const int32_t* cu_k, const int32_t* ctx_lens,
+                           int32_t num_seqs, int32_t max_q, int32_t num_heads, int32_t groups, int32_t kdim,
+                           int32_t vdim,
+                           int32_t mode, int32_t act_silu, const float* decay, const void* dt,
+                           int64_t dt_stride, const float* dt_bias, const float* a_log, const float* d_skip,
+                           int32_t qk_f32, int32_t dtype, int64_t total_q, b200_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------------
  * Multi-stream residuals, rotary positions, delta rule, latent attention, clamped gated unit

@@ -211,6 +211,40 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   while (!mbar_try_wait(bar, parity)) {
   }
 }
+// ---- waits that end by themselves
+constexpr int64_t kWaitNs = 4000000000ll;                  // a launch takes milliseconds at most
+constexpr int64_t kDrainNs = 1000000000ll;                 // copies and products that are under way when a wait has run out
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {      // does not suspend
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ int64_t global_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return (int64_t)t;
+}
+// false: the phase did not complete within limit_ns, or another role of the CTA gave up first (gave_up, where given). One
+// thread's answer: warps vote on it
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* gave_up, int64_t limit_ns) {
+  if (mbar_test_wait(bar, parity)) return true;
+  if (limit_ns > 0) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const int64_t t0 = global_ns();
+    do {
+      if (mbar_try_wait(bar, parity)) return true;
+      if (gave_up != nullptr && *gave_up) return false;
+    } while (global_ns() - t0 < limit_ns);
+  }
+  if (gave_up != nullptr) *gave_up = 1;
+  return false;
+}
 // generic-proxy writes to smem must be fenced before the async proxy (TMA) may overwrite
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -236,41 +236,6 @@ constexpr int kMwOut = 4 * 32 * 128;                        // epilogue: 32 rows
 constexpr int kMwMaxExperts = 256;
 constexpr int kMwSmem = 1024 + kMwStages * kMwStageBytes + kMwOut + 128 + (kMwMaxExperts + 4) * 4;
 
-constexpr int64_t kMwWaitNs = 4000000000ll;                  // a launch takes milliseconds at most
-constexpr int64_t kMwDrainNs = 1000000000ll;
-
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {      // does not suspend
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ int64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return (int64_t)t;
-}
-// false: the phase did not complete within limit_ns, or another role of the CTA gave up first (gave_up, where given). One
-// thread's answer: warps vote on it
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* gave_up, int64_t limit_ns) {
-  if (mbar_test_wait(bar, parity)) return true;
-  if (limit_ns > 0) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const int64_t t0 = global_ns();
-    do {
-      if (mbar_try_wait(bar, parity)) return true;
-      if (gave_up != nullptr && *gave_up) return false;
-    } while (global_ns() - t0 < limit_ns);
-  }
-  if (gave_up != nullptr) *gave_up = 1;
-  return false;
-}
-
 template <typename T, bool kGateUp>
 __global__ void __launch_bounds__(kMuThreads, 1)
 moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const MoeUmmaParams p) {
@@ -368,7 +333,7 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       // copies under way land before the CTA's shared memory is given back, whichever role leaves early: the last ones of
       // every stage, copies max(0, it - stages) .. it - 1
       for (int j = max(0, it - kMwStages); j < it; ++j)
-        mbar_wait_bounded(&full[j % kMwStages], (j / kMwStages) & 1, nullptr, kMwDrainNs);
+        mbar_wait_bounded(&full[j % kMwStages], (j / kMwStages) & 1, nullptr, kDrainNs);
     }
   } else if (warp == 1) {
     // =========================== MMA issuer ===========================
@@ -401,7 +366,7 @@ moe_umma_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     // products under way finish before the columns and the operands go, whichever role leaves early
     if (leader) umma::commit(drained);
     __syncwarp();
-    mbar_wait_bounded(drained, 0, nullptr, kMwDrainNs);
+    mbar_wait_bounded(drained, 0, nullptr, kDrainNs);
     __syncwarp();
   } else {
     // =========================== epilogue warps (2..5) ===========================
@@ -580,7 +545,7 @@ extern "C" int b200_moe_gather_rows(void* xs, const void* x, const int32_t* offs
 static int moe_umma_common(bool gate_up, void* out, const void* a, const void* w, const int32_t* offsets,
                            const int32_t* sorted_pair, const void* pair_scale, int32_t pairs, int32_t K,
                            int32_t n_out, int32_t num_local, int32_t dtype, b200_stream_t stream,
-                           int out_f32 = 0, const float* in_scale = nullptr, int64_t wait_ns = kMwWaitNs) {
+                           int out_f32 = 0, const float* in_scale = nullptr, int64_t wait_ns = kWaitNs) {
   B200_RETURN_IF(dtype != B200_DTYPE_BF16 && dtype != B200_DTYPE_F16, B200_ERR_BAD_DTYPE);
   B200_RETURN_IF(pairs < 0 || K <= 0 || n_out <= 0 || num_local <= 0, B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(K % 64 != 0 || n_out % (gate_up ? 64 : 128) != 0 || num_local > 256, B200_ERR_UNSUPPORTED);

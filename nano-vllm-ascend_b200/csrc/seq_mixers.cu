@@ -13,6 +13,7 @@
 //                      forget gate per key channel that also decides what is written (k = 1 - f: the tied form
 //                      of HGRN2), S_t = diag(f_t) S_(t-1) + (1 - f_t) v_t^T.
 #include "attn_tiled.cuh"
+#include "recurrence.cuh"
 #include "seq_common.cuh"
 
 namespace b200 {
@@ -143,24 +144,6 @@ attn_generic_kernel(T* __restrict__ out, const T* __restrict__ q, int64_t q_stri
 // registers while the current one is consumed.
 constexpr int kRecTok = 8;
 
-// silu for 16-bit activations: its result is rounded to 8 or 11 bits, the fast exponential is good to ~21
-__device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
-
-struct RecParams {
-  const void *q, *k, *v;            // q, k: [tokens, groups * kdim] of type T; v: [tokens, H * vdim] of type TV
-  int64_t q_stride, k_stride, v_stride;
-  float* out;                       // [tokens, H * vdim] fp32
-  float* state;                     // [slots, H, kdim, vdim] fp32 or nullptr (start from zero, keep nothing)
-  const int *state_slots, *cu_q, *cu_k, *ctx_lens;
-  int H, groups, kdim, vdim;
-  int mode;                         // 0: constant decay per head; 1: selective (dt); 2: `k` holds a forget gate f per
-                                    //    key channel (fp32): S <- diag(f) S + (1 - f) v^T
-  int act_silu;                     // silu on q, k, v as they are read (mode 0)
-  const float* decay;               // mode 0: [H]
-  const void* dt;                   // mode 1: [tokens, H] element type T, before bias and softplus
-  int64_t dt_stride;
-  const float *dt_bias, *a_log, *d_skip;   // mode 1: [H] each
-};
 
 template <typename T, typename TV, int KPT, int NS>
 __global__ void __launch_bounds__(128)
@@ -355,19 +338,6 @@ static void recurrence_launch_as(const RecParams& P, int num_seqs, cudaStream_t 
 // chunks of 16 (1420), 328 us with chunks of 32. Chunks of 64 would need 10 more score tiles per warp than there are registers.
 // The decays of a chunk are exponentials of sums over at most 16 tokens: across the two blocks they are multiplied, since a
 // prefix sum over 32 loses a bit (error of the outputs against 64 bits 4.2e-7 with it, 2.5e-7 so).
-// two fp32 -> three packed bf16 pairs hi, mid, lo (first value in the low half), each term the rounding of what the ones
-// before it leave. The packed conversion runs at half of the fp32 rate, the scalar one on the special-function unit at
-// an eighth (which is 3 % busy now).
-__device__ __forceinline__ void split3x2(float x, float y, uint32_t (&w)[3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(y), "f"(x));
-    if (i < 2) x -= __uint_as_float(w[i] << 16), y -= __uint_as_float(w[i] & 0xffff0000u);
-  }
-}
-__device__ __forceinline__ uint32_t bf16_bits(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
-__device__ __forceinline__ float bits_f32(uint32_t b16) { return __uint_as_float(b16 << 16); }
-
 constexpr int kChunk = 32;             // two 16-token blocks
 
 // VEC: q, k, v rows start on 16-byte boundaries (strides, sizes and slice offsets % 8 == 0): the tiles of the next
@@ -813,14 +783,14 @@ extern "C" int b200_attn_generic(void* out, const void* q, int64_t q_stride, con
   return finish_launch();
 }
 
-extern "C" int b200_linear_recurrence(float* out, const void* q, int64_t q_stride, const void* k,
+extern "C" int b200_linear_recurrence_step(float* out, const void* q, int64_t q_stride, const void* k,
                                       int64_t k_stride, const void* v, int64_t v_stride, float* state,
                                       const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k,
                                       const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q,
                                       int32_t num_heads, int32_t groups, int32_t kdim, int32_t vdim, int32_t mode,
                                       int32_t act_silu, const float* decay, const void* dt, int64_t dt_stride,
                                       const float* dt_bias, const float* a_log, const float* d_skip,
-                                      int32_t qk_f32, int32_t dtype, b200_stream_t stream) {
+                                      int32_t qk_f32, int32_t dtype, int64_t total_q, b200_stream_t stream) {
   B200_RETURN_IF(num_seqs < 0 || num_heads <= 0 || groups <= 0 || num_heads % groups != 0 || kdim <= 0 ||
                      vdim <= 0 || mode < 0 || mode > 2, B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(kdim > 256, B200_ERR_UNSUPPORTED);
@@ -840,7 +810,19 @@ extern "C" int b200_linear_recurrence(float* out, const void* q, int64_t q_strid
     if (dtype == B200_DTYPE_F16) return recurrence_launch<float, __half>(P, num_seqs, (cudaStream_t)stream);
     return B200_ERR_BAD_DTYPE;
   }
+  if (recurrence_umma_ok(P, dtype, num_seqs, max_q, total_q)) return recurrence_umma_launch(P, num_seqs, (cudaStream_t)stream);
   if (chunk_recurrence_ok(P, dtype, max_q)) return chunk_recurrence_launch(P, num_seqs, (cudaStream_t)stream);
   B200_DISPATCH_3(dtype, T, return recurrence_launch<T>(P, num_seqs, (cudaStream_t)stream));
   return B200_OK;
+}
+
+extern "C" int b200_linear_recurrence(float* out, const void* q, int64_t q_stride, const void* k,
+                                      int64_t k_stride, const void* v, int64_t v_stride, float* state,
+                                      const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k,
+                                      const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q,
+                                      int32_t num_heads, int32_t groups, int32_t kdim, int32_t vdim, int32_t mode,
+                                      int32_t act_silu, const float* decay, const void* dt, int64_t dt_stride,
+                                      const float* dt_bias, const float* a_log, const float* d_skip,
+                                      int32_t qk_f32, int32_t dtype, b200_stream_t stream) {
+  return b200_linear_recurrence_step(out, q, q_stride, k, k_stride, v, v_stride, state, state_slots, cu_q, cu_k, ctx_lens, num_seqs, max_q, num_heads, groups, kdim, vdim, mode, act_silu, decay, dt, dt_stride, dt_bias, a_log, d_skip, qk_f32, dtype, 0, stream);
 }

@@ -1,0 +1,61 @@
+"""ops.linear_recurrence in chunks of 64 tokens on the tensor cores (csrc/recurrence_umma.cu): spans around its chunks, its 16-token
+blocks and the length from which it takes a span, beside spans that chunk_recurrence_kernel keeps; two heads per CTA and one,
+key sizes that are padded, in two portions with a carried state, against the recurrence in 64 bits, token by token. Tolerance:
+fp32 sums of a few hundred terms, as the other tests of these recurrences."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+F64 = torch.float64
+
+
+@pytest.mark.parametrize("H,G,N,V,selective,silu,lens", [
+    (4, 2, 128, 64, True, False, [130, 1, 200, 95, 96, 97, 17, 0, 385]),
+    (4, 1, 72, 64, True, True, [128, 191, 1]),
+    (2, 2, 128, 128, False, True, [96, 1, 129, 64]),
+    (2, 1, 128, 128, True, False, [257]),
+    (4, 2, 64, 64, False, False, [255, 256, 257, 1, 320]),
+    (2, 1, 40, 128, True, False, [321, 1, 63]),
+    (2, 2, 64, 128, False, True, [449]),
+])
+def test_against_64_bit_in_portions(H, G, N, V, selective, silu, lens):
+    from nanovllm import ops
+    g = torch.Generator(device="cuda").manual_seed(N + V + len(lens))
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    S = len(lens)
+    state = torch.full((S + 1, H, N, V), float("nan"), device="cuda")
+    slots = torch.tensor(list(range(S, 0, -1)), dtype=torch.int32, device="cuda")
+    rows = [dict(q=rand(2 * n, G * N).bfloat16(), k=(rand(2 * n, G * N) * N ** -0.5).bfloat16(), v=rand(2 * n, H * V).bfloat16(),
+                 dt=rand(2 * n, H).bfloat16()) for n in lens]
+    decay = 0.699 + 0.3 * torch.rand(H, device="cuda", generator=g)
+    bias, alog, skip = rand(H) * 0.5, -torch.rand(H, device="cuda", generator=g), rand(H)
+    par = dict(dt_bias=bias, a_log=alog, d_skip=skip) if selective else dict(decay=decay, act_silu=silu)
+    cu = lambda x: torch.tensor([0] + x).cumsum(0).to(torch.int32).cuda()  # noqa: E731
+    act = (lambda x: torch.nn.functional.silu(x.float()).bfloat16().to(F64)) if silu and not selective else (lambda x: x.to(F64))
+    tol = 1e-2 if silu and not selective else 5e-6             # silu: one bf16 step of an operand now and then
+    want_state = torch.zeros(S, H, N, V, dtype=F64, device="cuda")
+    for part in range(2):
+        at = [slice(part * n, (part + 1) * n) for n in lens]
+        d = {x: torch.cat([r[x][a] for r, a in zip(rows, at)]) for x in ("q", "k", "v", "dt")}
+        sp = ops.StepSpans(cu(lens), cu([n * (part + 1) for n in lens]), None, max(lens))
+        o = ops.linear_recurrence(d["q"], d["k"], d["v"], sp, H, G, N, V, state, slots, **(dict(par, dt=d["dt"]) if selective else par))
+        begin = 0
+        for s, n in enumerate(lens):
+            q, k, v = (act(rows[s][x][at[s]]) for x in "qkv")
+            step = torch.nn.functional.softplus(rows[s]["dt"][at[s]].to(F64) + bias.to(F64)) if selective else torch.ones(n, H, dtype=F64, device="cuda")
+            a = torch.exp(-torch.exp(alog.to(F64)) * step) if selective else decay.to(F64).expand(n, H)
+            st, want = want_state[s], torch.zeros(n, H, V, dtype=F64, device="cuda")
+            q, k = (x.view(n, G, N).repeat_interleave(H // G, 1) for x in (q, k))
+            vx = step[:, :, None] * v.view(n, H, V)
+            for t in range(n):
+                st.mul_(a[t][:, None, None]).add_(k[t][:, :, None] * vx[t][:, None, :])
+                want[t] = torch.matmul(q[t][:, None, :], st).squeeze(1)
+            if selective:
+                want += skip.to(F64)[:, None] * v.view(n, H, V)
+            if n:
+                x = o[begin:begin + n].to(F64).view(n, H, V)
+                assert float((x - want).norm() / want.norm()) < tol, (part, s, n)
+                kept = state[int(slots[s])].to(F64)
+                assert float((kept - st).norm() / st.norm()) < tol, (part, s, n)
+            begin += n
+    assert bool(torch.isnan(state[0]).all())                   # a slot that no sequence holds
