@@ -17,8 +17,9 @@
 // order of issue is O2(i) | SC(i+1) | O1(i) | dS(i+1): the score warps work under O1 and dS, the state warps store outputs under
 // dS(i+1) and turn S(i) into terms under O2(i+1), k and x come two chunks ahead. What also counts is code size: 24 warps of six
 // roles run through their code once per chunk, and with everything unrolled (164 KB) instruction fetches took three quarters of
-// the time (16 x 1024 tokens, 32 heads of 128 x 64: 265 us; 190 with short loops; 135 with the roles spread over 24 warps).
-// Measured there: 329 us (chunk_recurrence_kernel, mma.sync, chunks of 32) -> 135 us; 8 heads of 128 x 128 195 -> 114; errors against
+// the time (16 x 1024 tokens, 32 heads of 128 x 64: 265 us; 190 with short loops; 135 with the roles spread over 24 warps; 133 with an add per
+// operand and MMA).
+// Measured there: 329 us (chunk_recurrence_kernel, mma.sync, chunks of 32) -> 133 us; 8 heads of 128 x 128 195 -> 113; errors against
 // 64 bits 2.2e-7 (2.5e-7).
 // Warps: 0-7 state and outputs (a warp: 32 channels x half of the keys, then half of the tokens; D / 2 state registers a thread);
 // 8, 9 and 12, 13 P of a head's diagonal blocks, 17 and 21 of the others (only warps w with w % 4 < 2 may read TMEM lanes 0-63);
@@ -166,7 +167,7 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
-  const uint32_t tb = *tmem_slot;
+  constexpr uint32_t tb = 0;                            // all 512 columns: they start at 0
   const int chunks = (sp.q_len + kRuL - 1) / kRuL;
   // Whole warps wait, and leave together. A try is suspended for up to 4 us (measured); counting them takes less code than a clock
   auto wait = [&](uint64_t* bar, int parity) {
@@ -444,16 +445,16 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
       // =========================== issue ===========================
       const uint32_t id_sc = umma::make_idesc<T>(128, 64, 0, 0), id_o2 = umma::make_idesc<T>(128, 64, 1, 0),
                      id_d = umma::make_idesc<T>(128, D, 1, 1);
-      const uint64_t dq = umma::desc_kmajor(smem_u32(sQ)), dk = umma::desc_kmajor(smem_u32(sK)),
-                     dk_mn = umma::desc_mnmajor(smem_u32(sK), kRuPanel), dx = umma::desc_mnmajor(smem_u32(sX), kRuPanel),
-                     dp = umma::desc_kmajor(smem_u32(sP)), dw = umma::desc_mnmajor(smem_u32(sW), kRuPanel);
+      const uint32_t dq = umma::desc_low(smem_u32(sQ), 16), dk = umma::desc_low(smem_u32(sK), 16), dk_mn = umma::desc_low(smem_u32(sK), kRuPanel),
+                     dx = umma::desc_low(smem_u32(sX), kRuPanel), dp = umma::desc_low(smem_u32(sP), 16), dw = umma::desc_low(smem_u32(sW), kRuPanel);
       const bool leader = umma::elect_one();
       auto issue_sc = [&](int j) {
         if (leader) {
+          const uint32_t at = (j & 1) * (kQK >> 4), a0 = dq + at, b0 = dk + at;
 #pragma unroll
           for (int ks = 0; ks < D / 16; ++ks) {
-            const uint32_t at = (j & 1) * kQK + (ks >> 2) * kRuPanel + (ks & 3) * 32;
-            umma::mma_ss(tb + kTmSC, umma::desc_advance(dq, at), umma::desc_advance(dk, at), id_sc, ks > 0);
+            constexpr int kPanel = kRuPanel >> 4;
+            umma::mma_ss_low(tb + kTmSC, a0 + (ks >> 2) * kPanel + (ks & 3) * 2, b0 + (ks >> 2) * kPanel + (ks & 3) * 2, id_sc, ks > 0);
           }
           umma::commit(sc_full);
         }
@@ -461,12 +462,12 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
       };
       auto issue_d = [&](int j) {
         if (leader) {
-          const uint64_t bd = umma::desc_advance(dk_mn, (j & 1) * kQK);
+          const uint32_t b0 = dk_mn + (j & 1) * (kQK >> 4);
 #pragma unroll
           for (int p = 2; p >= 0; --p)
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
-              umma::mma_ss(tb + kTmD, umma::desc_advance(dw, p * 2 * kRuPanel + ks * 2048), umma::desc_advance(bd, ks * 2048), id_d, p < 2 || ks > 0);
+              umma::mma_ss_low(tb + kTmD, dw + ((p * 2 * kRuPanel + ks * 2048) >> 4), b0 + (ks * 2048 >> 4), id_d, p < 2 || ks > 0);
           umma::commit(d_done);
           umma::commit(&k_empty[j & 1]);                // the last reader of k, and of x of chunk j - 1
         }
@@ -474,12 +475,12 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
       };
       auto issue_o1 = [&](int j) {
         if (leader) {
-          const uint64_t bd = umma::desc_advance(dq, (j & 1) * kQK);
+          const uint32_t b0 = dq + (j & 1) * (kQK >> 4);
 #pragma unroll
           for (int p = 2; p >= 0; --p)
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks)
-              umma::mma_ts(tb + kTmO1, tb + kTmS + p * (D / 2) + ks * 8, umma::desc_advance(bd, (ks >> 2) * kRuPanel + (ks & 3) * 32), id_sc, p < 2 || ks > 0);
+              umma::mma_ts_low(tb + kTmO1, tb + kTmS + p * (D / 2) + ks * 8, b0 + (((ks >> 2) * kRuPanel + (ks & 3) * 32) >> 4), id_sc, p < 2 || ks > 0);
           umma::commit(o1_done);
           umma::commit(&q_empty[j & 1]);                // their last reader
         }
@@ -487,16 +488,16 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
       };
       auto issue_o2 = [&](int j) {
         if (leader) {
-          const uint64_t ad = umma::desc_advance(dx, (j % 3) * 2 * kRuPanel);
+          const uint32_t a0 = dx + (j % 3) * (2 * kRuPanel >> 4);
 #pragma unroll
           for (int p = 2; p >= 0; --p)
 #pragma unroll
             for (int hh = 0; hh < NH; ++hh)              // P of a head meets the values of both: half of the lanes are of use
 #pragma unroll
               for (int ks = 0; ks < 4; ++ks) {
-                const uint64_t b = umma::desc_advance(dp, (p * NH + hh) * kRuPanel + ks * 32);
-                if (NH == 2) umma::mma_ss_half(tb + kTmO2, umma::desc_advance(ad, ks * 2048), b, id_o2, p < 2 || ks > 0, hh);
-                else umma::mma_ss(tb + kTmO2, umma::desc_advance(ad, ks * 2048), b, id_o2, p < 2 || ks > 0);
+                const uint32_t a = a0 + (ks * 2048 >> 4), b = dp + (((p * NH + hh) * kRuPanel + ks * 32) >> 4);
+                if (NH == 2) umma::mma_ss_half_low(tb + kTmO2, a, b, id_o2, p < 2 || ks > 0, hh);
+                else umma::mma_ss_low(tb + kTmO2, a, b, id_o2, p < 2 || ks > 0);
               }
           umma::commit(o2_done);
         }

@@ -84,17 +84,6 @@ __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// the same, but only lanes 0-63 (half 0) or 64-127 (half 1) of D are written
-__device__ __forceinline__ void mma_ss_half(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate, int half) {
-  const uint32_t off0 = half == 0 ? 0u : 0xffffffffu, off1 = ~off0;        // lanes whose bit is set are left alone
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %6, %6}, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(off0), "r"(off1)
-      : "memory");
-}
 // D[tmem] (+)= A[tmem] * B[smem desc]: the ".ts" form (A is K-major by construction; a 16-bit A
 // operand packs two consecutive K elements per 32-bit column, lane = M row). The P V
 // products of prefill_umma.cu.
@@ -105,6 +94,43 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
       "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The same from the low word of each descriptor (address and leading byte offset; the high one is that of every SW128 panel here:
+// 1024 bytes between 8-row groups, version 1). A 32-bit add per operand is what an MMA costs the issuing lane then, and that lane
+// is what short MMAs wait for.
+__device__ __forceinline__ uint32_t desc_low(uint32_t smem_addr, uint32_t lbo_bytes) {
+  return ((smem_addr >> 4) & 0x3FFF) | (((lbo_bytes >> 4) & 0x3FFF) << 16);
+}
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ void mma_ss_low(uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "n"(kDescHigh)
+      : "memory");
+}
+// only lanes 0-63 (half 0) or 64-127 (half 1) of D are written
+__device__ __forceinline__ void mma_ss_half_low(uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate,
+                                                int half) {
+  const uint32_t off0 = half == 0 ? 0u : 0xffffffffu, off1 = ~off0;        // lanes whose bit is set are left alone
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %7};\n\tmov.b64 b, {%2, %7};\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, {%5, %5, %6, %6}, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(off0), "r"(off1), "n"(kDescHigh)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ts_low(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+      "mov.b64 b, {%2, %5};\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_low), "r"(idesc), "r"(accumulate), "n"(kDescHigh)
       : "memory");
 }
 // all previously issued MMAs of this thread arrive on `bar` when complete

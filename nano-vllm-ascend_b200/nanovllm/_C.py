@@ -144,6 +144,10 @@ PROTOTYPES = {
                                     c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
                                     c_int32, c_int32, c_int32, c_float, c_int32, c_int32, c_int32, c_float, c_void_p,
                                     c_void_p, c_int64, c_int32, c_void_p]),
+    "b200_attn_generic_step": (c_int32, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
+                                    c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
+                                    c_int32, c_int32, c_int32, c_float, c_int32, c_int32, c_int32, c_float, c_void_p,
+                                    c_void_p, c_int64, c_int32, c_int64, c_void_p]),
     "b200_linear_recurrence": (c_int32, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                                          c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
                                          c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p,

@@ -1044,12 +1044,11 @@ def attn_generic(q, k, v, spans: StepSpans, scale, num_kv_heads, vdim, block_tab
         raise ValueError("values inside the key rows: one kv head with vdim <= dim, or vdim == dim")
     out = torch.empty(T, H * vdim, dtype=q.dtype, device=q.device)
     cu_q, cu_k, ctx = spans.ptrs()
-    _C.check(_C.load().b200_attn_generic(out.data_ptr(), q.data_ptr(), q.stride(0) if T > 1 else H * dim,
-                                         k.data_ptr(), ks, _ptr(v), vs, bt_ptr, bt_stride, bs, cu_q, cu_k, ctx,
-                                         spans.num_seqs, spans.max_q, H, G, dim, vdim, float(scale), int(window),
-                                         int(keep_first), int(chunk), float(softcap), _ptr(sink), _ptr(gate),
-                                         (gate.stride(0) if T > 1 else H) if gate is not None else 0, _dt3(q),
-                                         _stream()), "b200_attn_generic")
+    _C.check(_C.load().b200_attn_generic_step(
+        out.data_ptr(), q.data_ptr(), q.stride(0) if T > 1 else H * dim, k.data_ptr(), ks, _ptr(v), vs, bt_ptr, bt_stride, bs, cu_q,
+        cu_k, ctx, spans.num_seqs, spans.max_q, H, G, dim, vdim, float(scale), int(window), int(keep_first), int(chunk),
+        float(softcap), _ptr(sink), _ptr(gate), (gate.stride(0) if T > 1 else H) if gate is not None else 0, _dt3(q), T,
+        _stream()), "b200_attn_generic_step")
     return out
 
 

@@ -1,0 +1,74 @@
+"""Prompt portions of ops.attn_generic in fp32 on the tensor cores (csrc/attn_split.cu): rows and keys around its 128-row and 64-key
+tiles, head sizes that are padded, sinks, gates, values inside the key rows, packed and paged keys, against a 64-bit evaluation;
+and values that three bf16 terms cannot carry. Tolerance: fp32 scores of a few units sum up to 128 products and enter an exponential."""
+import math
+
+import pytest
+import torch
+from test_attn_tiled_gpu import _want
+
+pytestmark = pytest.mark.gpu
+F64 = torch.float64
+
+
+def _run(H, G, dim, dv, spans, paged, sink=False, gate=False, latent=False, poke=None):
+    from nanovllm import ops
+    g = torch.Generator().manual_seed(dim * dv + H + len(spans))
+    rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    T = sum(n for n, _ in spans)
+    q, sk, gt = rnd(T, H, dim), rnd(H) if sink else None, rnd(T, H) if gate else None
+    ks = [rnd(m, G, dim) for _, m in spans]
+    vs = [k[:, :, :dv] if latent else rnd(m, G, dv) for k, (_, m) in zip(ks, spans)]
+    if poke:
+        poke(q, ks, vs)
+    cu = lambda i: torch.tensor([0] + [s[i] for s in spans]).cumsum(0).to(torch.int32).cuda()  # noqa: E731
+    sp = ops.StepSpans(cu(0), cu(1), None, max(n for n, _ in spans))
+    extra = dict(sink=None if sk is None else sk.cuda(), gate=None if gt is None else gt.cuda())
+    if paged:
+        need = [-(-m // paged) for _, m in spans]
+        order = torch.randperm(sum(need) + 2, generator=g).tolist()
+        table = torch.full((len(spans), max(need)), -1, dtype=torch.int32)
+        kc, vc = (torch.full((len(order), paged, G * n), math.nan) for n in (dim, dv))   # what no sequence owns is never used
+        for s, n in enumerate(need):
+            for b in range(n):
+                blk = order.pop()
+                table[s, b] = blk
+                for c, x in ((kc, ks), (vc, vs)):
+                    rows = x[s][b * paged:(b + 1) * paged]
+                    c[blk, :len(rows)] = rows.reshape(len(rows), -1)
+        got = ops.attn_generic(q.cuda(), kc.cuda(), vc.cuda(), sp, dim ** -0.5, G, dv, block_tables=table.cuda(), **extra)
+    else:
+        got = ops.attn_generic(q.cuda(), torch.cat(ks).cuda(), None if latent else torch.cat(vs).cuda(), sp, dim ** -0.5, G, dv, **extra)
+    at, out = 0, []
+    for s, (n, m) in enumerate(spans):
+        w = _want(q[at:at + n], ks[s], vs[s], m - n, dim ** -0.5, 0, 0, 0, 0.0, sk, None if gt is None else gt[at:at + n])
+        out.append((got[at:at + n].cpu().to(F64).view(n, H, dv), w))
+        at += n
+    return out
+
+
+@pytest.mark.parametrize("H,G,dim,dv,spans,paged,kw", [
+    (8, 2, 128, 128, [(32, 32), (33, 64), (65, 129), (1, 63)], 16, {}),
+    (2, 2, 64, 64, [(127, 127), (129, 192), (64, 65)], 0, dict(sink=True)),
+    (3, 3, 48, 48, [(130, 200)], 16, dict(gate=True)),
+    (6, 2, 20, 124, [(100, 100), (43, 300)], 64, dict(sink=True, gate=True)),
+    (5, 1, 128, 36, [(26, 26), (77, 90)], 0, dict(latent=True)),
+    (4, 1, 68, 128, [(64, 700)], 16, {}),
+])
+def test_against_64_bit(H, G, dim, dv, spans, paged, kw):
+    for s, (x, w) in enumerate(_run(H, G, dim, dv, spans, paged, **kw)):
+        assert float(((x - w).abs() / w.abs().clamp(min=1.0)).max()) < 2e-5, s
+
+
+@pytest.mark.parametrize("bad", [math.inf, -math.inf, math.nan, 1e-36])
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+def test_what_three_terms_cannot_carry(bad, where):
+    def poke(q, ks, vs):                                       # seen by the second half of the second sequence's rows
+        if where == "q":
+            q[200, 1, 5] = bad
+        else:
+            (ks if where == "k" else vs)[1][150, 0, 7] = bad
+    for s, (x, w) in enumerate(_run(4, 2, 64, 64, [(100, 100), (180, 200)], 16, poke=poke)):
+        fine = torch.isfinite(w)
+        assert torch.equal(torch.isfinite(x), fine), s
+        assert float(((x - w).abs() / w.abs().clamp(min=1.0))[fine].max()) < 2e-5, s
