@@ -38,12 +38,29 @@ struct DeltaParams {
   int H, groups, kdim, vdim;
 };
 
+// The sequence that `rank` of the `num` are longer than, of equal ones the first first. All threads of the CTA
+__device__ __forceinline__ int sequence_of_rank(const int* cu_q, int num, int rank) {
+  __shared__ int found;
+  for (int i = threadIdx.x; i < num; i += blockDim.x) {
+    const int own = cu_q[i + 1] - cu_q[i];
+    int before = 0;
+    for (int o = 0; o < num; ++o) {
+      const int len = cu_q[o + 1] - cu_q[o];
+      before += len > own || (len == own && o < i);
+    }
+    if (before == rank) found = i;
+  }
+  __syncthreads();
+  return __shfl_sync(0xffffffffu, found, 0);
+}
+
 __device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* gptr, bool pred) {
   const int bytes = pred ? 4 : 0;
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr), "l"(gptr), "r"(bytes) : "memory");
 }
 
-template <typename TV, int KPT, int NS, int NC, bool VEC, int MODE>
+// ORDER: CTAs start with the longest sequences (delta_launch_as)
+template <typename TV, int KPT, int NS, int NC, bool VEC, int MODE, bool ORDER = false>
 __global__ void __launch_bounds__(32 * NS)
 delta_rule_kernel(const DeltaParams P) {
   extern __shared__ __align__(16) float smem[];
@@ -52,7 +69,7 @@ delta_rule_kernel(const DeltaParams P) {
   constexpr int KS = KPT + 4;                        // slice stride: NS lanes, different banks
   constexpr int KP = NS * KS;                        // row of padded keys
   constexpr int CC = 32 * NC;                        // value columns per CTA
-  const int s = blockIdx.z, h = blockIdx.y;
+  const int s = ORDER ? sequence_of_rank(P.cu_q, gridDim.z, blockIdx.z) : blockIdx.z, h = blockIdx.y;
   const SeqSpan sp = seq_span(P.cu_q, P.cu_k, P.ctx_lens, s);
   if (sp.q_len == 0) return;
   const int kdim = P.kdim, vdim = P.vdim;
@@ -255,6 +272,19 @@ static void delta_launch_as(const DeltaParams& P, int num_seqs, cudaStream_t str
       cudaFuncSetAttribute(delta_rule_kernel<TV, KPT, NS, NC, true, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem);
       configured = true;
+    }
+    // Prompts that do not find an SM for every CTA start with the longest sequences: those share an SM with the shortest, and a token of
+    // a CTA that shares costs half as much again. States of 128 key rows alone: the others have room for more CTAs per SM.
+    if constexpr (KPT * NS == 128 && MODE != kWkv) {
+      if (P.cu_q != nullptr && num_seqs > 1 && num_seqs <= 32 && (int64_t)grid.x * grid.y * num_seqs > 148) {
+        static bool ordered = false;
+        if (!ordered && smem > 48 * 1024) {
+          cudaFuncSetAttribute(delta_rule_kernel<TV, KPT, NS, NC, true, MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          ordered = true;
+        }
+        launch_pdl(delta_rule_kernel<TV, KPT, NS, NC, true, MODE, true>, grid, dim3(32 * NS), smem, stream, P);
+        return;
+      }
     }
     launch_pdl(delta_rule_kernel<TV, KPT, NS, NC, true, MODE>, grid, dim3(32 * NS), smem, stream, P);
   } else {
