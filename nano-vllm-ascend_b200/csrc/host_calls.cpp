@@ -1,0 +1,171 @@
+// host_calls.cpp -- the attention entry points of ops.py as one native call each.
+//
+// A decode step of one row takes 12 us on the GPU and took 17 us of Python: 25 arguments through ctypes (3.6 us), some 35 tensor
+// attributes (4 us). Here the same attributes are looked at and the same library function is called without either. What ops.py
+// would refuse is not judged here: the functions return None for any argument that is not exactly what they expect, and ops.py goes its
+// own way, checks and errors included. An int is the library's status. Plain torch.Tensor only (subclasses, fake tensors and dispatch
+// modes take ops.py's way); nothing is kept between calls.
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <ATen/ATen.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include "../../include/b200attn.h"
+
+namespace {
+
+decltype(&b200_paged_decode_attn_windowed) g_decode = nullptr;
+decltype(&b200_paged_decode_attn_fp8) g_decode_fp8 = nullptr;
+decltype(&b200_prefill_varlen_attn_windowed) g_prefill = nullptr;
+
+// a plain CUDA tensor, or nullptr
+const at::Tensor* cuda_tensor(PyObject* o) {
+  if (!THPVariable_CheckExact(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !t.is_conj() ? &t : nullptr;
+}
+int element(const at::Tensor& t) {
+  return t.scalar_type() == at::kBFloat16 ? B200_DTYPE_BF16 : t.scalar_type() == at::kHalf ? B200_DTYPE_F16 : -1;
+}
+bool is_int(const at::Tensor& t) { return t.scalar_type() == at::kInt; }
+bool heads_fit(const at::Tensor& t, int64_t width) { return t.dim() == 3 && t.stride(2) == 1 && t.stride(1) == width; }
+// [blocks, block size, row] or [blocks, block size, heads, width], contiguous, with rows of `row` elements
+bool cache_fits(const at::Tensor& t, int64_t row) {
+  return (t.dim() == 3 || t.dim() == 4) && t.is_contiguous() && t.size(0) > 0 && t.size(1) > 0 &&
+         t.size(2) * (t.dim() == 4 ? t.size(3) : 1) == row;
+}
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+bool numbers(PyObject* const* a, int n) {
+  for (int i = 0; i < n; ++i) {
+    int over = 0;
+    if (PyLong_CheckExact(a[i])) PyLong_AsLongLongAndOverflow(a[i], &over);
+    else if (!PyFloat_CheckExact(a[i])) return false;
+    if (over != 0) return false;
+  }
+  return true;
+}
+// a number as int(x) and as float(x) give it
+int64_t whole(PyObject* o) { return PyLong_CheckExact(o) ? PyLong_AsLongLong(o) : (int64_t)PyFloat_AS_DOUBLE(o); }
+double real(PyObject* o) { return PyFloat_CheckExact(o) ? PyFloat_AS_DOUBLE(o) : PyLong_AsDouble(o); }
+
+PyObject* status(int rc, at::Tensor out) { return rc == B200_OK ? THPVariable_Wrap(std::move(out)) : PyLong_FromLong(rc); }
+
+// decode(workspace of ops.py, q, k_cache, v_cache, block_tables, context_lens, scale, num_kv_heads, num_ctas, softcap, window, keep_first,
+// chunk); decode_fp8 (.., num_ctas, k_scale, v_scale)
+template <bool FP8>
+PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != (FP8 ? 11 : 13) || !numbers(a + 6, (int)n - 6) || c10::impl::TorchDispatchModeTLS::any_modes_set()) Py_RETURN_NONE;
+  const at::Tensor *q = cuda_tensor(a[1]), *k = cuda_tensor(a[2]), *v = cuda_tensor(a[3]), *bt = cuda_tensor(a[4]), *lens = cuda_tensor(a[5]);
+  if (!q || !k || !v || !bt || !lens || element(*q) < 0 || q->dim() != 3) Py_RETURN_NONE;
+  const int64_t B = q->size(0), H = q->size(1), D = q->size(2), kv = whole(a[7]), ctas = whole(a[8]);
+  if (!heads_fit(*q, D) || !is_int(*bt) || !is_int(*lens) || bt->dim() != 2 || bt->stride(1) != 1 || !lens->is_contiguous()) Py_RETURN_NONE;
+  if (!cache_fits(*k, kv * D)) Py_RETURN_NONE;
+  if (FP8) {
+    for (const at::Tensor* c : {k, v})
+      if (c->scalar_type() != at::kByte && c->scalar_type() != at::kFloat8_e4m3fn) Py_RETURN_NONE;
+  }
+  PyObject* device = PyObject_GetAttrString(a[1], "device");
+  if (device == nullptr) return nullptr;
+  PyObject* held = PyObject_CallFunction(a[0], "LLLLO", (long long)B, (long long)H, (long long)kv, (long long)D, device);
+  Py_DECREF(device);
+  if (held == nullptr) return nullptr;
+  const at::Tensor* ws = cuda_tensor(held);
+  if (ws == nullptr) {
+    Py_DECREF(held);
+    Py_RETURN_NONE;
+  }
+  PyObject* got = nullptr;
+  try {
+    at::Tensor out = at::empty({B, H * D}, q->options());
+    const int64_t qs = B > 1 ? q->stride(0) : H * D;
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    if constexpr (FP8)
+      rc = g_decode_fp8(out.data_ptr(), q->data_ptr(), k->data_ptr(), v->data_ptr(), (const int32_t*)bt->data_ptr(),
+                        (const int32_t*)lens->data_ptr(), (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, qs, H * D, (int32_t)k->size(0),
+                        (int32_t)k->size(1), (int32_t)bt->stride(0), (float)real(a[6]), (float)real(a[9]), (float)real(a[10]),
+                        ws->data_ptr(), (size_t)ws->numel(), (int32_t)ctas, element(*q), stream());
+    else
+      rc = g_decode(out.data_ptr(), q->data_ptr(), k->data_ptr(), v->data_ptr(), (const int32_t*)bt->data_ptr(),
+                    (const int32_t*)lens->data_ptr(), (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, (int32_t)D, qs, H * D,
+                    (int32_t)k->size(0), (int32_t)k->size(1), (int32_t)bt->stride(0), (float)real(a[6]), (float)real(a[9]), nullptr,
+                    (int32_t)whole(a[10]), (int32_t)whole(a[11]), (int32_t)whole(a[12]), ws->data_ptr(), (size_t)ws->numel(), (int32_t)ctas,
+                    element(*q), stream());
+    Py_END_ALLOW_THREADS
+    got = status(rc, std::move(out));
+  } catch (...) {
+    Py_DECREF(held);
+    throw;
+  }
+  Py_DECREF(held);
+  return got;
+  END_HANDLE_TH_ERRORS
+}
+
+// prefill(workspace tensor or None, q, k, v, cu_seqlens_q, cu_seqlens_k, block_tables or None, max_seqlen_q, max_seqlen_k, scale, num_kv_heads,
+// softcap, sink or None, window, keep_first, chunk)
+PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 16 || !numbers(a + 7, 5) || !numbers(a + 13, 3) || c10::impl::TorchDispatchModeTLS::any_modes_set()) Py_RETURN_NONE;
+  const bool paged = a[6] != Py_None;
+  const at::Tensor *q = cuda_tensor(a[1]), *k = cuda_tensor(a[2]), *v = cuda_tensor(a[3]), *cq = cuda_tensor(a[4]), *ck = cuda_tensor(a[5]),
+                   *bt = paged ? cuda_tensor(a[6]) : nullptr, *ws = a[0] != Py_None ? cuda_tensor(a[0]) : nullptr,
+                   *sink = a[12] != Py_None ? cuda_tensor(a[12]) : nullptr;
+  if (!q || !k || !v || !cq || !ck || (paged && !bt) || (a[0] != Py_None && !ws) || (a[12] != Py_None && !sink)) Py_RETURN_NONE;
+  if (element(*q) < 0 || q->dim() != 3 || !is_int(*cq) || !is_int(*ck)) Py_RETURN_NONE;
+  const int64_t T = q->size(0), H = q->size(1), D = q->size(2), kv = whole(a[10]);
+  if (!heads_fit(*q, D)) Py_RETURN_NONE;
+  if (sink && (sink->numel() != H || sink->scalar_type() != at::kFloat || !sink->is_contiguous())) Py_RETURN_NONE;
+  int64_t ks = kv * D, vs = kv * D, nb = 0, bs = 0, total_k = 0;
+  if (paged) {
+    if (!is_int(*bt) || bt->dim() != 2 || bt->stride(1) != 1 || !cache_fits(*k, kv * D) || !cache_fits(*v, kv * D)) Py_RETURN_NONE;
+    nb = k->size(0), bs = k->size(1);
+  } else {
+    if (!heads_fit(*k, D) || !heads_fit(*v, D)) Py_RETURN_NONE;
+    total_k = k->size(0);
+    if (k->size(0) > 1) ks = k->stride(0);
+    if (v->size(0) > 1) vs = v->stride(0);
+  }
+  at::Tensor out = at::empty({T, H * D}, q->options());
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = g_prefill(out.data_ptr(), q->data_ptr(), k->data_ptr(), v->data_ptr(), (const int32_t*)cq->data_ptr(), (const int32_t*)ck->data_ptr(),
+                 (int32_t)(cq->numel() - 1), (int32_t)T, (int32_t)total_k, (int32_t)whole(a[7]), (int32_t)whole(a[8]), (int32_t)H,
+                 (int32_t)kv, (int32_t)D, (int32_t)D, T > 1 ? q->stride(0) : H * D, ks, vs, H * D,
+                 paged ? (const int32_t*)bt->data_ptr() : nullptr, paged ? (int32_t)bt->stride(0) : 0, (int32_t)nb, (int32_t)bs,
+                 (float)real(a[9]), (float)real(a[11]), sink ? (const float*)sink->data_ptr() : nullptr, (int32_t)whole(a[13]),
+                 (int32_t)whole(a[14]), (int32_t)whole(a[15]), element(*q), ws ? ws->data_ptr() : nullptr, ws ? ws->numel() : 0, stream());
+  Py_END_ALLOW_THREADS
+  return status(rc, std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// bind(addresses of the three library functions)
+PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 3) {
+    PyErr_SetString(PyExc_TypeError, "bind takes three addresses");
+    return nullptr;
+  }
+  void* p[3];
+  for (int i = 0; i < 3; ++i)
+    if ((p[i] = PyLong_AsVoidPtr(a[i])) == nullptr) {
+      if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address");
+      return nullptr;
+    }
+  g_decode = (decltype(g_decode))p[0], g_decode_fp8 = (decltype(g_decode_fp8))p[1], g_prefill = (decltype(g_prefill))p[2];
+  Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"decode", (PyCFunction)(void (*)())decode<false>, METH_FASTCALL, nullptr},
+    {"decode_fp8", (PyCFunction)(void (*)())decode<true>, METH_FASTCALL, nullptr},
+    {"prefill", (PyCFunction)(void (*)())prefill, METH_FASTCALL, nullptr},
+    {"bind", (PyCFunction)(void (*)())bind, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_b200calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__b200calls() { return PyModule_Create(&module); }

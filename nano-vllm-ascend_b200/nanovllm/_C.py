@@ -264,6 +264,27 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_calls = None
+
+
+def calls():
+    """The native calls of the attention entry points (csrc/host_calls.cpp), bound to the library's functions."""
+    global _calls
+    if _calls is None:
+        import importlib.util
+        path = os.path.join(os.path.dirname(DEFAULT_LIB_PATH), "_b200calls.so")
+        if not os.path.exists(path):
+            raise B200Error(f"_b200calls.so not found at {path}: build it as libb200attn.so is built")
+        spec = importlib.util.spec_from_file_location("_b200calls", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        lib = load()
+        module.bind(*(ctypes.cast(f, c_void_p).value for f in (lib.b200_paged_decode_attn_windowed, lib.b200_paged_decode_attn_fp8,
+                                                               lib.b200_prefill_varlen_attn_windowed)))
+        _calls = module
+    return _calls
+
+
 def check(code: int, what: str) -> None:
     if code != 0:
         msg = load().b200_error_string(code).decode()

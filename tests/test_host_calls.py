@@ -1,0 +1,81 @@
+"""The native calls of ops' attention entry points (csrc/host_calls.cpp): what they take gives what ops' own way gives, bit for bit; what they
+do not take is left to ops' own checks."""
+import pytest
+import torch
+
+
+def test_nothing_but_cuda_tensors_and_numbers():
+    from nanovllm import _C, ops
+    calls, t = _C.calls(), torch.zeros(1, 16, 128, dtype=torch.bfloat16)
+    never = lambda *a: pytest.fail("asked for a workspace")  # noqa: E731
+    assert calls.decode(never, t, t, t, t, t, 1.0, 8, 0, 0.0, 0, 0, 0) is None            # CPU tensors
+    assert calls.decode_fp8(never, t, t, t, t, t, 1.0, 8, 0, 1.0, 1.0) is None
+    assert calls.prefill(None, t, t, t, t, t, None, 1, 1, 1.0, 8, 0.0, None, 0, 0, 0) is None
+    assert calls.decode(never, t, t, t, t, t, "1", 8, 0, 0.0, 0, 0, 0) is None            # not numbers
+    assert calls.decode(never, t, t, t, t, t, 1.0, 1 << 70, 0, 0.0, 0, 0, 0) is None
+    assert calls.decode(never, 1, 2, 3, 4, 5, 1.0, 8, 0, 0.0, 0, 0, 0) is None            # not tensors
+    assert calls.decode() is None and calls.prefill() is None
+    with pytest.raises(RuntimeError, match="CUDA only"):
+        ops.paged_decode_attn(t, t, t, t, t, 1.0, 8)
+
+
+def _step(dtype=torch.bfloat16, fp8=False, B=3, H=8, G=2, D=64, bs=16):
+    g = torch.Generator(device="cuda").manual_seed(B)
+    q = torch.randn(B, H + 2, D, device="cuda", generator=g).to(dtype)[:, :H]             # a token-strided view
+    k, v = (torch.randn(40, bs, G * D, device="cuda", generator=g).to(dtype) for _ in range(2))
+    if fp8:
+        k, v = k.to(torch.float8_e4m3fn), v.to(torch.float8_e4m3fn).view(torch.uint8)
+    tables = torch.randperm(40, device="cuda", generator=g)[:B * 10].view(B, 10).to(torch.int32)
+    return q, k, v, tables, torch.tensor([150, 1, 77], dtype=torch.int32, device="cuda")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_decode_is_the_same_either_way(dtype):
+    from nanovllm import _C, ops
+    q, k, v, tables, lens = _step(dtype)
+    for kw in ({}, dict(window=20, keep_first=3), dict(chunk=32), dict(softcap=5), dict(num_ctas=64)):
+        got = ops.paged_decode_attn(q, k, v, tables, lens, 0.125, 2, **kw)
+        want = ops.paged_decode_attn(q, k, v, tables, lens, 0.125, 2, out=torch.empty_like(got), **kw)
+        assert torch.equal(got, want) and got.dtype == dtype and got.shape == (3, 512), kw
+    k4 = k.view(40, 16, 2, 64)
+    assert torch.equal(ops.paged_decode_attn(q, k4, v, tables, lens, 0.125, 2), ops.paged_decode_attn(q, k, v, tables, lens, 0.125, 2))
+    q8, k8, v8 = _step(dtype, fp8=True)[:3]
+    got = ops.paged_decode_attn_fp8(q8, k8, v8, tables, lens, 0.125, 2, 0.5, 2.0)
+    assert torch.equal(got, ops.paged_decode_attn_fp8(q8, k8, v8, tables, lens, 0.125, 2, 0.5, 2.0, out=torch.empty_like(got)))
+    with pytest.raises(TypeError):
+        ops.paged_decode_attn(q, k, v, tables.long(), lens, 0.125, 2)
+    with pytest.raises(ValueError):
+        ops.paged_decode_attn(q, k[:, :, :64], v, tables, lens, 0.125, 2)
+    with pytest.raises(TypeError):
+        ops.paged_decode_attn(q.float(), k, v, tables, lens, 0.125, 2)
+    with pytest.raises(TypeError):
+        ops.paged_decode_attn_fp8(q8, k, v, tables, lens, 0.125, 2)
+    with pytest.raises(_C.B200Error):
+        ops.paged_decode_attn(q[:, :3], k, v, tables, lens, 0.125, 2)                     # 3 heads over 2
+
+
+@pytest.mark.gpu
+def test_prompts_are_the_same_either_way():
+    from nanovllm import ops
+    g = torch.Generator(device="cuda").manual_seed(1)
+    T, H, G, D = 90, 4, 2, 64
+    qkv = torch.randn(T, (H + 2 * G) * D, device="cuda", generator=g).bfloat16()
+    q, k, v = (x.unflatten(1, (-1, D)) for x in qkv.split([H * D, G * D, G * D], dim=1))
+    cu = torch.tensor([0, 33, 90], dtype=torch.int32, device="cuda")
+    sink = torch.randn(H, device="cuda", generator=g)
+    for kw in ({}, dict(sink=sink, softcap=20.0), dict(window=16, keep_first=2), dict(chunk=24), dict(workspace=None)):
+        got = ops.prefill_varlen_attn(q, k, v, cu, cu, 57, 57, 0.125, G, **kw)
+        assert torch.equal(got, ops.prefill_varlen_attn(q, k, v, cu, cu, 57, 57, 0.125, G, out=torch.empty_like(got), **kw)), kw
+    one = ops.prefill_varlen_attn(q[:1], k[:1], v[:1], cu[:1].repeat(2) + torch.tensor([0, 1], dtype=torch.int32, device="cuda"),
+                                  torch.tensor([0, 1], dtype=torch.int32, device="cuda"), 1, 1, 0.125, G)
+    assert torch.allclose(one.view(H, D).float(), v[0].repeat_interleave(H // G, 0).float(), atol=1e-2)
+    cache = torch.randn(12, 16, G * D, device="cuda", generator=g).bfloat16()
+    table = torch.randperm(12, device="cuda", generator=g).view(2, 6).to(torch.int32)
+    ck = torch.tensor([0, 60, 150], dtype=torch.int32, device="cuda")
+    got = ops.prefill_varlen_attn(q, cache, cache, cu, ck, 57, 90, 0.125, G, block_tables=table)
+    assert torch.equal(got, ops.prefill_varlen_attn(q, cache, cache, cu, ck, 57, 90, 0.125, G, block_tables=table, out=torch.empty_like(got)))
+    with pytest.raises(TypeError):
+        ops.prefill_varlen_attn(q, k, v, cu.long(), cu, 57, 57, 0.125, G)
+    with pytest.raises(ValueError):
+        ops.prefill_varlen_attn(q, k.transpose(0, 1).contiguous().transpose(0, 1), v, cu, cu, 57, 57, 0.125, G)
