@@ -25,6 +25,8 @@
 //            d = 16c+2g and d = 16c+2g+1. A lane therefore ends up owning the 4 consecutive
 //            outputs d = 16c + 4t4 + {0,1,2,3} of every 16-wide column group c.
 //  * k_scale is folded into the softmax scale, v_scale into the final normalisation.
+#include <type_traits>
+
 #include "decode_common.cuh"
 
 namespace b200 {
@@ -259,97 +261,134 @@ paged_decode_fp8_kernel(const __grid_constant__ CUtensorMap tmK,
     for (int n = 0; n < NT; ++n) o_acc[n][0] = o_acc[n][1] = o_acc[n][2] = o_acc[n][3] = 0.f;
     float m_run = -INFINITY, l_run = 0.f;
 
-    for (int j = j0; j < j1; ++j) {
-      const int tok0 = j * TILE_TOKENS + tok_off;  // first token of this warp's unit
-      const bool active = tok0 < len;
-      mbar_wait(&full_k[stage], phase);
-      if (active) {
-        const uint32_t kb = smem_u32(kbuf + stage * TILE_BYTES) + unit_base;
-        float s[2][4];
-        uint32_t kw[2][KSTEPS];     // token rows g (n = 0) and g + 8 (n = 1): word ks feeds MMA step ks
+    // W tiles j .. j + W - 1 of the item at a time. A warp's way through a tile is one chain (copy -> de-quantise -> scores -> maximum ->
+    // weights -> de-quantise -> outputs) with two warps per scheduler: two tiles together are two chains through most of it, and one
+    // maximum and one rescale for both. Only the item's last tile can be short of tokens. For heads of 64 (us, one tile at a time / two: 64
+    // rows of 100-2048 tokens, 32 heads over 8, 29.5 / 27.4, 32 of 1000-2000 22.5 / 20.9); the registers of 128 do not go round (24 words
+    // spilled: 8 rows of 500-1500 13.2 / 14.1).
+    auto take = [&](int j, auto tiles) {
+      constexpr int W = decltype(tiles)::value;
+      int st[W], ph[W];
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
-          s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
-          const uint32_t rowaddr = kb + (n * 8 + g) * 128;
+      for (int w = 0; w < W; ++w) {
+        st[w] = stage, ph[w] = phase;
+        if (++stage == kStagesQ8) stage = 0, phase ^= 1;
+      }
+      const int valid = len - ((j + W - 1) * TILE_TOKENS + tok_off);  // tokens of this warp's unit in the last of the tiles
+      const bool active = valid > 0;
+      uint32_t kw[W][2][KSTEPS];    // token rows g (n = 0) and g + 8 (n = 1): word ks feeds MMA step ks
 #pragma unroll
-          for (int i = 0; i < KSTEPS / 4; ++i) {
-            const uint4 x = lds128(rowaddr + (((k_c16 + i) ^ g) << 4));
-            kw[n][4 * i] = x.x, kw[n][4 * i + 1] = x.y, kw[n][4 * i + 2] = x.z, kw[n][4 * i + 3] = x.w;
+      for (int w = 0; w < W; ++w) {
+        mbar_wait(&full_k[st[w]], ph[w]);
+        if (w < W - 1 || active) {
+          const uint32_t kb = smem_u32(kbuf + st[w] * TILE_BYTES) + unit_base;
+#pragma unroll
+          for (int n = 0; n < 2; ++n) {
+            const uint32_t rowaddr = kb + (n * 8 + g) * 128;
+#pragma unroll
+            for (int i = 0; i < KSTEPS / 4; ++i) {
+              const uint4 x = lds128(rowaddr + (((k_c16 + i) ^ g) << 4));
+              kw[w][n][4 * i] = x.x, kw[w][n][4 * i + 1] = x.y, kw[w][n][4 * i + 2] = x.z, kw[w][n][4 * i + 3] = x.w;
+            }
           }
         }
+      }
+      if (W > 1 || active) {
+        float s[W][2][4];
 #pragma unroll
-        for (int ks = 0; ks < KSTEPS; ++ks) {   // the two accumulator chains interleave
+        for (int w = 0; w < W; ++w)
 #pragma unroll
-          for (int n = 0; n < 2; ++n)
-            mma_16816<__half>(s[n], qa[ks][0], 0u, qa[ks][1], 0u, e4m3x2_to_f16x2(kw[n][ks] & 0xffffu),
-                              e4m3x2_to_f16x2(kw[n][ks] >> 16));
+          for (int n = 0; n < 2; ++n) s[w][n][0] = s[w][n][1] = s[w][n][2] = s[w][n][3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < KSTEPS; ++ks) {   // the accumulator chains interleave
+#pragma unroll
+          for (int w = 0; w < W; ++w)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+              if (w < W - 1 || active)
+                mma_16816<__half>(s[w][n], qa[ks][0], 0u, qa[ks][1], 0u, e4m3x2_to_f16x2(kw[w][n][ks] & 0xffffu),
+                                  e4m3x2_to_f16x2(kw[w][n][ks] >> 16));
         }
         // mask tokens beyond the context (only the last tile of a sequence)
-        const int valid = len - tok0;  // > 0
         if (valid < 16) {
 #pragma unroll
           for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int e = 0; e < 2; ++e)
-              if (n * 8 + 2 * t4 + e >= valid) s[n][e] = -INFINITY;
+              if (n * 8 + 2 * t4 + e >= valid) s[W - 1][n][e] = -INFINITY;
         }
         // online softmax for row g (rows 8..15 are padding)
-        float mx = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
+        float mx = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < W; ++w) mx = fmaxf(mx, fmaxf(fmaxf(s[w][0][0], s[w][0][1]), fmaxf(s[w][1][0], s[w][1][1])));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         const float m_new = fmaxf(m_run, mx);
         const float alpha = ex2_approx((m_run - m_new) * sl2);
         const float mb = m_new * sl2;
-        const float p00 = ex2_approx(fmaf(s[0][0], sl2, -mb));
-        const float p01 = ex2_approx(fmaf(s[0][1], sl2, -mb));
-        const float p10 = ex2_approx(fmaf(s[1][0], sl2, -mb));
-        const float p11 = ex2_approx(fmaf(s[1][1], sl2, -mb));
-        l_run = fmaf(l_run, alpha, (p00 + p01) + (p10 + p11));
+        l_run *= alpha;
+        uint32_t pa0[W], pa2[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const float p00 = ex2_approx(fmaf(s[w][0][0], sl2, -mb));
+          const float p01 = ex2_approx(fmaf(s[w][0][1], sl2, -mb));
+          const float p10 = ex2_approx(fmaf(s[w][1][0], sl2, -mb));
+          const float p11 = ex2_approx(fmaf(s[w][1][1], sl2, -mb));
+          l_run += (p00 + p01) + (p10 + p11);
+          pa0[w] = pack2<__half>(p00, p01), pa2[w] = pack2<__half>(p10, p11);
+        }
         m_run = m_new;
         if (alpha != 1.f) {
 #pragma unroll
           for (int n = 0; n < NT; ++n) o_acc[n][0] *= alpha, o_acc[n][1] *= alpha;
         }
-        const uint32_t pa0 = pack2<__half>(p00, p01), pa2 = pack2<__half>(p10, p11);
-
-        mbar_wait(&full_v[stage], phase);
-        uint8_t* vstage = vbuf + stage * TILE_BYTES + unit_base;
-        if (valid < 16) {
-          // rows past the context hold stale cache bytes (0x7f/0xff decode to NaN): zero this
-          // head's bytes of those rows so that 0 * garbage cannot poison the accumulator.
-          const int nz = (16 - valid) * NC;
-          for (int idx = lane; idx < nz; idx += 32) {
-            const int row = valid + idx / NC;
-            const int c = hb16 + idx % NC;
-            *reinterpret_cast<uint4*>(vstage + row * 128 + ((c ^ (row & 7)) << 4)) =
-                make_uint4(0, 0, 0, 0);
-          }
-          __syncwarp();
-        }
-        const uint32_t vb = smem_u32(vstage) + v_tok * 128;
 #pragma unroll
-        for (int jp = 0; jp < D / 32; ++jp) {
-          uint32_t r0_, r1_, r2_, r3_;
-          ldsm_x4_trans(vb + (((hb16 + 2 * jp + v_dc) ^ (v_tok & 7)) << 4), r0_, r1_, r2_, r3_);
-          const uint32_t e0 = __byte_perm(r0_, r1_, 0x6420), o0 = __byte_perm(r0_, r1_, 0x7531);
-          const uint32_t e1 = __byte_perm(r2_, r3_, 0x6420), o1 = __byte_perm(r2_, r3_, 0x7531);
-          mma_16816<__half>(o_acc[4 * jp + 0], pa0, 0u, pa2, 0u, e4m3x2_to_f16x2(e0 & 0xffffu),
-                            e4m3x2_to_f16x2(e0 >> 16));
-          mma_16816<__half>(o_acc[4 * jp + 1], pa0, 0u, pa2, 0u, e4m3x2_to_f16x2(o0 & 0xffffu),
-                            e4m3x2_to_f16x2(o0 >> 16));
-          mma_16816<__half>(o_acc[4 * jp + 2], pa0, 0u, pa2, 0u, e4m3x2_to_f16x2(e1 & 0xffffu),
-                            e4m3x2_to_f16x2(e1 >> 16));
-          mma_16816<__half>(o_acc[4 * jp + 3], pa0, 0u, pa2, 0u, e4m3x2_to_f16x2(o1 & 0xffffu),
-                            e4m3x2_to_f16x2(o1 >> 16));
+        for (int w = 0; w < W; ++w) {
+          mbar_wait(&full_v[st[w]], ph[w]);
+          if (w == W - 1 && !active) continue;
+          uint8_t* vstage = vbuf + st[w] * TILE_BYTES + unit_base;
+          if (w == W - 1 && valid < 16) {
+            // rows past the context hold stale cache bytes (0x7f/0xff decode to NaN): zero this
+            // head's bytes of those rows so that 0 * garbage cannot poison the accumulator.
+            const int nz = (16 - valid) * NC;
+            for (int idx = lane; idx < nz; idx += 32) {
+              const int row = valid + idx / NC;
+              const int c = hb16 + idx % NC;
+              *reinterpret_cast<uint4*>(vstage + row * 128 + ((c ^ (row & 7)) << 4)) =
+                  make_uint4(0, 0, 0, 0);
+            }
+            __syncwarp();
+          }
+          const uint32_t vb = smem_u32(vstage) + v_tok * 128;
+#pragma unroll
+          for (int jp = 0; jp < D / 32; ++jp) {
+            uint32_t r0_, r1_, r2_, r3_;
+            ldsm_x4_trans(vb + (((hb16 + 2 * jp + v_dc) ^ (v_tok & 7)) << 4), r0_, r1_, r2_, r3_);
+            const uint32_t e0 = __byte_perm(r0_, r1_, 0x6420), o0 = __byte_perm(r0_, r1_, 0x7531);
+            const uint32_t e1 = __byte_perm(r2_, r3_, 0x6420), o1 = __byte_perm(r2_, r3_, 0x7531);
+            mma_16816<__half>(o_acc[4 * jp + 0], pa0[w], 0u, pa2[w], 0u, e4m3x2_to_f16x2(e0 & 0xffffu),
+                              e4m3x2_to_f16x2(e0 >> 16));
+            mma_16816<__half>(o_acc[4 * jp + 1], pa0[w], 0u, pa2[w], 0u, e4m3x2_to_f16x2(o0 & 0xffffu),
+                              e4m3x2_to_f16x2(o0 >> 16));
+            mma_16816<__half>(o_acc[4 * jp + 2], pa0[w], 0u, pa2[w], 0u, e4m3x2_to_f16x2(e1 & 0xffffu),
+                              e4m3x2_to_f16x2(e1 >> 16));
+            mma_16816<__half>(o_acc[4 * jp + 3], pa0[w], 0u, pa2[w], 0u, e4m3x2_to_f16x2(o1 & 0xffffu),
+                              e4m3x2_to_f16x2(o1 >> 16));
+          }
+          if (w == W - 1 && valid < 16) fence_proxy_async_smem();
         }
-        if (valid < 16) fence_proxy_async_smem();
       } else {
-        mbar_wait(&full_v[stage], phase);
+        mbar_wait(&full_v[st[0]], ph[0]);
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[stage]);
-      if (++stage == kStagesQ8) stage = 0, phase ^= 1;
-    }
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        if (lane == 0) mbar_arrive(&empty[st[w]]);
+    };
+    int j = j0;
+    if constexpr (D == 64)
+      for (; j + 2 <= j1; j += 2) take(j, std::integral_constant<int, 2>{});
+    for (; j < j1; ++j) take(j, std::integral_constant<int, 1>{});
 
     // ---- finalise this segment. Lane (g, t4) owns, for every 16-wide column group c, the four
     // consecutive outputs d = 16c + 4t4 + {0,1,2,3} = {o_acc[2c][0], o_acc[2c+1][0], o_acc[2c][1],
