@@ -470,12 +470,14 @@ static int moe_sm_count() {
   return sms;
 }
 
-// The persistent kernel where its 256-column bands divide the output and full row tiles alone give every SM a tile; fewer
-// tiles than SMs leave it with idle SMs and one cold ring per tile, where the 128-column kernels (two CTAs per SM or a deep
-// ring) are the better ones. fp32 outputs (attention scores) stay there as well.
-static bool moe_umma_wide(bool gate_up, int pairs, int n_out, int out_f32) {
+// The persistent kernel where its 256-column bands divide the output and every SM can expect a tile: full row tiles, or one of every
+// expert where they have 16 rows on average (a layer of 128 experts, 2048 x 768, top 8, 256 tokens: 359 us with the 128-column
+// kernels, 209 so). Fewer tiles than SMs leave it with idle SMs and one cold ring per tile, where the
+// 128-column kernels (two CTAs per SM or a deep ring) are the better ones. fp32 outputs (attention scores) stay there as well.
+static bool moe_umma_wide(bool gate_up, int pairs, int num_local, int n_out, int out_f32) {
   const int band = gate_up ? 128 : 256;
-  return !out_f32 && n_out % band == 0 && (long long)(pairs / 128) * (n_out / band) >= moe_sm_count();
+  const int row_tiles = num_local > 1 && pairs / 16 >= num_local && num_local > pairs / 128 ? num_local : pairs / 128;
+  return !out_f32 && n_out % band == 0 && (long long)row_tiles * (n_out / band) >= moe_sm_count();
 }
 
 template <typename T, bool kGateUp, int kStages>
@@ -558,7 +560,7 @@ static int moe_umma_common(bool gate_up, void* out, const void* a, const void* w
   int rc = get_panel_map(a, pairs, (int64_t)K * 2, K / 64, 128, 1, dtype, &ma);
   if (rc != B200_OK) return rc;
   const int64_t w_rows = (int64_t)num_local * (gate_up ? 2 : 1) * n_out;
-  const bool wide = moe_umma_wide(gate_up, pairs, n_out, out_f32);
+  const bool wide = moe_umma_wide(gate_up, pairs, num_local, n_out, out_f32);
   rc = get_panel_map(w, w_rows, (int64_t)K * 2, K / 64, wide ? 128 : 64, 1, dtype, &mw);
   if (rc != B200_OK) return rc;
   MoeUmmaParams p{offsets, sorted_pair, pair_scale, out, num_local, K, n_out, out_f32, in_scale, wait_ns, wait_status()};

@@ -559,7 +559,7 @@ def moe_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_ids: 
     pairs = T * k
     lib = _C.load()
     in_w, out_w = (topk_weights, None) if weigh_input else (None, topk_weights)
-    if _MOE_BIG_GEMM != "stream" and pairs >= _MOE_BIG_GEMM_ROWS * n_local:
+    if _MOE_BIG_GEMM != "stream" and pairs >= _moe_big_rows(n_local, hidden * inter) * n_local:
         big = _moe_expert_gemms_umma if _MOE_BIG_GEMM == "umma" else _moe_expert_gemms_library
         y = big(x, w13, w2, out_w, plan, in_w)
         return _moe_combine(lib, y, topk_ids, plan, T, hidden, out, x)
@@ -575,16 +575,28 @@ def moe_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_ids: 
     return _moe_combine(lib, y, topk_ids, plan, T, hidden, out, x)
 
 
-# Prefill-sized batches (hundreds of rows per expert) are tensor-bound, not weight-streaming: from
-# _MOE_BIG_GEMM_ROWS average rows per local expert on they go through the tcgen05 grouped GEMMs of
-# csrc/moe_umma.cu. The line dates from the 128-column kernel alone and is a safe one: with the kernels as they are,
-# a layer takes (us, weight-streaming / tcgen05, by rows per expert; hidden 2048, inter 768, 128 experts) 16: 213 / 359,
-# 32: 241 / 221, 48: 324 / 227, 64: 386 / 235, 96: 518 / 248, 192: 951 / 386; (hidden 1024, inter 512, 16 experts) 16: 23 / 25,
-# 32: 27 / 25, 64: 50 / 25, 96: 60 / 27; (2048, 1024, 16) 16: 46 / 56, 32: 60 / 57, 64: 90 / 60, 96: 110 / 61. Module attributes, not
-# environment switches: "stream" forces the weight-streaming kernel for every size, "library" routes
-# through torch._grouped_mm (comparator for tools/moe_diag.py and the tests).
+# Batches of many rows per expert go through the tcgen05 grouped GEMMs of csrc/moe_umma.cu instead of the weight-streaming ones.
+# Module attributes, not environment switches: "stream" forces the weight-streaming kernel for every size, "library" routes
+# through torch._grouped_mm (comparator for tools/moe_diag.py and the tests); _MOE_BIG_GEMM_ROWS, if set, is the line in average rows
+# per local expert.
 _MOE_BIG_GEMM = "umma"
-_MOE_BIG_GEMM_ROWS = 96
+_MOE_BIG_GEMM_ROWS = None
+_MOE_OTHER_BIG_ROWS = 96            # experts without a gate and with the clamped unit: measured at prefill sizes only
+
+
+def _moe_big_rows(n_local: int, weights: int) -> int:
+    """The line for gated experts of `weights` = hidden x inter. A layer takes (us, weight-streaming / tcgen05, by rows per expert)
+      2048 x 768, 128 experts  16: 218 / 209, 24: 230 / 216, 32: 257 / 222, 64: 401 / 239, 95: 527 / 259
+      2048 x 768, 64           16: 125 / 117, 32: 148 / 120, 64: 227 / 130
+      1024 x 512, 64           16: 55 / 58, 20: 56.5 / 58.5, 24: 62 / 59, 32: 69 / 60, 64: 99 / 63
+      1024 x 512, 16           16: 26.7 / 28.2, 24: 29.5 / 29.2, 32: 33.5 / 29.2, 64: 46 / 30
+      2048 x 1024, 16          24: 55 / 62, 28: 60 / 62, 32: 64 / 62, 64: 96 / 64
+    Many experts fill the chip with a 128-row tile each, however few rows it has; below 16 rows the 128-column kernels would run."""
+    if _MOE_BIG_GEMM_ROWS is not None:
+        return _MOE_BIG_GEMM_ROWS
+    if n_local < 64:
+        return 32
+    return 16 if weights >= 1 << 20 else 24
 
 
 def _moe_expert_gemms_umma(x, w13, w2, topk_weights, plan: MoePlan, in_weights=None) -> torch.Tensor:
@@ -632,7 +644,7 @@ def moe_experts_ungated(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, top
     lib = _C.load()
     h = torch.empty(pairs, inter, dtype=x.dtype, device=x.device)
     y = torch.empty(pairs, hidden, dtype=x.dtype, device=x.device)
-    if _MOE_BIG_GEMM != "stream" and pairs >= _MOE_BIG_GEMM_ROWS * E:
+    if _MOE_BIG_GEMM != "stream" and pairs >= (_MOE_OTHER_BIG_ROWS if _MOE_BIG_GEMM_ROWS is None else _MOE_BIG_GEMM_ROWS) * E:
         xs = torch.empty(pairs, hidden, dtype=x.dtype, device=x.device)
         _C.check(lib.b200_moe_gather_rows(xs.data_ptr(), x.data_ptr(), plan.offsets.data_ptr(),
                                           plan.sorted_pair.data_ptr(), pairs, E, k, hidden,
@@ -676,7 +688,7 @@ def moe_experts_glu_clamped(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor
     pairs = T * k
     lib = _C.load()
     y = torch.empty(pairs, hidden, dtype=x.dtype, device=x.device)
-    if _MOE_BIG_GEMM == "stream" or pairs < _MOE_BIG_GEMM_ROWS * E:
+    if _MOE_BIG_GEMM == "stream" or pairs < (_MOE_OTHER_BIG_ROWS if _MOE_BIG_GEMM_ROWS is None else _MOE_BIG_GEMM_ROWS) * E:
         h = torch.empty(pairs, inter, dtype=x.dtype, device=x.device)
         _C.check(lib.b200_moe_gemm_gate_up_glu(h.data_ptr(), x.data_ptr(), w13.data_ptr(), plan.offsets.data_ptr(),
                                                plan.sorted_pair.data_ptr(), hidden, inter, E, k,

@@ -1,0 +1,36 @@
+"""ops.moe_experts on both sides of the line between the weight-streaming and the tcgen05 grouped kernels (ops._moe_big_rows), with experts of
+few and of no rows: plain fp32 experts, and the other kernels' answer."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("experts,top,hidden,inter,rows", [(64, 4, 1024, 1024, 15), (64, 4, 1024, 1024, 16), (64, 4, 128, 256, 23), (64, 4, 128, 256, 24),
+                                                           (8, 2, 256, 256, 31), (8, 2, 256, 256, 32)])
+@pytest.mark.parametrize("skewed", [False, True])
+def test_both_sides_of_the_line(experts, top, hidden, inter, rows, skewed, monkeypatch):
+    from nanovllm import ops
+    assert ops._moe_big_rows(experts, hidden * inter) in (rows, rows + 1)
+    T = rows * experts // top
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    x, logits = rand(T, hidden).bfloat16(), rand(T, experts)
+    if skewed:                                                 # a few experts take nearly all rows, many none
+        logits[:, :top + 1] += 8
+    w13, w2 = (rand(experts, 2 * inter, hidden) * hidden ** -0.5).bfloat16(), (rand(experts, hidden, inter) * inter ** -0.5).bfloat16()
+    ids, weights = ops.moe_route(logits.bfloat16(), top)
+    plan = ops.moe_align(ids, 0, experts)
+    got = ops.moe_experts(x, w13, w2, ids, weights, plan).float()
+    monkeypatch.setattr(ops, "_MOE_BIG_GEMM_ROWS", 1 << 30 if rows % 2 == 0 else 1)
+    other = ops.moe_experts(x, w13, w2, ids, weights, plan).float()
+    want = torch.zeros(T, hidden, device="cuda")
+    for e in range(experts):
+        t, j = (ids == e).nonzero(as_tuple=True)
+        if t.numel():
+            h = (x[t].float() @ w13[e].float().T).bfloat16().float()
+            h = (torch.nn.functional.silu(h[:, :inter]).bfloat16().float() * h[:, inter:]).bfloat16().float()
+            want.index_add_(0, t, (h @ w2[e].float().T).bfloat16().float() * weights[t, j, None].float())
+    # products and sums of bf16 roundings
+    assert float((got - want).norm() / want.norm()) < 1e-2
+    assert float((got - other).norm() / other.norm()) < 1e-2
