@@ -80,19 +80,22 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   try {
     at::Tensor out = at::empty({B, H * D}, q->options());
     const int64_t qs = B > 1 ? q->stride(0) : H * D;
+    // everything that Python holds or that can throw is read before the interpreter lock is given up
+    const float scale = (float)real(a[6]), f9 = (float)real(a[9]), f10 = FP8 ? (float)real(a[10]) : 0.f;
+    const int32_t window = FP8 ? 0 : (int32_t)whole(a[10]), keep_first = FP8 ? 0 : (int32_t)whole(a[11]), chunk = FP8 ? 0 : (int32_t)whole(a[12]);
+    void* const on = stream();
     int rc;
     Py_BEGIN_ALLOW_THREADS
     if constexpr (FP8)
       rc = g_decode_fp8(out.data_ptr(), q->data_ptr(), k->data_ptr(), v->data_ptr(), (const int32_t*)bt->data_ptr(),
                         (const int32_t*)lens->data_ptr(), (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, qs, H * D, (int32_t)k->size(0),
-                        (int32_t)k->size(1), (int32_t)bt->stride(0), (float)real(a[6]), (float)real(a[9]), (float)real(a[10]),
-                        ws->data_ptr(), (size_t)ws->numel(), (int32_t)ctas, element(*q), stream());
+                        (int32_t)k->size(1), (int32_t)bt->stride(0), scale, f9, f10, ws->data_ptr(),
+                        (size_t)ws->numel(), (int32_t)ctas, element(*q), on);
     else
       rc = g_decode(out.data_ptr(), q->data_ptr(), k->data_ptr(), v->data_ptr(), (const int32_t*)bt->data_ptr(),
                     (const int32_t*)lens->data_ptr(), (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, (int32_t)D, qs, H * D,
-                    (int32_t)k->size(0), (int32_t)k->size(1), (int32_t)bt->stride(0), (float)real(a[6]), (float)real(a[9]), nullptr,
-                    (int32_t)whole(a[10]), (int32_t)whole(a[11]), (int32_t)whole(a[12]), ws->data_ptr(), (size_t)ws->numel(), (int32_t)ctas,
-                    element(*q), stream());
+                    (int32_t)k->size(0), (int32_t)k->size(1), (int32_t)bt->stride(0), scale, f9, nullptr, window, keep_first,
+                    chunk, ws->data_ptr(), (size_t)ws->numel(), (int32_t)ctas, element(*q), on);
     Py_END_ALLOW_THREADS
     got = status(rc, std::move(out));
   } catch (...) {
@@ -129,14 +132,18 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (v->size(0) > 1) vs = v->stride(0);
   }
   at::Tensor out = at::empty({T, H * D}, q->options());
+  const int32_t max_q = (int32_t)whole(a[7]), max_k = (int32_t)whole(a[8]);
+  const float scale = (float)real(a[9]), softcap = (float)real(a[11]);
+  const int32_t window = (int32_t)whole(a[13]), keep_first = (int32_t)whole(a[14]), chunk = (int32_t)whole(a[15]);
+  void* const on = stream();
   int rc;
   Py_BEGIN_ALLOW_THREADS
   rc = g_prefill(out.data_ptr(), q->data_ptr(), k->data_ptr(), v->data_ptr(), (const int32_t*)cq->data_ptr(), (const int32_t*)ck->data_ptr(),
-                 (int32_t)(cq->numel() - 1), (int32_t)T, (int32_t)total_k, (int32_t)whole(a[7]), (int32_t)whole(a[8]), (int32_t)H,
+                 (int32_t)(cq->numel() - 1), (int32_t)T, (int32_t)total_k, max_q, max_k, (int32_t)H,
                  (int32_t)kv, (int32_t)D, (int32_t)D, T > 1 ? q->stride(0) : H * D, ks, vs, H * D,
                  paged ? (const int32_t*)bt->data_ptr() : nullptr, paged ? (int32_t)bt->stride(0) : 0, (int32_t)nb, (int32_t)bs,
-                 (float)real(a[9]), (float)real(a[11]), sink ? (const float*)sink->data_ptr() : nullptr, (int32_t)whole(a[13]),
-                 (int32_t)whole(a[14]), (int32_t)whole(a[15]), element(*q), ws ? ws->data_ptr() : nullptr, ws ? ws->numel() : 0, stream());
+                 scale, softcap, sink ? (const float*)sink->data_ptr() : nullptr, window, keep_first, chunk, element(*q),
+                 ws ? ws->data_ptr() : nullptr, ws ? ws->numel() : 0, on);
   Py_END_ALLOW_THREADS
   return status(rc, std::move(out));
   END_HANDLE_TH_ERRORS
