@@ -3,8 +3,10 @@
 // A decode step of one row takes 12 us on the GPU and took 17 us of Python: 25 arguments through ctypes (3.6 us), some 35 tensor
 // attributes (4 us). Here the same attributes are looked at and the same library function is called without either. What ops.py
 // would refuse is not judged here: the functions return None for any argument that is not exactly what they expect, and ops.py goes its
-// own way, checks and errors included. An int is the library's status. Plain torch.Tensor only (subclasses, fake tensors and dispatch
-// modes take ops.py's way); nothing is kept between calls.
+// own way, checks and errors included. An int is the library's status. Plain torch.Tensor with memory of its own only (subclasses, fake
+// tensors, dispatch modes and what torch.vmap and torch.func wrap take ops.py's way); nothing is kept between calls.
+// The interpreter lock is given up around the library's function alone: everything that can throw, addresses of tensors included,
+// is read before, since an exception that left the block would be handled without the lock.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ATen.h>
@@ -19,11 +21,11 @@ decltype(&b200_paged_decode_attn_windowed) g_decode = nullptr;
 decltype(&b200_paged_decode_attn_fp8) g_decode_fp8 = nullptr;
 decltype(&b200_prefill_varlen_attn_windowed) g_prefill = nullptr;
 
-// a plain CUDA tensor, or nullptr
+// a plain CUDA tensor with memory, or nullptr (the wrappers of torch.vmap, grad and jvp are torch.Tensor to Python, and have none)
 const at::Tensor* cuda_tensor(PyObject* o) {
   if (!THPVariable_CheckExact(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
-  return t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !t.is_conj() ? &t : nullptr;
+  return t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !t.is_conj() && t.has_storage() ? &t : nullptr;
 }
 int element(const at::Tensor& t) {
   return t.scalar_type() == at::kBFloat16 ? B200_DTYPE_BF16 : t.scalar_type() == at::kHalf ? B200_DTYPE_F16 : -1;
@@ -47,7 +49,7 @@ bool numbers(PyObject* const* a, int n) {
 }
 // a number as int(x) and as float(x) give it
 int64_t whole(PyObject* o) { return PyLong_CheckExact(o) ? PyLong_AsLongLong(o) : (int64_t)PyFloat_AS_DOUBLE(o); }
-double real(PyObject* o) { return PyFloat_CheckExact(o) ? PyFloat_AS_DOUBLE(o) : PyLong_AsDouble(o); }
+float real(PyObject* o) { return (float)(PyFloat_CheckExact(o) ? PyFloat_AS_DOUBLE(o) : PyLong_AsDouble(o)); }
 
 PyObject* status(int rc, at::Tensor out) { return rc == B200_OK ? THPVariable_Wrap(std::move(out)) : PyLong_FromLong(rc); }
 
@@ -56,7 +58,9 @@ PyObject* status(int rc, at::Tensor out) { return rc == B200_OK ? THPVariable_Wr
 template <bool FP8>
 PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != (FP8 ? 11 : 13) || !numbers(a + 6, (int)n - 6) || c10::impl::TorchDispatchModeTLS::any_modes_set()) Py_RETURN_NONE;
+  if (n != (FP8 ? 11 : 13) || !numbers(a + 6, (int)n - 6) ||
+      c10::impl::TorchDispatchModeTLS::any_modes_set())
+    Py_RETURN_NONE;
   const at::Tensor *q = cuda_tensor(a[1]), *k = cuda_tensor(a[2]), *v = cuda_tensor(a[3]), *bt = cuda_tensor(a[4]), *lens = cuda_tensor(a[5]);
   if (!q || !k || !v || !bt || !lens || element(*q) < 0 || q->dim() != 3) Py_RETURN_NONE;
   const int64_t B = q->size(0), H = q->size(1), D = q->size(2), kv = whole(a[7]), ctas = whole(a[8]);
@@ -80,22 +84,22 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   try {
     at::Tensor out = at::empty({B, H * D}, q->options());
     const int64_t qs = B > 1 ? q->stride(0) : H * D;
-    // everything that Python holds or that can throw is read before the interpreter lock is given up
-    const float scale = (float)real(a[6]), f9 = (float)real(a[9]), f10 = FP8 ? (float)real(a[10]) : 0.f;
+    const float scale = real(a[6]), f9 = real(a[9]), f10 = FP8 ? real(a[10]) : 0.f;
     const int32_t window = FP8 ? 0 : (int32_t)whole(a[10]), keep_first = FP8 ? 0 : (int32_t)whole(a[11]), chunk = FP8 ? 0 : (int32_t)whole(a[12]);
+    void *const to = out.data_ptr(), *const qp = q->data_ptr(), *const kp = k->data_ptr(), *const vp = v->data_ptr(), *const wp = ws->data_ptr();
+    const int32_t *const tables = (const int32_t*)bt->data_ptr(), *const rows = (const int32_t*)lens->data_ptr();
+    const int32_t nb = (int32_t)k->size(0), bs = (int32_t)k->size(1), bt_stride = (int32_t)bt->stride(0);
+    const size_t bytes = (size_t)ws->numel();
+    const int type = element(*q);
     void* const on = stream();
     int rc;
     Py_BEGIN_ALLOW_THREADS
     if constexpr (FP8)
-      rc = g_decode_fp8(out.data_ptr(), q->data_ptr(), k->data_ptr(), v->data_ptr(), (const int32_t*)bt->data_ptr(),
-                        (const int32_t*)lens->data_ptr(), (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, qs, H * D, (int32_t)k->size(0),
-                        (int32_t)k->size(1), (int32_t)bt->stride(0), scale, f9, f10, ws->data_ptr(),
-                        (size_t)ws->numel(), (int32_t)ctas, element(*q), on);
+      rc = g_decode_fp8(to, qp, kp, vp, tables, rows, (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, qs, H * D, nb, bs, bt_stride, scale,
+                        f9, f10, wp, bytes, (int32_t)ctas, type, on);
     else
-      rc = g_decode(out.data_ptr(), q->data_ptr(), k->data_ptr(), v->data_ptr(), (const int32_t*)bt->data_ptr(),
-                    (const int32_t*)lens->data_ptr(), (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, (int32_t)D, qs, H * D,
-                    (int32_t)k->size(0), (int32_t)k->size(1), (int32_t)bt->stride(0), scale, f9, nullptr, window, keep_first,
-                    chunk, ws->data_ptr(), (size_t)ws->numel(), (int32_t)ctas, element(*q), on);
+      rc = g_decode(to, qp, kp, vp, tables, rows, (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, (int32_t)D, qs, H * D, nb, bs, bt_stride,
+                    scale, f9, nullptr, window, keep_first, chunk, wp, bytes, (int32_t)ctas, type, on);
     Py_END_ALLOW_THREADS
     got = status(rc, std::move(out));
   } catch (...) {
@@ -133,17 +137,22 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   at::Tensor out = at::empty({T, H * D}, q->options());
   const int32_t max_q = (int32_t)whole(a[7]), max_k = (int32_t)whole(a[8]);
-  const float scale = (float)real(a[9]), softcap = (float)real(a[11]);
+  const float scale = real(a[9]), softcap = real(a[11]);
   const int32_t window = (int32_t)whole(a[13]), keep_first = (int32_t)whole(a[14]), chunk = (int32_t)whole(a[15]);
+  void *const to = out.data_ptr(), *const qp = q->data_ptr(), *const kp = k->data_ptr(), *const vp = v->data_ptr(),
+             *const wp = ws ? ws->data_ptr() : nullptr;
+  const int32_t *const cqp = (const int32_t*)cq->data_ptr(), *const ckp = (const int32_t*)ck->data_ptr(),
+                *const tables = paged ? (const int32_t*)bt->data_ptr() : nullptr;
+  const float* const sinks = sink ? (const float*)sink->data_ptr() : nullptr;
+  const int32_t seqs = (int32_t)(cq->numel() - 1), bt_stride = paged ? (int32_t)bt->stride(0) : 0;
+  const int64_t qs = T > 1 ? q->stride(0) : H * D, bytes = ws ? ws->numel() : 0;
+  const int type = element(*q);
   void* const on = stream();
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = g_prefill(out.data_ptr(), q->data_ptr(), k->data_ptr(), v->data_ptr(), (const int32_t*)cq->data_ptr(), (const int32_t*)ck->data_ptr(),
-                 (int32_t)(cq->numel() - 1), (int32_t)T, (int32_t)total_k, max_q, max_k, (int32_t)H,
-                 (int32_t)kv, (int32_t)D, (int32_t)D, T > 1 ? q->stride(0) : H * D, ks, vs, H * D,
-                 paged ? (const int32_t*)bt->data_ptr() : nullptr, paged ? (int32_t)bt->stride(0) : 0, (int32_t)nb, (int32_t)bs,
-                 scale, softcap, sink ? (const float*)sink->data_ptr() : nullptr, window, keep_first, chunk, element(*q),
-                 ws ? ws->data_ptr() : nullptr, ws ? ws->numel() : 0, on);
+  rc = g_prefill(to, qp, kp, vp, cqp, ckp, seqs, (int32_t)T, (int32_t)total_k, max_q, max_k, (int32_t)H, (int32_t)kv, (int32_t)D, (int32_t)D,
+                 qs, ks, vs, H * D, tables, bt_stride, (int32_t)nb, (int32_t)bs, scale, softcap, sinks, window, keep_first, chunk, type, wp,
+                 bytes, on);
   Py_END_ALLOW_THREADS
   return status(rc, std::move(out));
   END_HANDLE_TH_ERRORS

@@ -79,3 +79,23 @@ def test_prompts_are_the_same_either_way():
         ops.prefill_varlen_attn(q, k, v, cu.long(), cu, 57, 57, 0.125, G)
     with pytest.raises(ValueError):
         ops.prefill_varlen_attn(q, k.transpose(0, 1).contiguous().transpose(0, 1), v, cu, cu, 57, 57, 0.125, G)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("transform", [lambda f, x: torch.vmap(f)(x[None]), lambda f, x: torch.func.grad(f)(x), lambda f, x: torch.func.jvp(f, (x,), (x,))],
+                         ids=["vmap", "grad", "jvp"])
+def test_wrapped_tensors_raise(transform):
+    """torch.vmap and torch.func wrap what they pass on: torch.Tensor to Python, and without memory."""
+    from nanovllm import ops
+    q, k, v, tables, lens = _step()
+    q8, k8, v8 = _step(fp8=True)[:3]
+    cu = torch.tensor([0, 3], dtype=torch.int32, device="cuda")
+    kv = torch.randn(3, 2, 64, device="cuda").bfloat16()
+    calls = ((q, lambda x: ops.paged_decode_attn(x, k, v, tables, lens, 0.125, 2)),
+             (q8, lambda x: ops.paged_decode_attn_fp8(x, k8, v8, tables, lens, 0.125, 2)),
+             (q, lambda x: ops.prefill_varlen_attn(x, kv, kv, cu, cu, 3, 3, 0.125, 2)))
+    for x, call in calls:
+        want = call(x)                                         # (the workspaces are there)
+        with pytest.raises(RuntimeError, match="storage"):
+            transform(lambda y: call(y).sum(), x)              # noqa: B023
+        assert torch.equal(call(x), want)
