@@ -38,17 +38,22 @@ bool cache_fits(const at::Tensor& t, int64_t row) {
          t.size(2) * (t.dim() == 4 ? t.size(3) : 1) == row;
 }
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
-bool numbers(PyObject* const* a, int n) {
+// ints that fit 64 bits (what int() would make of a float, and what ctypes would refuse, is ops.py's business)
+bool ints(PyObject* const* a, int n) {
   for (int i = 0; i < n; ++i) {
     int over = 0;
-    if (PyLong_CheckExact(a[i])) PyLong_AsLongLongAndOverflow(a[i], &over);
-    else if (!PyFloat_CheckExact(a[i])) return false;
+    if (!PyLong_CheckExact(a[i])) return false;
+    PyLong_AsLongLongAndOverflow(a[i], &over);
     if (over != 0) return false;
   }
   return true;
 }
-// a number as int(x) and as float(x) give it
-int64_t whole(PyObject* o) { return PyLong_CheckExact(o) ? PyLong_AsLongLong(o) : (int64_t)PyFloat_AS_DOUBLE(o); }
+bool reals(PyObject* const* a, int n) {
+  for (int i = 0; i < n; ++i)
+    if (!PyFloat_CheckExact(a[i]) && !ints(a + i, 1)) return false;
+  return true;
+}
+int64_t whole(PyObject* o) { return PyLong_AsLongLong(o); }
 float real(PyObject* o) { return (float)(PyFloat_CheckExact(o) ? PyFloat_AS_DOUBLE(o) : PyLong_AsDouble(o)); }
 
 PyObject* status(int rc, at::Tensor out) { return rc == B200_OK ? THPVariable_Wrap(std::move(out)) : PyLong_FromLong(rc); }
@@ -58,7 +63,7 @@ PyObject* status(int rc, at::Tensor out) { return rc == B200_OK ? THPVariable_Wr
 template <bool FP8>
 PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != (FP8 ? 11 : 13) || !numbers(a + 6, (int)n - 6) ||
+  if (n != (FP8 ? 11 : 13) || !reals(a + 6, 1) || !ints(a + 7, 2) || !reals(a + 9, FP8 ? 2 : 1) || (!FP8 && !ints(a + 10, 3)) ||
       c10::impl::TorchDispatchModeTLS::any_modes_set())
     Py_RETURN_NONE;
   const at::Tensor *q = cuda_tensor(a[1]), *k = cuda_tensor(a[2]), *v = cuda_tensor(a[3]), *bt = cuda_tensor(a[4]), *lens = cuda_tensor(a[5]);
@@ -115,7 +120,7 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // softcap, sink or None, window, keep_first, chunk)
 PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 16 || !numbers(a + 7, 5) || !numbers(a + 13, 3) || c10::impl::TorchDispatchModeTLS::any_modes_set()) Py_RETURN_NONE;
+  if (n != 16 || !ints(a + 7, 2) || !reals(a + 9, 1) || !ints(a + 10, 1) || !reals(a + 11, 1) || !ints(a + 13, 3) || c10::impl::TorchDispatchModeTLS::any_modes_set()) Py_RETURN_NONE;
   const bool paged = a[6] != Py_None;
   const at::Tensor *q = cuda_tensor(a[1]), *k = cuda_tensor(a[2]), *v = cuda_tensor(a[3]), *cq = cuda_tensor(a[4]), *ck = cuda_tensor(a[5]),
                    *bt = paged ? cuda_tensor(a[6]) : nullptr, *ws = a[0] != Py_None ? cuda_tensor(a[0]) : nullptr,

@@ -1,5 +1,7 @@
 """The native calls of ops' attention entry points (csrc/host_calls.cpp): what they take gives what ops' own way gives, bit for bit; what they
 do not take is left to ops' own checks."""
+import ctypes
+
 import pytest
 import torch
 
@@ -99,3 +101,14 @@ def test_wrapped_tensors_raise(transform):
         with pytest.raises(RuntimeError, match="storage"):
             transform(lambda y: call(y).sum(), x)              # noqa: B023
         assert torch.equal(call(x), want)
+
+
+@pytest.mark.gpu
+def test_numbers_are_what_ctypes_takes():
+    from nanovllm import ops
+    q, k, v, tables, lens = _step()
+    with pytest.raises(ctypes.ArgumentError):
+        ops.paged_decode_attn(q, k, v, tables, lens, 0.125, 2.0)
+    with pytest.raises(ValueError):
+        ops.paged_decode_attn(q, k, v, tables, lens, 0.125, 2, window=float("nan"))
+    assert torch.equal(ops.paged_decode_attn(q, k, v, tables, lens, 1, 2, window=20.0), ops.paged_decode_attn(q, k, v, tables, lens, 1.0, 2, window=20))
