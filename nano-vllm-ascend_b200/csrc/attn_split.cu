@@ -58,6 +58,12 @@ __device__ __forceinline__ bool beyond_split(float x) {
   return e - 0x0d800000u >= 0x7f000000u - 0x0d800000u && e != 0u;
 }
 
+// two fp32 operations in one instruction: a b + c
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(reinterpret_cast<uint64_t&>(c)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+  return c;
+}
+
 template <int DK, int DV>
 __global__ void __launch_bounds__(kAsThreads, 1)
 attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
@@ -128,12 +134,21 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     const int row = warp * 32 + lane, r = min(r0 + row, rows - 1);
     const uint32_t base = tb + ((uint32_t)(warp * 32) << 16);
     const int pos = sp.first_pos() + r / rep;
-    // scores in units of log2: S c with c in two parts, subtracted from the reference in one rounding (with the product of the
-    // rounded c and S the weights of short rows were off by a seventh more)
-    const float c = P.scale * kLog2e, c_low = fmaf(P.scale, kLog2e, -c) + P.scale * 1.925963033500e-8f;
-    const float sign = c < 0.f ? -1.f : 1.f, hidden = -3e38f * sign;      // (infinity times c_low could be anything)
-    // a sink is one more entry of the softmax that has a logit and no value: the running state starts from it
-    float m = P.sink != nullptr ? P.sink[g * rep + r % rep] * kLog2e : -INFINITY, l = P.sink != nullptr ? 1.f : 0.f;
+    // A key's weight is 2^(x c - top), top = m c of the largest score so far, with c in two parts that are subtracted from top in one
+    // rounding (with the rounded c alone the weights of short rows were off by a seventh more). Rows whose top has a spacing of 2^-7
+    // or more count from the largest score itself: 2^((x - m) c). Hidden keys, and visible ones whose score has overflowed,
+    // end at -FLT_MAX, which c turns into no weight and at which the small part stays finite (attn_split_fits); NaN stays NaN. Scores
+    // of a negative scale have changed sign in q
+    const float c = fabsf(P.scale) * kLog2e, c_low = fmaf(fabsf(P.scale), kLog2e, -c) + fabsf(P.scale) * 1.925963033500e-8f;
+    float top = -INFINITY, less = 0.f;
+    auto weights = [&](float& a, float& b) {                   // 2^(x c - less) of both
+      float2 x = make_float2(a, b);
+      asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.x) : "f"(-3.4028234e38f));
+      asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.y) : "f"(-3.4028234e38f));
+      const float2 e = fma2(x, make_float2(c, c), fma2(x, make_float2(c_low, c_low), make_float2(-less, -less)));
+      a = ex2_approx(e.x), b = ex2_approx(e.y);
+    };
+    float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < tiles; ++j) {
       ok = wait(&s_full[j & 1], j >> 1);
@@ -151,13 +166,23 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       if (j * kAsN + kAsN - 1 > min_pos) {
         const int last = pos - j * kAsN;
 #pragma unroll
-        for (int i = 0; i < kAsN; ++i) x[i] = i <= last ? x[i] : hidden;
+        for (int i = 0; i < kAsN; ++i) x[i] = i <= last ? x[i] : -INFINITY;
       }
-      float mx[4] = {x[0] * sign, x[1] * sign, x[2] * sign, x[3] * sign};
+      float mx[4] = {x[0], x[1], x[2], x[3]};
 #pragma unroll
-      for (int i = 4; i < kAsN; ++i) mx[i & 3] = fmaxf(mx[i & 3], x[i] * sign);
-      const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * fabsf(c));
-      const float corr = ex2_approx(m - m_new);          // key 0 is seen by all: m_new is finite
+      for (int i = 4; i < kAsN; ++i) mx[i & 3] = fmaxf(mx[i & 3], x[i]);
+      const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
+      const bool far = fabsf(m_new) * c >= 65536.f && m_new != -INFINITY;
+      less = far || m_new == -INFINITY ? 0.f : m_new * c;      // (-inf: every score so far has overflowed)
+      float corr = ex2_approx(top - less);
+      if (far) {
+        float none = 0.f;
+        corr = m - m_new;
+        weights(corr, none);
+#pragma unroll
+        for (int i = 0; i < kAsN; ++i) x[i] -= m_new;
+      }
+      top = m_new * c;
       m = m_new;
       s_corr[(j & (kAsCorr - 1)) * kAsM + row] = corr;
       if (j > 0) {
@@ -171,7 +196,8 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
         uint32_t w[3][8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const float a = ex2_approx(fmaf(x[i0 + 2 * i], c, fmaf(x[i0 + 2 * i], c_low, -m))), b = ex2_approx(fmaf(x[i0 + 2 * i + 1], c, fmaf(x[i0 + 2 * i + 1], c_low, -m)));
+          float a = x[i0 + 2 * i], b = x[i0 + 2 * i + 1];
+          weights(a, b);
           sum[0] += a, sum[1] += b;
           uint32_t y[3];
           split3x2(a, b, y);
@@ -185,7 +211,14 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       umma::fence_before_sync();
       mbar_arrive(p_ready);
     }
-    float inv = 1.0f / l;
+    // a sink is one more entry of the softmax that has a logit and no value (in units of log2, as top)
+    float share = 1.f;
+    if (P.sink != nullptr) {
+      const float sink = P.sink[g * rep + r % rep] * kLog2e;
+      if (sink > top) share = ex2_approx(top - sink), l = fmaf(l, share, 1.f);
+      else l += top == -INFINITY ? 1.f : ex2_approx(sink - top);
+    }
+    float inv = share / l;
     if (P.gate != nullptr)
       inv *= sigmoid_f(reinterpret_cast<const float*>(P.gate)[(int64_t)(sp.q_start + r / rep) * P.gate_stride + g * rep + r % rep]);
     s_corr[kAsCorr * kAsM + row] = inv;
@@ -274,8 +307,9 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
 #pragma unroll 4
     for (int row = DK == 128 ? w8 : 2 * w8 + (lane >> 4); row < kAsM; row += DK == 128 ? 8 : 16) {
       const int r = r0 + row, tok = r / rep, col = 4 * (DK == 128 ? lane : lane & 15);
-      const float4 y = fetch(qb + (int64_t)(sp.q_start + tok) * P.q_stride + (int64_t)(g * rep + r - tok * rep) * dim, col, dim, r < rows);
+      float4 y = fetch(qb + (int64_t)(sp.q_start + tok) * P.q_stride + (int64_t)(g * rep + r - tok * rep) * dim, col, dim, r < rows);
       look(y);
+      if (P.scale < 0.f) y = make_float4(-y.x, -y.y, -y.z, -y.w);
       store_split4(sQ + (col >> 6) * 2 * kAsPanel + umma::sw128(row, (col >> 3) & 7) + (col & 4) * 2, kQPlane, y);
     }
     fence_proxy_async_smem();
@@ -420,7 +454,7 @@ bool attn_split_fits(const AttnTiledParams& P, int num_seqs, int max_q, int64_t 
   if (dtype != B200_DTYPE_F32 || P.window > 0 || P.chunk > 0 || P.softcap > 0.f || P.dim > 128 || P.vdim > 128) return false;
   if (P.dim % 4 != 0 || P.vdim % 4 != 0 || P.q_stride % 4 != 0 || P.k_stride % 4 != 0 || (P.v != nullptr && P.v_stride % 4 != 0)) return false;
   if (!aligned16(P.q) || !aligned16(P.k) || !aligned16(P.v) || !aligned16(P.out)) return false;
-  if (!(fabsf(P.scale) > 1e-20f && fabsf(P.scale) < 1e20f)) return false;      // a hidden score times it has to vanish
+  if (!(fabsf(P.scale) > 1e-20f && fabsf(P.scale) < 1e6f)) return false;       // -FLT_MAX times c vanishes, times c_low stays finite
   const int rep = P.H / P.G;
   if (((int64_t)max_q * rep + kAsM - 1) / kAsM * P.G > 0x7fffffff / num_seqs) return false;
   const int64_t least = P.dim <= 64 && P.vdim <= 64 ? 64 : 192;

@@ -11,11 +11,11 @@ pytestmark = pytest.mark.gpu
 F64 = torch.float64
 
 
-def _run(H, G, dim, dv, spans, paged, sink=False, gate=False, latent=False, poke=None):
+def _run(H, G, dim, dv, spans, paged, sink=False, gate=False, latent=False, poke=None, scale=None):
     from nanovllm import ops
     g = torch.Generator().manual_seed(dim * dv + H + len(spans))
     rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
-    T = sum(n for n, _ in spans)
+    T, scale = sum(n for n, _ in spans), dim ** -0.5 if scale is None else scale
     q, sk, gt = rnd(T, H, dim), rnd(H) if sink else None, rnd(T, H) if gate else None
     ks = [rnd(m, G, dim) for _, m in spans]
     vs = [k[:, :, :dv] if latent else rnd(m, G, dv) for k, (_, m) in zip(ks, spans)]
@@ -36,12 +36,12 @@ def _run(H, G, dim, dv, spans, paged, sink=False, gate=False, latent=False, poke
                 for c, x in ((kc, ks), (vc, vs)):
                     rows = x[s][b * paged:(b + 1) * paged]
                     c[blk, :len(rows)] = rows.reshape(len(rows), -1)
-        got = ops.attn_generic(q.cuda(), kc.cuda(), vc.cuda(), sp, dim ** -0.5, G, dv, block_tables=table.cuda(), **extra)
+        got = ops.attn_generic(q.cuda(), kc.cuda(), vc.cuda(), sp, scale, G, dv, block_tables=table.cuda(), **extra)
     else:
-        got = ops.attn_generic(q.cuda(), torch.cat(ks).cuda(), None if latent else torch.cat(vs).cuda(), sp, dim ** -0.5, G, dv, **extra)
+        got = ops.attn_generic(q.cuda(), torch.cat(ks).cuda(), None if latent else torch.cat(vs).cuda(), sp, scale, G, dv, **extra)
     at, out = 0, []
     for s, (n, m) in enumerate(spans):
-        w = _want(q[at:at + n], ks[s], vs[s], m - n, dim ** -0.5, 0, 0, 0, 0.0, sk, None if gt is None else gt[at:at + n])
+        w = _want(q[at:at + n], ks[s], vs[s], m - n, scale, 0, 0, 0, 0.0, sk, None if gt is None else gt[at:at + n])
         out.append((got[at:at + n].cpu().to(F64).view(n, H, dv), w))
         at += n
     return out
@@ -72,3 +72,39 @@ def test_what_three_terms_cannot_carry(bad, where):
         fine = torch.isfinite(w)
         assert torch.equal(torch.isfinite(x), fine), s
         assert float(((x - w).abs() / w.abs().clamp(min=1.0))[fine].max()) < 2e-5, s
+
+
+@pytest.mark.parametrize("scale", [1e-19, 2e-4, 0.3, -0.3, 8e5, -9.9e5, 1.01e6, 3e7, 5e9, -5e9])
+def test_scales_up_to_the_guard_and_past_it(scale):
+    """Scores of a few units at every scale; past the guard another kernel takes over."""
+    def poke(q, ks, vs):
+        q *= 0.125 / scale
+    for s, (x, w) in enumerate(_run(4, 2, 64, 64, [(70, 70), (64, 200)], 16, sink=True, poke=poke, scale=scale)):
+        assert float(((x - w).abs() / w.abs().clamp(min=1.0)).max()) < 2e-5, s
+
+
+@pytest.mark.parametrize("dim,scale", [(128, None), (64, 0.1), (64, -0.1), (64, 1e5)])
+def test_scores_that_overflow(dim, scale):
+    """Finite operands, scores of -1e39: no weight, also where a whole tile of keys has nothing else."""
+    sign = -1.0 if scale is not None and scale < 0 else 1.0
+
+    def poke(q, ks, vs):
+        q[:, :, 0], q[:, :, 1:] = 1e20, q[:, :, 1:] * 1e20
+        for k in ks:
+            k[:, :, 1:] *= 1e-20 if scale != 1e5 else 1e6      # others of a few units; of 1e31 and more
+            k[:, :, 0] = 0.0
+            k[:66, :, 0] = -1e20 * sign
+            k[70::7, :, 0] = -1e20 * sign
+    for s, (x, w) in enumerate(_run(4, 2, dim, 64, [(100, 200), (64, 130)], 16, poke=poke, scale=scale)):
+        assert float(((x - w).abs() / w.abs().clamp(min=1.0)).max()) < 2e-5, s
+
+
+@pytest.mark.parametrize("sink", [False, True])
+def test_scores_of_many_digits(sink):
+    """Scores around 1e10, whose spacing in fp32 is a thousand: the largest takes all (the next are millions below)."""
+    def poke(q, ks, vs):
+        q *= 1e5
+        for k in ks:
+            k *= 1e5
+    for s, (x, w) in enumerate(_run(4, 2, 128, 128, [(100, 100), (64, 200)], 16, sink=sink, poke=poke)):
+        assert float(((x - w).abs() / w.abs().clamp(min=1.0)).max()) < 2e-5, s
