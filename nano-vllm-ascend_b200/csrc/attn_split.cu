@@ -20,9 +20,11 @@
 // heads over 2 of 128, paged, 288 us (attn_tiled_kernel) -> 71 (81 with 8 columns a lane, which read every sector twice, 78 with
 // that but block ids looked up a step ahead); 4 of 600-1000, 32 heads over 8 of 64, 490 -> 141.
 //
-// What is not finite, or so small that a term of it would not be normal, the split cannot carry (and 0 x inf would reach rows that
-// do not see the key). The copying warps look at every value; a CTA that met one computes its rows once more in plain fp32,
-// key by key as attn_generic_kernel does.
+// What the split cannot carry: what is not finite or close to the largest numbers (and 0 x inf would reach rows that do not see the key),
+// and what is so small that a term of it would not be normal. Values come times 2^27, which leaves nothing too small, and go back
+// at the end. A small element of Q or K (below 2^-100) is off by 2^-126 at most, which is nothing to a score unless it meets one of
+// 2^70 or more. The copying warps look at the magnitudes; a CTA that met such values computes its rows once more in plain fp32,
+// key by key as attn_generic_kernel does (4 prompts of 700-1024 tokens with an infinity in every head of each: 5.2 ms; attn_tiled_kernel 0.29).
 // Waits are bounded as in recurrence_umma_kernel.
 #include "attn_tiled.cuh"
 #include "recurrence.cuh"
@@ -32,6 +34,8 @@ namespace b200 {
 
 constexpr int kAsM = 128, kAsN = 64, kAsThreads = 640, kAsCorr = 4;
 constexpr int kAsPanel = 64 * 128;                     // bytes of 64 rows x 64 elements
+
+constexpr float kAsUp = 134217728.f;                    // 2^27: values come to the tensor core times it (see below)
 
 struct AttnSplitParams {
   AttnTiledParams a;
@@ -52,12 +56,6 @@ __device__ __forceinline__ void store_split4(uint8_t* to, int plane, float4 x) {
 #pragma unroll
   for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(to + p * plane) = make_uint2(w[0][p], w[1][p]);
 }
-// not below 2^127 (a first term could round to infinity), or below 2^-100 and not zero
-__device__ __forceinline__ bool beyond_split(float x) {
-  const uint32_t e = __float_as_uint(x) & 0x7fffffffu;
-  return e - 0x0d800000u >= 0x7f000000u - 0x0d800000u && e != 0u;
-}
-
 // two fp32 operations in one instruction: a b + c
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(reinterpret_cast<uint64_t&>(c)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
@@ -83,7 +81,8 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
            *p_ready = bars + 7, *o_full = bars + 8, *o_read = bars + 10, *done = bars + 12, *drained = bars + 13;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* wild = gave_up + 1;
+  volatile int *huge = gave_up + 1, *tiny = gave_up + 2, *large = gave_up + 3;
+  auto wild = [&] { return *huge != 0 || (*tiny != 0 && *large != 0); };
 
   pdl_wait();
   // the last row tiles see the most keys: those of every (sequence, kv head) start first
@@ -111,7 +110,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     for (int b = 0; b < 2; ++b) mbar_init(&s_full[b], 1), mbar_init(&o_full[b], 1), mbar_init(&o_read[b], kAsM);
     mbar_init(p_ready, kAsM), mbar_init(done, kAsM), mbar_init(drained, 1);
     mbar_fence_init();
-    *gave_up = 0, *wild = 0;
+    *gave_up = 0, *huge = 0, *tiny = 0, *large = 0;
   }
   if (warp == 16) umma::tmem_alloc(tmem_slot, 512);
   umma::fence_before_sync();
@@ -248,13 +247,13 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       umma::fence_before_sync();
       mbar_arrive(&o_read[j & 1]);
     }
-    if (ok && wait(done, 0) && r < rows && !*wild) {
+    if (ok && wait(done, 0) && r < rows && !wild()) {
       const float inv = s_corr[kAsCorr * kAsM + row];
       const int tok = r / rep;
       float* o = reinterpret_cast<float*>(P.out) + (int64_t)(sp.q_start + tok) * ((int64_t)P.H * vdim) + (int64_t)(g * rep + r - tok * rep) * vdim;
 #pragma unroll
       for (int i = 0; i < DV; i += 4)
-        if (i < vdim) *reinterpret_cast<float4*>(o + i) = make_float4(O[i] * inv, O[i + 1] * inv, O[i + 2] * inv, O[i + 3] * inv);
+        if (i < vdim) *reinterpret_cast<float4*>(o + i) = make_float4(O[i] / kAsUp * inv, O[i + 1] / kAsUp * inv, O[i + 2] / kAsUp * inv, O[i + 3] / kAsUp * inv);
     }
   } else if (warp < 16) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
@@ -262,8 +261,17 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     // A lane takes 4 columns, so that a warp reads whole rows (with 8, every 32-byte sector came twice); warp w of the eight takes
     // rows w, w + 8, .. of Q, K or V, for 64 columns two neighbouring rows at a time
     const int w8 = warp - 8;
-    bool odd = false;                                   // met a value that the split cannot carry
-    auto look = [&](float4 x) { odd |= beyond_split(x.x) || beyond_split(x.y) || beyond_split(x.z) || beyond_split(x.w); };
+    float most = 0.f, least = 1.f, most_v = 0.f;        // magnitudes met
+    auto look = [&](float4 x) {
+      asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(x.x), "f"(x.y));
+      asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(x.z), "f"(x.w));
+      asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(x.x), "f"(x.y));
+      asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(x.z), "f"(x.w));
+    };
+    auto look_v = [&](float4 x) {
+      asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most_v) : "f"(x.x), "f"(x.y));
+      asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most_v) : "f"(x.z), "f"(x.w));
+    };
     auto fetch = [&](const float* row, int col, int width, bool there) {       // zero past the width (a multiple of 4)
       return there && col < width ? __ldg(reinterpret_cast<const float4*>(row + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
@@ -320,10 +328,13 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       if (j > 0 && !wait(key ? k_empty : v_empty, j - 1)) return false;
       uint8_t* to = key ? sK : sV;
       each((key ? DK : DV) == 128, [&](int i, int row, int col, int) {
-        look(x[i]);
+        if (key) look(x[i]);
+        else x[i] = make_float4(x[i].x * kAsUp, x[i].y * kAsUp, x[i].z * kAsUp, x[i].w * kAsUp), look_v(x[i]);
         store_split4(to + (col >> 6) * kAsPanel + umma::sw128(row, (col >> 3) & 7) + (col & 4) * 2, plane, x[i]);
       });
-      if (odd) *wild = 1;
+      if (!(most < 0x1p127f) || !(most_v < 0x1p107f)) *huge = 1;
+      if (most >= 0x1p70f) *large = 1;
+      if (least < 0x1p-100f) *tiny = 1;
       fence_proxy_async_smem();
       mbar_arrive(key ? k_full : v_full);
       if (st + kAhead < steps) load(st + kAhead, x);
@@ -399,7 +410,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     *reinterpret_cast<volatile int*>(AP.wait_status) = 1;
     __threadfence_system();
   }
-  if (!*wild) return;
+  if (!wild()) return;
 
   // ---- plain fp32, one warp per row, a lane per key of 32 and then a lane per value column of 32 (see above)
 #pragma unroll 1
@@ -417,7 +428,10 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
         const float* k = kb + key_row(j0 + lane) * P.k_stride;
         float d = 0.f;
 #pragma unroll 1
-        for (int i = 0; i < dim; ++i) d += q[i] * k[i];
+        for (int i = 0; i < dim; i += 4) {
+          const float4 x = __ldg(reinterpret_cast<const float4*>(q + i)), y = __ldg(reinterpret_cast<const float4*>(k + i));
+          d += x.x * y.x, d += x.y * y.y, d += x.z * y.z, d += x.w * y.w;
+        }
         sc = d * P.scale;
       }
       const float m_new = fmaxf(m, warp_max(sc));

@@ -108,3 +108,19 @@ def test_scores_of_many_digits(sink):
             k *= 1e5
     for s, (x, w) in enumerate(_run(4, 2, 128, 128, [(100, 100), (64, 200)], 16, sink=sink, poke=poke)):
         assert float(((x - w).abs() / w.abs().clamp(min=1.0)).max()) < 2e-5, s
+
+
+@pytest.mark.parametrize("qs,ks,vs", [(1, 1, 1e-36), (1, 1, 2e-42), (1e-37, 1, 1), (1, 1e-40, 1), (2.0 ** 76, 2.0 ** -76, 1), (2.0 ** 76, 2.0 ** -110, 1),
+                                      (2.0 ** -110, 2.0 ** 100, 1), (1, 1, 2.0 ** 78), (1, 1, 2.0 ** 90), (1, 1, 2.0 ** 115)])
+def test_small_and_large_operands(qs, ks, vs):
+    """fp32 accuracy over fp32's range: one operand small or large, and small ones against large ones. Values end at 2^115, since the sums
+    of up to 200 weights of at most 1 and values of up to 5 times that are kept in fp32 before they are divided (2^115 x 1000 < 2^128)."""
+    def poke(q, kk, vv):
+        q *= qs
+        for k, v in zip(kk, vv):
+            k *= ks
+            v *= vs
+    for s, (x, w) in enumerate(_run(4, 2, 64, 64, [(70, 70), (64, 200)], 16, poke=poke)):
+        size = float(w.abs().max())
+        floor = 2.0 ** -149 / size                             # one step of the smallest numbers
+        assert float(((x - w).abs() / w.abs().clamp(min=0.3 * size)).max()) < 2e-5 + 4 * floor, s
