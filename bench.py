@@ -66,7 +66,7 @@ def moe_expert_roofline(runner, B, peak_gbs):
     scores = torch.rand(B, blk.num_experts, device="cuda", generator=g)
     ids = scores.topk(blk.top_k, dim=1).indices.to(torch.int32).contiguous()
     w = torch.full((B, blk.top_k), 1.0 / blk.top_k, device="cuda").to(runner.dtype)
-    plan = ops.moe_align(ids, blk.expert_begin, blk.num_local)
+    plan = ops.moe_align(ids, blk.expert_begin, blk.num_local, blk.num_experts)
     hit = int((plan.offsets[1:] > plan.offsets[:-1]).sum())
 
     def one_pass():

@@ -393,6 +393,16 @@ int b200_moe_gemm_down_umma(void* y, const void* h, const void* w2, const int32_
                             const int32_t* sorted_pair, const void* topk_weights, int32_t pairs,
                             int32_t inter, int32_t hidden, int32_t num_local, int32_t dtype,
                             b200_stream_t stream);
+/* The same where the caller expects only `expected` of the pairs to be of the local experts (expert parallelism: pairs x num_local /
+ * num_experts). It decides between kernels, and nothing else: any number of them may be. */
+int b200_moe_gemm_gate_up_umma_expected(void* h, const void* xs, const void* w13, const int32_t* offsets,
+                                        const int32_t* sorted_pair, const float* in_scale, int32_t pairs, int32_t expected,
+                                        int32_t hidden, int32_t inter, int32_t num_local, int32_t dtype, b200_stream_t stream);
+int b200_moe_gemm_down_umma_expected(void* y, const void* h, const void* w2, const int32_t* offsets,
+                                     const int32_t* sorted_pair, const void* topk_weights, int32_t pairs, int32_t expected,
+                                     int32_t inter, int32_t hidden, int32_t num_local, int32_t dtype, b200_stream_t stream);
+/* 1: such a product runs on the persistent kernel (256 columns at a time). n_out: inter for gate and up, hidden for down. */
+int32_t b200_moe_umma_persistent(int32_t gate_up, int32_t expected, int32_t num_local, int32_t n_out);
 /* down_umma without weights and with its own limit on a single wait of the persistent kernel. 0: a wait whose phase is
  * not complete at once gives up (how the way out is tested). */
 int b200_moe_gemm_down_umma_bounded(void* y, const void* h, const void* w2, const int32_t* offsets, int32_t pairs,

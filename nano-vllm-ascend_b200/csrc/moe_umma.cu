@@ -474,6 +474,7 @@ static int moe_sm_count() {
 // expert where they have 16 rows on average (a layer of 128 experts, 2048 x 768, top 8, 256 tokens: 359 us with the 128-column
 // kernels, 209 so). Fewer tiles than SMs leave it with idle SMs and one cold ring per tile, where the
 // 128-column kernels (two CTAs per SM or a deep ring) are the better ones. fp32 outputs (attention scores) stay there as well.
+// `pairs` of the local experts alone, as far as is known: under expert parallelism most of a plan's pairs are other ranks'.
 static bool moe_umma_wide(bool gate_up, int pairs, int num_local, int n_out, int out_f32) {
   const int band = gate_up ? 128 : 256;
   const int row_tiles = num_local > 1 && pairs / 16 >= num_local && num_local > pairs / 128 ? num_local : pairs / 128;
@@ -507,10 +508,10 @@ static int moe_umma_wide_launch(const CUtensorMap& ma, const CUtensorMap& mw, co
 
 template <typename T>
 static int moe_umma_launch(bool gate_up, const CUtensorMap& ma, const CUtensorMap& mw,
-                           const MoeUmmaParams& p, int pairs, cudaStream_t stream) {
+                           const MoeUmmaParams& p, int pairs, int expected, cudaStream_t stream) {
   const int row_tiles = (pairs + 127) / 128 + p.num_local;      // upper bound; surplus CTAs exit at once
   const dim3 grid(p.n_out / (gate_up ? 64 : 128), row_tiles);
-  const bool deep = (long long)grid.x * ((pairs + 127) / 128) <= 2ll * moe_sm_count();   // few live CTAs: latency-bound
+  const bool deep = (long long)grid.x * ((expected + 127) / 128) <= 2ll * moe_sm_count();   // few live CTAs: latency-bound
   if (gate_up)
     return deep ? moe_umma_launch_s<T, true, 6>(ma, mw, p, grid, stream)
                 : moe_umma_launch_s<T, true, 3>(ma, mw, p, grid, stream);
@@ -547,7 +548,8 @@ extern "C" int b200_moe_gather_rows(void* xs, const void* x, const int32_t* offs
 static int moe_umma_common(bool gate_up, void* out, const void* a, const void* w, const int32_t* offsets,
                            const int32_t* sorted_pair, const void* pair_scale, int32_t pairs, int32_t K,
                            int32_t n_out, int32_t num_local, int32_t dtype, b200_stream_t stream,
-                           int out_f32 = 0, const float* in_scale = nullptr, int64_t wait_ns = kWaitNs) {
+                           int out_f32 = 0, const float* in_scale = nullptr, int64_t wait_ns = kWaitNs, int32_t expected = -1) {
+  if (expected < 0 || expected > pairs) expected = pairs;
   B200_RETURN_IF(dtype != B200_DTYPE_BF16 && dtype != B200_DTYPE_F16, B200_ERR_BAD_DTYPE);
   B200_RETURN_IF(pairs < 0 || K <= 0 || n_out <= 0 || num_local <= 0, B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(K % 64 != 0 || n_out % (gate_up ? 64 : 128) != 0 || num_local > 256, B200_ERR_UNSUPPORTED);
@@ -560,7 +562,7 @@ static int moe_umma_common(bool gate_up, void* out, const void* a, const void* w
   int rc = get_panel_map(a, pairs, (int64_t)K * 2, K / 64, 128, 1, dtype, &ma);
   if (rc != B200_OK) return rc;
   const int64_t w_rows = (int64_t)num_local * (gate_up ? 2 : 1) * n_out;
-  const bool wide = moe_umma_wide(gate_up, pairs, num_local, n_out, out_f32);
+  const bool wide = moe_umma_wide(gate_up, expected, num_local, n_out, out_f32);
   rc = get_panel_map(w, w_rows, (int64_t)K * 2, K / 64, wide ? 128 : 64, 1, dtype, &mw);
   if (rc != B200_OK) return rc;
   MoeUmmaParams p{offsets, sorted_pair, pair_scale, out, num_local, K, n_out, out_f32, in_scale, wait_ns, wait_status()};
@@ -572,25 +574,45 @@ static int moe_umma_common(bool gate_up, void* out, const void* a, const void* w
     return gate_up ? moe_umma_wide_launch<__half, true>(ma, mw, p, (cudaStream_t)stream)
                    : moe_umma_wide_launch<__half, false>(ma, mw, p, (cudaStream_t)stream);
   }
-  return dtype == B200_DTYPE_BF16 ? moe_umma_launch<__nv_bfloat16>(gate_up, ma, mw, p, pairs, (cudaStream_t)stream)
-                                  : moe_umma_launch<__half>(gate_up, ma, mw, p, pairs, (cudaStream_t)stream);
+  return dtype == B200_DTYPE_BF16 ? moe_umma_launch<__nv_bfloat16>(gate_up, ma, mw, p, pairs, expected, (cudaStream_t)stream)
+                                  : moe_umma_launch<__half>(gate_up, ma, mw, p, pairs, expected, (cudaStream_t)stream);
+}
+
+extern "C" int b200_moe_gemm_gate_up_umma_expected(void* h, const void* xs, const void* w13, const int32_t* offsets,
+                                                   const int32_t* sorted_pair, const float* in_scale, int32_t pairs, int32_t expected,
+                                                   int32_t hidden, int32_t inter, int32_t num_local, int32_t dtype,
+                                                   b200_stream_t stream) {
+  B200_RETURN_IF(in_scale && !sorted_pair, B200_ERR_NULL_POINTER);
+  return moe_umma_common(true, h, xs, w13, offsets, sorted_pair, nullptr, pairs, hidden, inter, num_local, dtype, stream, 0, in_scale,
+                         kWaitNs, expected);
 }
 
 extern "C" int b200_moe_gemm_gate_up_umma(void* h, const void* xs, const void* w13, const int32_t* offsets,
                                           const int32_t* sorted_pair, const float* in_scale, int32_t pairs,
                                           int32_t hidden, int32_t inter, int32_t num_local, int32_t dtype,
                                           b200_stream_t stream) {
-  B200_RETURN_IF(in_scale && !sorted_pair, B200_ERR_NULL_POINTER);
-  return moe_umma_common(true, h, xs, w13, offsets, sorted_pair, nullptr, pairs, hidden, inter, num_local, dtype,
-                         stream, 0, in_scale);
+  return b200_moe_gemm_gate_up_umma_expected(h, xs, w13, offsets, sorted_pair, in_scale, pairs, pairs, hidden, inter, num_local, dtype,
+                                             stream);
+}
+
+extern "C" int b200_moe_gemm_down_umma_expected(void* y, const void* h, const void* w2, const int32_t* offsets,
+                                                const int32_t* sorted_pair, const void* topk_weights, int32_t pairs, int32_t expected,
+                                                int32_t inter, int32_t hidden, int32_t num_local, int32_t dtype,
+                                                b200_stream_t stream) {
+  return moe_umma_common(false, y, h, w2, offsets, sorted_pair, topk_weights, pairs, inter, hidden, num_local, dtype, stream, 0, nullptr,
+                         kWaitNs, expected);
 }
 
 extern "C" int b200_moe_gemm_down_umma(void* y, const void* h, const void* w2, const int32_t* offsets,
                                        const int32_t* sorted_pair, const void* topk_weights, int32_t pairs,
                                        int32_t inter, int32_t hidden, int32_t num_local, int32_t dtype,
                                        b200_stream_t stream) {
-  return moe_umma_common(false, y, h, w2, offsets, sorted_pair, topk_weights, pairs, inter, hidden, num_local,
-                         dtype, stream);
+  return b200_moe_gemm_down_umma_expected(y, h, w2, offsets, sorted_pair, topk_weights, pairs, pairs, inter, hidden, num_local, dtype,
+                                          stream);
+}
+
+extern "C" int32_t b200_moe_umma_persistent(int32_t gate_up, int32_t expected, int32_t num_local, int32_t n_out) {
+  return num_local > 0 && moe_umma_wide(gate_up != 0, expected, num_local, n_out, 0);
 }
 
 extern "C" int b200_moe_gemm_down_umma_bounded(void* y, const void* h, const void* w2, const int32_t* offsets,

@@ -102,6 +102,11 @@ PROTOTYPES = {
                                         c_int32, c_void_p]),
     "b200_moe_gemm_down_umma": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                           c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p]),
+    "b200_moe_gemm_gate_up_umma_expected": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32,
+                                                      c_int32, c_int32, c_int32, c_int32, c_void_p]),
+    "b200_moe_gemm_down_umma_expected": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32,
+                                                   c_int32, c_int32, c_int32, c_int32, c_void_p]),
+    "b200_moe_umma_persistent": (c_int32, [c_int32, c_int32, c_int32, c_int32]),
     "b200_moe_gemm_down_umma_bounded": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
                                                   c_int32, c_int32, c_int64, c_void_p]),
     "b200_moe_combine": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,

@@ -89,7 +89,7 @@ class SparseMoeBlock(nn.Module):
         tokens, hidden = x.shape
         router_logits = F.linear(x, self.gate.weight)
         topk_ids, topk_w = ops.moe_route(router_logits, self.top_k)
-        plan = ops.moe_align(topk_ids, self.expert_begin, self.num_local)
+        plan = ops.moe_align(topk_ids, self.expert_begin, self.num_local, self.num_experts)
         out = None
         if self.ep_size > 1 and self.defer_allreduce:
             from ..comm import get_comm

@@ -497,15 +497,18 @@ def scores_umma(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor | None =
 class MoePlan:
     """Device-side dispatch plan of one MoE layer call (b200_moe_align): fixed-capacity buffers,
     nothing is read back by the host."""
-    __slots__ = ("offsets", "sorted_pair", "pos_of_pair", "counts", "num_local", "expert_begin", "top_k")
+    __slots__ = ("offsets", "sorted_pair", "pos_of_pair", "counts", "num_local", "expert_begin", "top_k", "local_pairs", "sharded")
 
-    def __init__(self, num_pairs: int, num_local: int, expert_begin: int, top_k: int, device):
+    def __init__(self, num_pairs: int, num_local: int, expert_begin: int, top_k: int, device, num_experts: int | None = None):
         i32 = dict(dtype=torch.int32, device=device)
         self.offsets = torch.empty(num_local + 1, **i32)
         self.sorted_pair = torch.zeros(num_pairs, **i32)     # tail beyond offsets[-1] stays 0 (a valid pair index)
         self.pos_of_pair = torch.empty(num_pairs, **i32)
         self.counts = torch.empty(num_local, **i32)
         self.num_local, self.expert_begin, self.top_k = num_local, expert_begin, top_k
+        num_experts = max(num_experts or 0, expert_begin + num_local)
+        self.local_pairs = num_pairs * num_local // num_experts      # how many of the pairs the local experts can expect
+        self.sharded = num_local < num_experts
 
 
 def moe_route(router_logits: torch.Tensor, top_k: int):
@@ -523,13 +526,14 @@ def moe_route(router_logits: torch.Tensor, top_k: int):
     return ids, w
 
 
-def moe_align(topk_ids: torch.Tensor, expert_begin: int, num_local: int) -> MoePlan:
-    """Pairs (t, j) stably sorted by local expert; see include/b200attn.h."""
+def moe_align(topk_ids: torch.Tensor, expert_begin: int, num_local: int, num_experts: int | None = None) -> MoePlan:
+    """Pairs (t, j) stably sorted by local expert; see include/b200attn.h. num_experts: of the whole layer, where other ranks hold
+    some (by default no more than expert_begin + num_local)."""
     _need_cuda(topk_ids)
     if topk_ids.dtype != torch.int32 or not topk_ids.is_contiguous():
         raise TypeError("topk_ids must be a contiguous int32 tensor")
     T, k = topk_ids.shape
-    plan = MoePlan(T * k, num_local, expert_begin, k, topk_ids.device)
+    plan = MoePlan(T * k, num_local, expert_begin, k, topk_ids.device, num_experts)
     _C.check(_C.load().b200_moe_align(plan.offsets.data_ptr(), plan.sorted_pair.data_ptr(),
                                       plan.pos_of_pair.data_ptr(), plan.counts.data_ptr(),
                                       topk_ids.data_ptr(), T * k, expert_begin, num_local, _stream()),
@@ -559,7 +563,7 @@ def moe_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_ids: 
     pairs = T * k
     lib = _C.load()
     in_w, out_w = (topk_weights, None) if weigh_input else (None, topk_weights)
-    if _MOE_BIG_GEMM != "stream" and pairs >= _moe_big_rows(n_local, hidden * inter) * n_local:
+    if _MOE_BIG_GEMM != "stream" and _moe_big(plan, hidden, inter):
         big = _moe_expert_gemms_umma if _MOE_BIG_GEMM == "umma" else _moe_expert_gemms_library
         y = big(x, w13, w2, out_w, plan, in_w)
         return _moe_combine(lib, y, topk_ids, plan, T, hidden, out, x)
@@ -585,18 +589,40 @@ _MOE_OTHER_BIG_ROWS = 96            # experts without a gate and with the clampe
 
 
 def _moe_big_rows(n_local: int, weights: int) -> int:
-    """The line for gated experts of `weights` = hidden x inter. A layer takes (us, weight-streaming / tcgen05, by rows per expert)
-      2048 x 768, 128 experts  16: 218 / 209, 24: 230 / 216, 32: 257 / 222, 64: 401 / 239, 95: 527 / 259
-      2048 x 768, 64           16: 125 / 117, 32: 148 / 120, 64: 227 / 130
-      1024 x 512, 64           16: 55 / 58, 20: 56.5 / 58.5, 24: 62 / 59, 32: 69 / 60, 64: 99 / 63
-      1024 x 512, 16           16: 26.7 / 28.2, 24: 29.5 / 29.2, 32: 33.5 / 29.2, 64: 46 / 30
-      2048 x 1024, 16          24: 55 / 62, 28: 60 / 62, 32: 64 / 62, 64: 96 / 64
+    """The line for gated experts of `weights` = hidden x inter, in rows that a local expert can expect, where the persistent kernel
+    runs or the 128-column kernels find room for all their CTAs. A layer takes (us, weights not in L2, weight-streaming / tcgen05, by rows)
+      2048 x 768, 128 experts    16: 216 / 209, 24: 231 / 214, 32: 248 / 217, 64: 424 / 233, 96: 548 / 248
+      2048 x 768, 64 and 64 of 128  16: 119 / 113, 32: 141 / 117, 64: 223 / 123
+      2048 x 768, 32 and 32 of 128  8: 71 / 85, 16: 73.6 / 69.6, 32: 91 / 72, 64: 124 / 75
+      1024 x 512, 64             16: 48.6 / 52.5, 24: 57 / 53, 32: 60 / 55, 64: 90 / 56
+      1024 x 512, 16             24: 19.2 / 22.8, 32: 24.3 / 22.8, 64: 48 / 24
+      2048 x 1024, 16            24: 50 / 57, 32: 59 / 57, 64: 90 / 61
+      2048 x 768, 16 of 128      16: 38.7 / 51.9, 24: 39-46 / 54, 32: 55 / 56.5, 48: 57-71 / 60
+      2048 x 1024, 8             24: 30 / 31.6, 32: 37.7 / 32, 64: 59 / 32
     Many experts fill the chip with a 128-row tile each, however few rows it has; below 16 rows the 128-column kernels would run."""
     if _MOE_BIG_GEMM_ROWS is not None:
         return _MOE_BIG_GEMM_ROWS
-    if n_local < 64:
+    if n_local < 32:
         return 32
     return 16 if weights >= 1 << 20 else 24
+
+
+def _moe_big(plan: MoePlan, hidden: int, inter: int) -> bool:
+    """Do gated experts take the tcgen05 side? (us as above.)
+    A few experts of many, a plan most of whose pairs are other ranks', pay for the tcgen05 side earlier (their weight-streaming products take a
+    quarter more than as many experts that are all there are):
+      2048 x 768, 8 of 128   2: 24-27 / 25, 4: 26.7 / 26.7, 8: 35 / 27, 32: 50 / 31; 2048 x 1024, 8 of 64   4: 36 / 28, 16: 36 / 31; 2048 x 512, 8 of 256   4: 24.2 / 23.8, 8: 28.7 / 24.9
+      1024 x 512, 4 of 64   16: 17.2 / 17.4, 24: 19.8 / 17.5; 8 of 16   16: 16.8 / 19.0, 24: 19.8 / 19.2; 16 of 64   16: 23.4 / 22.5, 24: 24-30 / 23.6
+      4096 x 1792, 8 of 64   8: 70 / 82, 24: 72 / 84, 32: 102 / 85 (as 8 of 8)"""
+    n, weights = plan.num_local, hidden * inter
+    rows = plan.local_pairs // n
+    line = _moe_big_rows(n, weights)
+    if _MOE_BIG_GEMM_ROWS is None:
+        if plan.sharded and n < 32 and weights < 1 << 20:
+            line = 24
+        elif plan.sharded and n <= 8 and weights <= 1 << 21:
+            line = 4
+    return rows >= line
 
 
 def _moe_expert_gemms_umma(x, w13, w2, topk_weights, plan: MoePlan, in_weights=None) -> torch.Tensor:
@@ -612,13 +638,14 @@ def _moe_expert_gemms_umma(x, w13, w2, topk_weights, plan: MoePlan, in_weights=N
                                       plan.sorted_pair.data_ptr(), pairs, n_local, k, hidden,
                                       x.stride(0) if T > 1 else hidden, _dt(x), _stream()),
              "b200_moe_gather_rows")
-    _C.check(lib.b200_moe_gemm_gate_up_umma(h.data_ptr(), xs.data_ptr(), w13.data_ptr(),
-                                            plan.offsets.data_ptr(), plan.sorted_pair.data_ptr(), _ptr(in_weights),
-                                            pairs, hidden, inter, n_local, _dt(x), _stream()),
+    _C.check(lib.b200_moe_gemm_gate_up_umma_expected(h.data_ptr(), xs.data_ptr(), w13.data_ptr(),
+                                                     plan.offsets.data_ptr(), plan.sorted_pair.data_ptr(), _ptr(in_weights),
+                                                     pairs, plan.local_pairs, hidden, inter, n_local, _dt(x), _stream()),
              "b200_moe_gemm_gate_up_umma")
-    _C.check(lib.b200_moe_gemm_down_umma(y.data_ptr(), h.data_ptr(), w2.data_ptr(), plan.offsets.data_ptr(),
-                                         plan.sorted_pair.data_ptr() if topk_weights is not None else None,
-                                         _ptr(topk_weights), pairs, inter, hidden, n_local, _dt(x), _stream()),
+    _C.check(lib.b200_moe_gemm_down_umma_expected(y.data_ptr(), h.data_ptr(), w2.data_ptr(), plan.offsets.data_ptr(),
+                                                  plan.sorted_pair.data_ptr() if topk_weights is not None else None,
+                                                  _ptr(topk_weights), pairs, plan.local_pairs, inter, hidden, n_local, _dt(x),
+                                                  _stream()),
              "b200_moe_gemm_down_umma")
     return y
 

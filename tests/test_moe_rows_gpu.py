@@ -34,3 +34,24 @@ def test_both_sides_of_the_line(experts, top, hidden, inter, rows, skewed, monke
     # products and sums of bf16 roundings
     assert float((got - want).norm() / want.norm()) < 1e-2
     assert float((got - other).norm() / other.norm()) < 1e-2
+
+
+@pytest.mark.parametrize("experts,ranks,tokens", [(16, 4, 256), (64, 2, 512), (16, 2, 1500)])
+def test_shares_of_the_ranks_add_up(experts, ranks, tokens):
+    """Expert parallelism with skewed routing: a rank gets more rows than the ones that its kernels were chosen for, others none."""
+    from nanovllm import ops
+    top, hidden, inter = 4, 512, 256
+    g = torch.Generator(device="cuda").manual_seed(experts)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    x, logits = rand(tokens, hidden).bfloat16(), rand(tokens, experts)
+    logits[:, :experts // ranks] += 8
+    w13, w2 = (rand(experts, 2 * inter, hidden) * hidden ** -0.5).bfloat16(), (rand(experts, hidden, inter) * inter ** -0.5).bfloat16()
+    ids, weights = ops.moe_route(logits.bfloat16(), top)
+    want = ops.moe_experts(x, w13, w2, ids, weights, ops.moe_align(ids, 0, experts)).float()
+    n, got, sides = experts // ranks, torch.zeros(tokens, hidden, device="cuda"), set()
+    for r in range(ranks):
+        plan = ops.moe_align(ids, r * n, n, experts)
+        sides.add(ops._moe_big(plan, hidden, inter))
+        got += ops.moe_experts(x, w13[r * n:(r + 1) * n].contiguous(), w2[r * n:(r + 1) * n].contiguous(), ids, weights, plan).float()
+    assert sides == {True}
+    assert float((got - want).norm() / want.norm()) < 1e-2     # sums of bf16 roundings
