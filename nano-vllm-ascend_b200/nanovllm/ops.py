@@ -608,7 +608,12 @@ def _moe_big_rows(n_local: int, weights: int) -> int:
 
 
 def _moe_big(plan: MoePlan, hidden: int, inter: int) -> bool:
-    """Do gated experts take the tcgen05 side? (us as above.)
+    """Do gated experts take the tcgen05 side? (us as above.) Where a product of 32 experts or more runs on the 128-column kernels, the
+    line is higher:
+      only down persistent: 4096 x 256, 64 experts   24: 101 / 108, 32: 115 / 113, 64: 186 / 122; 2048 x 704, 128   24: 217 / 266, 32: 231 / 226, 48: 287 / 240
+      only gate and up: 1920 x 768, 128   32: 256 / 266, 48: 281 / 290, 64: 372 / 309; of 64   32: 135 / 143, 48: 150 / 132
+      neither, all CTAs at once: 1024 x 512, 32   32: 36.5 / 42, 48: 44.2 / 43.5
+      neither: 1152 x 576, 64   48: 74 / 107, 64: 108 / 112, 72: 112 / 91; of 128   72: 207 / 217, 96: 244 / 247; 640 x 448, 64   64: 63 / 70, 72: 70 / 71.5, 80: 76 / 74
     A few experts of many, a plan most of whose pairs are other ranks', pay for the tcgen05 side earlier (their weight-streaming products take a
     quarter more than as many experts that are all there are):
       2048 x 768, 8 of 128   2: 24-27 / 25, 4: 26.7 / 26.7, 8: 35 / 27, 32: 50 / 31; 2048 x 1024, 8 of 64   4: 36 / 28, 16: 36 / 31; 2048 x 512, 8 of 256   4: 24.2 / 23.8, 8: 28.7 / 24.9
@@ -622,6 +627,11 @@ def _moe_big(plan: MoePlan, hidden: int, inter: int) -> bool:
             line = 24
         elif plan.sharded and n <= 8 and weights <= 1 << 21:
             line = 4
+        elif n >= 32 and line <= rows < 72:
+            wide = _C.load().b200_moe_umma_persistent
+            gate_up, down = wide(1, plan.local_pairs, n, inter), wide(0, plan.local_pairs, n, hidden)
+            if not (gate_up and down):
+                line = 32 if down else 48 if gate_up or n * max(inter // 64, hidden // 128) <= 296 else 72
     return rows >= line
 
 

@@ -13,7 +13,8 @@ def _plan(tokens, top, experts, ranks=1):
     (128, 8, 2048, 768, 1, 16), (128, 8, 2048, 768, 2, 16), (128, 8, 2048, 768, 4, 16), (128, 8, 2048, 768, 8, 32),
     (128, 8, 2048, 768, 16, 4),                       # 8 of 128
     (64, 4, 1024, 512, 1, 24), (64, 4, 1024, 512, 4, 24), (16, 2, 1024, 512, 1, 32), (8, 2, 2048, 1024, 1, 32),
-    (64, 8, 4096, 1792, 8, 32)])
+    (64, 4, 4096, 256, 1, 32), (128, 8, 2048, 704, 1, 32), (128, 8, 1920, 768, 1, 48), (64, 4, 1152, 576, 1, 72),
+    (32, 4, 1024, 512, 1, 48), (64, 8, 4096, 1792, 8, 32)])
 def test_the_line_is_in_rows_of_a_local_expert(experts, top, hidden, inter, ranks, line):
     from nanovllm import ops
     for rows, side in ((line - 1, False), (line, True), (line + 1, True), (1000, True), (1, False)):
