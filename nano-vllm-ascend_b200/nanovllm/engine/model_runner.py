@@ -601,7 +601,8 @@ class ModelRunner:
     # ------------------------------------------------------------------ run
     @staticmethod
     def _tokens(out: torch.Tensor) -> list[int]:
-        """The sampled tokens of a prompt step on the host, where no kernel of the step gave up a wait."""
+        """The sampled tokens of a step on the host, where no kernel of the step gave up a wait (a replayed decode step's too: its
+        grouped products' own entry points do not run)."""
         tokens = out.tolist()
         ops.check_waits()
         return tokens
@@ -659,9 +660,12 @@ class ModelRunner:
             if not logit_rows:
                 # the next step refills the pinned staging buffer: this step's upload must have left it
                 torch.cuda.current_stream().synchronize()
+                ops.check_waits()
                 return None
-            return self.d_logits[torch.tensor(logit_rows, dtype=torch.int64, device=self.device)].cpu()
+            logits = self.d_logits[torch.tensor(logit_rows, dtype=torch.int64, device=self.device)].cpu()
+            ops.check_waits()
+            return logits
         self.h_out[:n].copy_(self.d_out[:n], non_blocking=True)
         self.d2h_bytes += n * 8
         torch.cuda.current_stream().synchronize()
-        return self.h_out[:n].tolist()
+        return self._tokens(self.h_out[:n])

@@ -64,7 +64,7 @@ def launch_count() -> int:
 
 def check_waits() -> None:
     """Raises if a bounded wait ran out in a kernel that has finished since the last question: what that kernel was to write
-    is not valid. The engine asks once a prompt step's results are on the host."""
+    is not valid. The engine asks once a step's results are on the host."""
     _C.check(_C.load().b200_take_wait_status(), "a kernel of this step")
 
 
