@@ -8,6 +8,7 @@ absent, ``layers/attention.py:2-3`` of the reference).
 from __future__ import annotations
 
 import ctypes
+import logging
 import os
 from ctypes import c_char_p, c_double, c_float, c_int32, c_int64, c_size_t, c_uint64, c_void_p
 
@@ -269,25 +270,41 @@ def load() -> ctypes.CDLL:
     return lib
 
 
-_calls = None
+_calls = None          # the module; False: it cannot be had
+
+
+def calls_path() -> str:
+    """The native calls beside the library, built against this torch and this interpreter (csrc/Makefile names them so)."""
+    import sysconfig
+
+    import torch
+    name = "_b200calls-" + torch.__version__.replace("+", "_") + sysconfig.get_config_var("EXT_SUFFIX")
+    return os.path.join(os.path.dirname(lib_path()), name)
 
 
 def calls():
-    """The native calls of the attention entry points (csrc/host_calls.cpp), bound to the library's functions."""
+    """The native calls of the attention entry points (csrc/host_calls.cpp), bound to the library's functions; None where there are none:
+    ops goes through ctypes then, which is a few microseconds slower and needs the library alone."""
     global _calls
     if _calls is None:
         import importlib.util
-        path = os.path.join(os.path.dirname(DEFAULT_LIB_PATH), "_b200calls.so")
-        if not os.path.exists(path):
-            raise B200Error(f"_b200calls.so not found at {path}: build it as libb200attn.so is built")
-        spec = importlib.util.spec_from_file_location("_b200calls", path)
-        module = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(module)
-        lib = load()
+        try:
+            lib = load()
+        except B200Error:
+            return None                            # ops says what is missing
+        path = calls_path()
+        try:
+            spec = importlib.util.spec_from_file_location("_b200calls", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+        except (ImportError, OSError) as e:
+            logging.getLogger(__name__).warning("no native calls (%s): attention goes through ctypes", e)
+            _calls = False
+            return None
         module.bind(*(ctypes.cast(f, c_void_p).value for f in (lib.b200_paged_decode_attn_windowed, lib.b200_paged_decode_attn_fp8,
                                                                lib.b200_prefill_varlen_attn_windowed)))
         _calls = module
-    return _calls
+    return _calls or None
 
 
 def check(code: int, what: str) -> None:

@@ -152,9 +152,9 @@ def paged_decode_attn(q, k_cache, v_cache, block_tables, context_lens, scale, nu
     softcap > 0: scores become softcap * tanh(score / softcap); sink fp32 [H]: exp(sink[h]) joins the softmax denominator
     (no key, no value). window > 0: a row sees its last `window` keys and those below keep_first; chunk > 0 (without a
     window): the keys of its own chunk, counted from position 0."""
-    if out is None and workspace is None and sink is None and vdim is None:
-        got = _C.calls().decode(decode_workspace, q, k_cache, v_cache, block_tables, context_lens, scale, num_kv_heads, num_ctas,
-                                softcap, window, keep_first, chunk)
+    if out is None and workspace is None and sink is None and vdim is None and (calls := _C.calls()) is not None:
+        got = calls.decode(decode_workspace, q, k_cache, v_cache, block_tables, context_lens, scale, num_kv_heads, num_ctas,
+                           softcap, window, keep_first, chunk)
         if got is not None:                        # None: not quite what that call takes
             return got if type(got) is not int else _C.check(got, "b200_paged_decode_attn")
     _need_cuda(q, k_cache, v_cache, block_tables, context_lens, sink)
@@ -188,9 +188,9 @@ def paged_decode_attn(q, k_cache, v_cache, block_tables, context_lens, scale, nu
 def paged_decode_attn_fp8(q, k_cache, v_cache, block_tables, context_lens, scale, num_kv_heads,
                           k_scale=1.0, v_scale=1.0, out=None, workspace=None, num_ctas=0):
     """K6 over an e4m3 cache. q [B, H, D] bf16/fp16 -> out [B, H*D] in q's dtype."""
-    if out is None and workspace is None:
-        got = _C.calls().decode_fp8(decode_workspace, q, k_cache, v_cache, block_tables, context_lens, scale, num_kv_heads, num_ctas,
-                                    k_scale, v_scale)
+    if out is None and workspace is None and (calls := _C.calls()) is not None:
+        got = calls.decode_fp8(decode_workspace, q, k_cache, v_cache, block_tables, context_lens, scale, num_kv_heads, num_ctas,
+                               k_scale, v_scale)
         if got is not None:
             return got if type(got) is not int else _C.check(got, "b200_paged_decode_attn_fp8")
     _need_cuda(q, k_cache, v_cache, block_tables, context_lens)
@@ -263,10 +263,10 @@ def prefill_varlen_attn(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_s
     split-KV workspace), None (never split the keys across CTAs) or a uint8 CUDA tensor. softcap, sink, vdim, window,
     keep_first, chunk as in paged_decode_attn (the tcgen05 kernel only); position i sees j <= i with i - j < window or
     j < keep_first, or with j // chunk == i // chunk."""
-    if out is None and vdim is None and q.is_cuda and (workspace is None or isinstance(workspace, str)):
+    if out is None and vdim is None and q.is_cuda and (workspace is None or isinstance(workspace, str)) and (calls := _C.calls()) is not None:
         ws = prefill_workspace(q.device, q.shape[-1]) if workspace is not None else None
-        got = _C.calls().prefill(ws, q, k, v, cu_seqlens_q, cu_seqlens_k, block_tables, max_seqlen_q, max_seqlen_k, scale, num_kv_heads,
-                                 softcap, sink, window, keep_first, chunk)
+        got = calls.prefill(ws, q, k, v, cu_seqlens_q, cu_seqlens_k, block_tables, max_seqlen_q, max_seqlen_k, scale, num_kv_heads,
+                            softcap, sink, window, keep_first, chunk)
         if got is not None:
             return got if type(got) is not int else _C.check(got, "b200_prefill_varlen_attn")
     _need_cuda(q, k, v, cu_seqlens_q, cu_seqlens_k, block_tables, sink)

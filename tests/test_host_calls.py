@@ -21,6 +21,38 @@ def test_nothing_but_cuda_tensors_and_numbers():
         ops.paged_decode_attn(t, t, t, t, t, 1.0, 8)
 
 
+def test_without_the_module_ops_goes_its_own_way(monkeypatch, tmp_path, caplog):
+    from nanovllm import _C, ops
+    assert _C.calls() is not None
+    t = torch.zeros(1, 16, 128, dtype=torch.bfloat16)
+    _C.load()
+    monkeypatch.setenv("B200ATTN_LIB", str(tmp_path / "libb200attn.so"))      # a library elsewhere, without native calls beside it
+    for there in (None, "not a module"):
+        if there:
+            open(_C.calls_path(), "w").write(there)
+        monkeypatch.setattr(_C, "_calls", None)
+        caplog.clear()
+        assert _C.calls() is None and _C.calls() is None and len(caplog.records) == 1
+        with pytest.raises(RuntimeError, match="CUDA only"):
+            ops.paged_decode_attn(t, t, t, t, t, 1.0, 8)
+        with pytest.raises(RuntimeError, match="CUDA only"):
+            ops.prefill_varlen_attn(t, t, t, t, t, 1, 1, 1.0, 8)
+    monkeypatch.setattr(_C, "_calls", None)
+    monkeypatch.setattr(_C, "_lib", None)                                     # and none at all
+    assert _C.calls() is None
+    with pytest.raises(RuntimeError, match="CUDA only"):
+        ops.paged_decode_attn_fp8(t, t, t, t, t, 1.0, 8)
+
+
+@pytest.mark.gpu
+def test_without_the_module_the_answer_is_the_same(monkeypatch):
+    from nanovllm import _C, ops
+    q, k, v, tables, lens = _step()
+    want = ops.paged_decode_attn(q, k, v, tables, lens, 0.125, 2)
+    monkeypatch.setattr(_C, "_calls", False)
+    assert torch.equal(ops.paged_decode_attn(q, k, v, tables, lens, 0.125, 2), want)
+
+
 def _step(dtype=torch.bfloat16, fp8=False, B=3, H=8, G=2, D=64, bs=16):
     g = torch.Generator(device="cuda").manual_seed(B)
     q = torch.randn(B, H + 2, D, device="cuda", generator=g).to(dtype)[:, :H]             # a token-strided view
