@@ -61,8 +61,9 @@ const char* b200_error_string(int code);
  * (host-side counter; lets bench.py report `gpu_launches`). */
 int64_t b200_launch_count(void);
 void b200_reset_launch_count(void);
-/* Waits of the persistent grouped GEMM (b200_moe_gemm_*_umma on prompt-sized batches) are bounded. When one runs out, the
- * kernel returns without having written its output and sets a word of page-locked host memory. b200_take_wait_status asks
+/* Waits inside the persistent grouped GEMM (b200_moe_gemm_*_umma), b200_linear_recurrence_step and b200_attn_generic_step on tensor-core
+ * prompts are bounded. When one runs out, the kernel returns without having written its output (a recurrence may have written part of its
+ * state) and sets a word of page-locked host memory. b200_take_wait_status asks
  * and clears it: B200_ERR_WAIT or B200_OK, meaningful for kernels that the host has waited for. The same entry points ask it
  * first of all, so that a call after the failed one returns B200_ERR_WAIT. b200_wait_status_word: the word itself. */
 int b200_take_wait_status(void);
@@ -622,6 +623,15 @@ int b200_attn_generic_step(void* out, const void* q, int64_t q_stride, const voi
                       int32_t num_seqs, int32_t max_q, int32_t num_heads, int32_t num_kv_heads, int32_t dim,
                       int32_t vdim, float scale, int32_t window, int32_t keep_first, int32_t chunk, float softcap,
                       const float* sink, const void* gate, int64_t gate_stride, int32_t dtype, int64_t total_q, b200_stream_t stream);
+/* and with its own limit on a single wait of the tensor-core kernel, in steps of about 4 us. 0 is how the way
+ * out is tested: tiles stop coming after the first few, and the waits for them give up. */
+int b200_attn_generic_bounded(void* out, const void* q, int64_t q_stride, const void* k, int64_t k_stride,
+                      const void* v, int64_t v_stride, const int32_t* block_tables, int32_t bt_stride,
+                      int32_t block_size, const int32_t* cu_q, const int32_t* cu_k, const int32_t* ctx_lens,
+                      int32_t num_seqs, int32_t max_q, int32_t num_heads, int32_t num_kv_heads, int32_t dim,
+                      int32_t vdim, float scale, int32_t window, int32_t keep_first, int32_t chunk, float softcap,
+                      const float* sink, const void* gate, int64_t gate_stride, int32_t dtype, int64_t total_q, int64_t wait_ns,
+                      b200_stream_t stream);
 
 /* Per head S_t = a_t S_(t-1) + k_t (b_t v_t)^T, o_t = S_t^T q_t; S fp32 [kdim, vdim] in state
  * [slots, H, kdim, vdim]. q, k [T, groups*kdim] (head h reads group h / (H / groups)), v [T, H*vdim];
@@ -651,6 +661,17 @@ int b200_linear_recurrence_step(float* out, const void* q, int64_t q_stride, con
                            int32_t mode, int32_t act_silu, const float* decay, const void* dt,
                            int64_t dt_stride, const float* dt_bias, const float* a_log, const float* d_skip,
                            int32_t qk_f32, int32_t dtype, int64_t total_q, b200_stream_t stream);
+/* and with its own limit on a single wait of the tensor-core kernel, in steps of about 4 us. 0 is how the way
+ * out is tested: tiles stop coming after the first few, and the waits for them give up. */
+int b200_linear_recurrence_bounded(float* out, const void* q, int64_t q_stride, const void* k, int64_t k_stride,
+                           const void* v, int64_t v_stride, float* state, const int32_t* state_slots,
+                           const int32_t* cu_q, const int32_t* cu_k, const int32_t* ctx_lens,
+                           int32_t num_seqs, int32_t max_q, int32_t num_heads, int32_t groups, int32_t kdim,
+                           int32_t vdim,
+                           int32_t mode, int32_t act_silu, const float* decay, const void* dt,
+                           int64_t dt_stride, const float* dt_bias, const float* a_log, const float* d_skip,
+                           int32_t qk_f32, int32_t dtype, int64_t total_q, int64_t wait_ns,
+                      b200_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------------
  * Multi-stream residuals, rotary positions, delta rule, latent attention, clamped gated unit

@@ -39,7 +39,7 @@ constexpr float kAsUp = 134217728.f;                    // 2^27: values come to 
 
 struct AttnSplitParams {
   AttnTiledParams a;
-  int wait_tries;                                      // of one wait, 4 us each
+  int wait_tries;                                      // of one wait
   int* wait_status;
 };
 
@@ -117,14 +117,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
   __syncthreads();
   umma::fence_after_sync();
   constexpr uint32_t tb = 0;                            // all 512 columns: they start at 0
-  // whole warps wait, and leave together
-  auto wait = [&](uint64_t* bar, int parity) {
-    int left = AP.wait_tries;
-    while (!mbar_try_wait(bar, parity & 1) && --left >= 0) {
-    }
-    if (left < 0) *gave_up = 1;
-    return __all_sync(0xffffffffu, left >= 0) != 0;
-  };
+  auto wait = [&](uint64_t* bar, int parity) { return mbar_warp_wait(bar, parity & 1, AP.wait_tries, gave_up); };
 
   // Registers: 640 x 96 at launch = 128 x (112 softmax + 160 sums + 2 x 80 copies + 48)
   if (warp < 4) {
@@ -341,8 +334,9 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       if (st + kAhead + 1 < steps) look_up(st + kAhead + 1);
       return true;
     };
+    const int come = AP.wait_tries > 0 ? steps : min(steps, 4);       // (a limit of 0 tests the way out: nothing comes any more)
 #pragma unroll 1
-    for (int st = 0; st < steps; st += kAhead) {        // (steps is even)
+    for (int st = 0; st < come; st += kAhead) {         // (steps is even)
       if (!put(st, x0)) break;
       if (kAhead == 2 && !put(st + 1, x1)) break;
     }
@@ -476,25 +470,25 @@ bool attn_split_fits(const AttnTiledParams& P, int num_seqs, int max_q, int64_t 
 }
 
 template <int DK, int DV>
-static int attn_split_launch_as(const AttnTiledParams& P, dim3 grid, cudaStream_t stream) {
+static int attn_split_launch_as(const AttnTiledParams& P, dim3 grid, int64_t wait_ns, cudaStream_t stream) {
   auto kern = attn_split_kernel<DK, DV>;
   constexpr int smem = as_smem<DK, DV>();
   static_assert(smem <= 227 * 1024, "one CTA's shared memory");
   static std::atomic<uint64_t> devices{0};
   const cudaError_t allowed = allow_smem(kern, smem, devices);
   if (allowed != cudaSuccess) return (int)allowed;
-  const AttnSplitParams AP{P, 1 << 20, wait_status()};
+  const AttnSplitParams AP{P, wait_tries(wait_ns), wait_status()};
   B200_RETURN_IF(AP.wait_status == nullptr, B200_ERR_DRIVER);
   launch_pdl(kern, grid, dim3(kAsThreads), (size_t)smem, stream, AP);
   return finish_launch();
 }
 
-int attn_split_launch(AttnTiledParams P, int num_seqs, int max_q, cudaStream_t stream) {
+int attn_split_launch(AttnTiledParams P, int num_seqs, int max_q, int64_t wait_ns, cudaStream_t stream) {
   B200_RETURN_IF(take_wait_status(), B200_ERR_WAIT);             // of an earlier call
   P.num_seqs = num_seqs;
   const dim3 grid((unsigned)(((int64_t)max_q * (P.H / P.G) + kAsM - 1) / kAsM * P.G * num_seqs));
-  if (P.dim <= 64) return P.vdim <= 64 ? attn_split_launch_as<64, 64>(P, grid, stream) : attn_split_launch_as<64, 128>(P, grid, stream);
-  return P.vdim <= 64 ? attn_split_launch_as<128, 64>(P, grid, stream) : attn_split_launch_as<128, 128>(P, grid, stream);
+  if (P.dim <= 64) return P.vdim <= 64 ? attn_split_launch_as<64, 64>(P, grid, wait_ns, stream) : attn_split_launch_as<64, 128>(P, grid, wait_ns, stream);
+  return P.vdim <= 64 ? attn_split_launch_as<128, 64>(P, grid, wait_ns, stream) : attn_split_launch_as<128, 128>(P, grid, wait_ns, stream);
 }
 
 }  // namespace b200

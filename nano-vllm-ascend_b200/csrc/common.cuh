@@ -245,6 +245,19 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   if (gave_up != nullptr) *gave_up = 1;
   return false;
 }
+// The same counted in tries, a try being suspended for up to 4 us (measured): less code than a clock, for roles that go round a loop per
+// tile. Whole warps wait, and leave together. Nobody looks at gave_up on the way: roles that wait for one that has left started
+// to wait when it did, and their own count ends with its; a look per failed try cost 4 to 8 % (recurrence_umma_kernel 132 -> 138 us,
+// attn_split_kernel 66 -> 72), and so did a test without suspension before the first (143, 71)
+constexpr int64_t kTryNs = 4000;
+__device__ __forceinline__ bool mbar_warp_wait(uint64_t* bar, uint32_t parity, int tries, volatile int* gave_up) {
+  int left = tries;
+  while (!mbar_try_wait(bar, parity) && --left >= 0) {
+  }
+  if (left < 0) *gave_up = 1;
+  return __all_sync(0xffffffffu, left >= 0) != 0;
+}
+inline int wait_tries(int64_t limit_ns) { return (int)((limit_ns < 1000000 * kTryNs ? limit_ns + kTryNs - 1 : 1000000 * kTryNs) / kTryNs); }
 // generic-proxy writes to smem must be fenced before the async proxy (TMA) may overwrite
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -53,6 +53,6 @@ __device__ __forceinline__ float bits_f32(uint32_t b16) { return __uint_as_float
 // The form on the 5th-generation tensor cores (recurrence_umma.cu), for chunks of 64 tokens. total_q: the step's tokens, 0 if the
 // caller has not said
 bool recurrence_umma_ok(const RecParams& P, int dtype, int num_seqs, int max_q, int64_t total_q);
-int recurrence_umma_launch(const RecParams& P, int num_seqs, cudaStream_t stream);
+int recurrence_umma_launch(const RecParams& P, int num_seqs, int64_t wait_ns, cudaStream_t stream);
 
 }  // namespace b200

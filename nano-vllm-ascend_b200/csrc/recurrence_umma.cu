@@ -30,8 +30,8 @@
 // A value x that is not finite spoils all outputs of its channel in its chunk, the tokens before it too (0 x inf), as in
 // chunk_recurrence_kernel, whose chunks are half as long.
 //
-// Waits are bounded as in moe_umma_wide_kernel: one that runs out makes every role leave its loop, the products under way are
-// waited for, the CTA sets the host's word and the library reports it.
+// Waits are bounded (mbar_warp_wait): one that runs out makes its role leave its loop, those that wait for that role run out as well, the
+// products under way are waited for, the CTA sets the host's word and the library reports it.
 #include <type_traits>
 
 #include "recurrence.cuh"
@@ -58,7 +58,7 @@ struct RuDecay {                                       // of one head and chunk;
 
 struct RuParams {
   RecParams r;
-  int wait_tries;                                      // of one wait, 4 us each
+  int wait_tries;                                      // of one wait
   int* wait_status;
 };
 
@@ -169,20 +169,14 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
   umma::fence_after_sync();
   constexpr uint32_t tb = 0;                            // all 512 columns: they start at 0
   const int chunks = (sp.q_len + kRuL - 1) / kRuL;
-  // Whole warps wait, and leave together. A try is suspended for up to 4 us (measured); counting them takes less code than a clock
-  auto wait = [&](uint64_t* bar, int parity) {
-    int left = RP.wait_tries;
-    while (!mbar_try_wait(bar, parity & 1) && --left >= 0) {
-    }
-    if (left < 0) *gave_up = 1;
-    return __all_sync(0xffffffffu, left >= 0) != 0;
-  };
+  auto wait = [&](uint64_t* bar, int parity) { return mbar_warp_wait(bar, parity & 1, RP.wait_tries, gave_up); };
   // Copies: k and x of chunk j (kQ false) once the products of chunk j - 2 that read them have retired, or q; thread li of kThreads
   auto copies = [&](auto is_q, auto threads, int li) {
     constexpr bool kQ = decltype(is_q)::value;
     constexpr int kThreads = decltype(threads)::value;
     uint64_t *full = kQ ? q_full : k_full, *empty = kQ ? q_empty : k_empty;
-    for (int j = 0; j < chunks; ++j) {
+    const int come = RP.wait_tries > 0 ? chunks : min(chunks, 2);     // (a limit of 0 tests the way out: nothing comes any more)
+    for (int j = 0; j < come; ++j) {
       if (j >= 2 && !wait(&empty[j & 1], (j >> 1) - 1)) break;
       const int nt = min(kRuL, sp.q_len - j * kRuL);
       const int64_t tok0 = sp.q_start + j * kRuL;
@@ -611,26 +605,26 @@ bool recurrence_umma_ok(const RecParams& P, int dtype, int num_seqs, int max_q, 
 }
 
 template <int D, int NH, int MODE, bool SILU>
-static int recurrence_umma_launch_as(const RecParams& P, int num_seqs, cudaStream_t stream) {
+static int recurrence_umma_launch_as(const RecParams& P, int num_seqs, int64_t wait_ns, cudaStream_t stream) {
   auto kern = recurrence_umma_kernel<D, NH, MODE, SILU>;
   constexpr int smem = ru_smem<D, NH>();
   static_assert(smem <= 227 * 1024, "one CTA's shared memory");
   static std::atomic<uint64_t> devices{0};
   const cudaError_t allowed = allow_smem(kern, smem, devices);
   if (allowed != cudaSuccess) return (int)allowed;
-  const RuParams RP{P, 1 << 20, wait_status()};
+  const RuParams RP{P, wait_tries(wait_ns), wait_status()};
   B200_RETURN_IF(RP.wait_status == nullptr, B200_ERR_DRIVER);
   launch_pdl(kern, dim3((unsigned)(P.H / NH), (unsigned)num_seqs), dim3(kRuThreads), (size_t)smem, stream, RP);
   return finish_launch();
 }
 
-int recurrence_umma_launch(const RecParams& P, int num_seqs, cudaStream_t stream) {
+int recurrence_umma_launch(const RecParams& P, int num_seqs, int64_t wait_ns, cudaStream_t stream) {
   B200_RETURN_IF(take_wait_status(), B200_ERR_WAIT);             // of an earlier call
 #define B200_RU(D, NH)                                                                                                   \
-  (P.mode == 1 ? (P.act_silu ? recurrence_umma_launch_as<D, NH, 1, true>(P, num_seqs, stream)                            \
-                             : recurrence_umma_launch_as<D, NH, 1, false>(P, num_seqs, stream))                          \
-               : (P.act_silu ? recurrence_umma_launch_as<D, NH, 0, true>(P, num_seqs, stream)                            \
-                             : recurrence_umma_launch_as<D, NH, 0, false>(P, num_seqs, stream)))
+  (P.mode == 1 ? (P.act_silu ? recurrence_umma_launch_as<D, NH, 1, true>(P, num_seqs, wait_ns, stream)                            \
+                             : recurrence_umma_launch_as<D, NH, 1, false>(P, num_seqs, wait_ns, stream))                          \
+               : (P.act_silu ? recurrence_umma_launch_as<D, NH, 0, true>(P, num_seqs, wait_ns, stream)                            \
+                             : recurrence_umma_launch_as<D, NH, 0, false>(P, num_seqs, wait_ns, stream)))
   if (P.vdim == 128) return P.kdim <= 64 ? B200_RU(64, 1) : B200_RU(128, 1);
   return P.kdim <= 64 ? B200_RU(64, 2) : B200_RU(128, 2);
 #undef B200_RU

@@ -744,13 +744,15 @@ static int recurrence_launch(const RecParams& P, int num_seqs, cudaStream_t stre
 
 using namespace b200;
 
-extern "C" int b200_attn_generic_step(void* out, const void* q, int64_t q_stride, const void* k, int64_t k_stride,
+extern "C" int b200_attn_generic_bounded(void* out, const void* q, int64_t q_stride, const void* k, int64_t k_stride,
                                  const void* v, int64_t v_stride, const int32_t* block_tables,
                                  int32_t bt_stride, int32_t block_size, const int32_t* cu_q,
                                  const int32_t* cu_k, const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q,
                                  int32_t num_heads, int32_t num_kv_heads, int32_t dim, int32_t vdim,
                                  float scale, int32_t window, int32_t keep_first, int32_t chunk, float softcap,
-                                 const float* sink, const void* gate, int64_t gate_stride, int32_t dtype, int64_t total_q, b200_stream_t stream) {
+                                 const float* sink, const void* gate, int64_t gate_stride, int32_t dtype, int64_t total_q, int64_t wait_ns,
+                                 b200_stream_t stream) {
+  B200_RETURN_IF(wait_ns < 0, B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(num_seqs < 0 || max_q < 0 || num_heads <= 0 || num_kv_heads <= 0 || dim <= 0 || vdim <= 0 ||
                      num_heads % num_kv_heads != 0, B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(vdim > 32 * kAttnMaxVChunks, B200_ERR_UNSUPPORTED);
@@ -767,7 +769,7 @@ extern "C" int b200_attn_generic_step(void* out, const void* q, int64_t q_stride
     A.block_tables = block_tables, A.bt_stride = bt_stride, A.block_size = block_size, A.cu_q = cu_q, A.cu_k = cu_k;
     A.H = num_heads, A.G = num_kv_heads, A.dim = dim, A.vdim = vdim, A.scale = scale, A.window = window;
     A.keep_first = keep_first, A.chunk = chunk, A.softcap = softcap, A.sink = sink, A.gate = gate, A.gate_stride = gate_stride;
-    if (attn_split_fits(A, num_seqs, max_q, total_q, dtype)) return attn_split_launch(A, num_seqs, max_q, (cudaStream_t)stream);
+    if (attn_split_fits(A, num_seqs, max_q, total_q, dtype)) return attn_split_launch(A, num_seqs, max_q, wait_ns, (cudaStream_t)stream);
     return attn_tiled_launch(A, num_seqs, max_q, dtype, (cudaStream_t)stream);
   }
   const dim3 grid((max_q * rep + kAttnRows - 1) / kAttnRows, num_kv_heads, num_seqs);
@@ -784,6 +786,18 @@ extern "C" int b200_attn_generic_step(void* out, const void* q, int64_t q_stride
   return finish_launch();
 }
 
+extern "C" int b200_attn_generic_step(void* out, const void* q, int64_t q_stride, const void* k, int64_t k_stride,
+                                 const void* v, int64_t v_stride, const int32_t* block_tables,
+                                 int32_t bt_stride, int32_t block_size, const int32_t* cu_q,
+                                 const int32_t* cu_k, const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q,
+                                 int32_t num_heads, int32_t num_kv_heads, int32_t dim, int32_t vdim,
+                                 float scale, int32_t window, int32_t keep_first, int32_t chunk, float softcap,
+                                 const float* sink, const void* gate, int64_t gate_stride, int32_t dtype, int64_t total_q, b200_stream_t stream) {
+  return b200_attn_generic_bounded(out, q, q_stride, k, k_stride, v, v_stride, block_tables, bt_stride, block_size, cu_q, cu_k,
+          ctx_lens, num_seqs, max_q, num_heads, num_kv_heads, dim, vdim, scale, window, keep_first, chunk, softcap, sink, gate,
+          gate_stride, dtype, total_q, kWaitNs, stream);
+}
+
 extern "C" int b200_attn_generic(void* out, const void* q, int64_t q_stride, const void* k, int64_t k_stride,
                                  const void* v, int64_t v_stride, const int32_t* block_tables,
                                  int32_t bt_stride, int32_t block_size, const int32_t* cu_q,
@@ -794,14 +808,16 @@ extern "C" int b200_attn_generic(void* out, const void* q, int64_t q_stride, con
   return b200_attn_generic_step(out, q, q_stride, k, k_stride, v, v_stride, block_tables, bt_stride, block_size, cu_q, cu_k, ctx_lens, num_seqs, max_q, num_heads, num_kv_heads, dim, vdim, scale, window, keep_first, chunk, softcap, sink, gate, gate_stride, dtype, 0, stream);
 }
 
-extern "C" int b200_linear_recurrence_step(float* out, const void* q, int64_t q_stride, const void* k,
+extern "C" int b200_linear_recurrence_bounded(float* out, const void* q, int64_t q_stride, const void* k,
                                       int64_t k_stride, const void* v, int64_t v_stride, float* state,
                                       const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k,
                                       const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q,
                                       int32_t num_heads, int32_t groups, int32_t kdim, int32_t vdim, int32_t mode,
                                       int32_t act_silu, const float* decay, const void* dt, int64_t dt_stride,
                                       const float* dt_bias, const float* a_log, const float* d_skip,
-                                      int32_t qk_f32, int32_t dtype, int64_t total_q, b200_stream_t stream) {
+                                      int32_t qk_f32, int32_t dtype, int64_t total_q, int64_t wait_ns,
+                                 b200_stream_t stream) {
+  B200_RETURN_IF(wait_ns < 0, B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(num_seqs < 0 || num_heads <= 0 || groups <= 0 || num_heads % groups != 0 || kdim <= 0 ||
                      vdim <= 0 || mode < 0 || mode > 2, B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(kdim > 256, B200_ERR_UNSUPPORTED);
@@ -821,10 +837,23 @@ extern "C" int b200_linear_recurrence_step(float* out, const void* q, int64_t q_
     if (dtype == B200_DTYPE_F16) return recurrence_launch<float, __half>(P, num_seqs, (cudaStream_t)stream);
     return B200_ERR_BAD_DTYPE;
   }
-  if (recurrence_umma_ok(P, dtype, num_seqs, max_q, total_q)) return recurrence_umma_launch(P, num_seqs, (cudaStream_t)stream);
+  if (recurrence_umma_ok(P, dtype, num_seqs, max_q, total_q)) return recurrence_umma_launch(P, num_seqs, wait_ns, (cudaStream_t)stream);
   if (chunk_recurrence_ok(P, dtype, max_q)) return chunk_recurrence_launch(P, num_seqs, (cudaStream_t)stream);
   B200_DISPATCH_3(dtype, T, return recurrence_launch<T>(P, num_seqs, (cudaStream_t)stream));
   return B200_OK;
+}
+
+extern "C" int b200_linear_recurrence_step(float* out, const void* q, int64_t q_stride, const void* k,
+                                      int64_t k_stride, const void* v, int64_t v_stride, float* state,
+                                      const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k,
+                                      const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q,
+                                      int32_t num_heads, int32_t groups, int32_t kdim, int32_t vdim, int32_t mode,
+                                      int32_t act_silu, const float* decay, const void* dt, int64_t dt_stride,
+                                      const float* dt_bias, const float* a_log, const float* d_skip,
+                                      int32_t qk_f32, int32_t dtype, int64_t total_q, b200_stream_t stream) {
+  return b200_linear_recurrence_bounded(out, q, q_stride, k, k_stride, v, v_stride, state, state_slots, cu_q, cu_k, ctx_lens,
+          num_seqs, max_q, num_heads, groups, kdim, vdim, mode, act_silu, decay, dt, dt_stride, dt_bias, a_log, d_skip, qk_f32,
+          dtype, total_q, kWaitNs, stream);
 }
 
 extern "C" int b200_linear_recurrence(float* out, const void* q, int64_t q_stride, const void* k,

@@ -154,6 +154,10 @@ PROTOTYPES = {
                                     c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
                                     c_int32, c_int32, c_int32, c_float, c_int32, c_int32, c_int32, c_float, c_void_p,
                                     c_void_p, c_int64, c_int32, c_int64, c_void_p]),
+    "b200_attn_generic_bounded": (c_int32, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
+                                    c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
+                                    c_int32, c_int32, c_int32, c_float, c_int32, c_int32, c_int32, c_float, c_void_p,
+                                    c_void_p, c_int64, c_int32, c_int64, c_int64, c_void_p]),
     "b200_linear_recurrence": (c_int32, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                                          c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
                                          c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p,
@@ -162,6 +166,10 @@ PROTOTYPES = {
                                          c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
                                          c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p,
                                          c_int64, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int64, c_void_p]),
+    "b200_linear_recurrence_bounded": (c_int32, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
+                                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
+                                         c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p, c_void_p,
+                                         c_int64, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int64, c_int64, c_void_p]),
     # multi-stream residual, rotary, delta rule, latent attention, clamped unit, generic MoE
     "b200_stream_mix_norm": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_void_p, c_void_p, c_float, c_float, c_int32, c_int32, c_int32, c_int32,
