@@ -81,6 +81,12 @@ inline cudaError_t allow_smem(Kernel kernel, int bytes, std::atomic<uint64_t>& d
   return e;
 }
 
+inline int sm_count() {                                    // of the current device
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---------------------------------------------------------------- dtype traits

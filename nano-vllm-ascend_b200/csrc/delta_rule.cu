@@ -274,14 +274,14 @@ static void delta_launch_as(const DeltaParams& P, int num_seqs, cudaStream_t str
       configured = true;
     }
     // Prompts that do not find an SM for every CTA start with the longest sequences: those share an SM with the shortest, and a token of
-    // a CTA that shares costs half as much again. States of 128 key rows alone: the others have room for more CTAs per SM.
+    // a CTA that shares costs half as much again. States of 128 key rows alone: the others have room for more CTAs per SM. Up to 32
+    // sequences, where equal lengths lose nothing and every CTA finds its rank with a handful of comparisons per thread. us in order of
+    // arrival / of length, 8 heads of 128 (a decay per channel): 10 prompts of 500-1300 tokens 768 / 706, 16 792 / 726, 32 of 100-900
+    // 850 / 586. Beyond, ragged prompts would still gain (48 of 100-600 723 / 640, 128 of 16-300 785 / 725), but equal ones lose (64 of
+    // 128 339 / 345), and so do many (256 of 16-200 1028 / 1109: comparisons of every pair in every CTA).
     if constexpr (KPT * NS == 128 && MODE != kWkv) {
-      if (P.cu_q != nullptr && num_seqs > 1 && num_seqs <= 32 && (int64_t)grid.x * grid.y * num_seqs > 148) {
-        static bool ordered = false;
-        if (!ordered && smem > 48 * 1024) {
-          cudaFuncSetAttribute(delta_rule_kernel<TV, KPT, NS, NC, true, MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-          ordered = true;
-        }
+      static_assert(2 * kDeltaTok * ((2 * KP + GT + 1) * sizeof(float) + CC * sizeof(TV)) <= 47 * 1024, "no more than a launch may have unasked");
+      if (P.cu_q != nullptr && num_seqs > 1 && num_seqs <= 32 && (int64_t)grid.x * grid.y * num_seqs > sm_count()) {
         launch_pdl(delta_rule_kernel<TV, KPT, NS, NC, true, MODE, true>, grid, dim3(32 * NS), smem, stream, P);
         return;
       }

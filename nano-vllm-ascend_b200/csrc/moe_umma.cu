@@ -464,12 +464,6 @@ moe_gather_rows_kernel(T* __restrict__ xs, const T* __restrict__ x, const int32_
   }
 }
 
-static int moe_sm_count() {
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 // The persistent kernel where its 256-column bands divide the output and every SM can expect a tile: full row tiles, or one of every
 // expert where they have 16 rows on average (a layer of 128 experts, 2048 x 768, top 8, 256 tokens: 359 us with the 128-column
 // kernels, 209 so). Fewer tiles than SMs leave it with idle SMs and one cold ring per tile, where the
@@ -478,7 +472,7 @@ static int moe_sm_count() {
 static bool moe_umma_wide(bool gate_up, int pairs, int num_local, int n_out, int out_f32) {
   const int band = gate_up ? 128 : 256;
   const int row_tiles = num_local > 1 && pairs / 16 >= num_local && num_local > pairs / 128 ? num_local : pairs / 128;
-  return !out_f32 && n_out % band == 0 && (long long)row_tiles * (n_out / band) >= moe_sm_count();
+  return !out_f32 && n_out % band == 0 && (long long)row_tiles * (n_out / band) >= sm_count();
 }
 
 template <typename T, bool kGateUp, int kStages>
@@ -502,7 +496,7 @@ static int moe_umma_wide_launch(const CUtensorMap& ma, const CUtensorMap& mw, co
   static std::atomic<uint64_t> devices{0};
   const cudaError_t allowed = allow_smem(kern, kMwSmem, devices);
   if (allowed != cudaSuccess) return (int)allowed;
-  launch_pdl(kern, dim3(moe_sm_count()), dim3(kMuThreads), (size_t)kMwSmem, stream, ma, mw, p);
+  launch_pdl(kern, dim3(sm_count()), dim3(kMuThreads), (size_t)kMwSmem, stream, ma, mw, p);
   return finish_launch();
 }
 
@@ -511,7 +505,7 @@ static int moe_umma_launch(bool gate_up, const CUtensorMap& ma, const CUtensorMa
                            const MoeUmmaParams& p, int pairs, int expected, cudaStream_t stream) {
   const int row_tiles = (pairs + 127) / 128 + p.num_local;      // upper bound; surplus CTAs exit at once
   const dim3 grid(p.n_out / (gate_up ? 64 : 128), row_tiles);
-  const bool deep = (long long)grid.x * ((expected + 127) / 128) <= 2ll * moe_sm_count();   // few live CTAs: latency-bound
+  const bool deep = (long long)grid.x * ((expected + 127) / 128) <= 2ll * sm_count();   // few live CTAs: latency-bound
   if (gate_up)
     return deep ? moe_umma_launch_s<T, true, 6>(ma, mw, p, grid, stream)
                 : moe_umma_launch_s<T, true, 3>(ma, mw, p, grid, stream);
