@@ -674,12 +674,16 @@ chunk_recurrence_kernel(const RecParams P) {
   }
 }
 
-static bool chunk_recurrence_ok(const RecParams& P, int dtype, int max_q) {
+// B200_CHUNK_RECURRENCE=0: every recurrence token by token
+static bool recurrence_in_chunks() {
   static const bool off = [] {
     const char* e = getenv("B200_CHUNK_RECURRENCE");
     return e != nullptr && e[0] == '0';
   }();
-  return !off && P.mode != 2 && dtype == B200_DTYPE_BF16 && P.cu_q != nullptr && max_q >= 16 && P.kdim <= 128 && P.vdim <= 128;
+  return !off;
+}
+static bool chunk_recurrence_ok(const RecParams& P, int dtype, int max_q) {
+  return P.mode != 2 && dtype == B200_DTYPE_BF16 && P.cu_q != nullptr && max_q >= 16 && P.kdim <= 128 && P.vdim <= 128;
 }
 
 static int chunk_recurrence_launch(const RecParams& P, int num_seqs, cudaStream_t stream) {
@@ -837,8 +841,10 @@ extern "C" int b200_linear_recurrence_bounded(float* out, const void* q, int64_t
     if (dtype == B200_DTYPE_F16) return recurrence_launch<float, __half>(P, num_seqs, (cudaStream_t)stream);
     return B200_ERR_BAD_DTYPE;
   }
-  if (recurrence_umma_ok(P, dtype, num_seqs, max_q, total_q)) return recurrence_umma_launch(P, num_seqs, wait_ns, (cudaStream_t)stream);
-  if (chunk_recurrence_ok(P, dtype, max_q)) return chunk_recurrence_launch(P, num_seqs, (cudaStream_t)stream);
+  if (recurrence_in_chunks()) {
+    if (recurrence_umma_ok(P, dtype, num_seqs, max_q, total_q)) return recurrence_umma_launch(P, num_seqs, wait_ns, (cudaStream_t)stream);
+    if (chunk_recurrence_ok(P, dtype, max_q)) return chunk_recurrence_launch(P, num_seqs, (cudaStream_t)stream);
+  }
   B200_DISPATCH_3(dtype, T, return recurrence_launch<T>(P, num_seqs, (cudaStream_t)stream));
   return B200_OK;
 }

@@ -59,3 +59,27 @@ def test_against_64_bit_in_portions(H, G, N, V, selective, silu, lens):
                 assert float((kept - st).norm() / st.norm()) < tol, (part, s, n)
             begin += n
     assert bool(torch.isnan(state[0]).all())                   # a slot that no sequence holds
+
+
+def test_the_switch_that_turns_chunks_off():
+    """B200_CHUNK_RECURRENCE=0: token by token, whatever the length (the fp32 model's kernel gives the same bits for the same inputs)."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import sys; sys.path.insert(0, "nano-vllm-ascend_b200")
+import torch
+from nanovllm import ops
+g = torch.Generator(device="cuda").manual_seed(1)
+rand = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+T, H, N, V = 300, 2, 128, 128
+q, k, v, decay = rand(T, H * N), rand(T, H * N), rand(T, H * V), torch.tensor([0.9, 0.99], device="cuda")
+cu = torch.tensor([0, T], dtype=torch.int32, device="cuda")
+sp = ops.StepSpans(cu, cu, None, T)
+a, b = (ops.linear_recurrence(*t, sp, H, H, N, V, None, None, decay=decay) for t in ((q, k, v), (q.float(), k.float(), v.float())))
+print("SAME" if torch.equal(a, b) else "OTHER")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for value, want in (("0", "SAME"), ("1", "OTHER")):
+        done = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, B200_CHUNK_RECURRENCE=value), capture_output=True, text=True)
+        assert done.stdout.split() == [want], (value, done.stdout, done.stderr[-2000:])
