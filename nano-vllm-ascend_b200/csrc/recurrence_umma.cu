@@ -27,8 +27,8 @@
 // TMEM: dS 128 columns, S terms 192, O1 64, O2 64 (both heads: MMAs that write half of the lanes), SC 64. Shared memory: q, k two
 // stages, x three (its last reader is O2), P and the scaled values one.
 //
-// A value x that is not finite spoils all outputs of its channel in its chunk, the tokens before it too (0 x inf), as in
-// chunk_recurrence_kernel, whose chunks are half as long.
+// A value x that is not finite must not reach the tokens before it (0 x inf): the warps that scale the values put a zero in its place,
+// and the outputs of its channel from its token on are NaN (the state takes the value itself).
 //
 // Waits are bounded (mbar_warp_wait): one that runs out makes its role leave its loop, those that wait for that role run out as well, the
 // products under way are waited for, the CTA sets the host's word and the library reports it.
@@ -89,7 +89,7 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
            *sc_read = bars + 13, *p_ready = bars + 14, *w_ready = bars + 15, *d_done = bars + 16, *d_read = bars + 17,
            *s_ready = bars + 18, *o1_done = bars + 19, *o2_done = bars + 20, *o_read = bars + 21, *drained = bars + 22;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
-  volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int *gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1), *odd = gave_up + 1;
 
   pdl_wait();
   const int s = blockIdx.y, h0 = blockIdx.x * NH;
@@ -161,7 +161,7 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
     mbar_init(o1_done, 1), mbar_init(o2_done, 1), mbar_init(o_read, 256);
     mbar_init(drained, 1);
     mbar_fence_init();
-    *gave_up = 0;
+    *gave_up = 0, *odd = 0;
   }
   if (warp == 16) umma::tmem_alloc(tmem_slot, 512);
   umma::fence_before_sync();
@@ -317,6 +317,17 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
       for (int i = 0; i < D / 2; ++i)
         if (i < rows) mine[i * VD] = S[i];
     }
+    if (*odd) {                                         // a value that is not finite: from its token on (beyond the chunk it is all NaN)
+      int first = sp.q_len;
+      for (int t = (*odd - 1) * kRuL; t < sp.q_len && first == sp.q_len; t += 16)
+#pragma unroll
+        for (int i = 15; i >= 0; --i) {                 // 16 on their way
+          const float x = t + i < sp.q_len ? __bfloat162float(v[(sp.q_start + t + i) * P.v_stride + c]) : 0.f;
+          if (!isfinite(SILU ? silu_fast(x) : x)) first = t + i;
+        }
+      for (int t = first; t < min(sp.q_len, (first / kRuL + 1) * kRuL); ++t)
+        if ((t & 32) == 32 * half) out[(sp.q_start + t) * out_stride + c] = NAN;
+    }
   } else if (warp < 16) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     const int wq = warp & 3, wg = (warp - 8) >> 2;
@@ -327,12 +338,15 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
         const RuDecay* dec = s_dec + (j & (kRuDec - 1)) * NH;
         if (!wait(&dec_full[j & (kRuDec - 1)], j / kRuDec) || !wait(&k_full[j & 1], j >> 1)) break;
         if (j > 0 && !wait(d_done, j - 1)) break;       // the last chunk's are consumed
-        const uint8_t* x = sX + (j % 3) * 2 * kRuPanel;
+        uint8_t* x = sX + (j % 3) * 2 * kRuPanel;
+        uint32_t seen = 0;                              // the largest magnitude of either half
 #pragma unroll 1
         for (int e0 = 0; e0 < 8; ++e0) {
           const int e = e0 * 128 + wi, row = e >> 4, panel = (e >> 3) & 1;
           const uint32_t at = panel * kRuPanel + umma::sw128(row, e & 7);
           const uint4 u = *reinterpret_cast<const uint4*>(x + at);
+          seen = __vimax3_u16x2(seen, u.x & 0x7fff7fffu, u.y & 0x7fff7fffu);
+          seen = __vimax3_u16x2(seen, u.z & 0x7fff7fffu, u.w & 0x7fff7fffu);
           const float w = dec[NH == 2 ? panel : 0].to_end[row];
           const uint32_t in[4] = {u.x, u.y, u.z, u.w};
           uint32_t y[4][3];
@@ -341,6 +355,15 @@ recurrence_umma_kernel(const __grid_constant__ RuParams RP) {
 #pragma unroll
           for (int p = 0; p < 3; ++p)
             *reinterpret_cast<uint4*>(sW + p * 2 * kRuPanel + at) = make_uint4(y[0][p], y[1][p], y[2][p], y[3][p]);
+        }
+        if ((seen & 0xffffu) >= 0x7f80u || seen >= 0x7f800000u) {      // the tokens before see zero instead (0 x inf), see the outputs
+          if (*odd == 0) *odd = j + 1;                  // the first chunk that has one
+#pragma unroll 1
+          for (int e = wi; e < 1024; e += 128) {
+            uint16_t* h = reinterpret_cast<uint16_t*>(x + ((e >> 3) & 1) * kRuPanel + umma::sw128(e >> 4, e & 7));
+            for (int i = 0; i < 8; ++i)
+              if ((h[i] & 0x7f80u) == 0x7f80u) h[i] = 0;
+          }
         }
         fence_proxy_async_smem();
         mbar_arrive(w_ready);

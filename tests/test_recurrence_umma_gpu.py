@@ -83,3 +83,32 @@ print("SAME" if torch.equal(a, b) else "OTHER")
     for value, want in (("0", "SAME"), ("1", "OTHER")):
         done = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, B200_CHUNK_RECURRENCE=value), capture_output=True, text=True)
         assert done.stdout.split() == [want], (value, done.stdout, done.stderr[-2000:])
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("V,silu,at", [(64, False, 60), (64, False, 64), (128, True, 127), (128, False, 0), (128, False, 299)])
+def test_a_value_that_is_not_finite_spoils_nothing_before_it(bad, V, silu, at):
+    from nanovllm import ops
+    g = torch.Generator(device="cuda").manual_seed(at)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()  # noqa: E731
+    lens, H, N, c = [300, 97], 2, 128, V + 5                   # a channel of the second head
+    T = sum(lens)
+    q, k, v, decay = rand(T, H * N), rand(T, H * N), rand(T, H * V), torch.tensor([0.9, 0.99], device="cuda")
+    cu = torch.tensor([0, 300, 397], dtype=torch.int32, device="cuda")
+    sp = ops.StepSpans(cu, cu, None, 300)
+    slots = torch.arange(2, dtype=torch.int32, device="cuda")
+    run = lambda v, s: ops.linear_recurrence(q, k, v, sp, H, 1 if V == 64 else H, N, V, s, slots, decay=decay, act_silu=silu)  # noqa: E731
+    if V == 64:
+        q, k = q[:, :N], k[:, :N]                              # two heads per CTA share q and k
+    fine, kept = torch.zeros(2, H, N, V, device="cuda"), torch.zeros(2, H, N, V, device="cuda")
+    want = run(v, fine)
+    v2 = v.clone()
+    v2[at, c] = bad
+    got = run(v2, kept)
+    spoilt = torch.zeros(T, H * V, dtype=torch.bool, device="cuda")
+    spoilt[at:300, c] = True
+    assert torch.equal(torch.isfinite(got), ~spoilt)
+    assert torch.equal(got[~spoilt], want[~spoilt])
+    column = torch.zeros_like(kept, dtype=torch.bool)
+    column[0, 1, :, 5] = True
+    assert not bool(torch.isfinite(kept[column]).any()) and torch.equal(kept[~column], fine[~column])
