@@ -17,10 +17,10 @@
 // order of issue is O2(i) | SC(i+1) | O1(i) | dS(i+1): the score warps work under O1 and dS, the state warps store outputs under
 // dS(i+1) and turn S(i) into terms under O2(i+1), k and x come two chunks ahead. What also counts is code size: 24 warps of six
 // roles run through their code once per chunk, and with everything unrolled (164 KB) instruction fetches took three quarters of
-// the time (16 x 1024 tokens, 32 heads of 128 x 64: 265 us; 190 with short loops; 135 with the roles spread over 24 warps; 133 with an add per
+// the time (16 x 1024 tokens, 32 heads of 128 x 64: 265 us; 190 with short loops; 135 with the roles spread over 24 warps; 132 with an add per
 // operand and MMA).
-// Measured there: 329 us (chunk_recurrence_kernel, mma.sync, chunks of 32) -> 133 us; 8 heads of 128 x 128 195 -> 113; errors against
-// 64 bits 2.2e-7 (2.5e-7).
+// Measured there (ten calls in a graph; 5 us more where the inputs change from call to call): 329 us (chunk_recurrence_kernel, mma.sync,
+// chunks of 32) -> 132, 133 with the look at the values (see below); 8 heads of 128 x 128 195 -> 114; errors against 64 bits 2.1e-7 (2.5e-7).
 // Warps: 0-7 state and outputs (a warp: 32 channels x half of the keys, then half of the tokens; D / 2 state registers a thread);
 // 8, 9 and 12, 13 P of a head's diagonal blocks, 17 and 21 of the others (only warps w with w % 4 < 2 may read TMEM lanes 0-63);
 // 10, 11, 14, 15 the scaled values; 16 issues; 20 decays; 18, 19 copy k and x, 22, 23 q. With one head of 128, 12 and 13 copy too.
