@@ -6,7 +6,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("experts,top,hidden,inter,rows", [(64, 4, 1024, 1024, 15), (64, 4, 1024, 1024, 16), (64, 4, 128, 256, 23), (64, 4, 128, 256, 24),
+@pytest.mark.parametrize("experts,top,hidden,inter,rows", [(64, 4, 1024, 1024, 15), (64, 4, 1024, 1024, 16), (64, 4, 768, 384, 23), (64, 4, 768, 384, 24),
                                                            (8, 2, 256, 256, 31), (8, 2, 256, 256, 32)])
 @pytest.mark.parametrize("skewed", [False, True])
 def test_both_sides_of_the_line(experts, top, hidden, inter, rows, skewed, monkeypatch):
@@ -21,6 +21,7 @@ def test_both_sides_of_the_line(experts, top, hidden, inter, rows, skewed, monke
     w13, w2 = (rand(experts, 2 * inter, hidden) * hidden ** -0.5).bfloat16(), (rand(experts, hidden, inter) * inter ** -0.5).bfloat16()
     ids, weights = ops.moe_route(logits.bfloat16(), top)
     plan = ops.moe_align(ids, 0, experts)
+    assert ops._moe_big(plan, hidden, inter) is (rows % 2 == 0)
     got = ops.moe_experts(x, w13, w2, ids, weights, plan).float()
     monkeypatch.setattr(ops, "_MOE_BIG_GEMM_ROWS", 1 << 30 if rows % 2 == 0 else 1)
     other = ops.moe_experts(x, w13, w2, ids, weights, plan).float()
