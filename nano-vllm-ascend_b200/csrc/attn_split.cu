@@ -17,8 +17,9 @@
 // 96, P V 2 x 128. Shared memory at 128: Q 96 KB, K 48, V 48: one CTA per SM.
 // Bound: the tensor pipe (24 x 74 + 48 x 75 = 5376 cycles per tile of 64 keys at heads of 128, where the fp32 FMA pipes need 16384),
 // and the copying warps' load -> split -> store beside it (a tile takes 6300). Measured: 4 ragged prompts of 700-1024 tokens, 8
-// heads over 2 of 128, paged, 288 us (attn_tiled_kernel) -> 66 (20 calls in a graph; 70 where the inputs change from call to call; 10 more with 8 columns a
-// lane, which read every sector twice, 7 with that but block ids looked up a step ahead); 4 of 600-1000, 32 heads over 8 of 64, 490 -> 132.
+// heads over 2 of 128, paged, 288 us (attn_tiled_kernel) -> 66 (20 calls in a graph; 70 where the inputs change from call to call;
+// 10 more with 8 columns a lane, which read every sector twice, 7 with that but block ids looked up a step ahead); 4 of 600-1000, 32
+// heads over 8 of 64, 490 -> 132.
 //
 // What the split cannot carry: what is not finite or close to the largest numbers (and 0 x inf would reach rows that do not see the key),
 // and what is so small that a term of it would not be normal. Values come times 2^27, which leaves nothing too small, and go back

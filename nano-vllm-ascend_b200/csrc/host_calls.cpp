@@ -1,10 +1,11 @@
 // host_calls.cpp -- the attention entry points of ops.py as one native call each.
 //
 // A decode call of one row takes 8.7 us on the device (100 of them in a graph) and took 17 us of Python: 25 arguments through ctypes (3.6
-// us), some 35 tensor attributes (4 us); 9.2 us now, all in all. Captured steps never paid it. Here the same attributes are looked at and the same library function is called without either. What ops.py
-// would refuse is not judged here: the functions return None for any argument that is not exactly what they expect, and ops.py goes its
-// own way, checks and errors included. An int is the library's status. Plain torch.Tensor with memory of its own only (subclasses, fake
-// tensors, dispatch modes and what torch.vmap and torch.func wrap take ops.py's way); nothing is kept between calls.
+// us), some 35 tensor attributes (4 us); 9.2 us now, all in all. Captured steps never paid it. Here the same attributes are looked at
+// and the same library function is called without either. What ops.py would refuse is not judged here: the functions return None for
+// any argument that is not exactly what they expect, and ops.py goes its own way, checks and errors included. An int is the library's
+// status. Plain torch.Tensor with memory of its own only (subclasses, fake tensors, dispatch modes and what torch.vmap and torch.func
+// wrap take ops.py's way); nothing is kept between calls.
 // The interpreter lock is given up around the library's function alone: everything that can throw, addresses of tensors included,
 // is read before, since an exception that left the block would be handled without the lock.
 #include <torch/csrc/Exceptions.h>
