@@ -61,8 +61,8 @@ const char* b200_error_string(int code);
  * (host-side counter; lets bench.py report `gpu_launches`). */
 int64_t b200_launch_count(void);
 void b200_reset_launch_count(void);
-/* Waits inside the persistent grouped GEMM (b200_moe_gemm_*_umma), b200_linear_recurrence_step and b200_attn_generic_step on tensor-core
- * prompts are bounded. When one runs out, the kernel returns without having written its output (a recurrence may have written part of its
+/* Waits inside the persistent grouped GEMM (b200_moe_gemm_*_umma), b200_linear_recurrence_step, b200_delta_rule_step and
+ * b200_attn_generic_step on tensor-core prompts are bounded. When one runs out, the kernel returns without having written its output (a recurrence may have written part of its
  * state) and sets a word of page-locked host memory. b200_take_wait_status asks
  * and clears it: B200_ERR_WAIT or B200_OK, meaningful for kernels that the host has waited for. The same entry points ask it
  * first of all, so that a call after the failed one returns B200_ERR_WAIT. b200_wait_status_word: the word itself. */
@@ -716,6 +716,25 @@ int b200_delta_rule(float* out, const float* q, int64_t q_stride, const float* k
                     const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k,
                     const int32_t* ctx_lens, int32_t num_seqs, int32_t num_heads, int32_t groups, int32_t kdim,
                     int32_t vdim, int32_t mode, int32_t dtype, b200_stream_t stream);
+/* The same where the caller knows the step's longest span and its tokens (total_q >= cu_q[num_seqs]) and lends a workspace
+ * (16-byte aligned; b200_delta_rule_workspace_size bytes, 0: none is of use): modes 0 and 1 with bf16 values, kdim = vdim = 128, or 64 with
+ * an even number of heads, rows on 16-byte boundaries and spans that are long on average run 64 tokens at a time on the 5th-generation
+ * tensor cores. A smaller workspace that holds one chunk of every head and one state will do, in several passes; without one, token by token. */
+int64_t b200_delta_rule_workspace_size(int32_t num_seqs, int32_t max_q, int64_t total_q, int32_t num_heads, int32_t groups,
+                                       int32_t kdim, int32_t vdim, int32_t mode, int32_t dtype);
+int b200_delta_rule_step(float* out, const float* q, int64_t q_stride, const float* k, int64_t k_stride,
+                         const void* v, int64_t v_stride, const float* g, const float* beta, float* state,
+                         const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k,
+                         const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q, int64_t total_q, int32_t num_heads,
+                         int32_t groups, int32_t kdim, int32_t vdim, int32_t mode, int32_t dtype, void* workspace,
+                         int64_t workspace_bytes, b200_stream_t stream);
+/* and with its own limit on a single wait, as b200_linear_recurrence_bounded. */
+int b200_delta_rule_bounded(float* out, const float* q, int64_t q_stride, const float* k, int64_t k_stride,
+                            const void* v, int64_t v_stride, const float* g, const float* beta, float* state,
+                            const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k,
+                            const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q, int64_t total_q, int32_t num_heads,
+                            int32_t groups, int32_t kdim, int32_t vdim, int32_t mode, int32_t dtype, void* workspace,
+                            int64_t workspace_bytes, int64_t wait_ns, b200_stream_t stream);
 
 /* Inputs of the wkv mode from projected activations r, k [T, H*dim] (row strides) and z fp32 [T, H*dim]: r and k in fp32,
  * decay = exp(-exp(z + w0)), bonus [T, H] = sum_i r_i u_i k_i per head; w0, u fp32 [H*dim]. */

@@ -1,0 +1,920 @@
+// delta_chunks.cu -- the gated delta rule over prompts on the 5th-generation tensor cores, 64 tokens at a time.
+//
+// With P_i the decay from a chunk's start to and with token i (a vector per key channel, or a number), S0 the state before the chunk and
+// w_i what token i writes,
+//   w_i = beta_i (v_i - (P_i k_i) S0 - sum_(j<i) A_ij w_j)       A_ij = sum_d k_id (P_i / P_j)_d k_jd
+//   o_i = (P_i q_i) S0 + sum_(j<=i) B_ij w_j                     B_ij = sum_d q_id (P_i / P_j)_d k_jd
+//   S   = P_end S0 + sum_j (P_end / P_j) k_j w_j^T
+// so that with X = [I; B] (I + diag(beta) A)^-1 diag(beta), 128 x 64,
+//   [U; O0] = X V        [W; Y] = X (P k)        w = U - W S0        o = O0 + (P q - Y) S0.
+// All of X, U, O0, W and P q - Y is independent of S0: delta_chunk_kernel computes it for all chunks at once, and delta_scan_kernel walks
+// the chunks of a head with two products each.
+//
+// delta_chunk_kernel, one CTA of 8 warps per (chunk, head), two CTAs per SM:
+//   scores [K~; Q~] K^^T   M128 N64 K = D, 32 channels to an accumulator (the tensor core cuts sums off: the small products of later
+//                          channels on top of a full sum would cost 6e-7). Decays per channel are split at the chunk's middle,
+//                          K~ = k P_i / P_mid, K^ = k P_mid / P_j, each a product of decays or its reciprocal. Where such a product
+//                          leaves 2^-80 .. 2^80 the scores are summed up in fp32 instead (no reciprocal). One decay per head:
+//                          K~ = K^ = k, and the decay goes on the scores.
+//   X                      a thread per row: back substitution over columns, 64 x 64 / 2 packed multiply-adds, rows of A as broadcasts
+//   [W; Y], [U; O0]        M128 N = D K64, X from tensor memory
+// delta_scan_kernel, one CTA per (sequence, 128 value channels = one head of 128 or two of 64), S^T in fp32 registers:
+//   E^T = S0^T [W; P q - Y]^T    M128 (channels) N128 K = D, S0 in three terms from tensor memory
+//   w -> three terms; o out;  dS^T = w^T (P_end / P_j k_j)    M128 N = D K64;   S = P_end S + dS in registers.
+// Every fp32 operand is three bf16 terms by cutting off (24 bits, exact), six products, small ones first; values are bf16 as they are.
+//
+// What bounds them, 16 prompts of 500-1300 tokens, 8 heads of 128 (delta_rule_kernel 650 us): delta_chunk_kernel 205, a CTA's phases behind
+// one another (loads, scores, substitution, products, 48000 cycles, of which 11000 are issue); delta_scan_kernel 108, the chain
+// E -> w -> dS -> S -> E, 72 MMAs of 64 cycles and four conversions a chunk. The records that pass between them (216 KB per chunk and head
+// of 128, written and read once) would take 2 x 63 at HBM's rate.
+//
+// Not for chunks, and left to delta_rule_kernel, which runs behind them over the heads that a record flags: values that are not finite
+// (0 x inf would reach tokens before them) or beyond 2^60, decays of 2 and more, keys, queries or values all below 2^-60 (the low terms
+// would be lost).
+//
+// Waits are bounded (mbar_warp_wait): one that runs out makes its role leave, those that wait for it run out as well, the products under
+// way are waited for, the CTA sets the host's word and the library reports it.
+#include <limits.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "delta_rule.cuh"
+#include "recurrence.cuh"
+#include "umma.cuh"
+
+namespace b200 {
+
+// ---- a record: bytes of its parts
+template <int D>
+struct DcRecord {
+  static constexpr int kWq = 3 * 2 * D * 128;            // [W; P q - Y]: [3 terms][2 panels of 64 rows r][D rows n][128 bytes]
+  static constexpr int kKe = 3 * (D / 64) * 8192;        // P_end / P_j k_j: [3 terms][D / 64 panels][64 rows j][128 bytes]
+  static constexpr int kUoRow = 132;                     // floats of a row of [U; O0]: 16-byte groups of eight rows in different banks
+  static constexpr int kUo = D * kUoRow * 4;             // [U; O0]: [D rows c][128 r] fp32
+  static constexpr int kPe = 1024;                       // P_end [D] fp32, the flag
+  static constexpr int kKeAt = kWq, kUoAt = kWq + kKe, kPeAt = kUoAt + kUo, kFlagAt = kPeAt + D * 4, kBytes = kPeAt + kPe;
+};
+// terms of A and B in the i-th of six products, small ones first: 0 2, 1 1, 2 0, 0 1, 1 0, 0 0
+__device__ __forceinline__ uint32_t term_a(int i) { return i == 2 ? 2 : (i == 1 || i == 4); }
+__device__ __forceinline__ uint32_t term_b(int i) { return i == 0 ? 2 : (i == 1 || i == 3); }
+
+struct DcParams {
+  DeltaParams d;
+  DeltaChunks c;
+  int num_seqs, wait_tries;
+  int* wait_status;
+};
+
+__device__ __forceinline__ void mma_ts_half_low(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_low, uint32_t idesc, uint32_t accumulate, int half) {
+  const uint32_t off0 = half == 0 ? 0u : 0xffffffffu, off1 = ~off0;        // lanes whose bit is set are left alone
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+      "mov.b64 b, {%2, %7};\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, {%5, %5, %6, %6}, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(off0), "r"(off1), "n"(umma::kDescHigh)
+      : "memory");
+}
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)), "l"(src),
+               "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+// The tensor core cuts a sum off after every 16 products; on average results lack this part of them. Measured as the mean relative difference
+// from 64-bit products of random operands, for sums of 8, 4 and 2 times 16 products, and for one large product among small ones. Added back,
+// in fp32: outputs 2.6e-7 -> 2.2e-7 off, states 2.2e-7 -> 1.9e-7, where the token form is 2.2e-7 and 2.0e-7 off (the case above).
+constexpr float kCut8 = 1.4e-7f, kCut4 = 0.9e-7f, kCut2 = 0.45e-7f, kCut1 = 0.42e-7f;
+__device__ __forceinline__ float uncut(uint32_t x, float part) { return fmaf(__uint_as_float(x), part, __uint_as_float(x)); }
+__device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ float largest(float most, float2 x) {             // of |x|; NaN stays
+  asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(fabsf(x.x)), "f"(fabsf(x.y)));
+  return most;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(r)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+  return r;
+}
+constexpr uint32_t kBig = (127u + 60u) << 23, kSmall = (127u - 60u) << 23, kTwo = 128u << 23;
+constexpr float kFar = 1.2089258e24f, kNear = 8.2718061e-25f;              // 2^80, 2^-80
+
+constexpr int kDcThreads = 256;
+constexpr int kDcARow = 68;                              // floats of a row of A: 16-byte groups of eight rows in different banks
+template <int D>
+struct DcSmem {
+  static constexpr int kScores = 3 * 16384 + 3 * 8192;   // [K~; Q~] [3 terms][128 rows], K^ [3 terms][64 rows], 64 channels at a time
+  static constexpr int kKb = 3 * (D / 64) * 8192;        // behind it: P k [3 terms][D / 64 panels][64 rows j]
+  static constexpr int kA = kDcL * kDcARow * 4;          // A (then V)
+  static constexpr int kQRow = D + 4;
+  static constexpr int kQs = kDcL * kQRow * 4;           // P q
+  static constexpr int kAAt = kKb, kQsAt = kKb + kA, kEnd = kQsAt + kQs > kScores ? kQsAt + kQs : kScores;
+  static constexpr int kTau = (D / 64) * 8 * 64 * 4;     // decays of 8 tokens
+  static constexpr int kBytes = 1024 + kEnd + kTau + 4 * 64 * 4 + 256;
+};
+
+template <int D, bool PER_HEAD>
+__global__ void __launch_bounds__(kDcThreads, 2)
+delta_chunk_kernel(const __grid_constant__ DcParams DP) {
+  using T = __nv_bfloat16;
+  using R = DcRecord<D>;
+  using M = DcSmem<D>;
+  const DeltaParams& P = DP.d;
+  extern __shared__ __align__(1024) uint8_t dc_smem_raw[];
+  uint8_t* smem = dc_smem_raw + (-smem_u32(dc_smem_raw) & 1023u);       // (not through an integer: the compiler has to know that it is shared memory)
+  float* sA = reinterpret_cast<float*>(smem + M::kAAt);
+  float* sQs = reinterpret_cast<float*>(smem + M::kQsAt);
+  float* s_tau = reinterpret_cast<float*>(smem + M::kEnd);             // [D / 64][8][64]
+  float* s_beta = s_tau + (D / 64) * 8 * 64;
+  float *s_g = s_beta + 64, *s_p = s_g + 64, *s_e = s_p + 64;          // one decay per head: of a token, P, P_end / P
+  uint64_t *scored = reinterpret_cast<uint64_t*>(s_e + 64), *made = scored + 1, *drained = made + 1;
+  uint32_t* s_max = reinterpret_cast<uint32_t*>(drained + 1);          // largest magnitudes: k, q, v, and what must stay below two
+  uint32_t* tmem_slot = s_max + 4;
+  int *s_far = reinterpret_cast<int*>(tmem_slot + 1), *s_where = s_far + 1, *s_next = s_where + 2;
+  volatile int* gave_up = s_next + 1;
+
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = blockIdx.x % P.H, lin = DP.c.first + blockIdx.x / P.H;
+  if (warp == 0) {                                       // the sequence of chunk `lin`
+    int base = 0, found = -1, at = 0;
+    for (int s0 = 0; s0 < DP.num_seqs && found < 0; s0 += 32) {
+      const int n = s0 + lane < DP.num_seqs ? chunks_of(P.cu_q[s0 + lane + 1] - P.cu_q[s0 + lane]) : 0;
+      int to = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, to, o);
+        if (lane >= o) to += up;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, lin < base + to);
+      if (hit != 0) {
+        const int l = __ffs(hit) - 1;
+        found = s0 + l, at = lin - base - __shfl_sync(0xffffffffu, to - n, l);
+      }
+      base += __shfl_sync(0xffffffffu, to, 31);
+    }
+    if (lane == 0) s_where[0] = found, s_where[1] = at;
+  }
+  if (threadIdx.x == 32) {
+    mbar_init(scored, 1), mbar_init(made, 1), mbar_init(drained, 1);
+    mbar_fence_init();
+    for (int i = 0; i < 4; ++i) s_max[i] = 0;
+    *s_far = 0, *s_next = 0, *gave_up = 0;
+  }
+  __syncthreads();
+  const int s = s_where[0], chunk = s_where[1];
+  if (s < 0) return;                                     // the grid has room for sequences that all end in a chunk of their own
+  if (warp == 1) umma::tmem_alloc(tmem_slot, 256);
+  const int64_t tok0 = P.cu_q[s] + chunk * kDcL;
+  const int nt = min(kDcL, P.cu_q[s + 1] - (int)tok0);
+  const int grp = h / (P.H / P.groups);
+  const float* q = P.q + tok0 * P.q_stride + (int64_t)grp * D;
+  const float* k = P.k + tok0 * P.k_stride + (int64_t)grp * D;
+  const float* g = P.g + tok0 * ((int64_t)P.H * (PER_HEAD ? 1 : D)) + (int64_t)h * (PER_HEAD ? 1 : D);
+  const int64_t g_stride = (int64_t)P.H * (PER_HEAD ? 1 : D);
+  const T* v = (const T*)P.v + tok0 * P.v_stride + (int64_t)h * D;
+  uint8_t* record = DP.c.records + ((int64_t)(lin - DP.c.first) * P.H + h) * DP.c.bytes;
+  const bool issuer = warp == 0 && umma::elect_one();
+  auto wait = [&](uint64_t* bar, int parity) { return mbar_warp_wait(bar, parity & 1, DP.wait_tries, gave_up); };
+
+  if (threadIdx.x < kDcL) {
+    const int t = threadIdx.x;
+    const float b = t < nt ? P.beta[(tok0 + t) * P.H + h] : 0.f;
+    s_beta[t] = b;
+    uint32_t most = magnitude(b);
+    if (PER_HEAD) {
+      const float d = t < nt ? g[t * g_stride] : 1.f;
+      s_g[t] = d;
+      most = max(most, magnitude(d));
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) atomicMax(&s_max[3], most);
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tb = *tmem_slot;
+  constexpr uint32_t kTmSC = 0, kTmX = 128;              // scores of 64 channels each, then [W; Y] and [U; O0], 128 columns; X 3 x 32
+  if (PER_HEAD && threadIdx.x < kDcL) {
+    float p = 1.f, e = 1.f;
+    for (int i = 0; i <= (int)threadIdx.x; ++i) p *= s_g[i];
+    for (int i = kDcL - 1; i > (int)threadIdx.x; --i) e *= s_g[i];
+    s_p[threadIdx.x] = p, s_e[threadIdx.x] = e;
+  }
+
+  // 8 tokens of two channels; rows are found by 32-bit offsets from the chunk's first
+  const uint32_t k_step = (uint32_t)P.k_stride * 4, q_step = (uint32_t)P.q_stride * 4, g_step = (uint32_t)g_stride * 4;
+  auto fetch = [&](int t0, int ch, float2 (&kk)[8], float2 (&qq)[8], float2 (&gg)[8]) {
+    auto rows = [&](auto all) {
+      uint32_t ka = t0 * k_step + ch * 4, qa = t0 * q_step + ch * 4, ga = t0 * g_step + ch * 4;
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const bool ok = decltype(all)::value || t0 + x < nt;
+        kk[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(k) + ka) : make_float2(0.f, 0.f);
+        qq[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(q) + qa) : make_float2(0.f, 0.f);
+        if (!PER_HEAD) gg[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(g) + ga) : make_float2(1.f, 1.f);
+        ka += k_step, qa += q_step, ga += g_step;
+      }
+    };
+    if (t0 + 8 <= nt) rows(std::true_type{});
+    else rows(std::false_type{});
+  };
+  bool alive = true;
+  // ------------------------------------------------ scores, 64 channels at a time; a thread has two channels and 8 tokens
+  float most_k = 0.f, most_q = 0.f, most_g = 0.f;
+  bool far = false;
+  const float2 one = make_float2(1.f, 1.f);
+#pragma unroll 1
+  for (int half = 0; half < D / 64; ++half) {
+    const int ch = half * 64 + 2 * lane;
+    float2 kk[8], qq[8], gg[8];
+    fetch(8 * warp, ch, kk, qq, gg);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      most_k = largest(most_k, kk[x]), most_q = largest(most_q, qq[x]);
+      if (!PER_HEAD) most_g = largest(most_g, gg[x]);
+    }
+    // the decay between a token and the chunk's middle, between tokens 31 and 32: of this warp's nearest token `f`, of its farthest 1 / `r`
+    float2 f = one, r = one;
+    if (!PER_HEAD) {
+      float2 but = one;                                  // of the tokens but the nearest (before the middle) or the first (behind it)
+      const bool first = warp < 4;
+#pragma unroll
+      for (int x = 1; x < 8; ++x) but = mul2(but, gg[x]);
+      const float2 all = mul2(but, gg[0]);
+      float2* tau = reinterpret_cast<float2*>(s_tau + half * 512) + lane;      // [8][32] pairs
+      tau[warp * 32] = all;
+      __syncthreads();
+      for (int w = first ? warp + 1 : 4; w < (first ? 4 : warp); ++w) f = mul2(f, tau[w * 32]);
+      r = mul2(f, first ? but : all);
+      far = far || !(fabsf(r.x) >= kNear && fabsf(r.x) <= kFar && fabsf(r.y) >= kNear && fabsf(r.y) <= kFar);
+      r = make_float2(1.f / r.x, 1.f / r.y);
+    }
+    if (half > 0) {                                      // the products of the channels before have read their operands
+      alive = alive && wait(scored, half - 1);
+      umma::fence_after_sync();
+    }
+    uint8_t* sKQ = smem + (lane & 3) * 4 + warp * 1024;
+    auto put_up = [&](int x, float2 up) {
+      uint32_t a[3], b[3];
+      const float2 kx = mul2(kk[x], up), qx = mul2(qq[x], up);
+      split3cut(kx.x, kx.y, a);
+      split3cut(qx.x, qx.y, b);
+      const uint32_t at = x * 128 + (((lane >> 2) ^ x) << 4);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        *reinterpret_cast<uint32_t*>(sKQ + p * 16384 + at) = a[p];
+        *reinterpret_cast<uint32_t*>(sKQ + p * 16384 + 8192 + at) = b[p];
+      }
+    };
+    auto put_dn = [&](int x, float2 dn) {
+      uint32_t c[3];
+      const float2 kx = mul2(kk[x], dn);
+      split3cut(kx.x, kx.y, c);
+      const uint32_t at = x * 128 + (((lane >> 2) ^ x) << 4);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(sKQ + 49152 + p * 8192 + at) = c[p];
+    };
+    if (PER_HEAD) {
+#pragma unroll
+      for (int x = 0; x < 8; ++x) put_up(x, one), put_dn(x, one);
+    } else if (warp < 4) {
+#pragma unroll
+      for (int x = 7; x >= 0; --x) {
+        put_dn(x, f);
+        f = mul2(f, gg[x]);
+      }
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        if (x > 0) r = mul2(r, gg[x]);
+        put_up(x, r);
+      }
+    } else {
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        f = mul2(f, gg[x]);
+        put_up(x, f);
+      }
+#pragma unroll
+      for (int x = 7; x >= 0; --x) {
+        put_dn(x, r);
+        r = mul2(r, gg[x]);
+      }
+    }
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (issuer && alive) {
+      const uint32_t id = umma::make_idesc<T>(128, 64, 0, 0);
+      const uint32_t a0 = umma::desc_low(smem_u32(smem), 16), b0 = umma::desc_low(smem_u32(smem + 49152), 16);
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          umma::mma_ss_low(tb + kTmSC + half * 128 + (ks >> 1) * 64, a0 + ((term_a(i) * 16384 + ks * 32) >> 4), b0 + ((term_b(i) * 8192 + ks * 32) >> 4), id,
+                           i > 0 || (ks & 1) > 0);
+      umma::commit(scored);
+    }
+    __syncwarp();
+  }
+  const uint32_t mk = __reduce_max_sync(0xffffffffu, magnitude(most_k)), mq = __reduce_max_sync(0xffffffffu, magnitude(most_q)),
+                 mg = __reduce_max_sync(0xffffffffu, magnitude(most_g));
+  if (lane == 0) atomicMax(&s_max[0], mk), atomicMax(&s_max[1], mq), atomicMax(&s_max[3], mg);
+  if (__any_sync(0xffffffffu, far) && lane == 0) *s_far = 1;
+  alive = alive && wait(scored, D / 64 - 1);
+  umma::fence_after_sync();
+  __syncthreads();                                       // s_far; all that the scores were made of is free
+  const bool direct = !PER_HEAD && *s_far != 0;
+  float* sB = reinterpret_cast<float*>(smem);            // [64][kDcARow], where P k comes later
+  if (direct) {
+    // a warp per column j: k_j decays from token to token and meets k_i and q_i
+    constexpr int C = D / 32;
+    for (int j = warp; j < kDcL; j += 8) {
+      float x[C];
+#pragma unroll
+      for (int c = 0; c < C; ++c) x[c] = j < nt ? k[j * P.k_stride + c * 32 + lane] : 0.f;
+      for (int i = j; i < kDcL; ++i) {
+        float a = 0.f, b = 0.f;
+        if (i < nt) {
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            const int d = c * 32 + lane;
+            if (i > j) x[c] *= g[i * g_stride + d];
+            a = fmaf(k[i * P.k_stride + d], x[c], a), b = fmaf(q[i * P.q_stride + d], x[c], b);
+          }
+        }
+        a = warp_sum(a), b = warp_sum(b);
+        if (lane == 0) sA[i * kDcARow + j] = a, sB[i * kDcARow + j] = b;
+      }
+    }
+    __syncthreads();
+  }
+
+  uint4 held[D / 16];                                    // values on their way to where A is
+  float2 X[32];                                          // warps 0-3: a row of X
+  if (warp < 4) {
+    const int i = threadIdx.x & 63;                      // token; rows 0-63: of T = (I + beta A)^-1, 64-127: of B T
+    const bool of_k = warp < 2;
+    const uint32_t base = tb + ((uint32_t)(warp * 32) << 16);
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+      uint32_t w[32];
+      if (!direct) {
+#pragma unroll
+        for (int c0 = 0; c0 < 32; c0 += 16) {
+          uint32_t y[D / 32][16];
+#pragma unroll
+          for (int z = 0; z < D / 32; ++z) umma::ld16(base + kTmSC + 64 * z + 32 * part + c0, y[z]);
+          umma::wait_ld();
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            float sum = __uint_as_float(y[0][c]) + __uint_as_float(y[1][c]);
+            if (D == 128) sum += __uint_as_float(y[D / 32 - 2][c]) + __uint_as_float(y[D / 32 - 1][c]);
+            w[c0 + c] = __float_as_uint(fmaf(sum, kCut2, sum));
+          }
+        }
+      } else {
+        const float* row = (of_k ? sA : sB) + i * kDcARow + 32 * part;
+#pragma unroll
+        for (int c = 0; c < 32; ++c) w[c] = __float_as_uint(row[c]);
+      }
+#pragma unroll
+      for (int c = 0; c < 16; ++c) X[16 * part + c] = make_float2(__uint_as_float(w[2 * c]), __uint_as_float(w[2 * c + 1]));
+    }
+    if (PER_HEAD) {                                      // the decay from j to i
+      float d = 1.f;
+#pragma unroll
+      for (int j = 63; j >= 0; --j) {
+        if (j < i) d *= s_g[j + 1];
+        (j & 1 ? X[j / 2].y : X[j / 2].x) *= d;
+      }
+    }
+    const float beta = of_k ? s_beta[i] : 1.f;
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+      X[c].x = 2 * c < i + (of_k ? 0 : 1) ? X[c].x * beta : 0.f;
+      X[c].y = 2 * c + 1 < i + (of_k ? 0 : 1) ? X[c].y * beta : 0.f;
+    }
+    if (direct) named_bar_sync(1, 128), named_bar_arrive(2, 256);      // the rows of A are replaced, those of B become P k
+    if (of_k) {
+#pragma unroll
+      for (int c = 0; c < 16; ++c)
+        *reinterpret_cast<float4*>(sA + i * kDcARow + 4 * c) = make_float4(X[2 * c].x, X[2 * c].y, X[2 * c + 1].x, X[2 * c + 1].y);
+#pragma unroll
+      for (int c = 0; c < 32; ++c) X[c] = make_float2(2 * c == i ? 1.f : 0.f, 2 * c + 1 == i ? 1.f : 0.f);
+    }
+    named_bar_sync(1, 128);
+    // X (I + beta A) = [I; B]: column l is final once those behind it are, and leaves the columns before it
+    auto column = [&](int l) {
+      const float xl = -(l & 1 ? X[l / 2].y : X[l / 2].x);
+      const float2 x2 = make_float2(xl, xl);
+      const float* row = sA + l * kDcARow;
+#pragma unroll
+      for (int c = 0; c < (l + 3) / 4; ++c) {
+        const float4 a = *reinterpret_cast<const float4*>(row + 4 * c);
+        const float2 a0 = make_float2(a.x, a.y), a1 = make_float2(a.z, a.w);
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(reinterpret_cast<uint64_t&>(X[2 * c])) : "l"(reinterpret_cast<const uint64_t&>(x2)), "l"(reinterpret_cast<const uint64_t&>(a0)));
+        if (4 * c + 2 < l) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(reinterpret_cast<uint64_t&>(X[2 * c + 1])) : "l"(reinterpret_cast<const uint64_t&>(x2)), "l"(reinterpret_cast<const uint64_t&>(a1)));
+      }
+    };
+    if (warp & 1) {                                      // tokens 32 and later
+#pragma unroll
+      for (int l = 63; l >= 32; --l) column(l);
+    }
+#pragma unroll
+    for (int l = 31; l >= 1; --l) column(l);
+    // times beta, as the A operand: packed pairs along j
+#pragma unroll
+    for (int part = 0; part < 4; ++part) {
+      uint32_t w[3][8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float2 b = *reinterpret_cast<const float2*>(s_beta + 16 * part + 2 * c);
+        uint32_t y[3];
+        split3cut(X[8 * part + c].x * b.x, X[8 * part + c].y * b.y, y);
+        w[0][c] = y[0], w[1][c] = y[1], w[2][c] = y[2];
+      }
+#pragma unroll
+      for (int p = 0; p < 3; ++p) umma::st8(base + kTmX + p * 32 + 8 * part, w[p]);
+    }
+    umma::wait_st();
+  } else {
+    if (direct) named_bar_sync(2, 256);                  // (the scores have been read)
+#pragma unroll
+    for (int i = 0; i < D / 16; ++i) {
+      const int e = i * 128 + threadIdx.x - 128, row = e / (D / 8), c16 = e % (D / 8);
+      held[i] = row < nt ? ld_nc_v4(v + row * P.v_stride + c16 * 8) : make_uint4(0, 0, 0, 0);
+    }
+    uint32_t most_v = 0;
+#pragma unroll
+    for (int i = 0; i < D / 16; ++i) {
+      most_v = __vimax3_u16x2(most_v, held[i].x & 0x7fff7fffu, held[i].y & 0x7fff7fffu);
+      most_v = __vimax3_u16x2(most_v, held[i].z & 0x7fff7fffu, held[i].w & 0x7fff7fffu);
+    }
+    most_v = max(most_v & 0xffffu, most_v >> 16) << 16;
+    most_v = __reduce_max_sync(0xffffffffu, most_v);
+    if (lane == 0) atomicMax(&s_max[2], most_v);
+  }
+  // ------------------------------------------------ P k for [W; Y], P q, P_end / P k for the scan: 8 tokens of 64 channels to a warp that is free
+  uint8_t* kb = smem + (lane & 3) * 4;
+  while (true) {
+    int u = lane == 0 ? atomicAdd(s_next, 1) : 0;
+    u = __shfl_sync(0xffffffffu, u, 0);
+    if (u >= 8 * (D / 64)) break;
+    const int half = u >> 3, e = u & 7, ch = half * 64 + 2 * lane;
+    float2 kk[8], qq[8], gg[8], to_end[8], p = one, post = one;
+    fetch(8 * e, ch, kk, qq, gg);
+    if (!PER_HEAD) {
+      const float2* tau = reinterpret_cast<const float2*>(s_tau + half * 512) + lane;
+      for (int w = 0; w < e; ++w) p = mul2(p, tau[w * 32]);
+      for (int w = 7; w > e; --w) post = mul2(post, tau[w * 32]);
+#pragma unroll
+      for (int x = 7; x >= 0; --x) to_end[x] = post, post = mul2(post, gg[x]);
+      if (e == 0) *reinterpret_cast<float2*>(record + R::kPeAt + ch * 4) = post;
+    } else if (e == 0) {
+      *reinterpret_cast<float2*>(record + R::kPeAt + ch * 4) = make_float2(s_p[63], s_p[63]);
+    }
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      const int t = 8 * e + x;
+      if (!PER_HEAD) p = mul2(p, gg[x]);
+      else p = make_float2(s_p[t], s_p[t]), to_end[x] = make_float2(s_e[t], s_e[t]);
+      uint32_t a[3], b[3];
+      const float2 kp = mul2(kk[x], p), kend = mul2(kk[x], to_end[x]);
+      split3cut(kp.x, kp.y, a);
+      split3cut(kend.x, kend.y, b);
+      const uint32_t at = half * 8192 + e * 1024 + x * 128 + (((lane >> 2) ^ x) << 4);
+#pragma unroll
+      for (int y = 0; y < 3; ++y) {
+        *reinterpret_cast<uint32_t*>(kb + y * (D / 64) * 8192 + at) = a[y];
+        *reinterpret_cast<uint32_t*>(record + (R::kKeAt + (lane & 3) * 4 + y * (D / 64) * 8192 + at)) = b[y];
+      }
+      *reinterpret_cast<float2*>(sQs + t * M::kQRow + ch) = mul2(qq[x], p);
+    }
+  }
+  umma::fence_before_sync();
+  __syncthreads();                                       // A has been read
+  umma::fence_after_sync();
+  uint8_t* sV = smem + M::kAAt;                          // [D / 64 panels][64 rows j]
+  static_assert(M::kAAt % 1024 == 0 && M::kA >= (D / 64) * 8192, "values");
+  if (warp >= 4) {
+#pragma unroll
+    for (int i = 0; i < D / 16; ++i) {
+      const int e = i * 128 + threadIdx.x - 128, row = e / (D / 8), c16 = e % (D / 8);
+      *reinterpret_cast<uint4*>(sV + (c16 >> 3) * 8192 + umma::sw128(row, c16 & 7)) = held[i];
+    }
+  }
+  fence_proxy_async_smem();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const bool odd = s_max[0] >= kBig || s_max[1] >= kBig || s_max[2] >= kBig || s_max[3] >= kTwo || (s_max[0] > 0 && s_max[0] < kSmall) ||
+                     (s_max[1] > 0 && s_max[1] < kSmall) || (s_max[2] > 0 && s_max[2] < kSmall);
+    *reinterpret_cast<int*>(record + R::kFlagAt) = odd ? 1 : 0;
+  }
+  const uint32_t id_w = umma::make_idesc<T>(128, D, 0, 1);
+  if (issuer && alive) {
+    const uint32_t b0 = umma::desc_low(smem_u32(smem), 8192);
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks)
+        umma::mma_ts_low(tb + kTmSC, tb + kTmX + term_a(i) * 32 + ks * 8, b0 + ((term_b(i) * (D / 64) * 8192 + ks * 2048) >> 4), id_w,
+                         i > 0 || ks > 0);
+    umma::commit(made);
+  }
+  __syncwarp();
+  // ------------------------------------------------ out: lane = row r, a warp half of the columns
+  const int quarter = warp & 3, side = warp >> 2, r = quarter * 32 + lane, i = r & 63, odd = lane & 1;
+  const uint32_t group = ((i >> 3) ^ odd) << 4;          // sw128 of row n + odd, n even, but for n & 6
+  const uint32_t base = tb + ((uint32_t)(quarter * 32) << 16) + kTmSC + side * (D / 2);
+  alive = alive && wait(made, 0);
+  umma::fence_after_sync();
+#pragma unroll 1
+  for (int c0 = 0; c0 < D / 2; c0 += 16) {
+    uint32_t w[16];
+    umma::ld16(base + c0, w);
+    umma::wait_ld();
+    const int n0 = side * (D / 2) + c0;
+    float x[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) x[c] = uncut(w[c], quarter >= 2 ? kCut4 : kCut1);      // (rows of T: mostly their diagonal)
+    if (quarter >= 2) {
+#pragma unroll
+      for (int c = 0; c < 16; c += 4) {
+        const float4 qs = *reinterpret_cast<const float4*>(sQs + i * M::kQRow + n0 + c);
+        x[c] = qs.x - x[c], x[c + 1] = qs.y - x[c + 1], x[c + 2] = qs.z - x[c + 2], x[c + 3] = qs.w - x[c + 3];
+      }
+    }
+    // rows of the record run along r: a lane gets its neighbour's value of one of two channels and writes the pair, in row n0 + c + odd
+    const uint32_t at = (quarter >> 1) * (D * 128) + (n0 + odd) * 128 + (i & 6) * 2;
+#pragma unroll
+    for (int c = 0; c < 16; c += 2) {
+      const float other = __shfl_xor_sync(0xffffffffu, odd ? x[c] : x[c + 1], 1);
+      uint32_t y[3];
+      split3cut(odd ? other : x[c], odd ? x[c + 1] : other, y);
+      uint8_t* to = record + (at + c * 128 + (group ^ ((c & 6) << 4)));
+#pragma unroll
+      for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(to + p * (2 * D * 128)) = y[p];
+    }
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  if (issuer && alive) {
+    const uint32_t b0 = umma::desc_low(smem_u32(sV), 8192);
+#pragma unroll
+    for (int p = 2; p >= 0; --p)
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks)
+        umma::mma_ts_low(tb + kTmSC, tb + kTmX + p * 32 + ks * 8, b0 + ((ks * 2048) >> 4), id_w, p < 2 || ks > 0);
+    umma::commit(made);
+  }
+  __syncwarp();
+  alive = alive && wait(made, 1);
+  umma::fence_after_sync();
+  const uint32_t uo = R::kUoAt + (side * (D / 2) * R::kUoRow + r) * 4;
+#pragma unroll 1
+  for (int c0 = 0; c0 < D / 2; c0 += 16) {
+    uint32_t w[16];
+    umma::ld16(base + c0, w);
+    umma::wait_ld();
+    float* to = reinterpret_cast<float*>(record + (uo + c0 * R::kUoRow * 4));
+#pragma unroll
+    for (int c = 0; c < 16; ++c) to[c * R::kUoRow] = uncut(w[c], quarter >= 2 ? kCut4 : kCut1);
+  }
+  umma::fence_before_sync();
+  if (*gave_up) {                                        // products under way finish before the columns and the operands go
+    if (issuer) umma::commit(drained);
+    if (warp == 0) __syncwarp(), mbar_wait_bounded(drained, 0, nullptr, kDrainNs);
+  }
+  __syncthreads();
+  if (warp == 1) umma::tmem_dealloc(tb, 256);
+  if (threadIdx.x == 0 && *gave_up) {
+    *reinterpret_cast<volatile int*>(DP.wait_status) = 1;
+    __threadfence_system();
+  }
+}
+
+
+constexpr int kDsThreads = 288;
+template <int D, int NH>
+constexpr int ds_smem() {
+  return 1024 + NH * (DcRecord<D>::kWq + DcRecord<D>::kKe + DcRecord<D>::kUo) + 2 * NH * D * 4 + 256;
+}
+
+template <int D, int NH>
+__global__ void __launch_bounds__(kDsThreads, 1)
+delta_scan_kernel(const __grid_constant__ DcParams DP) {
+  using T = __nv_bfloat16;
+  using R = DcRecord<D>;
+  static_assert(D * NH == 128, "128 value channels");
+  const DeltaParams& P = DP.d;
+  extern __shared__ __align__(1024) uint8_t ds_smem_raw[];
+  uint8_t* smem = ds_smem_raw + (-smem_u32(ds_smem_raw) & 1023u);       // (not through an integer: the compiler has to know that it is shared memory)
+  uint8_t *sWq = smem, *sKe = sWq + NH * R::kWq, *sUo = sKe + NH * R::kKe;
+  float* sPe = reinterpret_cast<float*>(sUo + NH * R::kUo);            // [2][NH * D]
+  uint64_t *wq_full = reinterpret_cast<uint64_t*>(sPe + 2 * NH * D), *ke_full = wq_full + 1, *uo_full = wq_full + 2, *s_ready = wq_full + 3,
+           *e_done = wq_full + 4, *w_ready = wq_full + 5, *d_done = wq_full + 6, *uo_read = wq_full + 7, *drained = wq_full + 8;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wq_full + 9);
+  volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  constexpr float kCut = D == 128 ? kCut8 : kCut4;
+  constexpr uint32_t kTmS = 0, kTmW = 0, kTmE = 256, kTmD = 384;       // S 3 x D / 2 (w 3 x 32 in its place), E 128, dS D
+
+  pdl_wait();
+  const int s = blockIdx.y, h0 = blockIdx.x * NH, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const SeqSpan sp = seq_span(P.cu_q, P.cu_k, nullptr, s);
+  const int before = chunks_before(P.cu_q, s);
+  const int lo = max(0, DP.c.first - before), hi = min(chunks_of(sp.q_len), DP.c.first + DP.c.count - before), chunks = hi - lo;
+  if (chunks <= 0) return;
+  uint8_t* records = DP.c.records + ((int64_t)(before + lo - DP.c.first) * P.H + h0) * DP.c.bytes;       // of chunk lo; a chunk on: P.H records
+  const int64_t step = (int64_t)P.H * DP.c.bytes;
+  const bool first_pass = lo == 0, last_pass = hi == chunks_of(sp.q_len);
+
+  const int c = (warp & 3) * 32 + lane, half = warp >> 2, hh = NH == 2 ? (c >> 6) : 0;
+  float S[D / 2];                                        // S[n][c], n = half * D / 2 + i
+  float* mine = nullptr;
+  bool odd = false;
+  if (warp < 8) {
+#pragma unroll
+    for (int i = 0; i < D / 2; ++i) S[i] = 0.f;
+    if (P.state != nullptr || !(first_pass && last_pass)) mine = chunk_state(P, DP.c, s, h0 + hh) + (int64_t)half * (D / 2) * D + (c & (D - 1));
+    if (first_pass ? P.state != nullptr && sp.first_pos() > 0 : true) {
+#pragma unroll
+      for (int i = 0; i < D / 2; ++i) S[i] = mine[i * D];
+#pragma unroll
+      for (int i = 0; i < D / 2; ++i) odd = odd || magnitude(S[i]) >= kBig;
+    }
+    if (P.state == nullptr && last_pass) mine = nullptr;
+  }
+  for (int j = threadIdx.x; j < chunks * NH; j += kDsThreads)
+    odd = odd || *reinterpret_cast<const int*>(records + (int64_t)(j / NH) * step + (j % NH) * DP.c.bytes + R::kFlagAt) != 0;
+  if (threadIdx.x == 0) {
+    mbar_init(wq_full, 1), mbar_init(ke_full, 1), mbar_init(uo_full, 1), mbar_init(s_ready, 256), mbar_init(e_done, 1), mbar_init(w_ready, 256);
+    mbar_init(d_done, 1), mbar_init(uo_read, 256), mbar_init(drained, 1);
+    mbar_fence_init();
+    *gave_up = 0;
+  }
+  if (__syncthreads_or(odd)) {                           // one token at a time, behind this kernel
+    if (threadIdx.x < NH) *reinterpret_cast<int*>(records + threadIdx.x * DP.c.bytes + R::kFlagAt) = 1;
+    return;
+  }
+  if (warp == 8) umma::tmem_alloc(tmem_slot, 512);
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  constexpr uint32_t tb = 0;                             // all 512 columns: they start at 0
+  auto wait = [&](uint64_t* bar, int parity) { return mbar_warp_wait(bar, parity & 1, DP.wait_tries, gave_up); };
+
+  if (warp < 8) {
+    const uint32_t base = tb + ((uint32_t)((warp & 3) * 32) << 16);
+    const int64_t out_stride = (int64_t)P.H * D;
+    float* out = P.out + (int64_t)h0 * D + c;
+    const float4* uo = reinterpret_cast<const float4*>(sUo + c * (R::kUoRow * 4));
+    for (int j = 0;; ++j) {
+      if (j > 0) {
+        if (!wait(d_done, j - 1)) break;
+        umma::fence_after_sync();
+        const float* pe = sPe + ((j - 1) & 1) * (NH * D) + hh * D + half * (D / 2);
+#pragma unroll
+        for (int i0 = 0; i0 < D / 2; i0 += 16) {
+          uint32_t w[16];
+          umma::ld16(base + kTmD + half * (D / 2) + i0, w);
+          umma::wait_ld();
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            const float4 p = *reinterpret_cast<const float4*>(pe + i0 + i);
+            S[i0 + i] = fmaf(p.x, S[i0 + i], uncut(w[i], kCut4));
+            S[i0 + i + 1] = fmaf(p.y, S[i0 + i + 1], uncut(w[i + 1], kCut4));
+            S[i0 + i + 2] = fmaf(p.z, S[i0 + i + 2], uncut(w[i + 2], kCut4));
+            S[i0 + i + 3] = fmaf(p.w, S[i0 + i + 3], uncut(w[i + 3], kCut4));
+          }
+        }
+      }
+      if (j == chunks) break;
+#pragma unroll
+      for (int i0 = 0; i0 < D / 2; i0 += 16) {           // as the A operand: packed pairs along n
+        uint32_t w[3][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          uint32_t x[3];
+          split3cut(S[i0 + 2 * i], S[i0 + 2 * i + 1], x);
+          w[0][i] = x[0], w[1][i] = x[1], w[2][i] = x[2];
+        }
+#pragma unroll
+        for (int p = 0; p < 3; ++p) umma::st8(base + kTmS + p * (D / 2) + half * (D / 4) + i0 / 2, w[p]);
+      }
+      umma::wait_st();
+      umma::fence_before_sync();
+      mbar_arrive(s_ready);
+      if (!wait(uo_full, j) || !wait(e_done, j)) break;
+      umma::fence_after_sync();
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {                      // what is written: this thread's 32 tokens
+        uint32_t e[16], w[3][8];
+        umma::ld16(base + kTmE + half * 32 + 16 * u, e);
+        float4 x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = uo[half * 8 + 4 * u + i];
+        umma::wait_ld();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t y[3];
+          split3cut(x[i].x - uncut(e[4 * i], kCut), x[i].y - uncut(e[4 * i + 1], kCut), y);
+          w[0][2 * i] = y[0], w[1][2 * i] = y[1], w[2][2 * i] = y[2];
+          split3cut(x[i].z - uncut(e[4 * i + 2], kCut), x[i].w - uncut(e[4 * i + 3], kCut), y);
+          w[0][2 * i + 1] = y[0], w[1][2 * i + 1] = y[1], w[2][2 * i + 1] = y[2];
+        }
+#pragma unroll
+        for (int p = 0; p < 3; ++p) umma::st8(base + kTmW + p * 32 + half * 16 + 8 * u, w[p]);
+      }
+      umma::wait_st();
+      umma::fence_before_sync();
+      mbar_arrive(w_ready);
+      const int t0 = (lo + j) * kDcL + half * 32, left = sp.q_len - t0;
+      float* to = out + (sp.q_start + (int64_t)t0) * out_stride;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        uint32_t e[16];
+        umma::ld16(base + kTmE + 64 + half * 32 + 16 * u, e);
+        float4 x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = uo[16 + half * 8 + 4 * u + i];
+        umma::wait_ld();
+        const float o[16] = {x[0].x, x[0].y, x[0].z, x[0].w, x[1].x, x[1].y, x[1].z, x[1].w,
+                             x[2].x, x[2].y, x[2].z, x[2].w, x[3].x, x[3].y, x[3].z, x[3].w};
+        if (left >= 32) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i, to += out_stride) *to = o[i] + uncut(e[i], kCut);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i, to += out_stride)
+            if (16 * u + i < left) *to = o[i] + uncut(e[i], kCut);
+        }
+      }
+      umma::fence_before_sync();
+      mbar_arrive(uo_read);
+    }
+    if (mine != nullptr) {
+#pragma unroll
+      for (int i = 0; i < D / 2; ++i) mine[i * D] = S[i];
+    }
+  } else {
+    const uint32_t id_e = umma::make_idesc<T>(128, 128, 0, 1), id_d = umma::make_idesc<T>(128, D, 0, 1);
+    const uint32_t dwq = umma::desc_low(smem_u32(sWq), D * 128), dke = umma::desc_low(smem_u32(sKe), 8192);
+    const bool leader = umma::elect_one();
+    auto load = [&](int j, int at, int bytes, uint8_t* to, uint64_t* bar, bool ends) {       // (ends: with P_end)
+      if (leader) {
+        mbar_expect_tx(bar, NH * (bytes + (ends ? D * 4 : 0)));
+        for (int n = 0; n < NH; ++n) {
+          const uint8_t* from = records + j * step + n * DP.c.bytes;
+          bulk_load(to + n * bytes, from + at, bytes, bar);
+          if (ends) bulk_load(sPe + (j & 1) * (NH * D) + n * D, from + R::kPeAt, D * 4, bar);
+        }
+      }
+      __syncwarp();
+    };
+    auto load_wq = [&](int j) { load(j, 0, R::kWq, sWq, wq_full, false); };
+    auto load_ke = [&](int j) { load(j, R::kKeAt, R::kKe, sKe, ke_full, false); };
+    auto load_uo = [&](int j) { load(j, R::kUoAt, R::kUo, sUo, uo_full, true); };
+    int wq = 0, ke = 0, uo = 0;                          // copies begun
+    if (DP.wait_tries > 0) load_wq(wq++), load_uo(uo++), load_ke(ke++);      // (a limit of 0 tests the way out: nothing comes)
+    for (int j = 0; j < chunks; ++j) {
+      const bool more = j + 1 < chunks;
+      if (!wait(wq_full, j) || !wait(s_ready, j)) break;
+      umma::fence_after_sync();
+      if (leader) {
+#pragma unroll 1
+        for (int i = 0; i < 6; ++i) {
+          const uint32_t pa = term_a(i), pb = term_b(i);
+#pragma unroll
+          for (int n = 0; n < NH; ++n)
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks) {
+              const uint32_t a = tb + kTmS + pa * (D / 2) + ks * 8, b = dwq + ((n * R::kWq + pb * (2 * D * 128) + ks * 2048) >> 4);
+              if (NH == 2) mma_ts_half_low(tb + kTmE, a, b, id_e, i > 0 || ks > 0, n);
+              else umma::mma_ts_low(tb + kTmE, a, b, id_e, i > 0 || ks > 0);
+            }
+        }
+        umma::commit(e_done);
+      }
+      __syncwarp();
+      if (!wait(e_done, j)) break;
+      if (more) load_wq(wq++);
+      if (!wait(ke_full, j) || !wait(w_ready, j)) break;
+      umma::fence_after_sync();
+      if (leader) {
+#pragma unroll 1
+        for (int i = 0; i < 6; ++i) {
+          const uint32_t pa = term_a(i), pb = term_b(i);
+#pragma unroll
+          for (int n = 0; n < NH; ++n)
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) {
+              const uint32_t a = tb + kTmW + pa * 32 + ks * 8, b = dke + ((n * R::kKe + pb * (D / 64) * 8192 + ks * 2048) >> 4);
+              if (NH == 2) mma_ts_half_low(tb + kTmD, a, b, id_d, i > 0 || ks > 0, n);
+              else umma::mma_ts_low(tb + kTmD, a, b, id_d, i > 0 || ks > 0);
+            }
+        }
+        umma::commit(d_done);
+      }
+      __syncwarp();
+      if (!wait(uo_read, j)) break;
+      if (more) load_uo(uo++);
+      if (!wait(d_done, j)) break;
+      if (more) load_ke(ke++);
+    }
+    // copies and products under way finish before the columns and the operands go
+    if (*gave_up) {
+      if (wq > 0) mbar_wait_bounded(wq_full, (wq - 1) & 1, nullptr, kDrainNs);
+      if (ke > 0) mbar_wait_bounded(ke_full, (ke - 1) & 1, nullptr, kDrainNs);
+      if (uo > 0) mbar_wait_bounded(uo_full, (uo - 1) & 1, nullptr, kDrainNs);
+      __syncwarp();
+    }
+    if (leader) umma::commit(drained);
+    __syncwarp();
+    mbar_wait_bounded(drained, 0, nullptr, kDrainNs);
+    __syncwarp();
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  if (warp == 8) umma::tmem_dealloc(tb, 512);
+  if (threadIdx.x == 0 && *gave_up) {
+    *reinterpret_cast<volatile int*>(DP.wait_status) = 1;
+    __threadfence_system();
+  }
+}
+
+constexpr int64_t kDcWorkspace = 512ll << 20;           // more than this and a step takes several passes
+
+static int64_t dc_chunks(int num_seqs, int64_t total_q) { return total_q / kDcL + num_seqs; }      // no step has more
+static int64_t dc_record(int D) { return D == 128 ? DcRecord<128>::kBytes : DcRecord<64>::kBytes; }
+
+// Steps with a span of 96 tokens at least whose chunks are the faster way. Either way's time in ns, from prompts alone, of equal and of
+// ragged lengths and beside single tokens (us, tokens / chunks; a decay per channel, with one per head 2 to 10 % less on both sides):
+//   8 heads of 128:  1 x 96 37 / 36, x 256 93 / 45, x 1024 360 / 100;  16 x 96 61 / 54, x 256 153 / 103, x 1024 594 / 314;  64 x 128 304 / 192;
+//                    16 of 500-1300 699 / 306;  1024 beside 32 x 1 364 / 133, beside 64 x 16 396 / 173;  [64 x 32 83 / 112, kept to tokens]
+//   32 heads of 64:  1 x 96 31 / 31, x 256 77 / 42, x 1024 299 / 117;  4 x 256 77 / 67, x 1024 300 / 214;  1024 beside 64 x 16 389 / 262;
+//                    [16 x 128 68 / 115, x 1024 508 / 734, 16 of 500-1300 572 / 708, kept to tokens: a chunk of a head of 64 costs
+//                    delta_chunk_kernel 0.6 of one of 128, a token of it delta_rule_kernel a fifth]
+static bool dc_shape(int mode, int dtype, int num_seqs, int max_q, int64_t total_q, int H, int kdim, int vdim) {
+  if (mode == kWkv || dtype != B200_DTYPE_BF16 || num_seqs <= 0 || num_seqs > 65535 || kdim != vdim || max_q < 96) return false;
+  if (!(kdim == 128 || (kdim == 64 && H % 2 == 0)) || H > 65535 || (total_q / kDcL + num_seqs) * H > INT_MAX / 2) return false;
+  const int64_t chunks = (total_q / kDcL + num_seqs / 2) * H, more = std::max<int64_t>(chunks - 300, 0);       // 300 run at a time
+  const int64_t tokens_ns = kdim == 128 ? std::max<int64_t>(355ll * max_q, total_q * H * 44 / 10) : std::max<int64_t>(285ll * max_q, total_q * H * 97 / 100);
+  const int64_t chunks_ns = kdim == 128 ? 26000 + 72ll * max_q + 140 * more : 20000 + 85ll * max_q + 77 * more;
+  return chunks_ns < tokens_ns;
+}
+
+int64_t delta_chunks_workspace(int mode, int dtype, int num_seqs, int max_q, int64_t total_q, int H, int groups, int kdim, int vdim) {
+  if (H <= 0 || groups <= 0 || H % groups != 0 || !dc_shape(mode, dtype, num_seqs, max_q, total_q, H, kdim, vdim)) return 0;
+  const int64_t chunk = dc_record(kdim) * H, carry = (int64_t)H * kdim * vdim * 4, all = dc_chunks(num_seqs, total_q) * chunk;
+  return carry + std::min(all, std::max(chunk, kDcWorkspace / chunk * chunk));
+}
+
+bool delta_chunks_ok(const DeltaParams& P, int mode, int dtype, int num_seqs, int max_q, int64_t total_q, const void* workspace, int64_t bytes) {
+  if (P.cu_q == nullptr || workspace == nullptr || !aligned16(workspace)) return false;
+  if (!dc_shape(mode, dtype, num_seqs, max_q, total_q, P.H, P.kdim, P.vdim)) return false;
+  if (bytes < (int64_t)P.H * (dc_record(P.kdim) + (int64_t)P.kdim * P.vdim * 4)) return false;
+  if (std::max(P.q_stride, P.k_stride) >= 1 << 22 || (int64_t)P.H * P.kdim >= 1 << 22) return false;       // (32-bit offsets inside a chunk)
+  if (P.q_stride % 4 != 0 || P.k_stride % 4 != 0 || !aligned16(P.q) || !aligned16(P.k) || (mode == kDecayPerChannel && !aligned16(P.g))) return false;
+  return P.v_stride % 8 == 0 && aligned16(P.v);
+}
+
+template <int D, bool PER_HEAD>
+static int delta_chunks_launch_as(DcParams DP, int mode, int64_t total_q, int64_t bytes, cudaStream_t stream) {
+  constexpr int NH = 128 / D;
+  auto chunk = delta_chunk_kernel<D, PER_HEAD>;
+  auto scan = delta_scan_kernel<D, NH>;
+  constexpr int chunk_smem = DcSmem<D>::kBytes, scan_smem = ds_smem<D, NH>();
+  static_assert(2 * (chunk_smem + 1024) <= 228 * 1024 && scan_smem <= 227 * 1024, "two CTAs' shared memory, one's");
+  static std::atomic<uint64_t> chunk_devices{0}, scan_devices{0};
+  cudaError_t allowed = allow_smem(chunk, chunk_smem, chunk_devices);
+  if (allowed == cudaSuccess) allowed = allow_smem(scan, scan_smem, scan_devices);
+  if (allowed != cudaSuccess) return (int)allowed;
+  const DeltaParams& P = DP.d;
+  const int64_t chunks = dc_chunks(DP.num_seqs, total_q), record = DcRecord<D>::kBytes, carry = (int64_t)P.H * D * D * 4;
+  const int64_t room = (bytes - carry) / (record * P.H), passes = (chunks + room - 1) / room, count = (chunks + passes - 1) / passes;
+  DP.c.bytes = record, DP.c.flag_at = DcRecord<D>::kFlagAt, DP.c.count = (int)count;
+  DP.c.carry = reinterpret_cast<float*>(DP.c.records + count * record * P.H);
+  for (int64_t at = 0; at < chunks; at += count) {
+    DP.c.first = (int)at;
+    launch_pdl(chunk, dim3((unsigned)(count * P.H)), dim3(kDcThreads), (size_t)chunk_smem, stream, DP);
+    launch_pdl(scan, dim3((unsigned)(P.H / NH), (unsigned)DP.num_seqs), dim3(kDsThreads), (size_t)scan_smem, stream, DP);
+    const int code = delta_rest_launch(P, DP.c, mode, DP.num_seqs, stream);
+    if (code != B200_OK) return code;
+  }
+  return finish_launch((int)(2 * ((chunks + count - 1) / count)));
+}
+
+int delta_chunks_launch(const DeltaParams& P, int mode, int num_seqs, int64_t total_q, void* workspace, int64_t bytes, int64_t wait_ns,
+                        cudaStream_t stream) {
+  B200_RETURN_IF(take_wait_status(), B200_ERR_WAIT);     // of an earlier call
+  DcParams DP{};
+  DP.d = P, DP.num_seqs = num_seqs, DP.wait_tries = wait_tries(wait_ns), DP.wait_status = wait_status();
+  DP.c.records = reinterpret_cast<uint8_t*>(workspace);
+  B200_RETURN_IF(DP.wait_status == nullptr, B200_ERR_DRIVER);
+  if (mode == kDecayPerHead)
+    return P.kdim == 128 ? delta_chunks_launch_as<128, true>(DP, mode, total_q, bytes, stream) : delta_chunks_launch_as<64, true>(DP, mode, total_q, bytes, stream);
+  return P.kdim == 128 ? delta_chunks_launch_as<128, false>(DP, mode, total_q, bytes, stream) : delta_chunks_launch_as<64, false>(DP, mode, total_q, bytes, stream);
+}
+
+}  // namespace b200

@@ -19,24 +19,11 @@
 // row lie KPT + 4 floats apart: the NS lanes of a column group read different banks. Tokens are staged kDeltaTok at a
 // time; where the rows allow 16-byte copies (VEC) the next batch arrives by cp.async in a second set of buffers while the
 // current one is consumed, otherwise batches are loaded in place.
-#include "seq_common.cuh"
+#include "delta_rule.cuh"
 
 namespace b200 {
 
 constexpr int kDeltaTok = 8;
-enum { kDecayPerChannel = 0, kDecayPerHead = 1, kWkv = 2 };
-
-struct DeltaParams {
-  const float *q, *k;               // [tokens, groups * kdim]
-  const float* g;                   // [tokens, H * kdim]; one decay per head: [tokens, H]
-  const float* beta;                // [tokens, H]; wkv: the current token's coefficient
-  const void* v;                    // [tokens, H * vdim], element type
-  int64_t q_stride, k_stride, v_stride;
-  float* out;                       // [tokens, H * vdim] fp32
-  float* state;                     // [slots, H, kdim, vdim] fp32 or nullptr
-  const int *state_slots, *cu_q, *cu_k, *ctx_lens;
-  int H, groups, kdim, vdim;
-};
 
 // The sequence that `rank` of the `num` are longer than, of equal ones the first first. All threads of the CTA
 __device__ __forceinline__ int sequence_of_rank(const int* cu_q, int num, int rank) {
@@ -59,10 +46,11 @@ __device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* gptr,
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr), "l"(gptr), "r"(bytes) : "memory");
 }
 
-// ORDER: CTAs start with the longest sequences (delta_launch_as)
-template <typename TV, int KPT, int NS, int NC, bool VEC, int MODE, bool ORDER = false>
+// ORDER: CTAs start with the longest sequences (delta_launch_as). REST: only heads that a pass of chunks has left aside (delta_chunks.cu),
+// and the tokens of that pass
+template <typename TV, int KPT, int NS, int NC, bool VEC, int MODE, bool ORDER = false, bool REST = false>
 __global__ void __launch_bounds__(32 * NS)
-delta_rule_kernel(const DeltaParams P) {
+delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
   extern __shared__ __align__(16) float smem[];
   pdl_wait();
   constexpr int NTH = 32 * NS;
@@ -70,8 +58,19 @@ delta_rule_kernel(const DeltaParams P) {
   constexpr int KP = NS * KS;                        // row of padded keys
   constexpr int CC = 32 * NC;                        // value columns per CTA
   const int s = ORDER ? sequence_of_rank(P.cu_q, gridDim.z, blockIdx.z) : blockIdx.z, h = blockIdx.y;
-  const SeqSpan sp = seq_span(P.cu_q, P.cu_k, P.ctx_lens, s);
+  SeqSpan sp = seq_span(P.cu_q, P.cu_k, P.ctx_lens, s);
   if (sp.q_len == 0) return;
+  bool goes_on = false, ends = true;                 // from the pass before, with the span
+  if constexpr (REST) {
+    const int before = chunks_before(P.cu_q, s), n = chunks_of(sp.q_len);
+    const int lo = max(0, C.first - before), hi = min(n, C.first + C.count - before);
+    int flagged = 0;
+    for (int j = lo + threadIdx.x; j < hi; j += NTH)
+      flagged |= *reinterpret_cast<const int*>(C.records + ((int64_t)(before + j - C.first) * P.H + h) * C.bytes + C.flag_at);
+    if (!__syncthreads_or(flagged)) return;
+    goes_on = lo > 0, ends = hi == n;
+    sp.q_start += lo * kDcL, sp.q_len = min(sp.q_len, hi * kDcL) - lo * kDcL;
+  }
   const int kdim = P.kdim, vdim = P.vdim;
   const int ksl = threadIdx.x % NS, cl = (threadIdx.x / NS) * NC;
   const int c0 = blockIdx.x * CC, col = c0 + cl;
@@ -90,7 +89,11 @@ delta_rule_kernel(const DeltaParams P) {
   float* slot = P.state != nullptr
                     ? P.state + (((int64_t)P.state_slots[s] * P.H + h) * kdim) * (int64_t)vdim
                     : nullptr;
-  const bool carried = slot != nullptr && sp.first_pos() > 0;
+  bool carried = slot != nullptr && sp.first_pos() > 0;
+  if constexpr (REST) {
+    if (P.state == nullptr && !(ends && !goes_on)) slot = chunk_state(P, C, s, h);
+    carried = carried || goes_on;
+  }
 #pragma unroll
   for (int r = 0; r < KPT; ++r) {
     const int i = ksl * KPT + r;
@@ -246,7 +249,7 @@ delta_rule_kernel(const DeltaParams P) {
       }
     }
   }
-  if (slot != nullptr) {
+  if (slot != nullptr && (!REST || P.state != nullptr || !ends)) {
 #pragma unroll
     for (int r = 0; r < KPT; ++r) {
       const int i = ksl * KPT + r;
@@ -259,6 +262,7 @@ delta_rule_kernel(const DeltaParams P) {
 
 template <typename TV, int KPT, int NS, int NC, int MODE>
 static void delta_launch_as(const DeltaParams& P, int num_seqs, cudaStream_t stream) {
+  const DeltaChunks C{};                              // (REST alone reads them)
   constexpr int CC = 32 * NC, KP = NS * (KPT + 4);
   constexpr int VE = 16 / (int)sizeof(TV);
   const dim3 grid((P.vdim + CC - 1) / CC, P.H, num_seqs);
@@ -282,14 +286,14 @@ static void delta_launch_as(const DeltaParams& P, int num_seqs, cudaStream_t str
     if constexpr (KPT * NS == 128 && MODE != kWkv) {
       static_assert(2 * kDeltaTok * ((2 * KP + GT + 1) * sizeof(float) + CC * sizeof(TV)) <= 47 * 1024, "no more than a launch may have unasked");
       if (P.cu_q != nullptr && num_seqs > 1 && num_seqs <= 32 && (int64_t)grid.x * grid.y * num_seqs > sm_count()) {
-        launch_pdl(delta_rule_kernel<TV, KPT, NS, NC, true, MODE, true>, grid, dim3(32 * NS), smem, stream, P);
+        launch_pdl(delta_rule_kernel<TV, KPT, NS, NC, true, MODE, true>, grid, dim3(32 * NS), smem, stream, P, C);
         return;
       }
     }
-    launch_pdl(delta_rule_kernel<TV, KPT, NS, NC, true, MODE>, grid, dim3(32 * NS), smem, stream, P);
+    launch_pdl(delta_rule_kernel<TV, KPT, NS, NC, true, MODE>, grid, dim3(32 * NS), smem, stream, P, C);
   } else {
     const size_t smem = (size_t)kDeltaTok * (2 * KP + GT + 1 + CC) * sizeof(float);
-    launch_pdl(delta_rule_kernel<TV, KPT, NS, NC, false, MODE>, grid, dim3(32 * NS), smem, stream, P);
+    launch_pdl(delta_rule_kernel<TV, KPT, NS, NC, false, MODE>, grid, dim3(32 * NS), smem, stream, P, C);
   }
 }
 
@@ -308,15 +312,37 @@ static int delta_launch(const DeltaParams& P, int num_seqs, cudaStream_t stream)
   return finish_launch();
 }
 
+template <int NS, int MODE>
+static void delta_rest_launch_as(const DeltaParams& P, const DeltaChunks& C, int num_seqs, cudaStream_t stream) {
+  using TV = __nv_bfloat16;
+  constexpr int KP = NS * 36, CC = 64;
+  constexpr size_t smem = (size_t)2 * kDeltaTok * (2 * KP + (MODE == kDecayPerHead ? 1 : KP) + 1) * sizeof(float) + (size_t)2 * kDeltaTok * CC * sizeof(TV);
+  static_assert(smem <= 47 * 1024, "no more than a launch may have unasked");
+  launch_pdl(delta_rule_kernel<TV, 32, NS, 2, true, MODE, false, true>, dim3(P.vdim / CC, P.H, num_seqs), dim3(32 * NS), smem, stream, P, C);
+}
+int delta_rest_launch(const DeltaParams& P, const DeltaChunks& C, int mode, int num_seqs, cudaStream_t stream) {
+  if (P.kdim == 128 && mode == kDecayPerHead) delta_rest_launch_as<4, kDecayPerHead>(P, C, num_seqs, stream);
+  else if (P.kdim == 128) delta_rest_launch_as<4, kDecayPerChannel>(P, C, num_seqs, stream);
+  else if (mode == kDecayPerHead) delta_rest_launch_as<2, kDecayPerHead>(P, C, num_seqs, stream);
+  else delta_rest_launch_as<2, kDecayPerChannel>(P, C, num_seqs, stream);
+  return finish_launch();
+}
+
 }  // namespace b200
 
 using namespace b200;
 
-extern "C" int b200_delta_rule(float* out, const float* q, int64_t q_stride, const float* k, int64_t k_stride,
-                               const void* v, int64_t v_stride, const float* g, const float* beta, float* state,
-                               const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k,
-                               const int32_t* ctx_lens, int32_t num_seqs, int32_t num_heads, int32_t groups,
-                               int32_t kdim, int32_t vdim, int32_t mode, int32_t dtype, b200_stream_t stream) {
+extern "C" int64_t b200_delta_rule_workspace_size(int32_t num_seqs, int32_t max_q, int64_t total_q, int32_t num_heads, int32_t groups,
+                                                  int32_t kdim, int32_t vdim, int32_t mode, int32_t dtype) {
+  return delta_chunks_workspace(mode, dtype, num_seqs, max_q, total_q, num_heads, groups, kdim, vdim);
+}
+
+extern "C" int b200_delta_rule_bounded(float* out, const float* q, int64_t q_stride, const float* k, int64_t k_stride, const void* v,
+                                       int64_t v_stride, const float* g, const float* beta, float* state, const int32_t* state_slots,
+                                       const int32_t* cu_q, const int32_t* cu_k, const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q,
+                                       int64_t total_q, int32_t num_heads, int32_t groups, int32_t kdim, int32_t vdim, int32_t mode,
+                                       int32_t dtype, void* workspace, int64_t workspace_bytes, int64_t wait_ns, b200_stream_t stream) {
+  B200_RETURN_IF(wait_ns < 0, B200_ERR_BAD_SHAPE);
   B200_RETURN_IF(num_seqs < 0 || num_heads <= 0 || groups <= 0 || num_heads % groups != 0 || kdim <= 0 || vdim <= 0 ||
                      mode < kDecayPerChannel || mode > kWkv,
                  B200_ERR_BAD_SHAPE);
@@ -328,10 +354,30 @@ extern "C" int b200_delta_rule(float* out, const float* q, int64_t q_stride, con
   P.q = q, P.k = k, P.g = g, P.beta = beta, P.v = v, P.q_stride = q_stride, P.k_stride = k_stride;
   P.v_stride = v_stride, P.out = out, P.state = state, P.state_slots = state_slots, P.cu_q = cu_q, P.cu_k = cu_k;
   P.ctx_lens = ctx_lens, P.H = num_heads, P.groups = groups, P.kdim = kdim, P.vdim = vdim;
+  if (delta_chunks_ok(P, mode, dtype, num_seqs, max_q, total_q, workspace, workspace_bytes))
+    return delta_chunks_launch(P, mode, num_seqs, total_q, workspace, workspace_bytes, wait_ns, (cudaStream_t)stream);
   B200_DISPATCH_3(dtype, TV, {
     if (mode == kDecayPerHead) return delta_launch<TV, kDecayPerHead>(P, num_seqs, (cudaStream_t)stream);
     if (mode == kWkv) return delta_launch<TV, kWkv>(P, num_seqs, (cudaStream_t)stream);
     return delta_launch<TV, kDecayPerChannel>(P, num_seqs, (cudaStream_t)stream);
   });
   return B200_OK;
+}
+
+extern "C" int b200_delta_rule_step(float* out, const float* q, int64_t q_stride, const float* k, int64_t k_stride, const void* v,
+                                    int64_t v_stride, const float* g, const float* beta, float* state, const int32_t* state_slots,
+                                    const int32_t* cu_q, const int32_t* cu_k, const int32_t* ctx_lens, int32_t num_seqs, int32_t max_q,
+                                    int64_t total_q, int32_t num_heads, int32_t groups, int32_t kdim, int32_t vdim, int32_t mode, int32_t dtype,
+                                    void* workspace, int64_t workspace_bytes, b200_stream_t stream) {
+  return b200_delta_rule_bounded(out, q, q_stride, k, k_stride, v, v_stride, g, beta, state, state_slots, cu_q, cu_k, ctx_lens, num_seqs,
+                                     max_q, total_q, num_heads, groups, kdim, vdim, mode, dtype, workspace, workspace_bytes, kWaitNs, stream);
+}
+
+extern "C" int b200_delta_rule(float* out, const float* q, int64_t q_stride, const float* k, int64_t k_stride,
+                               const void* v, int64_t v_stride, const float* g, const float* beta, float* state,
+                               const int32_t* state_slots, const int32_t* cu_q, const int32_t* cu_k,
+                               const int32_t* ctx_lens, int32_t num_seqs, int32_t num_heads, int32_t groups,
+                               int32_t kdim, int32_t vdim, int32_t mode, int32_t dtype, b200_stream_t stream) {
+  return b200_delta_rule_step(out, q, q_stride, k, k_stride, v, v_stride, g, beta, state, state_slots, cu_q, cu_k, ctx_lens, num_seqs, 1, 0,
+                              num_heads, groups, kdim, vdim, mode, dtype, nullptr, 0, stream);
 }

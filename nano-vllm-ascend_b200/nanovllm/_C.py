@@ -185,6 +185,14 @@ PROTOTYPES = {
     "b200_delta_rule": (c_int32, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
                                   c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32,
                                   c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p]),
+    "b200_delta_rule_workspace_size": (c_int64, [c_int32, c_int32, c_int64, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32]),
+    "b200_delta_rule_step": (c_int32, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
+                                       c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int64,
+                                       c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p, c_int64, c_void_p]),
+    "b200_delta_rule_bounded": (c_int32, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
+                                          c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int64,
+                                          c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_void_p, c_int64, c_int64,
+                                          c_void_p]),
     "b200_latent_kv_prep": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_void_p, c_int64,
                                       c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32,
                                       c_int32, c_int32, c_int32, c_double, c_int32, c_float, c_int32, c_void_p]),
