@@ -82,9 +82,9 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint3
                : "memory");
 }
 // The tensor core cuts a sum off after every 16 products; on average results lack this part of them. Measured as the mean relative difference
-// from 64-bit products of random operands, for sums of 8, 4 and 2 times 16 products, and for one large product among small ones. Added back,
+// from 64-bit products of random operands: of 8, 4 and 2 times 16 products, and in W, U (mostly one product each) and O0. Added back,
 // in fp32: outputs 2.6e-7 -> 2.2e-7 off, states 2.2e-7 -> 1.9e-7, where the token form is 2.2e-7 and 2.0e-7 off (the case above).
-constexpr float kCut8 = 1.4e-7f, kCut4 = 0.9e-7f, kCut2 = 0.45e-7f, kCut1 = 0.42e-7f;
+constexpr float kCut8 = 1.5e-7f, kCut4 = 0.9e-7f, kCut2 = 0.45e-7f, kCutW = 0.42e-7f, kCutU = 0.5e-7f, kCutO = 0.6e-7f;
 __device__ __forceinline__ float uncut(uint32_t x, float part) { return fmaf(__uint_as_float(x), part, __uint_as_float(x)); }
 __device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 __device__ __forceinline__ float largest(float most, float2 x) {             // of |x|; NaN stays
@@ -536,7 +536,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     const int n0 = side * (D / 2) + c0;
     float x[16];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) x[c] = uncut(w[c], quarter >= 2 ? kCut4 : kCut1);      // (rows of T: mostly their diagonal)
+    for (int c = 0; c < 16; ++c) x[c] = uncut(w[c], quarter >= 2 ? kCut4 : kCutW);
     if (quarter >= 2) {
 #pragma unroll
       for (int c = 0; c < 16; c += 4) {
@@ -579,7 +579,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     umma::wait_ld();
     float* to = reinterpret_cast<float*>(record + (uo + c0 * R::kUoRow * 4));
 #pragma unroll
-    for (int c = 0; c < 16; ++c) to[c * R::kUoRow] = uncut(w[c], quarter >= 2 ? kCut4 : kCut1);
+    for (int c = 0; c < 16; ++c) to[c * R::kUoRow] = uncut(w[c], quarter >= 2 ? kCutO : kCutU);
   }
   umma::fence_before_sync();
   if (*gave_up) {                                        // products under way finish before the columns and the operands go
