@@ -631,6 +631,11 @@ extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const v
   p.sink = sink;
   p.window = window, p.keep_first = window > 0 ? keep_first : 0, p.chunk = chunk;
 
+  if (num_ctas <= 0 && head_dim == value_dim && window == 0 && chunk == 0) {
+    const int ctas = decode_small_ctas((int64_t)batch * num_kv_heads, (int64_t)block_table_stride * block_size, head_dim);
+    if (ctas > 0) return decode_small_launch(p, k_cache, v_cache, num_blocks, head_dim, dtype, ctas, stream);
+  }
+
   const int k_chunks = num_kv_heads * head_dim / 64, v_chunks = num_kv_heads * value_dim / 64;
   CUtensorMap mk, mv;
   int rc = get_panel_map(k_cache, (int64_t)num_blocks * block_size, (int64_t)k_chunks * 128, k_chunks,
@@ -640,7 +645,7 @@ extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const v
                      p.rows_box, hkv_cta * value_dim / 64, dtype, &mv);
   if (rc != B200_OK) return rc;
 
-  // num_ctas 0: the library's choice (us at 64 / 112 / 148 CTAs; contexts a third to all of the length named).
+  // num_ctas 0: the library's choice (few rows: decode_small.cu, above; us at 64 / 112 / 148 CTAs; contexts a third to all of the length named).
   // * A CTA's tiles of 8 heads of 128 (64 KB per stage) in batches of 16 and more: three quarters of the SMs, each with
   //   192 KB under way, keep HBM busier than all of them: 256 x 1074 tokens 152 / 114 / 119, 64 x 1074 46 / 37.6 / 38.7, 256 x
   //   50 21 / 16.9 / 18.3, 16 x 1024 17 / 14.8 / 15.3. Smaller tiles need every SM: 8 heads of 64 105 / 73 / 68.

@@ -138,6 +138,11 @@ decode_combine_kernel(const DecodeParams p, int rows /* = HKV_CTA*G */) {
   }
 }
 
+// decode_small.cu: one launch, a cluster of CTAs per (row, kv head); keys and values of one size, no window, no chunk. decode_small_ctas: how
+// many for `pairs` (row, kv head) whose block tables have room for `width` tokens (0: the step is not for it)
+int decode_small_ctas(int64_t pairs, int64_t width, int dim);
+int decode_small_launch(const DecodeParams& p, const void* k, const void* v, int num_blocks, int dim, int dtype, int ctas, cudaStream_t stream);
+
 static inline int hkv_cta_of(int Hkv) {
   if (Hkv >= 8) return Hkv % 8 == 0 ? 8 : 0;
   return (Hkv == 1 || Hkv == 2 || Hkv == 4) ? Hkv : 0;
