@@ -23,16 +23,17 @@
 //                                            B = V MN-major straight from its [key][d] rows
 //                     issue order  S0(0) S1(0) | PV0(0) S0(1) PV1(0) S1(1) | PV0(1) S0(2) ...
 //                     so that the tensor pipe works on tile 1-t while warpgroup t is in its softmax.
-//   warps 10, 11      give their registers away (prefill_threads)
+//   warp 10           finds the work items of the softmax warps, one ahead
+//   warp 11           gives its registers away (prefill_threads)
 //   TMEM (512 columns): O[t] at 128 t, S[t] at 256 + 128 t, P[t] aliases S[t] columns [0, 64).
 //   Shared memory: Q 2 x 32 KiB + K 2 x 32 KiB + V 2 x 32 KiB = 192 KiB at D = 128; one CTA per SM.
-// QT = 1: one query tile per CTA: warps 0-3 softmax, warp 4 TMA, warp 5 MMA; single-stage K / V rings; 256
+// QT = 1: one query tile per CTA: warps 0-3 softmax, warp 4 TMA, warp 5 MMA, warp 6 items; single-stage K / V rings; 256
 //   TMEM columns (O at 0, S at 128), 105 KiB of shared memory -> two CTAs per SM.
 // A CTA walks several work items (Q of the next one is loaded, and its first S computed, under the epilogue of the one
 // before); a row's sizes live in shared memory, since 128 scores leave no registers for them. Sums and products of scores are
-// packed fp32 pairs, row maxima four chains. What bounds it (16 x 1024 tokens, 16 heads over 8 of 128, inputs that rotate: 107 us =
-// 643 TFLOP/s; 129 us with one item per CTA and one head): the chain S -> softmax -> P V -> S of a tile, 3300 to 3700 cycles of which
-// the tensor pipe works 1448 for each of two tiles, and what goes with an item -- first loads, drain, epilogue -- at about 7 us
+// packed fp32 pairs, row maxima four chains. What bounds it (16 x 1024 tokens, 16 heads over 8 of 128, inputs that rotate: 104.5 us =
+// 657 TFLOP/s; 129 us with one item per CTA and one head): the chain S -> softmax -> P V -> S of a tile, 3300 to 3700 cycles of which
+// the tensor pipe works 1448 for each of two tiles, and what goes with an item -- first loads, drain, epilogue -- at about 3 us
 // (1024 items of 31 pair tiles per CTA against as many of 114).
 // Hazards: S[t](j+1) overwrites the columns PV[t](j) reads P from -- both are tcgen05.mma of the same
 // issuing thread and execute in issue order; softmax(j+1) of tile t starts only after S[t](j+1) has
@@ -73,6 +74,7 @@ struct PrefillUmmaParams {
   // optional: scores capped by cap * tanh(scale * s / cap) (cap_pre = scale / cap; 0 = off), and a sink logit per
   // query head (fp32 [H], natural-log units) that joins the softmax denominator without a value
   float cap = 0.f, cap_pre = 0.f;
+  float2 cap_poly[4] = {};          // cap tanh(cap_pre x) = x (cap_poly[0] + x^2 (cap_poly[1] + ..)), each twice, as packed operations take it
   const float* sink = nullptr;
   int window = 0, keep_first = 0;   // window 0: every earlier key
   int chunk = 0;                    // chunk > 0: only keys of the row's own chunk (counted from position 0)
@@ -84,6 +86,7 @@ struct PrefillUmmaParams {
 
 constexpr int kUBM = 128, kUBN = 128;
 constexpr int kOrderSeqs = 256;     // sequences that a launch orders by length
+constexpr int kItems = 2;           // slots of work items: the one in hand and the next
 
 // QT = query tiles per CTA. QT = 2: the layout described above (one CTA per SM, two tiles ping-pong, K/V
 // tiles shared, 2-stage rings). QT = 1: one 128-row tile per CTA, single-stage K/V rings (K(j+1) is loaded
@@ -154,6 +157,7 @@ struct Item {
   int seq, head, split, q0, Lq, k0, Lk, m0, off, kept, skip, ntq, j_lo, NT;
   int n_tiles[2];
   bool ends_here[2];     // this split holds the last key tile of query tile t
+  bool none;             // past the last item
 };
 
 template <typename T, int DK, int DV, int QT, bool CAP>
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(prefill_threads(QT), DK > 128 ? 1 : 3 - QT)
 prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const PrefillUmmaParams p) {
   constexpr int kUStages = prefill_stages(DK, QT);   // K/V ring depth
-  constexpr int kTmaWarp = 4 * QT, kMmaWarp = 4 * QT + 1;
+  constexpr int kTmaWarp = 4 * QT, kMmaWarp = 4 * QT + 1, kItemWarp = 4 * QT + 2;
   constexpr uint32_t kTmemCols = QT * 256;      // O[t] at 128 t, S[t] at QT * 128 + 128 t
   constexpr uint32_t kSBase = QT * 128;
   constexpr int CHK = DK / 64, CHV = DV / 64;   // 128-byte chunks per key / value head row
@@ -179,8 +183,8 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint8_t* s_out = sV + kUStages * VTILE;        // [4 QT warps][32 rows x 64 bytes]: the epilogue's way to whole sectors
   uint16_t* s_tiles = reinterpret_cast<uint16_t*>(s_out + 4 * QT * 2048);   // [kOrderSeqs] row tiles, most first
   uint16_t* s_order = s_tiles + kOrderSeqs;                                 // [kOrderSeqs] their sequences
-  Item* s_items = reinterpret_cast<Item*>(s_order + kOrderSeqs);            // [4 QT softmax warps][2]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_items + 8 * QT);
+  Item* s_items = reinterpret_cast<Item*>(s_order + kOrderSeqs);            // [kItems] for the softmax warps
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_items + kItems);
   uint64_t* q_full = bars;                       // [1]
   uint64_t* k_full = bars + 1;                   // [kUStages]
   uint64_t* v_full = k_full + kUStages;          // [kUStages]
@@ -190,9 +194,9 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* p_full = s_full + 2;                 // [2 tiles][2 halves]  128 softmax threads stored 64 keys of P[t](j)
   uint64_t* o_full = p_full + 4;                 // [2 tiles]  PV[t](j) retired
   uint64_t* q_empty = o_full + 2;                // [1] the item's last S has retired: Q may be overwritten
-  uint64_t* item_full = q_empty + 1;             // [1] every product of the item has retired
-  uint64_t* o_empty = item_full + 1;             // [2 tiles]  128 softmax threads have read O[t] of the item
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_empty + 2);
+  uint64_t* item_full = q_empty + 1;             // [kItems] the slot holds the next item
+  uint64_t* item_empty = item_full + kItems;     // [kItems] the softmax warps are through with it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(item_empty + kItems);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -208,10 +212,9 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(&p_full[2 * t], kUBM);
       mbar_init(&p_full[2 * t + 1], kUBM);
       mbar_init(&o_full[t], 1);
-      mbar_init(&o_empty[t], kUBM);
     }
     mbar_init(q_empty, 1);
-    mbar_init(item_full, 1);
+    for (int i = 0; i < kItems; ++i) mbar_init(&item_full[i], 1), mbar_init(&item_empty[i], 4 * QT);
     mbar_fence_init();
   }
   if (warp == kTmaWarp && lane == 0) {
@@ -463,10 +466,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       if (NT <= 1 && leader) umma::commit(q_empty);
       __syncwarp();
-      // O[t] of the item before has been read (one wait per item, so that no phase is ever skipped)
-#pragma unroll
-      for (int t = 0; t < QT; ++t) mbar_wait(&o_empty[t], (n & 1) ^ 1);
-      umma::fence_after_sync();
+      // (O[t] of the item before has been read: the softmax group of tile t stores P of this one afterwards)
       for (int j = 0; j < NT; ++j) {
         const int jr = base + j, s = jr % kUStages, s1 = (jr + 1) % kUStages;
         mbar_wait(&v_full[s], (jr / kUStages) & 1);
@@ -509,8 +509,6 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         __syncwarp();
       }
-      if (leader) umma::commit(item_full);
-      __syncwarp();
       base += NT;
       done[0] += it.n_tiles[0], done[1] += it.n_tiles[1];
       ++n;
@@ -529,21 +527,10 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const float sl2 = CAP ? kLog2e : p.scale_log2;      // capped scores are already scaled
     constexpr float kLazy = 8.f;                     // lazy rescale threshold (exp2 domain): O is rescaled only when the max grew by > 2^8
     int n = 0, done = 0;                             // items and S[t] tiles so far
-    // The items' sizes live in shared memory, two slots per warp: a row of 128 scores leaves no registers for them
-    Item* slots = s_items + 2 * warp;
-    Cursor cur = begin();
-    auto look_up = [&](int slot) -> bool {
-      Item x;
-      const bool found = next_item(cur, x);
-      __syncwarp();                                  // every lane has read what this slot held (an item with no key tiles
-                                                     // for this warp has no other meeting point of its lanes)
-      if (lane == 0) slots[slot] = x;
-      __syncwarp();
-      return found;
-    };
-    bool live = look_up(0);
-    while (live) {
-    const volatile Item& it = slots[n & 1];
+    for (;; ++n) {
+    mbar_wait(&item_full[n % kItems], (n / kItems) & 1);
+    const volatile Item& it = s_items[n % kItems];     // (in shared memory: a row of 128 scores leaves no registers for it)
+    if (it.none) break;
     const int nt = it.n_tiles[t];
 #define B200_QROW (it.m0 + t * row_step + row)             // row inside the sequence
     float m_ref = -INFINITY, l_run = 0.f;
@@ -555,14 +542,34 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
       for (int c = 0; c < 4; ++c) umma::ld32(s_addr + c * 32, sr[c]);
       umma::wait_ld();
+      float mx = -INFINITY;
+      bool found = false;                              // mx is the row's maximum
       if constexpr (CAP) {
         // tanh of small arguments is a short odd polynomial: while every score of the warp's rows stays below 0.35 caps, it
         // replaces the ex2 and the reciprocal per score that otherwise bind this loop to the special-function unit (3 of
-        // its 16 results per clock for each score instead of 1). Truncation: 1.2e-8 of the score at 0.35. The
-        // test is warp-uniform (per-score selection would pay for both sides) and ends with the first tile that fails it
-        // (12 ragged prompts of 37-1501 tokens, 32 heads of 64, cap 30: 232 -> 162 us).
-        if (small) small = __all_sync(0xffffffffu, row_max(sr) * p.cap_pre <= 0.35f && row_min(sr) * p.cap_pre >= -0.35f);
+        // its 16 results per clock for each score instead of 1). Truncation: 1.2e-8 of the score at 0.35, with terms up to x^11; below
+        // 0.17 caps, where most scores are, 1.5e-8 with those up to x^7, whose five packed operations a pair are what the loop has
+        // most of otherwise (nine). The tests are warp-uniform (per-score selection would pay for both sides) and end with the first
+        // tile that fails both. A capped maximum is the cap of the maximum: a tile without a mask needs no second search.
+        // (12 ragged prompts of 37-1501 tokens, 32 heads of 64, cap 30: 232 us without polynomials, 162 with the long one, 145 with both.)
+        float most = 0.f;
         if (small) {
+          mx = row_max(sr);
+          most = fmaxf(mx, -row_min(sr)) * p.cap_pre;
+          small = __all_sync(0xffffffffu, most <= 0.35f);
+        }
+        if (small && __all_sync(0xffffffffu, most <= 0.17f)) {
+          const float2 a0 = p.cap_poly[0], a1 = p.cap_poly[1], a2 = p.cap_poly[2], a3 = p.cap_poly[3];
+#pragma unroll
+          for (int c = 0; c < 128; c += 2) {
+            const float2 x = score_pair(sr, c), x2 = mul2(x, x);
+            const float2 t = mul2(x, fma2(x2, fma2(x2, fma2(x2, a3, a2), a1), a0));
+            sr[c >> 5][c & 31] = __float_as_uint(t.x), sr[c >> 5][(c + 1) & 31] = __float_as_uint(t.y);
+          }
+          const float x2 = mx * mx;
+          mx *= fmaf(x2, fmaf(x2, fmaf(x2, a3.x, a2.x), a1.x), a0.x);
+          found = true;
+        } else if (small) {
           const float2 pre = both(p.cap_pre), scale = both(p.cap * p.cap_pre);
 #pragma unroll
           for (int c = 0; c < 128; c += 2) {
@@ -591,6 +598,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // mask (warp-uniform test: does this tile touch the diagonal or the end of the keys?)
       const int warp_row0 = it.m0 + t * row_step + (warp & 3) * 32, Lk = it.Lk, off = it.off;
       if (n0 + kUBN > Lk || n0 + kUBN - 1 > warp_row0 + off) {
+        found = false;
         const int limit = min(Lk - 1, B200_QROW + off) - n0;   // last visible key (tile-relative)
         const int every = min(Lk - 1, warp_row0 + off) - n0;   // last key that all rows of the warp see
 #pragma unroll
@@ -603,12 +611,13 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
       if (p.limited() && n0 + kUBN > p.keep_first && n0 < p.seen_from(warp_row0 + 31 + off)) {
+        found = false;
         const int low = p.seen_from(B200_QROW + off) - 1 - n0, keep = p.keep_first - n0;   // hidden: keep <= c <= low
 #pragma unroll
         for (int c = 0; c < 128; ++c)
           if (c <= low && c >= keep) sr[c >> 5][c & 31] = 0xff800000u;
       }
-      const float mx = row_max(sr);
+      if (!CAP || !found) mx = row_max(sr);
       const bool grow = (mx - m_ref) * sl2 > kLazy;       // also true for the first finite max
       if (__any_sync(0xffffffffu, grow)) {
         const float m_new = grow ? mx : m_ref;
@@ -659,13 +668,13 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (m_ref == -INFINITY) m_ref = sink2 / sl2, l_run = 1.f;      // no key of this split is visible to the row
       else l_run += ex2_approx(sink2 - m_ref * sl2);
     }
-    // ---- epilogue: O / l -> global, or (split-KV) the un-normalised partial -> workspace. The next item is looked up first:
-    // its loads would queue behind the stores
-    live = look_up((n & 1) ^ 1);
-    mbar_wait(item_full, n & 1);
+    // ---- epilogue: O / l -> global, or (split-KV) the un-normalised partial -> workspace
+    if (nt > 0) mbar_wait(&o_full[t], (done + nt - 1) & 1);          // its own last product, not the other tile's
     umma::fence_after_sync();
     const int m0 = it.m0, Lq = it.Lq, q0 = it.q0, head = it.head + t * head_step, split = it.split, qrow = m0 + t * row_step + row;
     const int warp_row_base = m0 + t * row_step + (warp & 3) * 32;   // this warp's first row inside the sequence
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&item_empty[n % kItems]);
     if (m0 + t * row_step < Lq) {
       T* orow = reinterpret_cast<T*>(p.out) + (int64_t)(q0 + qrow) * p.out_stride + (int64_t)head * DV;
       const int64_t pidx = ((int64_t)(q0 + qrow) * p.H + head) * p.kv_splits + split;
@@ -728,9 +737,22 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
     umma::fence_before_sync();
-    mbar_arrive(&o_empty[t]);
     done += nt;
-    ++n;
+    }
+  } else if (warp == kItemWarp) {
+    // =========================== work items of the softmax warps ===========================
+    // Found one ahead by a warp of its own: the loads and divisions took a softmax warp 1200 cycles of every item
+    Cursor cur = begin();
+    Item x;
+    for (int n = 0;; ++n) {
+      const bool found = next_item(cur, x);
+      mbar_wait(&item_empty[n % kItems], ((n / kItems) & 1) ^ 1);
+      if (lane == 0) {
+        x.none = !found;
+        s_items[n % kItems] = x;
+        mbar_arrive(&item_full[n % kItems]);
+      }
+      if (!found) break;
     }
   }
   umma::fence_before_sync();
@@ -778,8 +800,8 @@ static int prefill_umma_launch_c(const CUtensorMap& mq, const CUtensorMap& mk, c
                                  cudaStream_t stream) {
   constexpr int CHK = DK / 64, CHV = DV / 64;
   constexpr size_t smem =
-      1024 + QT * CHK * kUBM * 128 + prefill_stages(DK, QT) * (CHK + CHV) * kUBN * 128 + 4 * QT * 2048 + kOrderSeqs * 4 + 8 * QT * sizeof(Item) + 36 * 8 + 16;
-  static_assert(8 * sizeof(Item) % 8 == 0, "barriers on 8-byte boundaries");
+      1024 + QT * CHK * kUBM * 128 + prefill_stages(DK, QT) * (CHK + CHV) * kUBN * 128 + 4 * QT * 2048 + kOrderSeqs * 4 + kItems * sizeof(Item) + 36 * 8 + 16;
+  static_assert(kItems * sizeof(Item) % 8 == 0, "barriers on 8-byte boundaries");
   auto kern = prefill_umma_kernel<T, DK, DV, QT, CAP>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -879,7 +901,12 @@ int prefill_umma_launch(void* out, const void* q, const void* k, const void* v,
   p.out = out, p.out_stride = out_stride;
   p.H = H, p.G = H / Hkv, p.block_size = block_size, p.bt_stride = bt_stride;
   p.scale_log2 = scale * 1.4426950408889634f;
-  if (softcap > 0.f) p.cap = softcap, p.cap_pre = scale / softcap;
+  if (softcap > 0.f) {
+    p.cap = softcap, p.cap_pre = scale / softcap;
+    const double y2 = (double)p.cap_pre * p.cap_pre, y = (double)softcap * p.cap_pre;
+    const double series[4] = {y, -y * y2 / 3., y * y2 * y2 * (2. / 15.), -y * y2 * y2 * y2 * (17. / 315.)};
+    for (int i = 0; i < 4; ++i) p.cap_poly[i] = make_float2((float)series[i], (float)series[i]);
+  }
   p.sink = sink;
   p.window = window, p.keep_first = window > 0 ? keep_first : 0, p.chunk = chunk;
   const int span = window > 0 ? window : chunk;

@@ -108,3 +108,34 @@ def test_cached_keys_in_blocks(H, block, D, spans, tiles):
         w = _want(q[at:at + n], k, v, D ** -0.5, 0.0, None)
         assert float((got[at:at + n] - w).abs().max()) < 4e-3, (n, m)
         at += n
+
+
+@pytest.mark.parametrize("tiles", [1, 2])
+@pytest.mark.parametrize("level", [0.05, 0.168, 0.172, 0.348, 0.352, 1.5])
+@pytest.mark.parametrize("D,window", [(64, 0), (128, 0), (64, 100)])
+def test_caps_on_either_side_of_both_polynomials(D, window, level, tiles):
+    """The largest score of a head is `level` caps: the short polynomial, the long one and the function itself, on tiles with and without a mask
+    (the maximum of a tile without one is capped by itself). A cap of 40 makes scores of up to 60: a wrong cap or maximum shows."""
+    from nanovllm import _C, ops
+    _C.load().b200_prefill_set_query_tiles(tiles)
+    g = torch.Generator().manual_seed(D + window)
+    H, G, lens, cap = 4, 2, [300, 129, 1], 40.0
+    T = sum(lens)
+    q, k, v = torch.randn(T, H, D, generator=g), torch.randn(T, G, D, generator=g), torch.randn(T, G, D, generator=g).half()
+    q, k = q.half(), k.half()
+    top = max(float((q[:, h].double() @ k[:, h * G // H].double().T).abs().max()) for h in range(H))
+    scale = level * cap / top
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).cuda()
+    got = ops.prefill_varlen_attn(q.cuda(), k.cuda(), v.cuda(), cu, cu, max(lens), max(lens), scale, G, softcap=cap, window=window).cpu().to(F64)
+    at = 0
+    for n in lens:
+        out = []
+        for h in range(H):
+            s = cap * torch.tanh(q[at:at + n, h].to(F64) @ k[at:at + n, h * G // H].to(F64).T * scale / cap)
+            i = torch.arange(n)
+            seen = (i[None] <= i[:, None]) & ((i[:, None] - i[None] < window) if window else True)
+            out.append(torch.softmax(s.masked_fill(~seen, -math.inf), -1) @ v[at:at + n, h * G // H].to(F64))
+        want = torch.stack(out, 1).reshape(n, -1)
+        # a probability is rounded to 2^-11, a result to 2^-11; scores of 32 bits move a probability of e^60 in all by 60 * 2^-23
+        assert float((got[at:at + n] - want).norm() / want.norm()) < 6e-4
+        at += n
