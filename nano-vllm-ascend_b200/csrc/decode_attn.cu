@@ -632,7 +632,7 @@ extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const v
   p.window = window, p.keep_first = window > 0 ? keep_first : 0, p.chunk = chunk;
 
   if (num_ctas <= 0 && head_dim == value_dim && window == 0 && chunk == 0) {
-    const int ctas = decode_small_ctas((int64_t)batch * num_kv_heads, (int64_t)block_table_stride * block_size, head_dim);
+    const int ctas = decode_small_ctas((int64_t)batch * num_kv_heads, (int64_t)block_table_stride * block_size, head_dim, false);
     if (ctas > 0) return decode_small_launch(p, k_cache, v_cache, num_blocks, head_dim, dtype, ctas, stream);
   }
 

@@ -33,37 +33,6 @@ namespace b200 {
 
 constexpr int kStagesQ8 = 6;
 
-__device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t two_bytes) {
-  uint32_t r;
-  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(r) : "h"((uint16_t)two_bytes));
-  return r;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(addr));
-  return v;
-}
-// two consecutive T elements (one 32-bit word) -> f16x2
-template <typename T>
-__device__ __forceinline__ uint32_t to_f16x2(uint32_t w);
-template <>
-__device__ __forceinline__ uint32_t to_f16x2<__half>(uint32_t w) {
-  return w;
-}
-template <>
-__device__ __forceinline__ uint32_t to_f16x2<__nv_bfloat16>(uint32_t w) {
-  const float2 f = unpack2<__nv_bfloat16>(w);
-  // |q| beyond the f16 range cannot come out of a normalised projection; clamp instead of inf
-  return pack2<__half>(fminf(fmaxf(f.x, -65504.f), 65504.f), fminf(fmaxf(f.y, -65504.f), 65504.f));
-}
-
 template <typename T, int D, int HKV_CTA>
 __global__ void __launch_bounds__(kDecodeThreads, 1)
 paged_decode_fp8_kernel(const __grid_constant__ CUtensorMap tmK,
@@ -653,6 +622,11 @@ extern "C" int b200_paged_decode_attn_fp8(void* out, const void* q, const void* 
   p.hg_count = hg_count;
   p.rows_box = block_size < tile_tokens ? block_size : tile_tokens;
   p.scale_log2 = scale * k_scale * 1.4426950408889634f;
+
+  if (num_ctas <= 0) {                                    // few rows
+    const int ctas = decode_small_ctas((int64_t)batch * num_kv_heads, (int64_t)block_table_stride * block_size, head_dim, true);
+    if (ctas > 0) return decode_small_fp8_launch(p, k_cache, v_cache, num_blocks, head_dim, v_scale, dtype, ctas, stream);
+  }
 
   const int chunks = num_kv_heads * head_dim / 128;
   const int chunks_box = hkv_cta * head_dim / 128;

@@ -64,6 +64,38 @@ __device__ __forceinline__ int find_item(const int* prefix, int items, int t) {
   return lo;
 }
 
+// ---- an e4m3 cache: its elements in f16, which holds them exactly
+__device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t two_bytes) {
+  uint32_t r;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(r) : "h"((uint16_t)two_bytes));
+  return r;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr));
+  return v;
+}
+// two consecutive T elements (one 32-bit word) -> f16x2
+template <typename T>
+__device__ __forceinline__ uint32_t to_f16x2(uint32_t w);
+template <>
+__device__ __forceinline__ uint32_t to_f16x2<__half>(uint32_t w) {
+  return w;
+}
+template <>
+__device__ __forceinline__ uint32_t to_f16x2<__nv_bfloat16>(uint32_t w) {
+  const float2 f = unpack2<__nv_bfloat16>(w);
+  // |q| beyond the f16 range cannot come out of a normalised projection; clamp instead of inf
+  return pack2<__half>(fminf(fmaxf(f.x, -65504.f), 65504.f), fminf(fmaxf(f.y, -65504.f), 65504.f));
+}
+
 // Combine kernel: merges the partial results of items whose tiles were split across CTAs.
 // One CTA per range boundary c | c+1: the item that straddles that boundary is merged by the
 // FIRST boundary it straddles -- the decode CTA on the left of that boundary records the item in
@@ -140,8 +172,11 @@ decode_combine_kernel(const DecodeParams p, int rows /* = HKV_CTA*G */) {
 
 // decode_small.cu: one launch, a cluster of CTAs per (row, kv head); keys and values of one size, no window, no chunk. decode_small_ctas: how
 // many for `pairs` (row, kv head) whose block tables have room for `width` tokens (0: the step is not for it)
-int decode_small_ctas(int64_t pairs, int64_t width, int dim);
+int decode_small_ctas(int64_t pairs, int64_t width, int dim, bool fp8);
 int decode_small_launch(const DecodeParams& p, const void* k, const void* v, int num_blocks, int dim, int dtype, int ctas, cudaStream_t stream);
+
+int decode_small_fp8_launch(const DecodeParams& p, const void* k, const void* v, int num_blocks, int dim, float v_scale, int dtype, int ctas,
+                            cudaStream_t stream);
 
 static inline int hkv_cta_of(int Hkv) {
   if (Hkv >= 8) return Hkv % 8 == 0 ? 8 : 0;

@@ -9,12 +9,14 @@
 namespace b200 {
 
 constexpr int kSmallWarps = 8;
-constexpr int kSmallStages = 2;                          // units of a warp under way
+template <bool FP8>
+constexpr int kSmallStages = FP8 ? 3 : 2;                // units of a warp under way
 
 struct DecodeSmallParams {
   DecodeParams p;
   const void *k, *v;                                    // [num_blocks * block_size][Hkv * D]
   int num_blocks;
+  float v_scale;
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -37,12 +39,12 @@ __device__ __forceinline__ float ld_peer(uint32_t addr, uint32_t rank) {       /
   return r;
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kSmallWarps * 32)
+template <typename T, int D, bool FP8>
+__global__ void __launch_bounds__(kSmallWarps * 32, FP8 || D == 64 ? 2 : 1)
 decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
   const DecodeParams& p = S.p;
-  constexpr int CH = D / 64, KSTEPS = D / 16, NT = D / 8;
-  constexpr int kUnit = 16 * D * 2;                      // bytes of 16 keys
+  constexpr int KSTEPS = D / 16, NT = D / 8, kStages = kSmallStages<FP8>;
+  constexpr int kRow = FP8 ? D : 2 * D, kUnit = 16 * kRow;             // bytes of a key, of 16 keys
   extern __shared__ __align__(128) uint8_t small_smem[]; // [warps][stages][K, V]; then the warps' results
   __shared__ float s_o[8][D], s_m[8], s_l[8];            // this CTA's
   __shared__ float w_m[kSmallWarps][8], w_l[kSmallWarps][8];
@@ -52,11 +54,11 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
   pdl_wait();
   const int len = p.context_lens[b];
   const int units = len > 0 ? (len + 15) / 16 : 0, step = (int)ctas * kSmallWarps;
-  uint8_t* buf = small_smem + warp * (kSmallStages * 2 * kUnit);
+  uint8_t* buf = small_smem + warp * (kStages * 2 * kUnit);
   const uint32_t buf_at = smem_u32(buf);
-  const uint8_t* kc = reinterpret_cast<const uint8_t*>(S.k) + (int64_t)kv_head * (D * 2);
-  const uint8_t* vc = reinterpret_cast<const uint8_t*>(S.v) + (int64_t)kv_head * (D * 2);
-  const int64_t row_bytes = (int64_t)p.Hkv * (D * 2);
+  const uint8_t* kc = reinterpret_cast<const uint8_t*>(S.k) + (int64_t)kv_head * kRow;
+  const uint8_t* vc = reinterpret_cast<const uint8_t*>(S.v) + (int64_t)kv_head * kRow;
+  const int64_t row_bytes = (int64_t)p.Hkv * kRow;
   const int first = (int)rank + (int)ctas * warp;        // this warp's units: first, first + step, ...
   int looked_up = 0, rows = -1;                          // first cache row of unit looked_up + lane (-1: keys of no block are zero)
   auto look_up = [&](int n) {                            // 32 units at a time: a table entry per unit would cost each a trip to L2
@@ -77,9 +79,9 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
       const int64_t at = (int64_t)max(row0, 0) * row_bytes;
       const uint32_t to = buf_at + stage * (2 * kUnit);
 #pragma unroll
-      for (int i = 0; i < 16 * D / 8 / 32; ++i) {
-        const int e = i * 32 + lane, row = e / (D / 8), c = e % (D / 8);
-        const uint32_t dst = (c >> 3) * 2048 + row * 128 + (((c & 7) ^ (row & 7)) << 4);
+      for (int i = 0; i < kUnit / 512; ++i) {
+        const int e = i * 32 + lane, row = e / (kRow / 16), c = e % (kRow / 16);
+        const uint32_t dst = kRow == 64 ? row * 64 + ((c ^ ((row >> 1) & 3)) << 4) : (c >> 3) * 2048 + row * 128 + (((c & 7) ^ (row & 7)) << 4);
         const bool ok = row < valid;
         const int64_t src = ok ? at + row * row_bytes + c * 16 : 0;
         cp_async_16(to + dst, kc + src, ok);
@@ -90,7 +92,7 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
   };
   look_up(0);
 #pragma unroll
-  for (int i = 0; i < kSmallStages; ++i) load(i, i);
+  for (int i = 0; i < kStages; ++i) load(i, i);
 
   const bool capped = p.cap > 0.f;
   const float sl2 = capped ? kLog2e : p.scale_log2;
@@ -99,6 +101,12 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
     const T* qrow = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_stride + (int64_t)(kv_head * G + g) * D;
 #pragma unroll
     for (int ks = 0; ks < KSTEPS; ++ks) {
+      if constexpr (FP8) {                               // the order of paged_decode_fp8_kernel: a lane has D / 4 neighbouring elements
+        uint2 w = make_uint2(0u, 0u);
+        if (g < G) w = *reinterpret_cast<const uint2*>(qrow + t4 * (D / 4) + 4 * ks);
+        qa[ks][0] = to_f16x2<T>(w.x), qa[ks][1] = to_f16x2<T>(w.y);
+        continue;
+      }
       qa[ks][0] = g < G ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 2 * t4) : 0u;
       qa[ks][1] = g < G ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8 + 2 * t4) : 0u;
     }
@@ -109,13 +117,26 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
   float m_run = -INFINITY, l_run = 0.f;
   const int k_tok = ((lane >> 4) << 3) + (lane & 7), k_half = (lane >> 3) & 1;       // ldmatrix: as in paged_decode_kernel
   const int v_tok = (((lane >> 3) & 1) << 3) + (lane & 7), v_dt = lane >> 4;
-  for (int n = 0, stage = 0; first + n * step < units; ++n, stage = stage + 1 == kSmallStages ? 0 : stage + 1) {
-    cp_async_wait<kSmallStages - 1>();
+  for (int n = 0, stage = 0; first + n * step < units; ++n, stage = stage + 1 == kStages ? 0 : stage + 1) {
+    cp_async_wait<kStages - 1>();
     __syncwarp();
     const uint32_t kb = buf_at + stage * (2 * kUnit), vb = kb + kUnit;
     float s[2][4];
 #pragma unroll
     for (int t = 0; t < 2; ++t) s[t][0] = s[t][1] = s[t][2] = s[t][3] = 0.f;
+    if constexpr (FP8) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int i = 0; i < KSTEPS / 4; ++i) {
+          const int c = t4 * (D / 64) + i;
+          const uint4 x = lds128(kb + (t * 8 + g) * kRow + ((D == 64 ? c ^ ((g >> 1) & 3) : c ^ g) << 4));
+          const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int y = 0; y < 4; ++y)
+            mma_16816<__half>(s[t], qa[4 * i + y][0], 0u, qa[4 * i + y][1], 0u, e4m3x2_to_f16x2(w[y] & 0xffffu), e4m3x2_to_f16x2(w[y] >> 16));
+        }
+    } else {
 #pragma unroll
     for (int ks = 0; ks < KSTEPS; ++ks) {
       const int c16 = ((ks & 3) << 1) + k_half;
@@ -123,6 +144,7 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
       ldsm_x4(kb + (ks >> 2) * 2048 + k_tok * 128 + ((c16 ^ (k_tok & 7)) << 4), r0, r1, r2, r3);
       mma_16816<T>(s[0], qa[ks][0], 0u, qa[ks][1], 0u, r0, r1);
       mma_16816<T>(s[1], qa[ks][0], 0u, qa[ks][1], 0u, r2, r3);
+    }
     }
     const int valid = len - (first + n * step) * 16;
 #pragma unroll
@@ -144,6 +166,21 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
 #pragma unroll
       for (int t = 0; t < NT; ++t) o_acc[t][0] *= alpha, o_acc[t][1] *= alpha, o_acc[t][2] *= alpha, o_acc[t][3] *= alpha;
     }
+    if constexpr (FP8) {
+      const uint32_t pa0 = pack2<__half>(p00, p01), pa2 = pack2<__half>(p10, p11);
+#pragma unroll
+      for (int jp = 0; jp < D / 32; ++jp) {
+        const int c = 2 * jp + v_dt;
+        uint32_t r0, r1, r2, r3;
+        ldsm_x4_trans(vb + v_tok * kRow + ((D == 64 ? c ^ ((v_tok >> 1) & 3) : c ^ (v_tok & 7)) << 4), r0, r1, r2, r3);
+        const uint32_t e0 = __byte_perm(r0, r1, 0x6420), o0 = __byte_perm(r0, r1, 0x7531);
+        const uint32_t e1 = __byte_perm(r2, r3, 0x6420), o1 = __byte_perm(r2, r3, 0x7531);
+        mma_16816<__half>(o_acc[4 * jp + 0], pa0, 0u, pa2, 0u, e4m3x2_to_f16x2(e0 & 0xffffu), e4m3x2_to_f16x2(e0 >> 16));
+        mma_16816<__half>(o_acc[4 * jp + 1], pa0, 0u, pa2, 0u, e4m3x2_to_f16x2(o0 & 0xffffu), e4m3x2_to_f16x2(o0 >> 16));
+        mma_16816<__half>(o_acc[4 * jp + 2], pa0, 0u, pa2, 0u, e4m3x2_to_f16x2(e1 & 0xffffu), e4m3x2_to_f16x2(e1 >> 16));
+        mma_16816<__half>(o_acc[4 * jp + 3], pa0, 0u, pa2, 0u, e4m3x2_to_f16x2(o1 & 0xffffu), e4m3x2_to_f16x2(o1 >> 16));
+      }
+    } else {
     // two 16-bit terms of the probabilities, the second in the rows of the tile that the group does not use
     const uint32_t pa0 = pack2<T>(p00, p01), pa2 = pack2<T>(p10, p11);
     const float2 h0 = unpack2<T>(pa0), h1 = unpack2<T>(pa2);
@@ -156,22 +193,29 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
       mma_16816<T>(o_acc[2 * jp], pa0, pa1, pa2, pa3, r0, r1);
       mma_16816<T>(o_acc[2 * jp + 1], pa0, pa1, pa2, pa3, r2, r3);
     }
+    }
     __syncwarp();
-    load(n + kSmallStages, stage);
+    load(n + kStages, stage);
   }
   cp_async_wait<0>();
+  if constexpr (!FP8) {
   // the second term is left out where an infinite value made it 0 x inf or inf - inf
 #pragma unroll
   for (int n = 0; n < NT; ++n)
 #pragma unroll
     for (int e = 0; e < 2; ++e)
       if (fabsf(o_acc[n][2 + e]) < INFINITY) o_acc[n][e] += o_acc[n][2 + e];
+  }
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
   // ---- the warps of this CTA: each into its own buffer
   float* mine = reinterpret_cast<float*>(buf);           // [8][D]
-  static_assert(8 * D * 4 <= kSmallStages * 2 * kUnit, "a warp's result fits its buffers");
-  if (g < G) {
+  static_assert(8 * D * 4 <= kStages * 2 * kUnit, "a warp's result fits its buffers");
+  if (FP8 && g < G) {
+#pragma unroll
+    for (int c = 0; c < D / 16; ++c)
+      *reinterpret_cast<float4*>(mine + g * D + 16 * c + 4 * t4) = make_float4(o_acc[2 * c][0], o_acc[2 * c + 1][0], o_acc[2 * c][1], o_acc[2 * c + 1][1]);
+  } else if (g < G) {
 #pragma unroll
     for (int n = 0; n < NT; ++n) *reinterpret_cast<float2*>(mine + g * D + n * 8 + 2 * t4) = make_float2(o_acc[n][0], o_acc[n][1]);
   }
@@ -186,7 +230,7 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
     for (int w = 0; w < kSmallWarps; ++w) {
       const float x = w_m[w][r], f = x == -INFINITY ? 0.f : ex2_approx(x - m);
       l = fmaf(w_l[w][r], f, l);
-      if (x != -INFINITY) o = fmaf(reinterpret_cast<const float*>(small_smem + w * (kSmallStages * 2 * kUnit))[e], f, o);
+      if (x != -INFINITY) o = fmaf(reinterpret_cast<const float*>(small_smem + w * (kStages * 2 * kUnit))[e], f, o);
     }
     s_o[0][e] = o;
     if (e % D == 0) s_m[r] = m, s_l[r] = l;
@@ -207,7 +251,7 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
       l = fmaf(ld_peer(al, c), f, l), o0 = fmaf(ld_peer(ao, c), f, o0), o1 = fmaf(ld_peer(ao + 4, c), f, o1);
     }
     if (p.sink != nullptr && len > 0) l += ex2_approx(p.sink[kv_head * G + r] * kLog2e - m);
-    const float inv = len > 0 ? 1.f / l : 0.f;
+    const float inv = len > 0 ? S.v_scale / l : 0.f;
     T* out = reinterpret_cast<T*>(p.out) + (int64_t)b * p.out_stride + (int64_t)kv_head * total + e0;
     *reinterpret_cast<uint32_t*>(out) = len > 0 ? pack2<T>(o0 * inv, o1 * inv) : 0u;
   }
@@ -215,10 +259,10 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
   cluster_wait();
 }
 
-template <typename T, int D>
+template <typename T, int D, bool FP8>
 static int decode_small_launch_as(const DecodeSmallParams& S, int ctas, cudaStream_t stream) {
-  auto kern = decode_small_kernel<T, D>;
-  constexpr int smem = kSmallWarps * kSmallStages * 2 * 16 * D * 2;
+  auto kern = decode_small_kernel<T, D, FP8>;
+  constexpr int smem = kSmallWarps * kSmallStages<FP8> * 2 * 16 * D * (FP8 ? 1 : 2);
   static std::atomic<uint64_t> devices{0};
   cudaError_t e = allow_smem(kern, smem, devices);
   if (e != cudaSuccess) return (int)e;
@@ -245,21 +289,33 @@ static int decode_small_launch_as(const DecodeSmallParams& S, int ctas, cudaStre
 //   8 / 2 of 128:   1 x 1000 8.3 / 6.2, x 4000 10.1 / 9.5, [x 8000 12.0 / 13.7]
 //   32 / 8 of 64:   1 x 1000 8.4 / 5.1, x 8000 12.5 / 11.2;  4 x 1000 12.2 / 7.0, x 8000 18.6 / 15.1;  16 x 2000 18.1 / 14.1;  32 x 1000 18.0 / 13.8
 //   8 / 8 of 64:    1 x 1000 7.7 / 4.5, x 8000 12.4 / 10.6;  8 x 4000 15.1 / 13.9, [x 8000 21.5 / 23.0];  32 x 1000 14.7 / 13.4, [x 2000 20.8 / 21.9]
-// An SM takes about 70 bytes per ns, and no more than one CTA (heads of 64: three), so what counts is the bytes per CTA: 131072 tokens of kv
+// An SM takes about 70 bytes per ns, and one CTA (heads of 64: two), so what counts is the bytes per CTA: 131072 tokens of kv
 // heads of 128 or 262144 of 64 in all, on up to 128 or 256 CTAs (clusters of 8 of 128 pack 64). More CTAs than eight warps' units of 16 keys
 // only wait for one another (1 row x 100: 4.3 with one, 4.9 with eight).
-int decode_small_ctas(int64_t pairs, int64_t width, int dim) {
-  const int64_t most = dim == 128 ? 128 : 256;
-  if (width <= 0 || width > most * 32 || pairs > most || pairs * width > most * 1024) return 0;
-  int ctas = pairs <= (dim == 128 ? 8 : 32) ? 8 : pairs <= (dim == 128 ? 32 : 64) ? 4 : pairs <= most / 2 ? 2 : 1;
+// An e4m3 cache, two CTAs per SM: 16 / 8 of 128: 1 x 1000 9.3 / 5.7, x 4000 12.1 / 9.4;  4 x 4000 14.3 / 13.5;  8 x 2000 14.1 / 12.9, [x 4000 19.1 /
+// 19.3];  16 x 1000 13.8 / 12.8, [x 2000 18.4 / 18.9];  32 x 500 13.9 / 12.0, [x 1000 18.4 / 18.4], [64 x 500 18.6 / 19.7];  32 / 8 of 64: 1 x 1000
+// 10.7 / 4.7;  8 x 4000 16.1 / 11.6;  16 x 4000 20.0 / 17.2;  32 x 2000 20.0 / 16.5;  64 x 1000 21.3 / 19.2, [x 2000 29.2 / 29.0].
+int decode_small_ctas(int64_t pairs, int64_t width, int dim, bool fp8) {
+  const int64_t tokens = dim == 128 ? 128 << 10 : fp8 ? 512 << 10 : 256 << 10, most = !fp8 && dim == 128 ? 128 : fp8 && dim == 64 ? 512 : 256;
+  if (width <= 0 || width > (dim == 128 ? 4096 : 8192) || pairs > most || pairs * width > tokens) return 0;
+  const bool one = !fp8 && dim == 128;                   // CTA per SM
+  int ctas = pairs <= (one ? 8 : 32) ? 8 : pairs <= (one ? 32 : 64) ? 4 : pairs <= (one ? 64 : 128) ? 2 : 1;
   while (ctas > 1 && (ctas / 2) * kSmallWarps * 16 >= width) ctas /= 2;
   return ctas;
 }
 
+template <bool FP8>
+static int decode_small_launch_for(const DecodeSmallParams& S, int dim, int dtype, int ctas, cudaStream_t stream) {
+  if (dtype == B200_DTYPE_BF16)
+    return dim == 128 ? decode_small_launch_as<__nv_bfloat16, 128, FP8>(S, ctas, stream) : decode_small_launch_as<__nv_bfloat16, 64, FP8>(S, ctas, stream);
+  return dim == 128 ? decode_small_launch_as<__half, 128, FP8>(S, ctas, stream) : decode_small_launch_as<__half, 64, FP8>(S, ctas, stream);
+}
 int decode_small_launch(const DecodeParams& p, const void* k, const void* v, int num_blocks, int dim, int dtype, int ctas, cudaStream_t stream) {
-  const DecodeSmallParams S{p, k, v, num_blocks};
-  if (dtype == B200_DTYPE_BF16) return dim == 128 ? decode_small_launch_as<__nv_bfloat16, 128>(S, ctas, stream) : decode_small_launch_as<__nv_bfloat16, 64>(S, ctas, stream);
-  return dim == 128 ? decode_small_launch_as<__half, 128>(S, ctas, stream) : decode_small_launch_as<__half, 64>(S, ctas, stream);
+  return decode_small_launch_for<false>(DecodeSmallParams{p, k, v, num_blocks, 1.f}, dim, dtype, ctas, stream);
+}
+int decode_small_fp8_launch(const DecodeParams& p, const void* k, const void* v, int num_blocks, int dim, float v_scale, int dtype, int ctas,
+                            cudaStream_t stream) {
+  return decode_small_launch_for<true>(DecodeSmallParams{p, k, v, num_blocks, v_scale}, dim, dtype, ctas, stream);
 }
 
 }  // namespace b200

@@ -85,3 +85,27 @@ def test_strided_queries_and_a_replayed_graph():
         out.zero_()
         graph.replay()
         assert torch.equal(out, want)
+
+
+# an e4m3 cache: 8, 4, 2 and 1 CTAs, one and several units of a warp, the widest tables of each line and one more
+@pytest.mark.parametrize("H,G,D,lens", [(16, 8, 128, [1]), (16, 8, 128, [16, 17, 0, 129]), (8, 2, 128, [4096, 31]), (16, 8, 128, [4097]), (32, 4, 128, [333, 2, 1025]),
+                                        (16, 8, 128, [2048, 5, 700, 31, 33, 1, 64, 90]), (16, 8, 128, [500] * 32), (8, 8, 64, [8192]), (32, 8, 64, [500, 1024, 15, 511, 513]),
+                                        (8, 2, 64, [700] * 9), (8, 8, 64, [1000 - 15 * i for i in range(64)]), (32, 8, 64, [90] * 65)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_e4m3_cache(H, G, D, lens, dtype):
+    """As close to 64 bits as paged_decode_fp8_kernel (num_ctas given): probabilities are f16 in both, 2^-11; results are rounded to `dtype`."""
+    from nanovllm import ops
+    q, k, v, table = _case(H, G, D, lens, dtype, len(lens) + D)
+    k8, v8, ctx = k.to(torch.float8_e4m3fn), v.to(torch.float8_e4m3fn), torch.tensor(lens, dtype=torch.int32)
+    for row in (i for i, n in enumerate(lens) if n % 16):     # stale bytes past a row's length decode to NaN
+        block = table[row, lens[row] // 16]
+        k8[block, lens[row] % 16:] = v8[block, lens[row] % 16:] = float("nan")
+    run = lambda ctas: ops.paged_decode_attn_fp8(q.cuda(), k8.cuda(), v8.cuda(), table.cuda(), ctx.cuda(), D ** -0.5, G, k_scale=0.5, v_scale=2.0, num_ctas=ctas).cpu()  # noqa: E731
+    got, ref = run(0), run(148)
+    live = [i for i, n in enumerate(lens) if n]
+    want = 2 * _want(q[live], k8.float() * 0.5, v8.float(), table[live], [lens[i] for i in live], H, G, D)
+    off = lambda x: float((x[live].double() - want).norm() / want.norm())  # noqa: E731
+    assert off(got) <= off(ref) * 1.05 + 1e-5, (off(got), off(ref))
+    for i, n in enumerate(lens):
+        if n == 0:
+            assert torch.equal(got[i], torch.zeros_like(got[i]))
