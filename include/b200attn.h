@@ -174,6 +174,18 @@ int b200_paged_decode_attn_fp8(void* out, const void* q, const void* k_cache, co
                                float scale, float k_scale, float v_scale, void* workspace,
                                size_t workspace_bytes, int32_t num_ctas, int32_t dtype,
                                b200_stream_t stream);
+/* Steps of few rows that take one launch and no workspace (what the entries above do with them by themselves): the same without a
+ * workspace, B200_ERR_UNSUPPORTED for any other step. */
+int b200_paged_decode_attn_few(void* out, const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
+                               const int32_t* context_lens, int32_t batch, int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
+                               int64_t q_stride, int64_t out_stride, int32_t num_blocks, int32_t block_size,
+                               int32_t block_table_stride, float scale, float softcap, const float* sink, int32_t dtype,
+                               b200_stream_t stream);
+int b200_paged_decode_attn_fp8_few(void* out, const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
+                                   const int32_t* context_lens, int32_t batch, int32_t num_heads, int32_t num_kv_heads,
+                                   int32_t head_dim, int64_t q_stride, int64_t out_stride, int32_t num_blocks, int32_t block_size,
+                                   int32_t block_table_stride, float scale, float k_scale, float v_scale, int32_t dtype,
+                                   b200_stream_t stream);
 
 /* Paged e4m3 cache -> packed 16-bit K/V for the prefill kernel (prefix-cache-hit / chunked prefill
  * over an fp8 cache; extension, the reference's caches are always the model dtype). For sequence i,

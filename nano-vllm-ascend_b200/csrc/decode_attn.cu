@@ -531,43 +531,14 @@ extern "C" size_t b200_paged_decode_attn_workspace_size(int32_t batch, int32_t n
          align_up((size_t)kMaxCtas * 2 * rows * 2 * 4, 256);
 }
 
-extern "C" int b200_paged_decode_attn(void* out, const void* q, const void* k_cache,
-                                      const void* v_cache, const int32_t* block_tables,
-                                      const int32_t* context_lens, int32_t batch,
-                                      int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
-                                      int64_t q_stride, int64_t out_stride, int32_t num_blocks,
-                                      int32_t block_size, int32_t block_table_stride, float scale,
-                                      void* workspace, size_t workspace_bytes, int32_t num_ctas,
-                                      int32_t dtype, b200_stream_t stream_) {
-  return b200_paged_decode_attn_capped(out, q, k_cache, v_cache, block_tables, context_lens, batch, num_heads,
-                                       num_kv_heads, head_dim, q_stride, out_stride, num_blocks, block_size,
-                                       block_table_stride, scale, 0.f, nullptr, workspace, workspace_bytes, num_ctas,
-                                       dtype, stream_);
-}
-
-extern "C" int b200_paged_decode_attn_capped(void* out, const void* q, const void* k_cache,
-                                             const void* v_cache, const int32_t* block_tables,
-                                             const int32_t* context_lens, int32_t batch,
-                                             int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
-                                             int64_t q_stride, int64_t out_stride, int32_t num_blocks,
-                                             int32_t block_size, int32_t block_table_stride, float scale,
-                                             float softcap, const float* sink, void* workspace,
-                                             size_t workspace_bytes, int32_t num_ctas, int32_t dtype,
-                                             b200_stream_t stream_) {
-  return b200_paged_decode_attn_windowed(out, q, k_cache, v_cache, block_tables, context_lens, batch, num_heads,
-                                         num_kv_heads, head_dim, head_dim, q_stride, out_stride, num_blocks, block_size,
-                                         block_table_stride, scale, softcap, sink, 0, 0, 0, workspace, workspace_bytes,
-                                         num_ctas, dtype, stream_);
-}
-
-extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const void* k_cache, const void* v_cache,
-                                               const int32_t* block_tables, const int32_t* context_lens, int32_t batch,
-                                               int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
-                                               int32_t value_dim, int64_t q_stride, int64_t out_stride,
-                                               int32_t num_blocks, int32_t block_size, int32_t block_table_stride,
-                                               float scale, float softcap, const float* sink, int32_t window,
-                                               int32_t keep_first, int32_t chunk, void* workspace, size_t workspace_bytes,
-                                               int32_t num_ctas, int32_t dtype, b200_stream_t stream_) {
+static int decode_windowed(void* out, const void* q, const void* k_cache, const void* v_cache,
+                           const int32_t* block_tables, const int32_t* context_lens, int32_t batch,
+                           int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
+                           int32_t value_dim, int64_t q_stride, int64_t out_stride,
+                           int32_t num_blocks, int32_t block_size, int32_t block_table_stride,
+                           float scale, float softcap, const float* sink, int32_t window,
+                           int32_t keep_first, int32_t chunk, void* workspace, size_t workspace_bytes,
+                           int32_t num_ctas, int32_t dtype, bool few, b200_stream_t stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   B200_RETURN_IF(dtype != B200_DTYPE_BF16 && dtype != B200_DTYPE_F16, B200_ERR_BAD_DTYPE);
   B200_RETURN_IF(batch < 0 || num_heads <= 0 || num_kv_heads <= 0 || num_blocks <= 0 ||
@@ -576,7 +547,7 @@ extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const v
   B200_RETURN_IF(num_heads % num_kv_heads != 0, B200_ERR_BAD_SHAPE);
   if (batch == 0) return B200_OK;
   B200_RETURN_IF(!out || !q || !k_cache || !v_cache || !block_tables || !context_lens ||
-                     !workspace,
+                     (!few && !workspace),
                  B200_ERR_NULL_POINTER);
   B200_RETURN_IF((head_dim != 64 && head_dim != 128) || (value_dim != 64 && value_dim != 128), B200_ERR_UNSUPPORTED);
   B200_RETURN_IF(window < 0 || keep_first < 0 || chunk < 0 || (window > 0 && chunk > 0), B200_ERR_BAD_SHAPE);
@@ -597,7 +568,7 @@ extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const v
                  B200_ERR_MISALIGNED);
   B200_RETURN_IF(!aligned16(k_cache) || !aligned16(v_cache) || !aligned16(workspace),
                  B200_ERR_MISALIGNED);
-  B200_RETURN_IF(workspace_bytes <
+  B200_RETURN_IF(!few && workspace_bytes <
                      b200_paged_decode_attn_workspace_size(batch, num_heads, num_kv_heads, value_dim),
                  B200_ERR_WORKSPACE);
 
@@ -635,6 +606,7 @@ extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const v
     const int ctas = decode_small_ctas((int64_t)batch * num_kv_heads, (int64_t)block_table_stride * block_size, head_dim, false);
     if (ctas > 0) return decode_small_launch(p, k_cache, v_cache, num_blocks, head_dim, dtype, ctas, stream);
   }
+  B200_RETURN_IF(few, B200_ERR_UNSUPPORTED);
 
   const int k_chunks = num_kv_heads * head_dim / 64, v_chunks = num_kv_heads * value_dim / 64;
   CUtensorMap mk, mv;
@@ -670,4 +642,55 @@ extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const v
                                        : decode_launch_d<T, 64, 64>(hkv_cta, mk, mv, p, grid, stream)))
   return dtype == B200_DTYPE_BF16 ? B200_DECODE_DISPATCH(__nv_bfloat16) : B200_DECODE_DISPATCH(__half);
 #undef B200_DECODE_DISPATCH
+}
+
+extern "C" int b200_paged_decode_attn(void* out, const void* q, const void* k_cache,
+                                      const void* v_cache, const int32_t* block_tables,
+                                      const int32_t* context_lens, int32_t batch,
+                                      int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
+                                      int64_t q_stride, int64_t out_stride, int32_t num_blocks,
+                                      int32_t block_size, int32_t block_table_stride, float scale,
+                                      void* workspace, size_t workspace_bytes, int32_t num_ctas,
+                                      int32_t dtype, b200_stream_t stream_) {
+  return b200_paged_decode_attn_capped(out, q, k_cache, v_cache, block_tables, context_lens, batch, num_heads,
+                                       num_kv_heads, head_dim, q_stride, out_stride, num_blocks, block_size,
+                                       block_table_stride, scale, 0.f, nullptr, workspace, workspace_bytes, num_ctas,
+                                       dtype, stream_);
+}
+
+extern "C" int b200_paged_decode_attn_capped(void* out, const void* q, const void* k_cache,
+                                             const void* v_cache, const int32_t* block_tables,
+                                             const int32_t* context_lens, int32_t batch,
+                                             int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
+                                             int64_t q_stride, int64_t out_stride, int32_t num_blocks,
+                                             int32_t block_size, int32_t block_table_stride, float scale,
+                                             float softcap, const float* sink, void* workspace,
+                                             size_t workspace_bytes, int32_t num_ctas, int32_t dtype,
+                                             b200_stream_t stream_) {
+  return b200_paged_decode_attn_windowed(out, q, k_cache, v_cache, block_tables, context_lens, batch, num_heads,
+                                         num_kv_heads, head_dim, head_dim, q_stride, out_stride, num_blocks, block_size,
+                                         block_table_stride, scale, softcap, sink, 0, 0, 0, workspace, workspace_bytes,
+                                         num_ctas, dtype, stream_);
+}
+
+extern "C" int b200_paged_decode_attn_windowed(void* out, const void* q, const void* k_cache, const void* v_cache,
+                                               const int32_t* block_tables, const int32_t* context_lens, int32_t batch,
+                                               int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
+                                               int32_t value_dim, int64_t q_stride, int64_t out_stride,
+                                               int32_t num_blocks, int32_t block_size, int32_t block_table_stride,
+                                               float scale, float softcap, const float* sink, int32_t window,
+                                               int32_t keep_first, int32_t chunk, void* workspace, size_t workspace_bytes,
+                                               int32_t num_ctas, int32_t dtype, b200_stream_t stream_) {
+  return decode_windowed(out, q, k_cache, v_cache, block_tables, context_lens, batch, num_heads, num_kv_heads, head_dim, value_dim, q_stride,
+                         out_stride, num_blocks, block_size, block_table_stride, scale, softcap, sink, window, keep_first, chunk, workspace,
+                         workspace_bytes, num_ctas, dtype, false, stream_);
+}
+
+extern "C" int b200_paged_decode_attn_few(void* out, const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
+                                          const int32_t* context_lens, int32_t batch, int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
+                                          int64_t q_stride, int64_t out_stride, int32_t num_blocks, int32_t block_size,
+                                          int32_t block_table_stride, float scale, float softcap, const float* sink, int32_t dtype,
+                                          b200_stream_t stream) {
+  return decode_windowed(out, q, k_cache, v_cache, block_tables, context_lens, batch, num_heads, num_kv_heads, head_dim, head_dim, q_stride,
+                         out_stride, num_blocks, block_size, block_table_stride, scale, softcap, sink, 0, 0, 0, nullptr, 0, 0, dtype, true, stream);
 }

@@ -553,15 +553,15 @@ static int decode_fp8_launch_d(int hkv_cta, const CUtensorMap& mk, const CUtenso
 
 using namespace b200;
 
-extern "C" int b200_paged_decode_attn_fp8(void* out, const void* q, const void* k_cache,
-                                          const void* v_cache, const int32_t* block_tables,
-                                          const int32_t* context_lens, int32_t batch,
-                                          int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
-                                          int64_t q_stride, int64_t out_stride, int32_t num_blocks,
-                                          int32_t block_size, int32_t block_table_stride, float scale,
-                                          float k_scale, float v_scale, void* workspace,
-                                          size_t workspace_bytes, int32_t num_ctas, int32_t dtype,
-                                          b200_stream_t stream_) {
+static int decode_fp8(void* out, const void* q, const void* k_cache,
+                      const void* v_cache, const int32_t* block_tables,
+                      const int32_t* context_lens, int32_t batch,
+                      int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
+                      int64_t q_stride, int64_t out_stride, int32_t num_blocks,
+                      int32_t block_size, int32_t block_table_stride, float scale,
+                      float k_scale, float v_scale, void* workspace,
+                      size_t workspace_bytes, int32_t num_ctas, int32_t dtype,
+                      bool few, b200_stream_t stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   B200_RETURN_IF(dtype != B200_DTYPE_BF16 && dtype != B200_DTYPE_F16, B200_ERR_BAD_DTYPE);
   B200_RETURN_IF(batch < 0 || num_heads <= 0 || num_kv_heads <= 0 || num_blocks <= 0 ||
@@ -571,7 +571,7 @@ extern "C" int b200_paged_decode_attn_fp8(void* out, const void* q, const void* 
   B200_RETURN_IF(!(k_scale > 0.f) || !(v_scale > 0.f), B200_ERR_BAD_SHAPE);
   if (batch == 0) return B200_OK;
   B200_RETURN_IF(!out || !q || !k_cache || !v_cache || !block_tables || !context_lens ||
-                     !workspace,
+                     (!few && !workspace),
                  B200_ERR_NULL_POINTER);
   B200_RETURN_IF(head_dim != 64 && head_dim != 128, B200_ERR_UNSUPPORTED);
   const int G = num_heads / num_kv_heads;
@@ -592,7 +592,7 @@ extern "C" int b200_paged_decode_attn_fp8(void* out, const void* q, const void* 
                  B200_ERR_MISALIGNED);
   B200_RETURN_IF(!aligned16(k_cache) || !aligned16(v_cache) || !aligned16(workspace),
                  B200_ERR_MISALIGNED);
-  B200_RETURN_IF(workspace_bytes <
+  B200_RETURN_IF(!few && workspace_bytes <
                      b200_paged_decode_attn_workspace_size(batch, num_heads, num_kv_heads, head_dim),
                  B200_ERR_WORKSPACE);
 
@@ -627,6 +627,7 @@ extern "C" int b200_paged_decode_attn_fp8(void* out, const void* q, const void* 
     const int ctas = decode_small_ctas((int64_t)batch * num_kv_heads, (int64_t)block_table_stride * block_size, head_dim, true);
     if (ctas > 0) return decode_small_fp8_launch(p, k_cache, v_cache, num_blocks, head_dim, v_scale, dtype, ctas, stream);
   }
+  B200_RETURN_IF(few, B200_ERR_UNSUPPORTED);
 
   const int chunks = num_kv_heads * head_dim / 128;
   const int chunks_box = hkv_cta * head_dim / 128;
@@ -646,6 +647,28 @@ extern "C" int b200_paged_decode_attn_fp8(void* out, const void* q, const void* 
                : decode_fp8_launch_d<__nv_bfloat16, 64>(hkv_cta, mk, mv, p, v_scale, grid, stream);
   return head_dim == 128 ? decode_fp8_launch_d<__half, 128>(hkv_cta, mk, mv, p, v_scale, grid, stream)
                          : decode_fp8_launch_d<__half, 64>(hkv_cta, mk, mv, p, v_scale, grid, stream);
+}
+
+extern "C" int b200_paged_decode_attn_fp8(void* out, const void* q, const void* k_cache,
+                                          const void* v_cache, const int32_t* block_tables,
+                                          const int32_t* context_lens, int32_t batch,
+                                          int32_t num_heads, int32_t num_kv_heads, int32_t head_dim,
+                                          int64_t q_stride, int64_t out_stride, int32_t num_blocks,
+                                          int32_t block_size, int32_t block_table_stride, float scale,
+                                          float k_scale, float v_scale, void* workspace,
+                                          size_t workspace_bytes, int32_t num_ctas, int32_t dtype,
+                                          b200_stream_t stream_) {
+  return decode_fp8(out, q, k_cache, v_cache, block_tables, context_lens, batch, num_heads, num_kv_heads, head_dim, q_stride, out_stride, num_blocks,
+                    block_size, block_table_stride, scale, k_scale, v_scale, workspace, workspace_bytes, num_ctas, dtype, false, stream_);
+}
+
+extern "C" int b200_paged_decode_attn_fp8_few(void* out, const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
+                                              const int32_t* context_lens, int32_t batch, int32_t num_heads, int32_t num_kv_heads,
+                                              int32_t head_dim, int64_t q_stride, int64_t out_stride, int32_t num_blocks, int32_t block_size,
+                                              int32_t block_table_stride, float scale, float k_scale, float v_scale, int32_t dtype,
+                                              b200_stream_t stream) {
+  return decode_fp8(out, q, k_cache, v_cache, block_tables, context_lens, batch, num_heads, num_kv_heads, head_dim, q_stride, out_stride, num_blocks,
+                    block_size, block_table_stride, scale, k_scale, v_scale, nullptr, 0, 0, dtype, true, stream);
 }
 
 extern "C" int b200_reshape_and_cache_fp8(const void* key, const void* value, void* k_cache,

@@ -1,7 +1,8 @@
 // host_calls.cpp -- the attention entry points of ops.py as one native call each.
 //
-// A decode call of one row takes 8.7 us on the device (100 of them in a graph) and took 17 us of Python: 25 arguments through ctypes (3.6
-// us), some 35 tensor attributes (4 us); 9.2 us now, all in all. Captured steps never paid it. Here the same attributes are looked at
+// A decode call of one row takes 6.4 us on the device (in a graph) and took 17 us of Python: 25 arguments through ctypes (3.6 us), some 35
+// tensor attributes (4 us); 6.4 us now, all in all (7.7 with the workspace looked up that its one launch does not take). Captured steps
+// never paid it. Here the same attributes are looked at
 // and the same library function is called without either. What ops.py would refuse is not judged here: the functions return None for
 // any argument that is not exactly what they expect, and ops.py goes its own way, checks and errors included. An int is the library's
 // status. Plain torch.Tensor with memory of its own only (subclasses, fake tensors, dispatch modes and what torch.vmap and torch.func
@@ -21,6 +22,8 @@ namespace {
 decltype(&b200_paged_decode_attn_windowed) g_decode = nullptr;
 decltype(&b200_paged_decode_attn_fp8) g_decode_fp8 = nullptr;
 decltype(&b200_prefill_varlen_attn_windowed) g_prefill = nullptr;
+decltype(&b200_paged_decode_attn_few) g_decode_few = nullptr;
+decltype(&b200_paged_decode_attn_fp8_few) g_decode_fp8_few = nullptr;
 
 // a plain CUDA tensor with memory, or nullptr (the wrappers of torch.vmap, grad and jvp are torch.Tensor to Python, and have none)
 const at::Tensor* cuda_tensor(PyObject* o) {
@@ -76,6 +79,27 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     for (const at::Tensor* c : {k, v})
       if (c->scalar_type() != at::kByte && c->scalar_type() != at::kFloat8_e4m3fn) Py_RETURN_NONE;
   }
+  at::Tensor out = at::empty({B, H * D}, q->options());
+  const int64_t qs = B > 1 ? q->stride(0) : H * D;
+  const float scale = real(a[6]), f9 = real(a[9]), f10 = FP8 ? real(a[10]) : 0.f;
+  const int32_t window = FP8 ? 0 : (int32_t)whole(a[10]), keep_first = FP8 ? 0 : (int32_t)whole(a[11]), chunk = FP8 ? 0 : (int32_t)whole(a[12]);
+  void *const to = out.data_ptr(), *const qp = q->data_ptr(), *const kp = k->data_ptr(), *const vp = v->data_ptr();
+  const int32_t *const tables = (const int32_t*)bt->data_ptr(), *const rows = (const int32_t*)lens->data_ptr();
+  const int32_t nb = (int32_t)k->size(0), bs = (int32_t)k->size(1), bt_stride = (int32_t)bt->stride(0);
+  const int type = element(*q);
+  void* const on = stream();
+  int rc = B200_ERR_UNSUPPORTED;
+  if (B > 0 && ctas == 0 && window == 0 && chunk == 0) { // few rows: one launch that takes no workspace
+    Py_BEGIN_ALLOW_THREADS
+    if constexpr (FP8)
+      rc = g_decode_fp8_few(to, qp, kp, vp, tables, rows, (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, qs, H * D, nb, bs, bt_stride, scale,
+                            f9, f10, type, on);
+    else
+      rc = g_decode_few(to, qp, kp, vp, tables, rows, (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, qs, H * D, nb, bs, bt_stride, scale, f9,
+                        nullptr, type, on);
+    Py_END_ALLOW_THREADS
+  }
+  if (rc != B200_ERR_UNSUPPORTED) return status(rc, std::move(out));
   PyObject* device = PyObject_GetAttrString(a[1], "device");
   if (device == nullptr) return nullptr;
   PyObject* held = PyObject_CallFunction(a[0], "LLLLO", (long long)B, (long long)H, (long long)kv, (long long)D, device);
@@ -88,17 +112,8 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   PyObject* got = nullptr;
   try {
-    at::Tensor out = at::empty({B, H * D}, q->options());
-    const int64_t qs = B > 1 ? q->stride(0) : H * D;
-    const float scale = real(a[6]), f9 = real(a[9]), f10 = FP8 ? real(a[10]) : 0.f;
-    const int32_t window = FP8 ? 0 : (int32_t)whole(a[10]), keep_first = FP8 ? 0 : (int32_t)whole(a[11]), chunk = FP8 ? 0 : (int32_t)whole(a[12]);
-    void *const to = out.data_ptr(), *const qp = q->data_ptr(), *const kp = k->data_ptr(), *const vp = v->data_ptr(), *const wp = ws->data_ptr();
-    const int32_t *const tables = (const int32_t*)bt->data_ptr(), *const rows = (const int32_t*)lens->data_ptr();
-    const int32_t nb = (int32_t)k->size(0), bs = (int32_t)k->size(1), bt_stride = (int32_t)bt->stride(0);
+    void* const wp = ws->data_ptr();
     const size_t bytes = (size_t)ws->numel();
-    const int type = element(*q);
-    void* const on = stream();
-    int rc;
     Py_BEGIN_ALLOW_THREADS
     if constexpr (FP8)
       rc = g_decode_fp8(to, qp, kp, vp, tables, rows, (int32_t)B, (int32_t)H, (int32_t)kv, (int32_t)D, qs, H * D, nb, bs, bt_stride, scale,
@@ -164,19 +179,20 @@ PyObject* prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(addresses of the three library functions)
+// bind(addresses of the five library functions)
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 3) {
-    PyErr_SetString(PyExc_TypeError, "bind takes three addresses");
+  if (n != 5) {
+    PyErr_SetString(PyExc_TypeError, "bind takes five addresses");
     return nullptr;
   }
-  void* p[3];
-  for (int i = 0; i < 3; ++i)
+  void* p[5];
+  for (int i = 0; i < 5; ++i)
     if ((p[i] = PyLong_AsVoidPtr(a[i])) == nullptr) {
       if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address");
       return nullptr;
     }
   g_decode = (decltype(g_decode))p[0], g_decode_fp8 = (decltype(g_decode_fp8))p[1], g_prefill = (decltype(g_prefill))p[2];
+  g_decode_few = (decltype(g_decode_few))p[3], g_decode_fp8_few = (decltype(g_decode_fp8_few))p[4];
   Py_RETURN_NONE;
 }
 

@@ -63,6 +63,10 @@ PROTOTYPES = {
                                                     c_int32, c_int64, c_int64, c_int64, c_int64, c_void_p, c_int32,
                                                     c_int32, c_int32, c_float, c_float, c_void_p, c_int32, c_int32,
                                                     c_int32, c_int32, c_void_p, c_int64, c_void_p]),
+    "b200_paged_decode_attn_few": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32,
+                                            c_int64, c_int64, c_int32, c_int32, c_int32, c_float, c_float, c_void_p, c_int32, c_void_p]),
+    "b200_paged_decode_attn_fp8_few": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32,
+                                                c_int64, c_int64, c_int32, c_int32, c_int32, c_float, c_float, c_float, c_int32, c_void_p]),
     "b200_paged_decode_attn_windowed": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32,
                                                   c_int32, c_int32, c_int32, c_int32, c_int64, c_int64, c_int32,
                                                   c_int32, c_int32, c_float, c_float, c_void_p, c_int32, c_int32,
@@ -318,7 +322,8 @@ def calls():
             _calls = False
             return None
         module.bind(*(ctypes.cast(f, c_void_p).value for f in (lib.b200_paged_decode_attn_windowed, lib.b200_paged_decode_attn_fp8,
-                                                               lib.b200_prefill_varlen_attn_windowed)))
+                                                               lib.b200_prefill_varlen_attn_windowed, lib.b200_paged_decode_attn_few,
+                                                               lib.b200_paged_decode_attn_fp8_few)))
         _calls = module
     return _calls or None
 

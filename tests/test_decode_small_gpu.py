@@ -109,3 +109,18 @@ def test_e4m3_cache(H, G, D, lens, dtype):
     for i, n in enumerate(lens):
         if n == 0:
             assert torch.equal(got[i], torch.zeros_like(got[i]))
+
+
+def test_the_workspace_is_asked_for_by_wide_steps_alone(monkeypatch):
+    """Through the native call: one row takes none, more (row, kv head) pairs than the rule holds do; no rows at all are refused as they were."""
+    from nanovllm import _C, ops
+    if _C.calls() is None:
+        pytest.skip("no native calls")
+    H, G, D, asked, real = 16, 8, 128, [], ops.decode_workspace
+    monkeypatch.setattr(ops, "decode_workspace", lambda *a: asked.append(a) or real(*a))
+    for rows, wanted in ((1, 0), (40, 1)):
+        q, k, v, table = (t.cuda() for t in _case(H, G, D, [90] * rows, torch.bfloat16, 1))
+        ops.paged_decode_attn(q, k, v, table, torch.full((rows,), 90, dtype=torch.int32, device="cuda"), D ** -0.5, G)
+        assert len(asked) == wanted
+    with pytest.raises(_C.B200Error):
+        ops.paged_decode_attn(q[:0], k, v, table[:0], torch.empty(0, dtype=torch.int32, device="cuda"), D ** -0.5, G)
