@@ -21,6 +21,9 @@
 // 10 more with 8 columns a lane, which read every sector twice, 7 with that but block ids looked up a step ahead); 4 of 600-1000, 32
 // heads over 8 of 64, 490 -> 132.
 //
+// Few row tiles (attn_split_shared) have their keys shared by a cluster of two CTAs: each runs as above over its part, leaves its rows' maxima
+// and sums in its shared memory, and the first one merges them, relative to the larger maximum.
+//
 // What the split cannot carry: what is not finite or close to the largest numbers (and 0 x inf would reach rows that do not see the key),
 // and what is so small that a term of it would not be normal. Values come times 2^27, which leaves nothing too small, and go back
 // at the end. A small element of Q or K (below 2^-100) is off by 2^-126 at most, which is nothing to a score unless it meets one of
@@ -35,6 +38,7 @@ namespace b200 {
 
 constexpr int kAsM = 128, kAsN = 64, kAsThreads = 640, kAsCorr = 4;
 constexpr int kAsPanel = 64 * 128;                     // bytes of 64 rows x 64 elements
+constexpr int kAsParts = 2;                             // CTAs that share a row tile's keys, where they do
 
 constexpr float kAsUp = 134217728.f;                    // 2^27: values come to the tensor core times it (see below)
 
@@ -46,7 +50,7 @@ struct AttnSplitParams {
 
 template <int DK, int DV>
 constexpr int as_smem() {
-  return 1024 + 3 * (2 * (DK / 64) + DK / 64 + DV / 64) * kAsPanel + (kAsCorr + 1) * kAsM * 4 + 256;
+  return 1024 + 3 * (2 * (DK / 64) + DK / 64 + DV / 64) * kAsPanel + (kAsCorr + 3 + kAsParts) * kAsM * 4 + 256;
 }
 
 // four fp32 -> half a 16-byte chunk of each of three planes
@@ -63,7 +67,8 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return c;
 }
 
-template <int DK, int DV>
+// SHARED: a cluster of kAsParts CTAs takes a row tile, each a part of its keys; the first merges the results over distributed shared memory
+template <int DK, int DV, bool SHARED>
 __global__ void __launch_bounds__(kAsThreads, 1)
 attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
   using T = __nv_bfloat16;
@@ -77,17 +82,27 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
   uint8_t* sK = sQ + 3 * kQPlane;                       // [3][CK][64 keys]
   uint8_t* sV = sK + 3 * kKPlane;                       // [3][CV][64 keys]
   float* s_corr = reinterpret_cast<float*>(sV + 3 * kVPlane);   // [kAsCorr][128], then [128] 1 / l
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_corr + (kAsCorr + 1) * kAsM);
+  float *s_m = s_corr + (kAsCorr + 1) * kAsM, *s_l = s_m + kAsM, *s_part = s_l + kAsM;   // keys shared: [128] m, l of this part; [kAsParts][128] what a part counts
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_part + kAsParts * kAsM);
   uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 2, *v_full = bars + 3, *v_empty = bars + 4, *s_full = bars + 5,
            *p_ready = bars + 7, *o_full = bars + 8, *o_read = bars + 10, *done = bars + 12, *drained = bars + 13;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int *huge = gave_up + 1, *tiny = gave_up + 2, *large = gave_up + 3;
-  auto wild = [&] { return *huge != 0 || (*tiny != 0 && *large != 0); };
+  int parts_met = 1;                                     // CTAs whose values count: set behind the meeting of a cluster's
+  auto wild = [&] {
+    bool any = *huge != 0 || (*tiny != 0 && *large != 0);
+    for (int p = 1; p < parts_met; ++p)
+      any = any || ld_peer_int(smem_u32(const_cast<int*>(huge)), p) != 0 ||
+            (ld_peer_int(smem_u32(const_cast<int*>(tiny)), p) != 0 && ld_peer_int(smem_u32(const_cast<int*>(large)), p) != 0);
+    return any;
+  };
 
   pdl_wait();
   // the last row tiles see the most keys: those of every (sequence, kv head) start first
-  const int units = P.G * P.num_seqs, tile = (int)(gridDim.x / units - 1 - blockIdx.x / units), unit = blockIdx.x % units;
+  constexpr int ctas = SHARED ? kAsParts : 1;
+  const int part = SHARED ? (int)cluster_rank() : 0;
+  const int units = P.G * P.num_seqs, index = blockIdx.x / ctas, tile = (int)(gridDim.x / ctas / units) - 1 - index / units, unit = index % units;
   const int s = unit / P.G, g = unit % P.G;
   const SeqSpan sp = seq_span(P.cu_q, P.cu_k, nullptr, s);
   const int rep = P.H / P.G, rows = sp.q_len * rep, r0 = tile * kAsM;
@@ -104,7 +119,10 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     return table != nullptr ? (int64_t)table[key / P.block_size] * P.block_size + key % P.block_size : k_base + key;
   };
   const int min_pos = sp.first_pos() + r0 / rep, max_pos = sp.first_pos() + (min(r0 + kAsM, rows) - 1) / rep;
-  const int tiles = (max_pos + kAsN) / kAsN;
+  // this CTA's key tiles: of a cluster, each takes three at least, and those behind take none
+  const int all_tiles = (max_pos + kAsN) / kAsN, parts = SHARED ? max(1, min(ctas, all_tiles / 3)) : 1, per = (all_tiles + parts - 1) / parts;
+  if (SHARED && part >= parts) return;
+  const int first_key = part * per * kAsN, tiles = min(per, all_tiles - part * per);
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 256), mbar_init(k_full, 256), mbar_init(k_empty, 1), mbar_init(v_full, 256), mbar_init(v_empty, 1);
@@ -156,8 +174,8 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[i0 + i] = __uint_as_float(w[i]);
       }
-      if (j * kAsN + kAsN - 1 > min_pos) {
-        const int last = pos - j * kAsN;
+      if (first_key + j * kAsN + kAsN - 1 > min_pos) {
+        const int last = pos - first_key - j * kAsN;
 #pragma unroll
         for (int i = 0; i < kAsN; ++i) x[i] = i <= last ? x[i] : -INFINITY;
       }
@@ -204,6 +222,27 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       umma::fence_before_sync();
       mbar_arrive(p_ready);
     }
+    if (SHARED && parts > 1) {                                    // the parts of the row's keys: what each counts, relative to the largest score of all
+      s_m[row] = m, s_l[row] = l;
+      cluster_arrive(), cluster_wait();
+      if (part == 0) {
+        float ms[kAsParts], m_all = m;
+#pragma unroll
+        for (int p = 0; p < kAsParts; ++p) {
+          ms[p] = p < parts ? ld_peer(smem_u32(s_m + row), p) : -INFINITY;
+          m_all = fmaxf(m_all, ms[p]);
+        }
+        const bool far = fabsf(m_all) * c >= 65536.f && m_all != -INFINITY;
+        less = 0.f, l = 0.f, top = m_all * c;
+#pragma unroll
+        for (int p = 0; p < kAsParts; ++p) {
+          float f = ms[p] == -INFINITY ? 0.f : ex2_approx(ms[p] * c - top), none = 0.f;
+          if (far && ms[p] != -INFINITY) f = ms[p] - m_all, weights(f, none);
+          if (p < parts) l = fmaf(ld_peer(smem_u32(s_l + row), p), f, l);
+          s_part[p * kAsM + row] = f;
+        }
+      }
+    }
     // a sink is one more entry of the softmax that has a logit and no value (in units of log2, as top)
     float share = 1.f;
     if (P.sink != nullptr) {
@@ -241,7 +280,32 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       umma::fence_before_sync();
       mbar_arrive(&o_read[j & 1]);
     }
-    if (ok && wait(done, 0) && r < rows && !wild()) {
+    if (SHARED && parts > 1) {
+      // other parts leave their sums where the operands were, which no product reads any more: [DV / 4][128 rows][4]
+      if (part > 0) {
+#pragma unroll
+        for (int i = 0; i < DV; i += 4) reinterpret_cast<float4*>(smem)[(i / 4) * kAsM + row] = make_float4(O[i], O[i + 1], O[i + 2], O[i + 3]);
+      }
+      cluster_arrive(), cluster_wait();
+    }
+    parts_met = parts;
+    ok = ok && part == 0 && wait(done, 0);
+    if (SHARED && ok && parts > 1) {
+      const float own = s_part[row];
+#pragma unroll
+      for (int i = 0; i < DV; ++i) O[i] *= own;
+#pragma unroll 1
+      for (int p = 1; p < parts; ++p) {
+        const float f = s_part[p * kAsM + row];
+        const uint32_t from = smem_u32(smem) + row * 16;
+#pragma unroll
+        for (int i = 0; i < DV; i += 4) {
+          const float4 x = ld_peer4(from + (i / 4) * kAsM * 16, p);
+          O[i] = fmaf(x.x, f, O[i]), O[i + 1] = fmaf(x.y, f, O[i + 1]), O[i + 2] = fmaf(x.z, f, O[i + 2]), O[i + 3] = fmaf(x.w, f, O[i + 3]);
+        }
+      }
+    }
+    if (ok && r < rows && !wild()) {
       const float inv = s_corr[kAsCorr * kAsM + row];
       const int tok = r / rep;
       float* o = reinterpret_cast<float*>(P.out) + (int64_t)(sp.q_start + tok) * ((int64_t)P.H * vdim) + (int64_t)(g * rep + r - tok * rep) * vdim;
@@ -281,7 +345,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     int64_t own_row;
     auto row_of = [&](int i, int wide) { return wide ? w8 + 8 * i : 2 * (w8 + 8 * (i >> 1)) + (i & 1); };
     auto look_up = [&](int st) {
-      own_row = key_row(min(tile_of(st) * kAsN + row_of(lane & 7, (is_key(st) ? DK : DV) == 128), max_pos));
+      own_row = key_row(min(first_key + tile_of(st) * kAsN + row_of(lane & 7, (is_key(st) ? DK : DV) == 128), max_pos));
     };
     auto each = [&](int wide, auto f) {                 // f(item, row of the tile, first column, which of the 8 rows)
 #pragma unroll
@@ -296,7 +360,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       const float* from = key ? kb : vb;
       const int64_t stride = key ? P.k_stride : v_stride, offset = own_row * stride;
       each((key ? DK : DV) == 128, [&](int i, int row, int col, int nth) {
-        x[i] = fetch(from + __shfl_sync(0xffffffffu, offset, nth), col, width, j * kAsN + row <= max_pos);
+        x[i] = fetch(from + __shfl_sync(0xffffffffu, offset, nth), col, width, first_key + j * kAsN + row <= max_pos);
       });
     };
     look_up(0);
@@ -341,6 +405,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       if (!put(st, x0)) break;
       if (kAhead == 2 && !put(st + 1, x1)) break;
     }
+    if (SHARED && parts > 1) cluster_arrive(), cluster_wait();
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
     if (warp == 16) {
@@ -397,6 +462,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       mbar_wait_bounded(drained, 0, nullptr, kDrainNs);
       __syncwarp();
     }
+    if (SHARED && parts > 1) cluster_arrive(), cluster_wait();
   }
   umma::fence_before_sync();
   __syncthreads();
@@ -405,7 +471,14 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     *reinterpret_cast<volatile int*>(AP.wait_status) = 1;
     __threadfence_system();
   }
-  if (!wild()) return;
+  if (SHARED && part > 0) {                              // nobody leaves while the first part reads
+    cluster_arrive(), cluster_wait();
+    return;
+  }
+  parts_met = parts;
+  const bool plain = wild();
+  if (SHARED && parts > 1) cluster_arrive(), cluster_wait();
+  if (!plain) return;
 
   // ---- plain fp32, one warp per row, a lane per key of 32 and then a lane per value column of 32 (see above)
 #pragma unroll 1
@@ -470,9 +543,9 @@ bool attn_split_fits(const AttnTiledParams& P, int num_seqs, int max_q, int64_t 
   return (int64_t)max_q * rep >= least && (num_seqs == 1 || total_q * rep >= num_seqs * least / 2);
 }
 
-template <int DK, int DV>
+template <int DK, int DV, bool SHARED>
 static int attn_split_launch_as(const AttnTiledParams& P, dim3 grid, int64_t wait_ns, cudaStream_t stream) {
-  auto kern = attn_split_kernel<DK, DV>;
+  auto kern = attn_split_kernel<DK, DV, SHARED>;
   constexpr int smem = as_smem<DK, DV>();
   static_assert(smem <= 227 * 1024, "one CTA's shared memory");
   static std::atomic<uint64_t> devices{0};
@@ -480,16 +553,42 @@ static int attn_split_launch_as(const AttnTiledParams& P, dim3 grid, int64_t wai
   if (allowed != cudaSuccess) return (int)allowed;
   const AttnSplitParams AP{P, wait_tries(wait_ns), wait_status()};
   B200_RETURN_IF(AP.wait_status == nullptr, B200_ERR_DRIVER);
-  launch_pdl(kern, grid, dim3(kAsThreads), (size_t)smem, stream, AP);
+  if (!SHARED) {
+    launch_pdl(kern, grid, dim3(kAsThreads), (size_t)smem, stream, AP);
+    return finish_launch();
+  }
+  constexpr unsigned ctas = kAsParts;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid.x * ctas), cfg.blockDim = dim3(kAsThreads), cfg.dynamicSmemBytes = smem, cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr, cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, kern, AP);
   return finish_launch();
 }
 
-int attn_split_launch(AttnTiledParams P, int num_seqs, int max_q, int64_t wait_ns, cudaStream_t stream) {
+// A CTA's time is 11 us and 3.6 for every tile of 64 keys at heads of 128, so two share a row tile's keys where both find an SM, from six
+// tiles on, or where one of them does and there are many tiles. us, alone / shared, paged:
+//   8 heads over 2 of 128: 1 x 200 25.0 / 25.2, x 500 41.6 / 32.1, x 1000 70 / 47.2, x 2000 124 / 88.2;  [4 x 500 41.6 / 57.0, x 1000 86.6 / 145.3]
+//   8 of 48: 1 x 500 23.8 / 20.6, x 1000 39.0 / 27.4;  [32 over 8 of 64: 1 x 500 26.2 / 33.0, x 1000 49.0 / 75.9]
+// (four CTAs: 33.5, 66.6, 157.8 and 21.2, 39.7 on what two gain from)
+static bool attn_split_shared(int64_t row_tiles, int most_tiles) {
+  const int sms = sm_count();
+  return (row_tiles * 2 <= sms && most_tiles >= 6) || (row_tiles <= sms && most_tiles >= 24);
+}
+
+int attn_split_launch(AttnTiledParams P, int num_seqs, int max_q, int64_t total_q, int64_t wait_ns, cudaStream_t stream) {
   B200_RETURN_IF(take_wait_status(), B200_ERR_WAIT);             // of an earlier call
   P.num_seqs = num_seqs;
   const dim3 grid((unsigned)(((int64_t)max_q * (P.H / P.G) + kAsM - 1) / kAsM * P.G * num_seqs));
-  if (P.dim <= 64) return P.vdim <= 64 ? attn_split_launch_as<64, 64>(P, grid, wait_ns, stream) : attn_split_launch_as<64, 128>(P, grid, wait_ns, stream);
-  return P.vdim <= 64 ? attn_split_launch_as<128, 64>(P, grid, wait_ns, stream) : attn_split_launch_as<128, 128>(P, grid, wait_ns, stream);
+  const bool shared = total_q > 0 && attn_split_shared((total_q * (P.H / P.G) + kAsM - 1) / kAsM * P.G, (max_q + kAsN - 1) / kAsN);
+#define B200_AS(DK, DV) (shared ? attn_split_launch_as<DK, DV, true>(P, grid, wait_ns, stream) : attn_split_launch_as<DK, DV, false>(P, grid, wait_ns, stream))
+  if (P.dim <= 64) return P.vdim <= 64 ? B200_AS(64, 64) : B200_AS(64, 128);
+  return P.vdim <= 64 ? B200_AS(128, 64) : B200_AS(128, 128);
+#undef B200_AS
 }
 
 }  // namespace b200

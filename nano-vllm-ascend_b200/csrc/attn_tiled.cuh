@@ -24,7 +24,7 @@ struct AttnTiledParams {
 
 // The form on the tensor cores (attn_split.cu). total_q: the step's tokens, 0 if the caller has not said
 bool attn_split_fits(const AttnTiledParams& P, int num_seqs, int max_q, int64_t total_q, int dtype);
-int attn_split_launch(AttnTiledParams P, int num_seqs, int max_q, int64_t wait_ns, cudaStream_t stream);
+int attn_split_launch(AttnTiledParams P, int num_seqs, int max_q, int64_t total_q, int64_t wait_ns, cudaStream_t stream);
 bool attn_tiled_fits(int max_q, int rep, int G, int num_seqs, int dim, int vdim);
 int attn_tiled_launch(AttnTiledParams P, int num_seqs, int max_q, int dtype, cudaStream_t stream);
 

@@ -264,6 +264,35 @@ __device__ __forceinline__ bool mbar_warp_wait(uint64_t* bar, uint32_t parity, i
   return __all_sync(0xffffffffu, left >= 0) != 0;
 }
 inline int wait_tries(int64_t limit_ns) { return (int)((limit_ns < 1000000 * kTryNs ? limit_ns + kTryNs - 1 : 1000000 * kTryNs) / kTryNs); }
+// ---- thread-block clusters
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float ld_peer(uint32_t addr, uint32_t rank) {       // a word of CTA `rank`'s shared memory
+  uint32_t at;
+  float r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(r) : "r"(at) : "memory");
+  return r;
+}
+__device__ __forceinline__ int ld_peer_int(uint32_t addr, uint32_t rank) { return __float_as_int(ld_peer(addr, rank)); }
+__device__ __forceinline__ float4 ld_peer4(uint32_t addr, uint32_t rank) {
+  uint32_t at;
+  float4 r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(at) : "memory");
+  return r;
+}
+
 // generic-proxy writes to smem must be fenced before the async proxy (TMA) may overwrite
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -19,26 +19,6 @@ struct DecodeSmallParams {
   float v_scale;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ float ld_peer(uint32_t addr, uint32_t rank) {       // a word of CTA `rank`'s shared memory
-  uint32_t at;
-  float r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(r) : "r"(at) : "memory");
-  return r;
-}
-
 template <typename T, int D, bool FP8>
 __global__ void __launch_bounds__(kSmallWarps * 32, FP8 || D == 64 ? 2 : 1)
 decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {

@@ -773,7 +773,7 @@ extern "C" int b200_attn_generic_bounded(void* out, const void* q, int64_t q_str
     A.block_tables = block_tables, A.bt_stride = bt_stride, A.block_size = block_size, A.cu_q = cu_q, A.cu_k = cu_k;
     A.H = num_heads, A.G = num_kv_heads, A.dim = dim, A.vdim = vdim, A.scale = scale, A.window = window;
     A.keep_first = keep_first, A.chunk = chunk, A.softcap = softcap, A.sink = sink, A.gate = gate, A.gate_stride = gate_stride;
-    if (attn_split_fits(A, num_seqs, max_q, total_q, dtype)) return attn_split_launch(A, num_seqs, max_q, wait_ns, (cudaStream_t)stream);
+    if (attn_split_fits(A, num_seqs, max_q, total_q, dtype)) return attn_split_launch(A, num_seqs, max_q, total_q, wait_ns, (cudaStream_t)stream);
     return attn_tiled_launch(A, num_seqs, max_q, dtype, (cudaStream_t)stream);
   }
   const dim3 grid((max_q * rep + kAttnRows - 1) / kAttnRows, num_kv_heads, num_seqs);

@@ -124,3 +124,55 @@ def test_small_and_large_operands(qs, ks, vs):
         size = float(w.abs().max())
         floor = 2.0 ** -149 / size                             # one step of the smallest numbers
         assert float(((x - w).abs() / w.abs().clamp(min=0.3 * size)).max()) < 2e-5 + 4 * floor, s
+
+
+# ---- row tiles whose keys two CTAs share: few of them, and spans of 384 rows and more (every test above stays below)
+LONG = [(390, 900), (5, 5), (200, 333)]
+
+
+@pytest.mark.parametrize("H,G,dim,dv,paged,kw", [(8, 2, 128, 128, 16, {}), (4, 2, 64, 64, 0, dict(sink=True)), (3, 3, 48, 48, 16, dict(gate=True)),
+                                                 (2, 1, 20, 124, 64, dict(sink=True, gate=True)), (2, 1, 128, 36, 0, dict(latent=True))])
+def test_shared_keys_against_64_bit(H, G, dim, dv, paged, kw):
+    """Key tiles from one (a CTA alone) to fifteen, in odd and even numbers, parts that some rows see nothing of."""
+    for s, (x, w) in enumerate(_run(H, G, dim, dv, LONG, paged, **kw)):
+        assert float(((x - w).abs() / w.abs().clamp(min=1.0)).max()) < 2e-5, s
+    (x, w), = _run(H, G, dim, dv, [(449, 449)], paged, **kw)
+    assert float(((x - w).abs() / w.abs().clamp(min=1.0)).max()) < 2e-5
+
+
+@pytest.mark.parametrize("bad", [math.inf, math.nan, 1e-36])
+@pytest.mark.parametrize("where,at", [("q", 300), ("k", 10), ("k", 880), ("v", 10), ("v", 880)])
+def test_shared_keys_that_three_terms_cannot_carry(bad, where, at):
+    """Met by either of the two CTAs: the rows are computed once more, from all keys."""
+    def poke(q, ks, vs):
+        if where == "q":
+            q[at, 1, 5] = bad
+        else:
+            (ks if where == "k" else vs)[0][at, 0, 7] = bad
+    for s, (x, w) in enumerate(_run(4, 2, 64, 64, LONG, 16, poke=poke)):
+        fine = torch.isfinite(w)
+        assert torch.equal(torch.isfinite(x), fine), s
+        assert float(((x - w).abs() / w.abs().clamp(min=1.0))[fine].max()) < 2e-5, s
+
+
+@pytest.mark.parametrize("kind", ["far", "overflow", "one part has it all", "negative scale"])
+@pytest.mark.parametrize("sink", [False, True])
+def test_shared_keys_and_scores_of_any_size(kind, sink):
+    scale = -0.3 if kind == "negative scale" else None
+
+    def poke(q, ks, vs):
+        if kind == "far":                                      # around 1e10: their spacing is a thousand
+            q *= 1e5
+            for k in ks:
+                k *= 1e5
+        elif kind == "overflow":                               # finite operands, scores of -1e39 in the first part alone
+            q[:, :, 0], q[:, :, 1:] = 1e20, q[:, :, 1:] * 1e20
+            for k in ks:
+                k[:, :, 1:] *= 1e-20
+                k[:, :, 0] = 0.0
+                k[:len(k) // 3 if len(k) > 5 else 0, :, 0] = -1e20      # (the span of five has rows that would see nothing else)
+        elif kind == "one part has it all":                    # a key of the second part, hundreds above the others
+            q[:, :, 0] = 8.0
+            ks[0][700, :, 0] = 1000.0
+    for s, (x, w) in enumerate(_run(4, 2, 128, 128, LONG, 16, sink=sink, poke=poke, scale=scale)):
+        assert float(((x - w).abs() / w.abs().clamp(min=1.0)).max()) < 2e-5, s
