@@ -17,7 +17,7 @@
 // 96, P V 2 x 128. Shared memory at 128: Q 96 KB, K 48, V 48: one CTA per SM.
 // Bound: the tensor pipe (24 x 74 + 48 x 75 = 5376 cycles per tile of 64 keys at heads of 128, where the fp32 FMA pipes need 16384),
 // and the copying warps' load -> split -> store beside it (a tile takes 6300). Measured: 4 ragged prompts of 700-1024 tokens, 8
-// heads over 2 of 128, paged, 288 us (attn_tiled_kernel) -> 66 (20 calls in a graph; 70 where the inputs change from call to call;
+// heads over 2 of 128, paged, 288 us (attn_tiled_kernel) -> 66 (20 calls in a graph; 68 where the inputs change from call to call;
 // 10 more with 8 columns a lane, which read every sector twice, 7 with that but block ids looked up a step ahead); 4 of 600-1000, 32
 // heads over 8 of 64, 490 -> 132.
 //
@@ -138,10 +138,44 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
   constexpr uint32_t tb = 0;                            // all 512 columns: they start at 0
   auto wait = [&](uint64_t* bar, int parity) { return mbar_warp_wait(bar, parity & 1, AP.wait_tries, gave_up); };
 
+  auto look = [&](float4 x, float& most, float& least) {
+    asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(x.x), "f"(x.y));
+    asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(x.z), "f"(x.w));
+    asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(x.x), "f"(x.y));
+    asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(x.z), "f"(x.w));
+  };
+  auto judge = [&](float most, float least) {           // of what was looked at in Q or K
+    if (!(most < 0x1p127f)) *huge = 1;
+    if (most >= 0x1p70f) *large = 1;
+    if (least < 0x1p-100f) *tiny = 1;
+  };
+  auto fetch = [&](const float* row, int col, int width, bool there) {       // zero past the width (a multiple of 4)
+    return there && col < width ? __ldg(reinterpret_cast<const float4*>(row + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  // Q. Rows of 128: by the eight warps that have nothing else to do before the first scores, and registers for many loads; four rows at a time
+  // by the copying warps, it held the first tiles up (graphs: 12 x 500 93.8 -> 79.5 us, 4 x 1000 84.2 -> 78.5, 4 x 700-1024 68.6 -> 67.2). Rows of 64 and
+  // shared keys are up to 5 % better off with the copying warps.
+  constexpr bool kEarlyQ = DK == 128 && !SHARED;
+  auto copy_q = [&](int w8) {
+    float most = 0.f, least = 1.f;
+#pragma unroll (kEarlyQ ? 8 : 4)
+    for (int row = DK == 128 ? w8 : 2 * w8 + (lane >> 4); row < kAsM; row += DK == 128 ? 8 : 16) {
+      const int r = r0 + row, tok = r / rep, col = 4 * (DK == 128 ? lane : lane & 15);
+      float4 y = fetch(qb + (int64_t)(sp.q_start + tok) * P.q_stride + (int64_t)(g * rep + r - tok * rep) * dim, col, dim, r < rows);
+      look(y, most, least);
+      if (P.scale < 0.f) y = make_float4(-y.x, -y.y, -y.z, -y.w);
+      store_split4(sQ + (col >> 6) * 2 * kAsPanel + umma::sw128(row, (col >> 3) & 7) + (col & 4) * 2, kQPlane, y);
+    }
+    judge(most, least);
+    fence_proxy_async_smem();
+    mbar_arrive(q_full);
+  };
+
   // Registers: 640 x 96 at launch = 128 x (112 softmax + 160 sums + 2 x 80 copies + 48)
   if (warp < 4) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     // =========================== softmax ===========================
+    if (kEarlyQ) copy_q(warp);
     const int row = warp * 32 + lane, r = min(r0 + row, rows - 1);
     const uint32_t base = tb + ((uint32_t)(warp * 32) << 16);
     const int pos = sp.first_pos() + r / rep;
@@ -258,6 +292,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
   } else if (warp < 8) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
     // =========================== sums ===========================
+    if (kEarlyQ) copy_q(warp);
     const int quarter = warp - 4, row = quarter * 32 + lane, r = r0 + row;
     const uint32_t base = tb + ((uint32_t)(quarter * 32) << 16);
     float O[DV];
@@ -320,18 +355,9 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     // rows w, w + 8, .. of Q, K or V, for 64 columns two neighbouring rows at a time
     const int w8 = warp - 8;
     float most = 0.f, least = 1.f, most_v = 0.f;        // magnitudes met
-    auto look = [&](float4 x) {
-      asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(x.x), "f"(x.y));
-      asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(x.z), "f"(x.w));
-      asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(x.x), "f"(x.y));
-      asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(x.z), "f"(x.w));
-    };
     auto look_v = [&](float4 x) {
       asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most_v) : "f"(x.x), "f"(x.y));
       asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(most_v) : "f"(x.z), "f"(x.w));
-    };
-    auto fetch = [&](const float* row, int col, int width, bool there) {       // zero past the width (a multiple of 4)
-      return there && col < width ? __ldg(reinterpret_cast<const float4*>(row + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     // steps: K0, K1, V0, K2, V1, .., the order in which the issuing warp takes them
     const int steps = 2 * tiles;
@@ -370,29 +396,19 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       load(1, x1);
       if (steps > 2) look_up(2);
     }
-#pragma unroll 4
-    for (int row = DK == 128 ? w8 : 2 * w8 + (lane >> 4); row < kAsM; row += DK == 128 ? 8 : 16) {
-      const int r = r0 + row, tok = r / rep, col = 4 * (DK == 128 ? lane : lane & 15);
-      float4 y = fetch(qb + (int64_t)(sp.q_start + tok) * P.q_stride + (int64_t)(g * rep + r - tok * rep) * dim, col, dim, r < rows);
-      look(y);
-      if (P.scale < 0.f) y = make_float4(-y.x, -y.y, -y.z, -y.w);
-      store_split4(sQ + (col >> 6) * 2 * kAsPanel + umma::sw128(row, (col >> 3) & 7) + (col & 4) * 2, kQPlane, y);
-    }
-    fence_proxy_async_smem();
-    mbar_arrive(q_full);
+    if (!kEarlyQ) copy_q(w8);
     auto put = [&](int st, float4 (&x)[kItems]) -> bool {
       const bool key = is_key(st);
       const int j = tile_of(st), plane = key ? kKPlane : kVPlane;
       if (j > 0 && !wait(key ? k_empty : v_empty, j - 1)) return false;
       uint8_t* to = key ? sK : sV;
       each((key ? DK : DV) == 128, [&](int i, int row, int col, int) {
-        if (key) look(x[i]);
+        if (key) look(x[i], most, least);
         else x[i] = make_float4(x[i].x * kAsUp, x[i].y * kAsUp, x[i].z * kAsUp, x[i].w * kAsUp), look_v(x[i]);
         store_split4(to + (col >> 6) * kAsPanel + umma::sw128(row, (col >> 3) & 7) + (col & 4) * 2, plane, x[i]);
       });
-      if (!(most < 0x1p127f) || !(most_v < 0x1p107f)) *huge = 1;
-      if (most >= 0x1p70f) *large = 1;
-      if (least < 0x1p-100f) *tiny = 1;
+      if (!(most_v < 0x1p107f)) *huge = 1;
+      judge(most, least);
       fence_proxy_async_smem();
       mbar_arrive(key ? k_full : v_full);
       if (st + kAhead < steps) load(st + kAhead, x);
