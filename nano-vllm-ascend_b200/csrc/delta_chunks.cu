@@ -19,13 +19,13 @@
 //   X                      a thread per row: back substitution over columns, 64 x 64 / 2 packed multiply-adds, rows of A as broadcasts
 //   [W; Y], [U; O0]        M128 N = D K64, X from tensor memory
 // delta_scan_kernel, one CTA per (sequence, 128 value channels = one head of 128 or two of 64), S^T in fp32 registers:
-//   E^T = S0^T [W; P q - Y]^T    M128 (channels) N128 K = D, S0 in three terms from tensor memory
+//   E^T = S0^T [W; P q - Y]^T    M128 (channels) N128 K = D, S0 in three terms from tensor memory, in two halves of its rows
 //   w -> three terms; o out;  dS^T = w^T (P_end / P_j k_j)    M128 N = D K64;   S = P_end S + dS in registers.
 // Every fp32 operand is three bf16 terms by cutting off (24 bits, exact), six products, small ones first; values are bf16 as they are.
 //
 // What bounds them, 16 prompts of 500-1300 tokens, 8 heads of 128 (delta_rule_kernel 650 us): delta_chunk_kernel 205, a CTA's phases behind
-// one another (loads, scores, substitution, products, 48000 cycles, of which 11000 are issue); delta_scan_kernel 108, the chain
-// E -> w -> dS -> S -> E, 72 MMAs of 64 cycles and four conversions a chunk. The records that pass between them (216 KB per chunk and head
+// one another (loads, scores, substitution, products, 48000 cycles, of which 11000 are issue); delta_scan_kernel 106, the chain
+// E -> w -> dS -> S -> E of 8500 cycles a chunk, 6000 of them for 72 MMAs. The records that pass between them (216 KB per chunk and head
 // of 128, written and read once) would take 2 x 63 at HBM's rate.
 //
 // Not for chunks, and left to delta_rule_kernel, which runs behind them over the heads that a record flags: values that are not finite
@@ -82,9 +82,9 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint3
                : "memory");
 }
 // The tensor core cuts a sum off after every 16 products; on average results lack this part of them. Measured as the mean relative difference
-// from 64-bit products of random operands: of 8, 4 and 2 times 16 products, and in W, U (mostly one product each) and O0. Added back,
+// from 64-bit products of random operands, for each product as it is summed here. Added back,
 // in fp32: outputs 2.6e-7 -> 2.2e-7 off, states 2.2e-7 -> 1.9e-7, where the token form is 2.2e-7 and 2.0e-7 off (the case above).
-constexpr float kCut8 = 1.5e-7f, kCut4 = 0.9e-7f, kCut2 = 0.45e-7f, kCutW = 0.42e-7f, kCutU = 0.5e-7f, kCutO = 0.6e-7f;
+constexpr float kCutY = 0.9e-7f, kCutScore = 0.45e-7f, kCutW = 0.42e-7f, kCutU = 0.5e-7f, kCutO = 0.6e-7f, kCutE = 1.0e-7f, kCutD = 0.75e-7f;
 __device__ __forceinline__ float uncut(uint32_t x, float part) { return fmaf(__uint_as_float(x), part, __uint_as_float(x)); }
 __device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 __device__ __forceinline__ float largest(float most, float2 x) {             // of |x|; NaN stays
@@ -369,7 +369,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
           for (int c = 0; c < 16; ++c) {
             float sum = __uint_as_float(y[0][c]) + __uint_as_float(y[1][c]);
             if (D == 128) sum += __uint_as_float(y[D / 32 - 2][c]) + __uint_as_float(y[D / 32 - 1][c]);
-            w[c0 + c] = __float_as_uint(fmaf(sum, kCut2, sum));
+            w[c0 + c] = __float_as_uint(fmaf(sum, kCutScore, sum));
           }
         }
       } else {
@@ -536,7 +536,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     const int n0 = side * (D / 2) + c0;
     float x[16];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) x[c] = uncut(w[c], quarter >= 2 ? kCut4 : kCutW);
+    for (int c = 0; c < 16; ++c) x[c] = uncut(w[c], quarter >= 2 ? kCutY : kCutW);
     if (quarter >= 2) {
 #pragma unroll
       for (int c = 0; c < 16; c += 4) {
@@ -612,12 +612,13 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
   uint8_t* smem = ds_smem_raw + (-smem_u32(ds_smem_raw) & 1023u);       // (not through an integer: the compiler has to know that it is shared memory)
   uint8_t *sWq = smem, *sKe = sWq + NH * R::kWq, *sUo = sKe + NH * R::kKe;
   float* sPe = reinterpret_cast<float*>(sUo + NH * R::kUo);            // [2][NH * D]
-  uint64_t *wq_full = reinterpret_cast<uint64_t*>(sPe + 2 * NH * D), *ke_full = wq_full + 1, *uo_full = wq_full + 2, *s_ready = wq_full + 3,
+  uint64_t *wq_full = reinterpret_cast<uint64_t*>(sPe + 2 * NH * D), *ke_full = wq_full + 1, *uo_full = wq_full + 2, *s_ready = wq_full + 9,
            *e_done = wq_full + 4, *w_ready = wq_full + 5, *d_done = wq_full + 6, *uo_read = wq_full + 7, *drained = wq_full + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wq_full + 9);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wq_full + 11);                     // (s_ready: two)
   volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  constexpr float kCut = D == 128 ? kCut8 : kCut4;
-  constexpr uint32_t kTmS = 0, kTmW = 0, kTmE = 256, kTmD = 384;       // S 3 x D / 2 (w 3 x 32 in its place), E 128, dS D
+  // S 3 x D / 2 (w 3 x 32 in its place), E in two accumulators of 128, dS in place of the second. E starts with the half of every warp's rows of S
+  // that is ready first: its accumulator has the products of those rows, largest last, and the other half has one of its own
+  constexpr uint32_t kTmS = 0, kTmW = 0, kTmE = 192, kTmD = 320;
 
   pdl_wait();
   const int s = blockIdx.y, h0 = blockIdx.x * NH, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -648,7 +649,7 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
   for (int j = threadIdx.x; j < chunks * NH; j += kDsThreads)
     odd = odd || *reinterpret_cast<const int*>(records + (int64_t)(j / NH) * step + (j % NH) * DP.c.bytes + R::kFlagAt) != 0;
   if (threadIdx.x == 0) {
-    mbar_init(wq_full, 1), mbar_init(ke_full, 1), mbar_init(uo_full, 1), mbar_init(s_ready, 256), mbar_init(e_done, 1), mbar_init(w_ready, 256);
+    mbar_init(wq_full, 1), mbar_init(ke_full, 1), mbar_init(uo_full, 1), mbar_init(s_ready, 256), mbar_init(s_ready + 1, 256), mbar_init(e_done, 1), mbar_init(w_ready, 256);
     mbar_init(d_done, 1), mbar_init(uo_read, 256), mbar_init(drained, 1);
     mbar_fence_init();
     *gave_up = 0;
@@ -669,62 +670,84 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
     const int64_t out_stride = (int64_t)P.H * D;
     float* out = P.out + (int64_t)h0 * D + c;
     const float4* uo = reinterpret_cast<const float4*>(sUo + c * (R::kUoRow * 4));
+    auto update = [&](int j, int piece) {                // a half of this thread's rows of S after chunk j - 1
+      const float* pe = sPe + ((j - 1) & 1) * (NH * D) + hh * D + half * (D / 2);
+#pragma unroll
+      for (int i0 = piece * (D / 4); i0 < (piece + 1) * (D / 4); i0 += 16) {
+        uint32_t w[16];
+        umma::ld16(base + kTmD + half * (D / 2) + i0, w);
+        umma::wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+          const float4 p = *reinterpret_cast<const float4*>(pe + i0 + i);
+          S[i0 + i] = fmaf(p.x, S[i0 + i], uncut(w[i], kCutD));
+          S[i0 + i + 1] = fmaf(p.y, S[i0 + i + 1], uncut(w[i + 1], kCutD));
+          S[i0 + i + 2] = fmaf(p.z, S[i0 + i + 2], uncut(w[i + 2], kCutD));
+          S[i0 + i + 3] = fmaf(p.w, S[i0 + i + 3], uncut(w[i + 3], kCutD));
+        }
+      }
+    };
     for (int j = 0;; ++j) {
       if (j > 0) {
         if (!wait(d_done, j - 1)) break;
         umma::fence_after_sync();
-        const float* pe = sPe + ((j - 1) & 1) * (NH * D) + hh * D + half * (D / 2);
+      }
+      if (j == chunks) {                                 // the last update
+        update(j, 0), update(j, 1);
+        break;
+      }
 #pragma unroll
-        for (int i0 = 0; i0 < D / 2; i0 += 16) {
-          uint32_t w[16];
-          umma::ld16(base + kTmD + half * (D / 2) + i0, w);
-          umma::wait_ld();
+      for (int piece = 0; piece < 2; ++piece) {          // as the A operand: packed pairs along n
+        if (j > 0) update(j, piece);
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
-            const float4 p = *reinterpret_cast<const float4*>(pe + i0 + i);
-            S[i0 + i] = fmaf(p.x, S[i0 + i], uncut(w[i], kCut4));
-            S[i0 + i + 1] = fmaf(p.y, S[i0 + i + 1], uncut(w[i + 1], kCut4));
-            S[i0 + i + 2] = fmaf(p.z, S[i0 + i + 2], uncut(w[i + 2], kCut4));
-            S[i0 + i + 3] = fmaf(p.w, S[i0 + i + 3], uncut(w[i + 3], kCut4));
+        for (int i0 = piece * (D / 4); i0 < (piece + 1) * (D / 4); i0 += 16) {
+          uint32_t w[3][8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            uint32_t x[3];
+            split3cut(S[i0 + 2 * i], S[i0 + 2 * i + 1], x);
+            w[0][i] = x[0], w[1][i] = x[1], w[2][i] = x[2];
           }
+#pragma unroll
+          for (int p = 0; p < 3; ++p) umma::st8(base + kTmS + p * (D / 2) + half * (D / 4) + i0 / 2, w[p]);
         }
+        umma::wait_st();
+        umma::fence_before_sync();
+        mbar_arrive(s_ready + piece);
       }
-      if (j == chunks) break;
-#pragma unroll
-      for (int i0 = 0; i0 < D / 2; i0 += 16) {           // as the A operand: packed pairs along n
-        uint32_t w[3][8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          uint32_t x[3];
-          split3cut(S[i0 + 2 * i], S[i0 + 2 * i + 1], x);
-          w[0][i] = x[0], w[1][i] = x[1], w[2][i] = x[2];
-        }
-#pragma unroll
-        for (int p = 0; p < 3; ++p) umma::st8(base + kTmS + p * (D / 2) + half * (D / 4) + i0 / 2, w[p]);
-      }
-      umma::wait_st();
-      umma::fence_before_sync();
-      mbar_arrive(s_ready);
       if (!wait(uo_full, j) || !wait(e_done, j)) break;
       umma::fence_after_sync();
 #pragma unroll
       for (int u = 0; u < 2; ++u) {                      // what is written: this thread's 32 tokens
-        uint32_t e[16], w[3][8];
+        uint32_t e[16], more[16], w[3][8];
         umma::ld16(base + kTmE + half * 32 + 16 * u, e);
+        umma::ld16(base + kTmE + 128 + half * 32 + 16 * u, more);
         float4 x[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) x[i] = uo[half * 8 + 4 * u + i];
         umma::wait_ld();
 #pragma unroll
+        for (int i = 0; i < 16; ++i) e[i] = __float_as_uint(__uint_as_float(e[i]) + __uint_as_float(more[i]));
+#pragma unroll
         for (int i = 0; i < 4; ++i) {
           uint32_t y[3];
-          split3cut(x[i].x - uncut(e[4 * i], kCut), x[i].y - uncut(e[4 * i + 1], kCut), y);
+          split3cut(x[i].x - uncut(e[4 * i], kCutE), x[i].y - uncut(e[4 * i + 1], kCutE), y);
           w[0][2 * i] = y[0], w[1][2 * i] = y[1], w[2][2 * i] = y[2];
-          split3cut(x[i].z - uncut(e[4 * i + 2], kCut), x[i].w - uncut(e[4 * i + 3], kCut), y);
+          split3cut(x[i].z - uncut(e[4 * i + 2], kCutE), x[i].w - uncut(e[4 * i + 3], kCutE), y);
           w[0][2 * i + 1] = y[0], w[1][2 * i + 1] = y[1], w[2][2 * i + 1] = y[2];
         }
 #pragma unroll
         for (int p = 0; p < 3; ++p) umma::st8(base + kTmW + p * 32 + half * 16 + 8 * u, w[p]);
+      }
+      float read[32];                                    // (P q - Y) S0 for the outputs: dS takes the place of its second half
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        uint32_t e[16], more[16];
+        umma::ld16(base + kTmE + 64 + half * 32 + 16 * u, e);
+        umma::ld16(base + kTmE + 128 + 64 + half * 32 + 16 * u, more);
+        umma::wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) read[16 * u + i] = __uint_as_float(e[i]) + __uint_as_float(more[i]);
       }
       umma::wait_st();
       umma::fence_before_sync();
@@ -732,23 +755,19 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
       const int t0 = (lo + j) * kDcL + half * 32, left = sp.q_len - t0;
       float* to = out + (sp.q_start + (int64_t)t0) * out_stride;
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        uint32_t e[16];
-        umma::ld16(base + kTmE + 64 + half * 32 + 16 * u, e);
-        float4 x[4];
+      for (int i = 0; i < 32; i += 4) {
+        const float4 x = uo[16 + half * 8 + i / 4];
+        const float o[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = uo[16 + half * 8 + 4 * u + i];
-        umma::wait_ld();
-        const float o[16] = {x[0].x, x[0].y, x[0].z, x[0].w, x[1].x, x[1].y, x[1].z, x[1].w,
-                             x[2].x, x[2].y, x[2].z, x[2].w, x[3].x, x[3].y, x[3].z, x[3].w};
-        if (left >= 32) {
+        for (int y = 0; y < 4; ++y) read[i + y] = o[y] + fmaf(read[i + y], kCutE, read[i + y]);
+      }
+      if (left >= 32) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i, to += out_stride) *to = o[i] + uncut(e[i], kCut);
-        } else {
+        for (int i = 0; i < 32; ++i, to += out_stride) *to = read[i];
+      } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i, to += out_stride)
-            if (16 * u + i < left) *to = o[i] + uncut(e[i], kCut);
-        }
+        for (int i = 0; i < 32; ++i, to += out_stride)
+          if (i < left) *to = read[i];
       }
       umma::fence_before_sync();
       mbar_arrive(uo_read);
@@ -779,24 +798,33 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
     if (DP.wait_tries > 0) load_wq(wq++), load_uo(uo++), load_ke(ke++);      // (a limit of 0 tests the way out: nothing comes)
     for (int j = 0; j < chunks; ++j) {
       const bool more = j + 1 < chunks;
-      if (!wait(wq_full, j) || !wait(s_ready, j)) break;
-      umma::fence_after_sync();
-      if (leader) {
+      if (!wait(wq_full, j)) break;
+      bool ready = true;
 #pragma unroll 1
-        for (int i = 0; i < 6; ++i) {
-          const uint32_t pa = term_a(i), pb = term_b(i);
+      for (int piece = 0; ready && piece < 2; ++piece) {
+        ready = wait(s_ready + piece, j);
+        if (!ready) break;
+        umma::fence_after_sync();
+        if (leader) {
+          const uint32_t to = tb + kTmE + 128 * piece;
+#pragma unroll 1
+          for (int i = 0; i < 6; ++i) {
+            const uint32_t pa = term_a(i), pb = term_b(i);
 #pragma unroll
-          for (int n = 0; n < NH; ++n)
+            for (int n = 0; n < NH; ++n)
 #pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) {
-              const uint32_t a = tb + kTmS + pa * (D / 2) + ks * 8, b = dwq + ((n * R::kWq + pb * (2 * D * 128) + ks * 2048) >> 4);
-              if (NH == 2) mma_ts_half_low(tb + kTmE, a, b, id_e, i > 0 || ks > 0, n);
-              else umma::mma_ts_low(tb + kTmE, a, b, id_e, i > 0 || ks > 0);
-            }
+              for (int x = 0; x < D / 32; ++x) {         // 16 rows each: those of the first four warps, then of the others
+                const int in = x % (D / 64), ks = (x / (D / 64)) * (D / 32) + piece * (D / 64) + in;
+                const uint32_t a = tb + kTmS + pa * (D / 2) + ks * 8, b = dwq + ((n * R::kWq + pb * (2 * D * 128) + ks * 2048) >> 4);
+                if (NH == 2) mma_ts_half_low(to, a, b, id_e, i > 0 || x > 0, n);
+                else umma::mma_ts_low(to, a, b, id_e, i > 0 || x > 0);
+              }
+          }
+          if (piece == 1) umma::commit(e_done);
         }
-        umma::commit(e_done);
+        __syncwarp();
       }
-      __syncwarp();
+      if (!ready) break;
       if (!wait(e_done, j)) break;
       if (more) load_wq(wq++);
       if (!wait(ke_full, j) || !wait(w_ready, j)) break;
