@@ -1260,14 +1260,22 @@ def _fp32_state_rule(mode, q, k, v, g, beta, spans: StepSpans, num_heads, groups
     out = torch.empty(T, num_heads * vdim, dtype=torch.float32, device=q.device)
     cu_q, cu_k, ctx = spans.ptrs()
     stride = lambda t: t.stride(0) if T > 1 else t.shape[1]
-    lib, dtype = _C.load(), _dt3(v)
-    # what the chunks of a prompt step pass from one kernel to the next (0 bytes where tokens are taken one at a time)
-    need = lib.b200_delta_rule_workspace_size(spans.num_seqs, spans.max_q, T, num_heads, groups, kdim, vdim, mode, dtype) if cu_q else 0
-    workspace = torch.empty(need, dtype=torch.uint8, device=q.device) if need > 0 else None
-    _C.check(lib.b200_delta_rule_step(out.data_ptr(), q.data_ptr(), stride(q), k.data_ptr(), stride(k), v.data_ptr(),
-                                      stride(v), g.data_ptr(), beta.data_ptr(), _ptr(state), _ptr(state_slots),
-                                      cu_q, cu_k, ctx, spans.num_seqs, spans.max_q, T, num_heads, groups, kdim, vdim, mode,
-                                      dtype, _ptr(workspace), need, _stream()), "b200_delta_rule_step")
+    if spans.max_q >= 96 and mode != 2:
+        # what the chunks of a prompt step pass from one kernel to the next (0 bytes: tokens one at a time; steps without a span of 96 tokens
+        # are, and short enough to notice the question)
+        lib, dtype = _C.load(), _dt3(v)
+        need = lib.b200_delta_rule_workspace_size(spans.num_seqs, spans.max_q, T, num_heads, groups, kdim, vdim, mode, dtype)
+        if need > 0:
+            workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
+            _C.check(lib.b200_delta_rule_step(out.data_ptr(), q.data_ptr(), stride(q), k.data_ptr(), stride(k), v.data_ptr(),
+                                              stride(v), g.data_ptr(), beta.data_ptr(), _ptr(state), _ptr(state_slots),
+                                              cu_q, cu_k, ctx, spans.num_seqs, spans.max_q, T, num_heads, groups, kdim, vdim, mode,
+                                              dtype, workspace.data_ptr(), need, _stream()), "b200_delta_rule_step")
+            return out
+    _C.check(_C.load().b200_delta_rule(out.data_ptr(), q.data_ptr(), stride(q), k.data_ptr(), stride(k), v.data_ptr(),
+                                       stride(v), g.data_ptr(), beta.data_ptr(), _ptr(state), _ptr(state_slots),
+                                       cu_q, cu_k, ctx, spans.num_seqs, num_heads, groups, kdim, vdim, mode,
+                                       _dt3(v), _stream()), "b200_delta_rule")
     return out
 
 
