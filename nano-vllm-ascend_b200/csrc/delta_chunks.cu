@@ -13,8 +13,7 @@
 // delta_chunk_kernel, one CTA of 8 warps per (chunk, head), two CTAs per SM:
 //   scores [K~; Q~] K^^T   M128 N64 K = D, 32 channels to an accumulator (the tensor core cuts sums off: the small products of later
 //                          channels on top of a full sum would cost 6e-7). Decays per channel are split at the chunk's middle,
-//                          K~ = k P_i / P_mid, K^ = k P_mid / P_j, each a product of decays or its reciprocal. Where such a product
-//                          leaves 2^-80 .. 2^80 the scores are summed up in fp32 instead (no reciprocal). One decay per head:
+//                          K~ = k P_i / P_mid, K^ = k P_mid / P_j, each a product of decays or its reciprocal. One decay per head:
 //                          K~ = K^ = k, and the decay goes on the scores.
 //   X                      a thread per row: back substitution over columns, 64 x 64 / 2 packed multiply-adds, rows of A as broadcasts
 //   [W; Y], [U; O0]        M128 N = D K64, X from tensor memory
@@ -30,7 +29,8 @@
 //
 // Not for chunks, and left to delta_rule_kernel, which runs behind them over the heads that a record flags: values that are not finite
 // (0 x inf would reach tokens before them) or beyond 2^60, decays of 2 and more, keys, queries or values all below 2^-60 (the low terms
-// would be lost).
+// would be lost), and decays per channel that come to less than 2^-90 over half a chunk (0.14 a token), or meet keys or queries from 2^30 on or all
+// below 2^-20, where a reciprocal or low terms would leave the range: a CTA with such decays leaves after their products.
 //
 // Waits are bounded (mbar_warp_wait): one that runs out makes its role leave, those that wait for it run out as well, the products under
 // way are waited for, the CTA sets the host's word and the library reports it.
@@ -97,7 +97,8 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return r;
 }
 constexpr uint32_t kBig = (127u + 60u) << 23, kSmall = (127u - 60u) << 23, kTwo = 128u << 23;
-constexpr float kFar = 1.2089258e24f, kNear = 8.2718061e-25f;              // 2^80, 2^-80
+constexpr float kFar = 0x1p90f, kNear = 0x1p-90f;
+constexpr uint32_t kBigUp = (127u + 30u) << 23, kSmallDn = (127u - 20u) << 23;       // of what meets kFar and, in its third term, kNear: within 2^+-126
 
 constexpr int kDcThreads = 256;
 constexpr int kDcARow = 68;                              // floats of a row of A: 16-byte groups of eight rows in different banks
@@ -301,8 +302,14 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
         r = mul2(r, gg[x]);
       }
     }
+    if (!PER_HEAD && __any_sync(0xffffffffu, far) && lane == 0) *s_far = 1;
     fence_proxy_async_smem();
     __syncthreads();
+    if (!PER_HEAD && *s_far && !*gave_up) {              // not for chunks (no product is under way)
+      if (threadIdx.x == 0) *reinterpret_cast<int*>(record + R::kFlagAt) = 1;
+      if (warp == 1) umma::tmem_dealloc(tb, 256);
+      return;
+    }
     if (issuer && alive) {
       const uint32_t id = umma::make_idesc<T>(128, 64, 0, 0);
       const uint32_t a0 = umma::desc_low(smem_u32(smem), 16), b0 = umma::desc_low(smem_u32(smem + 49152), 16);
@@ -319,35 +326,9 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
   const uint32_t mk = __reduce_max_sync(0xffffffffu, magnitude(most_k)), mq = __reduce_max_sync(0xffffffffu, magnitude(most_q)),
                  mg = __reduce_max_sync(0xffffffffu, magnitude(most_g));
   if (lane == 0) atomicMax(&s_max[0], mk), atomicMax(&s_max[1], mq), atomicMax(&s_max[3], mg);
-  if (__any_sync(0xffffffffu, far) && lane == 0) *s_far = 1;
   alive = alive && wait(scored, D / 64 - 1);
   umma::fence_after_sync();
-  __syncthreads();                                       // s_far; all that the scores were made of is free
-  const bool direct = !PER_HEAD && *s_far != 0;
-  float* sB = reinterpret_cast<float*>(smem);            // [64][kDcARow], where P k comes later
-  if (direct) {
-    // a warp per column j: k_j decays from token to token and meets k_i and q_i
-    constexpr int C = D / 32;
-    for (int j = warp; j < kDcL; j += 8) {
-      float x[C];
-#pragma unroll
-      for (int c = 0; c < C; ++c) x[c] = j < nt ? k[j * P.k_stride + c * 32 + lane] : 0.f;
-      for (int i = j; i < kDcL; ++i) {
-        float a = 0.f, b = 0.f;
-        if (i < nt) {
-#pragma unroll
-          for (int c = 0; c < C; ++c) {
-            const int d = c * 32 + lane;
-            if (i > j) x[c] *= g[i * g_stride + d];
-            a = fmaf(k[i * P.k_stride + d], x[c], a), b = fmaf(q[i * P.q_stride + d], x[c], b);
-          }
-        }
-        a = warp_sum(a), b = warp_sum(b);
-        if (lane == 0) sA[i * kDcARow + j] = a, sB[i * kDcARow + j] = b;
-      }
-    }
-    __syncthreads();
-  }
+  __syncthreads();                                       // all that the scores were made of is free
 
   uint4 held[D / 16];                                    // values on their way to where A is
   float2 X[32];                                          // warps 0-3: a row of X
@@ -358,24 +339,18 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
 #pragma unroll
     for (int part = 0; part < 2; ++part) {
       uint32_t w[32];
-      if (!direct) {
 #pragma unroll
-        for (int c0 = 0; c0 < 32; c0 += 16) {
-          uint32_t y[D / 32][16];
+      for (int c0 = 0; c0 < 32; c0 += 16) {
+        uint32_t y[D / 32][16];
 #pragma unroll
-          for (int z = 0; z < D / 32; ++z) umma::ld16(base + kTmSC + 64 * z + 32 * part + c0, y[z]);
-          umma::wait_ld();
+        for (int z = 0; z < D / 32; ++z) umma::ld16(base + kTmSC + 64 * z + 32 * part + c0, y[z]);
+        umma::wait_ld();
 #pragma unroll
-          for (int c = 0; c < 16; ++c) {
-            float sum = __uint_as_float(y[0][c]) + __uint_as_float(y[1][c]);
-            if (D == 128) sum += __uint_as_float(y[D / 32 - 2][c]) + __uint_as_float(y[D / 32 - 1][c]);
-            w[c0 + c] = __float_as_uint(fmaf(sum, kCutScore, sum));
-          }
+        for (int c = 0; c < 16; ++c) {
+          float sum = __uint_as_float(y[0][c]) + __uint_as_float(y[1][c]);
+          if (D == 128) sum += __uint_as_float(y[D / 32 - 2][c]) + __uint_as_float(y[D / 32 - 1][c]);
+          w[c0 + c] = __float_as_uint(fmaf(sum, kCutScore, sum));
         }
-      } else {
-        const float* row = (of_k ? sA : sB) + i * kDcARow + 32 * part;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) w[c] = __float_as_uint(row[c]);
       }
 #pragma unroll
       for (int c = 0; c < 16; ++c) X[16 * part + c] = make_float2(__uint_as_float(w[2 * c]), __uint_as_float(w[2 * c + 1]));
@@ -394,7 +369,6 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
       X[c].x = 2 * c < i + (of_k ? 0 : 1) ? X[c].x * beta : 0.f;
       X[c].y = 2 * c + 1 < i + (of_k ? 0 : 1) ? X[c].y * beta : 0.f;
     }
-    if (direct) named_bar_sync(1, 128), named_bar_arrive(2, 256);      // the rows of A are replaced, those of B become P k
     if (of_k) {
 #pragma unroll
       for (int c = 0; c < 16; ++c)
@@ -438,7 +412,6 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     }
     umma::wait_st();
   } else {
-    if (direct) named_bar_sync(2, 256);                  // (the scores have been read)
 #pragma unroll
     for (int i = 0; i < D / 16; ++i) {
       const int e = i * 128 + threadIdx.x - 128, row = e / (D / 8), c16 = e % (D / 8);
@@ -506,8 +479,9 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
   fence_proxy_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {
-    const bool odd = s_max[0] >= kBig || s_max[1] >= kBig || s_max[2] >= kBig || s_max[3] >= kTwo || (s_max[0] > 0 && s_max[0] < kSmall) ||
-                     (s_max[1] > 0 && s_max[1] < kSmall) || (s_max[2] > 0 && s_max[2] < kSmall);
+    constexpr uint32_t big = PER_HEAD ? kBig : kBigUp, small = PER_HEAD ? kSmall : kSmallDn;
+    const bool odd = s_max[0] >= big || s_max[1] >= big || s_max[2] >= kBig || s_max[3] >= kTwo || (s_max[0] > 0 && s_max[0] < small) ||
+                     (s_max[1] > 0 && s_max[1] < small) || (s_max[2] > 0 && s_max[2] < kSmall);
     *reinterpret_cast<int*>(record + R::kFlagAt) = odd ? 1 : 0;
   }
   const uint32_t id_w = umma::make_idesc<T>(128, D, 0, 1);
@@ -927,7 +901,7 @@ static int delta_chunks_launch_as(DcParams DP, int mode, int64_t total_q, int64_
     DP.c.first = (int)at;
     launch_pdl(chunk, dim3((unsigned)(count * P.H)), dim3(kDcThreads), (size_t)chunk_smem, stream, DP);
     launch_pdl(scan, dim3((unsigned)(P.H / NH), (unsigned)DP.num_seqs), dim3(kDsThreads), (size_t)scan_smem, stream, DP);
-    const int code = delta_rest_launch(P, DP.c, mode, DP.num_seqs, stream);
+    const int code = delta_rest_launch(P, DP.c, mode, DP.num_seqs, count >= chunks, stream);
     if (code != B200_OK) return code;
   }
   return finish_launch((int)(2 * ((chunks + count - 1) / count)));

@@ -47,8 +47,8 @@ __device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* gptr,
 }
 
 // ORDER: CTAs start with the longest sequences (delta_launch_as). REST: only heads that a pass of chunks has left aside (delta_chunks.cu),
-// and the tokens of that pass
-template <typename TV, int KPT, int NS, int NC, bool VEC, int MODE, bool ORDER = false, bool REST = false>
+// 1: of the only pass, 2: and the tokens of that pass
+template <typename TV, int KPT, int NS, int NC, bool VEC, int MODE, bool ORDER = false, int REST = 0>
 __global__ void __launch_bounds__(32 * NS)
 delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
   extern __shared__ __align__(16) float smem[];
@@ -61,15 +61,14 @@ delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
   SeqSpan sp = seq_span(P.cu_q, P.cu_k, P.ctx_lens, s);
   if (sp.q_len == 0) return;
   bool goes_on = false, ends = true;                 // from the pass before, with the span
-  if constexpr (REST) {
+  if constexpr (REST > 0) {                          // (the scan has set the flag of the span's first record in the pass)
     const int before = chunks_before(P.cu_q, s), n = chunks_of(sp.q_len);
-    const int lo = max(0, C.first - before), hi = min(n, C.first + C.count - before);
-    int flagged = 0;
-    for (int j = lo + threadIdx.x; j < hi; j += NTH)
-      flagged |= *reinterpret_cast<const int*>(C.records + ((int64_t)(before + j - C.first) * P.H + h) * C.bytes + C.flag_at);
-    if (!__syncthreads_or(flagged)) return;
-    goes_on = lo > 0, ends = hi == n;
-    sp.q_start += lo * kDcL, sp.q_len = min(sp.q_len, hi * kDcL) - lo * kDcL;
+    const int lo = REST == 1 ? 0 : max(0, C.first - before), hi = REST == 1 ? n : min(n, C.first + C.count - before);
+    if (lo >= hi || *reinterpret_cast<const int*>(C.records + ((int64_t)(before + lo - C.first) * P.H + h) * C.bytes + C.flag_at) == 0) return;
+    if (REST == 2) {
+      goes_on = lo > 0, ends = hi == n;
+      sp.q_start += lo * kDcL, sp.q_len = min(sp.q_len, hi * kDcL) - lo * kDcL;
+    }
   }
   const int kdim = P.kdim, vdim = P.vdim;
   const int ksl = threadIdx.x % NS, cl = (threadIdx.x / NS) * NC;
@@ -90,7 +89,7 @@ delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
                     ? P.state + (((int64_t)P.state_slots[s] * P.H + h) * kdim) * (int64_t)vdim
                     : nullptr;
   bool carried = slot != nullptr && sp.first_pos() > 0;
-  if constexpr (REST) {
+  if constexpr (REST == 2) {
     if (P.state == nullptr && !(ends && !goes_on)) slot = chunk_state(P, C, s, h);
     carried = carried || goes_on;
   }
@@ -249,7 +248,7 @@ delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
       }
     }
   }
-  if (slot != nullptr && (!REST || P.state != nullptr || !ends)) {
+  if (slot != nullptr && (REST != 2 || P.state != nullptr || !ends)) {
 #pragma unroll
     for (int r = 0; r < KPT; ++r) {
       const int i = ksl * KPT + r;
@@ -312,19 +311,31 @@ static int delta_launch(const DeltaParams& P, int num_seqs, cudaStream_t stream)
   return finish_launch();
 }
 
-template <int NS, int MODE>
+template <int NS, int MODE, int REST>
 static void delta_rest_launch_as(const DeltaParams& P, const DeltaChunks& C, int num_seqs, cudaStream_t stream) {
   using TV = __nv_bfloat16;
   constexpr int KP = NS * 36, CC = 64;
   constexpr size_t smem = (size_t)2 * kDeltaTok * (2 * KP + (MODE == kDecayPerHead ? 1 : KP) + 1) * sizeof(float) + (size_t)2 * kDeltaTok * CC * sizeof(TV);
   static_assert(smem <= 47 * 1024, "no more than a launch may have unasked");
-  launch_pdl(delta_rule_kernel<TV, 32, NS, 2, true, MODE, false, true>, dim3(P.vdim / CC, P.H, num_seqs), dim3(32 * NS), smem, stream, P, C);
+  const dim3 grid(P.vdim / CC, P.H, num_seqs);
+  if constexpr (NS == 4 && REST == 1) {               // the longest sequences first, as in delta_launch_as
+    if (num_seqs > 1 && num_seqs <= 32 && (int64_t)grid.x * grid.y * num_seqs > sm_count()) {
+      launch_pdl(delta_rule_kernel<TV, 32, NS, 2, true, MODE, true, REST>, grid, dim3(32 * NS), smem, stream, P, C);
+      return;
+    }
+  }
+  launch_pdl(delta_rule_kernel<TV, 32, NS, 2, true, MODE, false, REST>, grid, dim3(32 * NS), smem, stream, P, C);
 }
-int delta_rest_launch(const DeltaParams& P, const DeltaChunks& C, int mode, int num_seqs, cudaStream_t stream) {
-  if (P.kdim == 128 && mode == kDecayPerHead) delta_rest_launch_as<4, kDecayPerHead>(P, C, num_seqs, stream);
-  else if (P.kdim == 128) delta_rest_launch_as<4, kDecayPerChannel>(P, C, num_seqs, stream);
-  else if (mode == kDecayPerHead) delta_rest_launch_as<2, kDecayPerHead>(P, C, num_seqs, stream);
-  else delta_rest_launch_as<2, kDecayPerChannel>(P, C, num_seqs, stream);
+template <int REST>
+static void delta_rest_launch_of(const DeltaParams& P, const DeltaChunks& C, int mode, int num_seqs, cudaStream_t stream) {
+  if (P.kdim == 128 && mode == kDecayPerHead) delta_rest_launch_as<4, kDecayPerHead, REST>(P, C, num_seqs, stream);
+  else if (P.kdim == 128) delta_rest_launch_as<4, kDecayPerChannel, REST>(P, C, num_seqs, stream);
+  else if (mode == kDecayPerHead) delta_rest_launch_as<2, kDecayPerHead, REST>(P, C, num_seqs, stream);
+  else delta_rest_launch_as<2, kDecayPerChannel, REST>(P, C, num_seqs, stream);
+}
+int delta_rest_launch(const DeltaParams& P, const DeltaChunks& C, int mode, int num_seqs, bool only_pass, cudaStream_t stream) {
+  if (only_pass) delta_rest_launch_of<1>(P, C, mode, num_seqs, stream);
+  else delta_rest_launch_of<2>(P, C, mode, num_seqs, stream);
   return finish_launch();
 }
 

@@ -51,6 +51,6 @@ bool delta_chunks_ok(const DeltaParams& P, int mode, int dtype, int num_seqs, in
 int delta_chunks_launch(const DeltaParams& P, int mode, int num_seqs, int64_t total_q, void* workspace, int64_t bytes, int64_t wait_ns,
                         cudaStream_t stream);
 // delta_rule.cu: the tokens of the heads that the pass leaves aside, one at a time
-int delta_rest_launch(const DeltaParams& P, const DeltaChunks& C, int mode, int num_seqs, cudaStream_t stream);
+int delta_rest_launch(const DeltaParams& P, const DeltaChunks& C, int mode, int num_seqs, bool only_pass, cudaStream_t stream);
 
 }  // namespace b200
