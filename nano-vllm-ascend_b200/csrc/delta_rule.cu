@@ -60,6 +60,7 @@ delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
   const int s = ORDER ? sequence_of_rank(P.cu_q, gridDim.z, blockIdx.z) : blockIdx.z, h = blockIdx.y;
   SeqSpan sp = seq_span(P.cu_q, P.cu_k, P.ctx_lens, s);
   if (sp.q_len == 0) return;
+  const bool has_past = sp.first_pos() > 0;          // (of the whole span: below, it may be cut to a pass)
   bool goes_on = false, ends = true;                 // from the pass before, with the span
   if constexpr (REST > 0) {                          // (the scan has set the flag of the span's first record in the pass)
     const int before = chunks_before(P.cu_q, s), n = chunks_of(sp.q_len);
@@ -88,7 +89,7 @@ delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
   float* slot = P.state != nullptr
                     ? P.state + (((int64_t)P.state_slots[s] * P.H + h) * kdim) * (int64_t)vdim
                     : nullptr;
-  bool carried = slot != nullptr && sp.first_pos() > 0;
+  bool carried = slot != nullptr && has_past;
   if constexpr (REST == 2) {
     if (P.state == nullptr && !(ends && !goes_on)) slot = chunk_state(P, C, s, h);
     carried = carried || goes_on;

@@ -177,6 +177,42 @@ def test_heads_left_to_tokens(H, G, N, what, passes):
             assert torch.equal(out[150:, cols], clean[150:, cols]) and torch.equal(state[1, h], clean_state[1, h])
 
 
+@pytest.mark.parametrize("H,G,N", [(4, 2, 128), (8, 4, 64)])
+@pytest.mark.parametrize("with_state,past", [(True, [0, 0]), (True, [3, 5])])
+@pytest.mark.parametrize("room", [4, 1])
+def test_a_sequence_that_ends_and_one_that_goes_on_in_one_pass(H, G, N, with_state, past, room):
+    """Two sequences of six chunks in passes of four (or one): the second pass ends the first and has the start of the other. Heads of the first, of
+    the other, of both and of neither are left to tokens in that pass. A slot's earlier content is nothing to a sequence without a past. What a
+    chunk does is as near to 64 bits as the token form: 2.5e-7 at most each, their difference below 1e-6."""
+    from nanovllm import _C
+    lens = [330, 330]
+    q, k, v, gate, beta, g = _inputs(lens, H, G, N, False)
+    marks = gate.view(660, H, N)                            # (a decay of two is not for chunks)
+    each = H // 4
+    marks[4 * 64 + 10, 0 * each:1 * each, 5] = 2.0
+    marks[330 + 20, 1 * each:2 * each, 5] = 2.0
+    marks[4 * 64 + 10, 2 * each:3 * each, 5] = 2.0
+    marks[330 + 20, 2 * each:3 * each, 5] = 2.0
+    first = torch.randn(2, H, N, N, device="cuda", generator=g)
+    spans, slots = _spans(lens, past), torch.arange(2, dtype=torch.int32, device="cuda") if with_state else None
+    whole = _C.load().b200_delta_rule_workspace_size(2, 330, 660, H, G, N, N, 0, 0)
+    carry, chunks = H * N * N * 4, 660 // 64 + 2
+    state, tokens = (first.clone(), first.clone()) if with_state else (None, None)
+    for _ in range(3):
+        if with_state:
+            state.copy_(first)
+        out = _call("step", q, k, v, gate, beta, spans, H, G, N, state, slots, carry + (whole - carry) // chunks * room)
+    ref = _call("tokens", q, k, v, gate, beta, spans, H, G, N, tokens, slots)
+    for h in range(H):
+        cols = slice(h * N, (h + 1) * N)
+        for rows in (slice(0, 256), slice(256, 330), slice(330, 458), slice(458, 660)):
+            assert _off(out[rows, cols], ref[rows, cols].to(F64)) < 1e-6, (h, rows)
+        if with_state:
+            for s in range(2):
+                assert _off(state[s, h], tokens[s, h].to(F64)) < 1e-6, (h, s)
+    assert not torch.equal(out, ref)
+
+
 def test_a_wait_that_runs_out_is_reported(monkeypatch):
     from types import SimpleNamespace
 
