@@ -606,19 +606,18 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
 
   const int c = (warp & 3) * 32 + lane, half = warp >> 2, hh = NH == 2 ? (c >> 6) : 0;
   float S[D / 2];                                        // S[n][c], n = half * D / 2 + i
-  float* mine = nullptr;
+  const int64_t own = (int64_t)half * (D / 2) * D + (c & (D - 1));     // of a state [D, D]
   bool odd = false;
   if (warp < 8) {
 #pragma unroll
     for (int i = 0; i < D / 2; ++i) S[i] = 0.f;
-    if (P.state != nullptr || !(first_pass && last_pass)) mine = chunk_state(P, DP.c, s, h0 + hh) + (int64_t)half * (D / 2) * D + (c & (D - 1));
     if (first_pass ? P.state != nullptr && sp.first_pos() > 0 : true) {
+      const float* from = chunk_state_in(P, DP.c, s, h0 + hh) + own;
 #pragma unroll
-      for (int i = 0; i < D / 2; ++i) S[i] = mine[i * D];
+      for (int i = 0; i < D / 2; ++i) S[i] = from[i * D];
 #pragma unroll
       for (int i = 0; i < D / 2; ++i) odd = odd || magnitude(S[i]) >= kBig;
     }
-    if (P.state == nullptr && last_pass) mine = nullptr;
   }
   for (int j = threadIdx.x; j < chunks * NH; j += kDsThreads)
     odd = odd || *reinterpret_cast<const int*>(records + (int64_t)(j / NH) * step + (j % NH) * DP.c.bytes + R::kFlagAt) != 0;
@@ -746,9 +745,10 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
       umma::fence_before_sync();
       mbar_arrive(uo_read);
     }
-    if (mine != nullptr) {
+    if (P.state != nullptr || !last_pass) {
+      float* to = chunk_state_out(P, DP.c, s, h0 + hh) + own;
 #pragma unroll
-      for (int i = 0; i < D / 2; ++i) mine[i * D] = S[i];
+      for (int i = 0; i < D / 2; ++i) to[i * D] = S[i];
     }
   } else {
     const uint32_t id_e = umma::make_idesc<T>(128, 128, 0, 1), id_d = umma::make_idesc<T>(128, D, 0, 1);
@@ -894,11 +894,17 @@ static int delta_chunks_launch_as(DcParams DP, int mode, int64_t total_q, int64_
   if (allowed != cudaSuccess) return (int)allowed;
   const DeltaParams& P = DP.d;
   const int64_t chunks = dc_chunks(DP.num_seqs, total_q), record = DcRecord<D>::kBytes, carry = (int64_t)P.H * D * D * 4;
-  const int64_t room = (bytes - carry) / (record * P.H), passes = (chunks + room - 1) / room, count = (chunks + passes - 1) / passes;
+  int64_t room = (bytes - carry) / (record * P.H);
+  const bool two = P.state == nullptr && room > 1 && room < chunks;      // two carried states, the second in the place of a part of a chunk
+  if (two) room = (bytes - 2 * carry) / (record * P.H);
+  const int64_t passes = (chunks + room - 1) / room, count = (chunks + passes - 1) / passes;
+  static_assert(D * D * 4 < DcRecord<D>::kBytes, "a second carried state leaves one chunk of two");
   DP.c.bytes = record, DP.c.flag_at = DcRecord<D>::kFlagAt, DP.c.count = (int)count;
-  DP.c.carry = reinterpret_cast<float*>(DP.c.records + count * record * P.H);
-  for (int64_t at = 0; at < chunks; at += count) {
+  float* const carried = reinterpret_cast<float*>(DP.c.records + count * record * P.H);
+  const int64_t other = two ? carry / 4 : 0;
+  for (int64_t at = 0, pass = 0; at < chunks; at += count, ++pass) {
     DP.c.first = (int)at;
+    DP.c.carry_in = carried + (pass & 1 ? 0 : other), DP.c.carry_out = carried + (pass & 1 ? other : 0);
     launch_pdl(chunk, dim3((unsigned)(count * P.H)), dim3(kDcThreads), (size_t)chunk_smem, stream, DP);
     launch_pdl(scan, dim3((unsigned)(P.H / NH), (unsigned)DP.num_seqs), dim3(kDsThreads), (size_t)scan_smem, stream, DP);
     const int code = delta_rest_launch(P, DP.c, mode, DP.num_seqs, count >= chunks, stream);

@@ -90,16 +90,17 @@ delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
                     ? P.state + (((int64_t)P.state_slots[s] * P.H + h) * kdim) * (int64_t)vdim
                     : nullptr;
   bool carried = slot != nullptr && has_past;
+  const float* from = slot;
   if constexpr (REST == 2) {
-    if (P.state == nullptr && !(ends && !goes_on)) slot = chunk_state(P, C, s, h);
-    carried = carried || goes_on;
+    if (goes_on) from = chunk_state_in(P, C, s, h), carried = true;
+    if (P.state == nullptr && !ends) slot = chunk_state_out(P, C, s, h);
   }
 #pragma unroll
   for (int r = 0; r < KPT; ++r) {
     const int i = ksl * KPT + r;
 #pragma unroll
     for (int c = 0; c < NC; ++c)
-      S[c][r] = (carried && col + c < vdim && i < kdim) ? slot[(int64_t)i * vdim + col + c] : 0.f;
+      S[c][r] = (carried && col + c < vdim && i < kdim) ? from[(int64_t)i * vdim + col + c] : 0.f;
   }
   const float* q = P.q + (int64_t)grp * kdim;
   const float* k = P.k + (int64_t)grp * kdim;
@@ -249,7 +250,7 @@ delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
       }
     }
   }
-  if (slot != nullptr && (REST != 2 || P.state != nullptr || !ends)) {
+  if (slot != nullptr) {
 #pragma unroll
     for (int r = 0; r < KPT; ++r) {
       const int i = ksl * KPT + r;

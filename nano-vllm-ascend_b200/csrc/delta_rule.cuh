@@ -22,8 +22,12 @@ struct DeltaParams {
 // `count`; a (chunk, head) of the pass in hand has a record in the workspace.
 constexpr int kDcL = 64;                               // tokens per chunk
 struct DeltaChunks {
-  uint8_t* records;                                    // [count][H] of `bytes` each, then one state [H, kdim, vdim] fp32
-  float* carry;                                        // the state of a sequence that goes on in the next pass, where the caller keeps none
+  uint8_t* records;                                    // [count][H] of `bytes` each, then the two below
+  // Where the caller keeps no state, [H, kdim, vdim] fp32 of the sequence that came into this pass from the one before, and of the one that goes
+  // on into the next. Two places, for these may be two sequences whose CTAs (and launches, where a head is left aside) run in any order;
+  // one where a pass is a chunk, and so of one sequence
+  const float* carry_in;
+  float* carry_out;
   int64_t bytes;
   int first, count;                                    // the pass
   int flag_at;                                         // where a record says that its head's tokens are to be taken one at a time
@@ -38,10 +42,14 @@ __device__ __forceinline__ int chunks_before(const int* cu_q, int s) {
   for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
   return n;
 }
-// the state between spans of a pass and the next: the sequence's slot, or the one that is carried from pass to pass
-__device__ __forceinline__ float* chunk_state(const DeltaParams& P, const DeltaChunks& C, int s, int h) {
+// the state between spans of a pass and the next: the sequence's slot, or what is carried from pass to pass
+__device__ __forceinline__ const float* chunk_state_in(const DeltaParams& P, const DeltaChunks& C, int s, int h) {
   const int64_t size = (int64_t)P.kdim * P.vdim;
-  return P.state != nullptr ? P.state + ((int64_t)P.state_slots[s] * P.H + h) * size : C.carry + (int64_t)h * size;
+  return P.state != nullptr ? P.state + ((int64_t)P.state_slots[s] * P.H + h) * size : C.carry_in + (int64_t)h * size;
+}
+__device__ __forceinline__ float* chunk_state_out(const DeltaParams& P, const DeltaChunks& C, int s, int h) {
+  const int64_t size = (int64_t)P.kdim * P.vdim;
+  return P.state != nullptr ? P.state + ((int64_t)P.state_slots[s] * P.H + h) * size : C.carry_out + (int64_t)h * size;
 }
 
 // Bytes of workspace that the chunks would like for a step (0: such a step is not for them), and what they do with them: as many passes

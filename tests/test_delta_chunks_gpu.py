@@ -178,8 +178,8 @@ def test_heads_left_to_tokens(H, G, N, what, passes):
 
 
 @pytest.mark.parametrize("H,G,N", [(4, 2, 128), (8, 4, 64)])
-@pytest.mark.parametrize("with_state,past", [(True, [0, 0]), (True, [3, 5])])
-@pytest.mark.parametrize("room", [4, 1])
+@pytest.mark.parametrize("with_state,past", [(False, [0, 0]), (True, [0, 0]), (True, [3, 5])])
+@pytest.mark.parametrize("room", [5, 1])                 # (three passes of four, or one chunk at a time)
 def test_a_sequence_that_ends_and_one_that_goes_on_in_one_pass(H, G, N, with_state, past, room):
     """Two sequences of six chunks in passes of four (or one): the second pass ends the first and has the start of the other. Heads of the first, of
     the other, of both and of neither are left to tokens in that pass. A slot's earlier content is nothing to a sequence without a past. What a
