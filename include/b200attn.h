@@ -62,9 +62,10 @@ const char* b200_error_string(int code);
 int64_t b200_launch_count(void);
 void b200_reset_launch_count(void);
 /* Waits inside the persistent grouped GEMM (b200_moe_gemm_*_umma), b200_linear_recurrence_step, b200_delta_rule_step and
- * b200_attn_generic_step on tensor-core prompts are bounded. When one runs out, the kernel returns without having written its output (a recurrence may have written part of its
- * state) and sets a word of page-locked host memory. b200_take_wait_status asks
- * and clears it: B200_ERR_WAIT or B200_OK, meaningful for kernels that the host has waited for. The same entry points ask it
+ * b200_attn_generic_step on tensor-core prompts are bounded. When one runs out, the kernel returns and sets a word of page-locked
+ * host memory. The GEMM and the attention have then left the tile's output unwritten; the recurrence and the delta rule may have
+ * written wrong outputs and states from there on. Whatever such a call wrote is to be discarded. b200_take_wait_status asks
+ * and clears the word: B200_ERR_WAIT or B200_OK, meaningful for kernels that the host has waited for. The same entry points ask it
  * first of all, so that a call after the failed one returns B200_ERR_WAIT. b200_wait_status_word: the word itself. */
 int b200_take_wait_status(void);
 int32_t* b200_wait_status_word(void);

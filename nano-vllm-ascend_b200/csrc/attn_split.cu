@@ -98,6 +98,12 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     return any;
   };
 
+  auto peers_gave_up = [&] {
+    bool any = false;
+    for (int p = 1; p < parts_met; ++p) any = any || ld_peer_int(smem_u32(const_cast<int*>(gave_up)), p) != 0;
+    return any;
+  };
+
   pdl_wait();
   // the last row tiles see the most keys: those of every (sequence, kv head) start first
   constexpr int ctas = SHARED ? kAsParts : 1;
@@ -324,7 +330,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
       cluster_arrive(), cluster_wait();
     }
     parts_met = parts;
-    ok = ok && part == 0 && wait(done, 0);
+    ok = ok && part == 0 && wait(done, 0) && !peers_gave_up();     // (a part whose wait ran out has left nothing to merge)
     if (SHARED && ok && parts > 1) {
       const float own = s_part[row];
 #pragma unroll
@@ -492,7 +498,7 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
     return;
   }
   parts_met = parts;
-  const bool plain = wild();
+  const bool plain = wild() && !*gave_up && !peers_gave_up();
   if (SHARED && parts > 1) cluster_arrive(), cluster_wait();
   if (!plain) return;
 
