@@ -273,10 +273,11 @@ attn_split_kernel(const __grid_constant__ AttnSplitParams AP) {
           m_all = fmaxf(m_all, ms[p]);
         }
         const bool far = fabsf(m_all) * c >= 65536.f && m_all != -INFINITY;
-        less = 0.f, l = 0.f, top = m_all * c;
+        // (a part's weights count from the ROUNDED m c: with a product fused into the difference its residual would stay in the factor)
+        less = 0.f, l = 0.f, top = __fmul_rn(m_all, c);
 #pragma unroll
         for (int p = 0; p < kAsParts; ++p) {
-          float f = ms[p] == -INFINITY ? 0.f : ex2_approx(ms[p] * c - top), none = 0.f;
+          float f = ms[p] == -INFINITY ? 0.f : ex2_approx(__fmul_rn(ms[p], c) - top), none = 0.f;
           if (far && ms[p] != -INFINITY) f = ms[p] - m_all, weights(f, none);
           if (p < parts) l = fmaf(ld_peer(smem_u32(s_l + row), p), f, l);
           s_part[p * kAsM + row] = f;
