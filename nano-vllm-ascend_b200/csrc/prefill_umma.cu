@@ -74,7 +74,8 @@ struct PrefillUmmaParams {
   // optional: scores capped by cap * tanh(scale * s / cap) (cap_pre = scale / cap; 0 = off), and a sink logit per
   // query head (fp32 [H], natural-log units) that joins the softmax denominator without a value
   float cap = 0.f, cap_pre = 0.f;
-  float2 cap_poly[4] = {};          // cap tanh(cap_pre x) = x (cap_poly[0] + x^2 (cap_poly[1] + ..)), each twice, as packed operations take it
+  float cap_short = -1.f;           // up to so many caps, cap tanh(cap_pre x) = x (cap_poly[0] + x^2 (cap_poly[1] + ..)); each twice, as
+  float2 cap_poly[4] = {};          // packed operations take it
   const float* sink = nullptr;
   int window = 0, keep_first = 0;   // window 0: every earlier key
   int chunk = 0;                    // chunk > 0: only keys of the row's own chunk (counted from position 0)
@@ -85,6 +86,12 @@ struct PrefillUmmaParams {
 };
 
 constexpr int kUBM = 128, kUBN = 128;
+
+// tanh(y) = y (1 + c1 y^2 + c2 y^4 + c3 y^6) up to y = kCapShortTo, off by 1.4e-10 at most: the minimax polynomial of its form (Remez exchange;
+// cutting the series off after as many terms would leave 1.5e-8). In fp32, scores are off by 3.1e-8 (caps of 4 and 30) to 3.8e-8 (0.7) on
+// average, like those of the long polynomial below (3.1e-8, 3.1e-8 and 3.9e-8)
+constexpr double kCapShort[4] = {1., -0.33333323867490996, 0.13331341300491710, -0.05277317222556861};
+constexpr float kCapShortTo = 0.17f;
 constexpr int kOrderSeqs = 256;     // sequences that a launch orders by length
 constexpr int kItems = 2;           // slots of work items: the one in hand and the next
 
@@ -548,7 +555,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // tanh of small arguments is a short odd polynomial: while every score of the warp's rows stays below 0.35 caps, it
         // replaces the ex2 and the reciprocal per score that otherwise bind this loop to the special-function unit (3 of
         // its 16 results per clock for each score instead of 1). Truncation: 1.2e-8 of the score at 0.35, with terms up to x^11; below
-        // 0.17 caps, where most scores are, 1.5e-8 with those up to x^7, whose five packed operations a pair are what the loop has
+        // 0.17 caps, where most scores are, four coefficients do (kCapShort), and their five packed operations a pair are what the loop has
         // most of otherwise (nine). The tests are warp-uniform (per-score selection would pay for both sides) and end with the first
         // tile that fails both. A capped maximum is the cap of the maximum: a tile without a mask needs no second search.
         // (12 ragged prompts of 37-1501 tokens, 32 heads of 64, cap 30: 232 us without polynomials, 162 with the long one, 145 with both.)
@@ -558,7 +565,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           most = fmaxf(mx, -row_min(sr)) * p.cap_pre;
           small = __all_sync(0xffffffffu, most <= 0.35f);
         }
-        if (small && __all_sync(0xffffffffu, most <= 0.17f)) {
+        if (small && __all_sync(0xffffffffu, most <= p.cap_short)) {
           const float2 a0 = p.cap_poly[0], a1 = p.cap_poly[1], a2 = p.cap_poly[2], a3 = p.cap_poly[3];
 #pragma unroll
           for (int c = 0; c < 128; c += 2) {
@@ -903,9 +910,11 @@ int prefill_umma_launch(void* out, const void* q, const void* k, const void* v,
   p.scale_log2 = scale * 1.4426950408889634f;
   if (softcap > 0.f) {
     p.cap = softcap, p.cap_pre = scale / softcap;
-    const double y2 = (double)p.cap_pre * p.cap_pre, y = (double)softcap * p.cap_pre;
-    const double series[4] = {y, -y * y2 / 3., y * y2 * y2 * (2. / 15.), -y * y2 * y2 * y2 * (17. / 315.)};
-    for (int i = 0; i < 4; ++i) p.cap_poly[i] = make_float2((float)series[i], (float)series[i]);
+    const double y2 = (double)scale / softcap * ((double)scale / softcap);
+    double power = scale;
+    for (int i = 0; i < 4; ++i, power *= y2) p.cap_poly[i] = make_float2((float)(kCapShort[i] * power), (float)(kCapShort[i] * power));
+    // (coefficients and squares of scores have to be normal numbers: others leave it to the long polynomial, whose powers are of the quotient)
+    if (scale >= 0x1p-20f && scale <= 0x1p20f && p.cap_pre >= 0x1p-14f && p.cap_pre <= 0x1p14f) p.cap_short = kCapShortTo;
   }
   p.sink = sink;
   p.window = window, p.keep_first = window > 0 ? keep_first : 0, p.chunk = chunk;

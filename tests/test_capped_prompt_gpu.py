@@ -139,3 +139,20 @@ def test_caps_on_either_side_of_both_polynomials(D, window, level, tiles):
         # a probability is rounded to 2^-11, a result to 2^-11; scores of 32 bits move a probability of e^60 in all by 60 * 2^-23
         assert float((got[at:at + n] - want).norm() / want.norm()) < 6e-4
         at += n
+
+
+@pytest.mark.parametrize("cap", [1e-8, 1e-4, 3e4, 1e9])
+def test_caps_of_any_size(cap):
+    """Scores of up to 0.15 caps, however small or large the cap is: its powers leave the range of 32 bits."""
+    from nanovllm import ops
+    g = torch.Generator().manual_seed(3)
+    n, H, G, D = 200, 2, 1, 64
+    q, k, v = (torch.randn(n, h, D, generator=g).bfloat16() for h in (H, G, G))
+    top = max(float((q[:, h].double() @ k[:, 0].double().T).abs().max()) for h in range(H))
+    q = (q * (0.15 * cap / (top * D ** -0.5))).bfloat16()
+    cu = torch.tensor([0, n], dtype=torch.int32).cuda()
+    got = ops.prefill_varlen_attn(q.cuda(), k.cuda(), v.cuda(), cu, cu, n, n, D ** -0.5, G, softcap=cap).cpu().to(F64)
+    want = _want(q, k, v, D ** -0.5, cap, None)
+    # scores up to 1.5e8: their spacing is 16, so that only the largest of a row counts, and near ties fall either way
+    assert bool(got.isfinite().all())
+    assert float(((got - want).abs().amax(1) > 3e-2).double().mean()) <= (0.02 if cap > 1e6 else 0.0)
