@@ -74,8 +74,9 @@ struct PrefillUmmaParams {
   // optional: scores capped by cap * tanh(scale * s / cap) (cap_pre = scale / cap; 0 = off), and a sink logit per
   // query head (fp32 [H], natural-log units) that joins the softmax denominator without a value
   float cap = 0.f, cap_pre = 0.f;
-  float cap_short = -1.f;           // up to so many caps, cap tanh(cap_pre x) = x (cap_poly[0] + x^2 (cap_poly[1] + ..)); each twice, as
-  float2 cap_poly[4] = {};          // packed operations take it
+  // up to cap_short caps, the short polynomial (kCapShort) times cap_scale = cap * cap_pre. (The kernel makes its coefficients of these: 32 bytes of
+  // them among the arguments cost every call 0.5 us of host time, 15.6 for 15.1)
+  float cap_scale = 0.f, cap_short = -1.f;
   const float* sink = nullptr;
   int window = 0, keep_first = 0;   // window 0: every earlier key
   int chunk = 0;                    // chunk > 0: only keys of the row's own chunk (counted from position 0)
@@ -566,7 +567,8 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           small = __all_sync(0xffffffffu, most <= 0.35f);
         }
         if (small && __all_sync(0xffffffffu, most <= p.cap_short)) {
-          const float2 a0 = p.cap_poly[0], a1 = p.cap_poly[1], a2 = p.cap_poly[2], a3 = p.cap_poly[3];
+          const float y2 = p.cap_pre * p.cap_pre, b0 = p.cap_scale, b1 = b0 * y2, b2 = b1 * y2;
+          const float2 a0 = both(b0), a1 = both((float)kCapShort[1] * b1), a2 = both((float)kCapShort[2] * b2), a3 = both((float)kCapShort[3] * (b2 * y2));
 #pragma unroll
           for (int c = 0; c < 128; c += 2) {
             const float2 x = score_pair(sr, c), x2 = mul2(x, x);
@@ -910,11 +912,8 @@ int prefill_umma_launch(void* out, const void* q, const void* k, const void* v,
   p.scale_log2 = scale * 1.4426950408889634f;
   if (softcap > 0.f) {
     p.cap = softcap, p.cap_pre = scale / softcap;
-    const double y2 = (double)scale / softcap * ((double)scale / softcap);
-    double power = scale;
-    for (int i = 0; i < 4; ++i, power *= y2) p.cap_poly[i] = make_float2((float)(kCapShort[i] * power), (float)(kCapShort[i] * power));
     // (coefficients and squares of scores have to be normal numbers: others leave it to the long polynomial, whose powers are of the quotient)
-    if (scale >= 0x1p-20f && scale <= 0x1p20f && p.cap_pre >= 0x1p-14f && p.cap_pre <= 0x1p14f) p.cap_short = kCapShortTo;
+    if (scale >= 0x1p-20f && scale <= 0x1p20f && p.cap_pre >= 0x1p-14f && p.cap_pre <= 0x1p14f) p.cap_scale = scale, p.cap_short = kCapShortTo;
   }
   p.sink = sink;
   p.window = window, p.keep_first = window > 0 ? keep_first : 0, p.chunk = chunk;
