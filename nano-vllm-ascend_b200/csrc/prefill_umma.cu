@@ -563,7 +563,7 @@ prefill_umma_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         float most = 0.f;
         if (small) {
           mx = row_max(sr);
-          most = fmaxf(mx, -row_min(sr)) * p.cap_pre;
+          most = fmaxf(mx, -row_min(sr)) * fabsf(p.cap_pre);
           small = __all_sync(0xffffffffu, most <= 0.35f);
         }
         if (small && __all_sync(0xffffffffu, most <= p.cap_short)) {

@@ -156,3 +156,15 @@ def test_caps_of_any_size(cap):
     # scores up to 1.5e8: their spacing is 16, so that only the largest of a row counts, and near ties fall either way
     assert bool(got.isfinite().all())
     assert float(((got - want).abs().amax(1) > 3e-2).double().mean()) <= (0.02 if cap > 1e6 else 0.0)
+
+
+@pytest.mark.parametrize("scale", [-0.125, -0.004])
+def test_a_negative_scale(scale):
+    """Scores far beyond the polynomials' range, and within: what decides is their size, whatever the sign."""
+    from nanovllm import ops
+    g = torch.Generator().manual_seed(4)
+    n, H, G, D = 200, 2, 1, 64
+    q, k, v = (torch.randn(n, h, D, generator=g).half() * s for h, s in ((H, 4.0), (G, 1.0), (G, 1.0)))
+    cu = torch.tensor([0, n], dtype=torch.int32).cuda()
+    got = ops.prefill_varlen_attn(q.cuda(), k.cuda(), v.cuda(), cu, cu, n, n, scale, G, softcap=5.0).cpu().to(F64)
+    assert float((got - _want(q, k, v, scale, 5.0, None)).abs().max()) < 4e-3
