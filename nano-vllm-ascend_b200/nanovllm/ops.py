@@ -1243,6 +1243,16 @@ def wkv(r, k, v, decay, bonus, spans: StepSpans, num_heads, kdim, vdim, state=No
     return _fp32_state_rule(2, r, k, v, decay, bonus, spans, num_heads, num_heads, kdim, vdim, state, state_slots)
 
 
+def _lent(need, device):
+    """`need` bytes to work in, or what there is: a quarter, a sixteenth, .. (more passes), down to a MB. None: nothing is left."""
+    while need >= 1 << 20:
+        try:
+            return torch.empty(need, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            need //= 4
+    return None
+
+
 def _fp32_state_rule(mode, q, k, v, g, beta, spans: StepSpans, num_heads, groups, kdim, vdim, state, state_slots):
     _need_cuda(q, k, v, g, beta, state, state_slots)
     _f32(g, beta, state)
@@ -1265,12 +1275,12 @@ def _fp32_state_rule(mode, q, k, v, g, beta, spans: StepSpans, num_heads, groups
         # are, and short enough to notice the question)
         lib, dtype = _C.load(), _dt3(v)
         need = lib.b200_delta_rule_workspace_size(spans.num_seqs, spans.max_q, T, num_heads, groups, kdim, vdim, mode, dtype)
-        if need > 0:
-            workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
+        workspace = _lent(need, q.device) if need > 0 else None
+        if workspace is not None:
             _C.check(lib.b200_delta_rule_step(out.data_ptr(), q.data_ptr(), stride(q), k.data_ptr(), stride(k), v.data_ptr(),
                                               stride(v), g.data_ptr(), beta.data_ptr(), _ptr(state), _ptr(state_slots),
                                               cu_q, cu_k, ctx, spans.num_seqs, spans.max_q, T, num_heads, groups, kdim, vdim, mode,
-                                              dtype, workspace.data_ptr(), need, _stream()), "b200_delta_rule_step")
+                                              dtype, workspace.data_ptr(), workspace.numel(), _stream()), "b200_delta_rule_step")
             return out
     _C.check(_C.load().b200_delta_rule(out.data_ptr(), q.data_ptr(), stride(q), k.data_ptr(), stride(k), v.data_ptr(),
                                        stride(v), g.data_ptr(), beta.data_ptr(), _ptr(state), _ptr(state_slots),

@@ -255,3 +255,25 @@ def test_a_first_call_in_a_captured_graph():
         a.copy_(b)
     graph.replay()
     assert torch.equal(out, ops.delta_rule(*other[:5], spans, H, G, N, N))
+
+
+@pytest.mark.parametrize("free", [1 << 40, 12 << 20, 3 << 20, 0])
+def test_what_memory_there_is(monkeypatch, free):
+    """Where the workspace that a step would like is not to be had, it takes several passes (the same bits), and without any goes token by token."""
+    from nanovllm import ops
+    H, G, N, lens = 4, 2, 128, [500, 129, 700]
+    q, k, v, gate, beta, _ = _inputs(lens, H, G, N, False)
+    spans, empty, asked = _spans(lens, [0, 0, 0]), torch.empty, []
+    want = ops.delta_rule(q, k, v, gate, beta, spans, H, G, N, N)
+
+    def short(*size, **kw):
+        if kw.get("dtype") == torch.uint8:
+            asked.append(size[0])
+            if size[0] > free:
+                raise torch.OutOfMemoryError("CUDA out of memory")
+        return empty(*size, **kw)
+    with monkeypatch.context() as m:
+        m.setattr(torch, "empty", short)
+        got = ops.delta_rule(q, k, v, gate, beta, spans, H, G, N, N)
+    assert (len(asked) == 1) == (free > 1 << 30)
+    assert torch.equal(got, want if free else _call("tokens", q, k, v, gate, beta, spans, H, G, N, None, None))
