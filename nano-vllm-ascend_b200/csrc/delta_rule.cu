@@ -60,13 +60,13 @@ delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
   const int s = ORDER ? sequence_of_rank(P.cu_q, gridDim.z, blockIdx.z) : blockIdx.z, h = blockIdx.y;
   SeqSpan sp = seq_span(P.cu_q, P.cu_k, P.ctx_lens, s);
   if (sp.q_len == 0) return;
-  const bool has_past = sp.first_pos() > 0;          // (of the whole span: below, it may be cut to a pass)
-  bool goes_on = false, ends = true;                 // from the pass before, with the span
+  bool has_past = false, goes_on = false, ends = true;   // earlier tokens than the step's; from the pass before, with the span
   if constexpr (REST > 0) {                          // (the scan has set the flag of the span's first record in the pass)
     const int before = chunks_before(P.cu_q, s), n = chunks_of(sp.q_len);
     const int lo = REST == 1 ? 0 : max(0, C.first - before), hi = REST == 1 ? n : min(n, C.first + C.count - before);
     if (lo >= hi || *reinterpret_cast<const int*>(C.records + ((int64_t)(before + lo - C.first) * P.H + h) * C.bytes + C.flag_at) == 0) return;
     if (REST == 2) {
+      has_past = sp.first_pos() > 0;                 // (of the whole span, which is cut to the pass)
       goes_on = lo > 0, ends = hi == n;
       sp.q_start += lo * kDcL, sp.q_len = min(sp.q_len, hi * kDcL) - lo * kDcL;
     }
@@ -89,7 +89,7 @@ delta_rule_kernel(const DeltaParams P, const DeltaChunks C) {
   float* slot = P.state != nullptr
                     ? P.state + (((int64_t)P.state_slots[s] * P.H + h) * kdim) * (int64_t)vdim
                     : nullptr;
-  bool carried = slot != nullptr && has_past;
+  bool carried = slot != nullptr && (REST == 2 ? has_past : sp.first_pos() > 0);
   const float* from = slot;
   if constexpr (REST == 2) {
     if (goes_on) from = chunk_state_in(P, C, s, h), carried = true;
