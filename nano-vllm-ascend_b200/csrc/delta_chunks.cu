@@ -20,7 +20,10 @@
 // delta_scan_kernel, one CTA per (sequence, 128 value channels = one head of 128 or two of 64), S^T in fp32 registers:
 //   E^T = S0^T [W; P q - Y]^T    M128 (channels) N128 K = D, S0 in three terms from tensor memory, in two halves of its rows
 //   w -> three terms; o out;  dS^T = w^T (P_end / P_j k_j)    M128 N = D K64;   S = P_end S + dS in registers.
-// Every fp32 operand is three bf16 terms by cutting off (24 bits, exact), six products, small ones first; values are bf16 as they are.
+// Every fp32 operand is three bf16 terms (24 bits, exact), six products, small ones first; values are bf16 as they are. One operand of every
+// product is split by rounding: where both are by cutting off, the three products left out have one sign and lack 6e-8 on average.
+// Outputs are 0.8 to 0.98 times as far from 64 bits as the token form's, states 0.4 to 1.15 times, where the last token is nearly all of a
+// state 1.4 (test_no_precision_is_lost; the inputs of 16 prompts below: 2.0e-7 of either).
 //
 // What bounds them, 16 prompts of 500-1300 tokens, 8 heads of 128 (delta_rule_kernel 650 us): delta_chunk_kernel 205, a CTA's phases behind
 // one another (loads, scores, substitution, products, 48000 cycles, of which 11000 are issue); delta_scan_kernel 106, the chain
@@ -81,11 +84,9 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint3
                "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
-// The tensor core cuts a sum off after every 16 products; on average results lack this part of them. Measured as the mean relative difference
-// from 64-bit products of random operands, for each product as it is summed here. Added back,
-// in fp32: outputs 2.6e-7 -> 2.2e-7 off, states 2.2e-7 -> 1.9e-7, where the token form is 2.2e-7 and 2.0e-7 off (the case above).
-constexpr float kCutY = 0.9e-7f, kCutScore = 0.45e-7f, kCutW = 0.42e-7f, kCutU = 0.5e-7f, kCutO = 0.6e-7f, kCutE = 1.0e-7f, kCutD = 0.75e-7f;
-__device__ __forceinline__ float uncut(uint32_t x, float part) { return fmaf(__uint_as_float(x), part, __uint_as_float(x)); }
+// The tensor core cuts a sum off where fp32 arithmetic rounds it: half a unit of the last place is lost on average, ln 2 / 2 x 2^-23 of a number. It is
+// given back where the sum meets another number or is split in terms (alone, 24 bits could not hold it).
+constexpr float kCut = 4.13e-8f;
 __device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 __device__ __forceinline__ float largest(float most, float2 x) {             // of |x|; NaN stays
   asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(most) : "f"(fabsf(x.x)), "f"(fabsf(x.y)));
@@ -95,6 +96,33 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   float2 r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(r)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
   return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(r)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(reinterpret_cast<uint64_t&>(c)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+  return c;
+}
+__device__ __forceinline__ float2 both(uint32_t x, uint32_t y) { return make_float2(__uint_as_float(x), __uint_as_float(y)); }
+// split3x2 (each term the rounding of what those before leave) of x (1 + part)
+__device__ __forceinline__ void split3more(float2 x, float2 part, uint32_t (&w)[3]) {
+  float2 r = x;
+  const float2 less = make_float2(-1.f, -1.f);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    if (i == 2) r = fma2(x, part, r);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(r.y), "f"(r.x));
+    if (i < 2) r = fma2(both(w[i] << 16, w[i] & 0xffff0000u), less, r);
+  }
+}
+// 1 / x to within a unit: an approximation, and Newton's step from it
+__device__ __forceinline__ float rcp_newton(float x) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(fmaf(-x, r, 1.f), r, r);
 }
 constexpr uint32_t kBig = (127u + 60u) << 23, kSmall = (127u - 60u) << 23, kTwo = 128u << 23;
 constexpr float kFar = 0x1p90f, kNear = 0x1p-90f;
@@ -235,21 +263,16 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
       most_k = largest(most_k, kk[x]), most_q = largest(most_q, qq[x]);
       if (!PER_HEAD) most_g = largest(most_g, gg[x]);
     }
-    // the decay between a token and the chunk's middle, between tokens 31 and 32: of this warp's nearest token `f`, of its farthest 1 / `r`
-    float2 f = one, r = one;
+    // the decay between a token and the chunk's middle, between tokens 31 and 32: of this warp's nearest tokens `f`
+    float2 f = one;
     if (!PER_HEAD) {
-      float2 but = one;                                  // of the tokens but the nearest (before the middle) or the first (behind it)
-      const bool first = warp < 4;
+      float2 all = gg[0];
 #pragma unroll
-      for (int x = 1; x < 8; ++x) but = mul2(but, gg[x]);
-      const float2 all = mul2(but, gg[0]);
+      for (int x = 1; x < 8; ++x) all = mul2(all, gg[x]);
       float2* tau = reinterpret_cast<float2*>(s_tau + half * 512) + lane;      // [8][32] pairs
       tau[warp * 32] = all;
       __syncthreads();
-      for (int w = first ? warp + 1 : 4; w < (first ? 4 : warp); ++w) f = mul2(f, tau[w * 32]);
-      r = mul2(f, first ? but : all);
-      far = far || !(fabsf(r.x) >= kNear && fabsf(r.x) <= kFar && fabsf(r.y) >= kNear && fabsf(r.y) <= kFar);
-      r = make_float2(1.f / r.x, 1.f / r.y);
+      for (int w = warp < 4 ? warp + 1 : 4; w < (warp < 4 ? 4 : warp); ++w) f = mul2(f, tau[w * 32]);
     }
     if (half > 0) {                                      // the products of the channels before have read their operands
       alive = alive && wait(scored, half - 1);
@@ -271,7 +294,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     auto put_dn = [&](int x, float2 dn) {
       uint32_t c[3];
       const float2 kx = mul2(kk[x], dn);
-      split3cut(kx.x, kx.y, c);
+      split3x2(kx.x, kx.y, c);
       const uint32_t at = x * 128 + (((lane >> 2) ^ x) << 4);
 #pragma unroll
       for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(sKQ + 49152 + p * 8192 + at) = c[p];
@@ -279,28 +302,29 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     if (PER_HEAD) {
 #pragma unroll
       for (int x = 0; x < 8; ++x) put_up(x, one), put_dn(x, one);
-    } else if (warp < 4) {
-#pragma unroll
-      for (int x = 7; x >= 0; --x) {
-        put_dn(x, f);
-        f = mul2(f, gg[x]);
-      }
-#pragma unroll
-      for (int x = 0; x < 8; ++x) {
-        if (x > 0) r = mul2(r, gg[x]);
-        put_up(x, r);
-      }
     } else {
+      // (a token's two factors are one and its reciprocal: between tokens that are near each other, no rounding but those of the decays in between)
+      float near = 1.f, most = 1.f;
+      auto inverse = [&](float2 x) {
+        near = fminf(near, fminf(fabsf(x.x), fabsf(x.y))), most = fmaxf(most, fmaxf(fabsf(x.x), fabsf(x.y)));
+        return make_float2(rcp_newton(x.x), rcp_newton(x.y));
+      };
+      if (warp < 4) {
 #pragma unroll
-      for (int x = 0; x < 8; ++x) {
-        f = mul2(f, gg[x]);
-        put_up(x, f);
-      }
+        for (int x = 7; x >= 0; --x) {
+          put_dn(x, f);
+          put_up(x, inverse(f));
+          f = mul2(f, gg[x]);
+        }
+      } else {
 #pragma unroll
-      for (int x = 7; x >= 0; --x) {
-        put_dn(x, r);
-        r = mul2(r, gg[x]);
+        for (int x = 0; x < 8; ++x) {
+          f = mul2(f, gg[x]);
+          put_up(x, f);
+          put_dn(x, inverse(f));
+        }
       }
+      far = far || !(near >= kNear && most <= kFar);
     }
     if (!PER_HEAD && __any_sync(0xffffffffu, far) && lane == 0) *s_far = 1;
     fence_proxy_async_smem();
@@ -347,9 +371,9 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
         umma::wait_ld();
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
-          float sum = __uint_as_float(y[0][c]) + __uint_as_float(y[1][c]);
-          if (D == 128) sum += __uint_as_float(y[D / 32 - 2][c]) + __uint_as_float(y[D / 32 - 1][c]);
-          w[c0 + c] = __float_as_uint(fmaf(sum, kCutScore, sum));
+          float a = __uint_as_float(y[0][c]), b = __uint_as_float(y[1][c]);
+          if (D == 128) a += b, b = __uint_as_float(y[D / 32 - 2][c]) + __uint_as_float(y[D / 32 - 1][c]);
+          w[c0 + c] = __float_as_uint(a + fmaf(a + b, kCut, b));
         }
       }
 #pragma unroll
@@ -453,8 +477,8 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
       else p = make_float2(s_p[t], s_p[t]), to_end[x] = make_float2(s_e[t], s_e[t]);
       uint32_t a[3], b[3];
       const float2 kp = mul2(kk[x], p), kend = mul2(kk[x], to_end[x]);
-      split3cut(kp.x, kp.y, a);
-      split3cut(kend.x, kend.y, b);
+      split3x2(kp.x, kp.y, a);
+      split3x2(kend.x, kend.y, b);
       const uint32_t at = half * 8192 + e * 1024 + x * 128 + (((lane >> 2) ^ x) << 4);
 #pragma unroll
       for (int y = 0; y < 3; ++y) {
@@ -510,12 +534,14 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     const int n0 = side * (D / 2) + c0;
     float x[16];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) x[c] = uncut(w[c], quarter >= 2 ? kCutY : kCutW);
+    for (int c = 0; c < 16; ++c) x[c] = __uint_as_float(w[c]);
+    const float part = quarter >= 2 ? 0.f : kCut;
     if (quarter >= 2) {
 #pragma unroll
       for (int c = 0; c < 16; c += 4) {
         const float4 qs = *reinterpret_cast<const float4*>(sQs + i * M::kQRow + n0 + c);
-        x[c] = qs.x - x[c], x[c + 1] = qs.y - x[c + 1], x[c + 2] = qs.z - x[c + 2], x[c + 3] = qs.w - x[c + 3];
+        x[c] = fmaf(x[c], -kCut, qs.x) - x[c], x[c + 1] = fmaf(x[c + 1], -kCut, qs.y) - x[c + 1];
+        x[c + 2] = fmaf(x[c + 2], -kCut, qs.z) - x[c + 2], x[c + 3] = fmaf(x[c + 3], -kCut, qs.w) - x[c + 3];
       }
     }
     // rows of the record run along r: a lane gets its neighbour's value of one of two channels and writes the pair, in row n0 + c + odd
@@ -524,7 +550,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     for (int c = 0; c < 16; c += 2) {
       const float other = __shfl_xor_sync(0xffffffffu, odd ? x[c] : x[c + 1], 1);
       uint32_t y[3];
-      split3cut(odd ? other : x[c], odd ? x[c + 1] : other, y);
+      split3more(make_float2(odd ? other : x[c], odd ? x[c + 1] : other), make_float2(part, part), y);
       uint8_t* to = record + (at + c * 128 + (group ^ ((c & 6) << 4)));
 #pragma unroll
       for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(to + p * (2 * D * 128)) = y[p];
@@ -553,7 +579,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     umma::wait_ld();
     float* to = reinterpret_cast<float*>(record + (uo + c0 * R::kUoRow * 4));
 #pragma unroll
-    for (int c = 0; c < 16; ++c) to[c * R::kUoRow] = uncut(w[c], quarter >= 2 ? kCutO : kCutU);
+    for (int c = 0; c < 16; ++c) to[c * R::kUoRow] = __uint_as_float(w[c]);
   }
   umma::fence_before_sync();
   if (*gave_up) {                                        // products under way finish before the columns and the operands go
@@ -643,6 +669,7 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
     const int64_t out_stride = (int64_t)P.H * D;
     float* out = P.out + (int64_t)h0 * D + c;
     const float4* uo = reinterpret_cast<const float4*>(sUo + c * (R::kUoRow * 4));
+    const float2 part = make_float2(kCut, kCut);
     auto update = [&](int j, int piece) {                // a half of this thread's rows of S after chunk j - 1
       const float* pe = sPe + ((j - 1) & 1) * (NH * D) + hh * D + half * (D / 2);
 #pragma unroll
@@ -653,10 +680,12 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
 #pragma unroll
         for (int i = 0; i < 16; i += 4) {
           const float4 p = *reinterpret_cast<const float4*>(pe + i0 + i);
-          S[i0 + i] = fmaf(p.x, S[i0 + i], uncut(w[i], kCutD));
-          S[i0 + i + 1] = fmaf(p.y, S[i0 + i + 1], uncut(w[i + 1], kCutD));
-          S[i0 + i + 2] = fmaf(p.z, S[i0 + i + 2], uncut(w[i + 2], kCutD));
-          S[i0 + i + 3] = fmaf(p.w, S[i0 + i + 3], uncut(w[i + 3], kCutD));
+#pragma unroll
+          for (int y = 0; y < 4; y += 2) {
+            const float2 d = both(w[i + y], w[i + y + 1]);
+            const float2 r = add2(fma2(y ? make_float2(p.z, p.w) : make_float2(p.x, p.y), make_float2(S[i0 + i + y], S[i0 + i + y + 1]), mul2(d, part)), d);
+            S[i0 + i + y] = r.x, S[i0 + i + y + 1] = r.y;
+          }
         }
       }
     };
@@ -700,15 +729,14 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
         for (int i = 0; i < 4; ++i) x[i] = uo[half * 8 + 4 * u + i];
         umma::wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) e[i] = __float_as_uint(__uint_as_float(e[i]) + __uint_as_float(more[i]));
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint32_t y[3];
-          split3cut(x[i].x - uncut(e[4 * i], kCutE), x[i].y - uncut(e[4 * i + 1], kCutE), y);
-          w[0][2 * i] = y[0], w[1][2 * i] = y[1], w[2][2 * i] = y[2];
-          split3cut(x[i].z - uncut(e[4 * i + 2], kCutE), x[i].w - uncut(e[4 * i + 3], kCutE), y);
-          w[0][2 * i + 1] = y[0], w[1][2 * i + 1] = y[1], w[2][2 * i + 1] = y[2];
-        }
+          for (int z = 0; z < 4; z += 2) {
+            const float2 read_ = add2(both(e[4 * i + z], e[4 * i + z + 1]), both(more[4 * i + z], more[4 * i + z + 1]));
+            uint32_t y[3];
+            split3more(fma2(read_, make_float2(-1.f, -1.f), z ? make_float2(x[i].z, x[i].w) : make_float2(x[i].x, x[i].y)), part, y);
+            w[0][2 * i + z / 2] = y[0], w[1][2 * i + z / 2] = y[1], w[2][2 * i + z / 2] = y[2];
+          }
 #pragma unroll
         for (int p = 0; p < 3; ++p) umma::st8(base + kTmW + p * 32 + half * 16 + 8 * u, w[p]);
       }
@@ -732,7 +760,7 @@ delta_scan_kernel(const __grid_constant__ DcParams DP) {
         const float4 x = uo[16 + half * 8 + i / 4];
         const float o[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int y = 0; y < 4; ++y) read[i + y] = o[y] + fmaf(read[i + y], kCutE, read[i + y]);
+        for (int y = 0; y < 4; ++y) read[i + y] = o[y] + fmaf(o[y] + read[i + y], kCut, read[i + y]);
       }
       if (left >= 32) {
 #pragma unroll
