@@ -30,10 +30,12 @@
 // E -> w -> dS -> S -> E of 8500 cycles a chunk, 6000 of them for 72 MMAs. The records that pass between them (216 KB per chunk and head
 // of 128, written and read once) would take 2 x 63 at HBM's rate.
 //
+// Decays per channel that come to less than 2^-83 over half a chunk (0.17 a token) would take the reciprocals, or low terms, out of the range: a CTA
+// that meets them computes its scores in blocks of 16 tokens (dc_block_scores), for which no decay is too small.
+//
 // Not for chunks, and left to delta_rule_kernel, which runs behind them over the heads that a record flags: values that are not finite
 // (0 x inf would reach tokens before them) or beyond 2^60, decays of 2 and more, keys, queries or values all below 2^-60 (the low terms
-// would be lost), and decays per channel that come to less than 2^-90 over half a chunk (0.14 a token), or meet keys or queries from 2^30 on or all
-// below 2^-20, where a reciprocal or low terms would leave the range: a CTA with such decays leaves after their products.
+// would be lost), and, where scores go by reciprocals, keys or queries from 2^30 on or all below 2^-20.
 //
 // Waits are bounded (mbar_warp_wait): one that runs out makes its role leave, those that wait for it run out as well, the products under
 // way are waited for, the CTA sets the host's word and the library reports it.
@@ -125,8 +127,8 @@ __device__ __forceinline__ float rcp_newton(float x) {
   return fmaf(fmaf(-x, r, 1.f), r, r);
 }
 constexpr uint32_t kBig = (127u + 60u) << 23, kSmall = (127u - 60u) << 23, kTwo = 128u << 23;
-constexpr float kFar = 0x1p90f, kNear = 0x1p-90f;
-constexpr uint32_t kBigUp = (127u + 30u) << 23, kSmallDn = (127u - 20u) << 23;       // of what meets kFar and, in its third term, kNear: within 2^+-126
+constexpr float kNear = 0x1p-83f;                        // between eight tokens and the middle: with each of those, 2^-90 and more
+constexpr uint32_t kBigUp = (127u + 30u) << 23, kSmallDn = (127u - 20u) << 23;       // of what meets 2^90 and, in its third term, 2^-90: within 2^+-126
 
 constexpr int kDcThreads = 256;
 constexpr int kDcARow = 68;                              // floats of a row of A: 16-byte groups of eight rows in different banks
@@ -137,222 +139,279 @@ struct DcSmem {
   static constexpr int kA = kDcL * kDcARow * 4;          // A (then V)
   static constexpr int kQRow = D + 4;
   static constexpr int kQs = kDcL * kQRow * 4;           // P q
-  static constexpr int kAAt = kKb, kQsAt = kKb + kA, kEnd = kQsAt + kQs > kScores ? kQsAt + kQs : kScores;
+  static constexpr int kAAt = kKb, kQsAt = kKb + kA;
+  // strong decays: scores inside blocks of 16 tokens, [4 parts][16 i][4 groups of j][k, q][4 blocks][4 j], and, where A will be, their sum in rows of kBlockRow and
+  // [k, q][tokens 16-31, 48-63] those of the block before
+  static constexpr int kParts = 4 * 2 * kDcL * 16 * 4, kPartsAt = kScores, kBlockRow = 20, kBlocks = 2 * kDcL * kBlockRow * 4, kNear = kBlocks / 2;
+  static constexpr int kEnd = kQsAt + kQs > kPartsAt + kParts ? kQsAt + kQs : kPartsAt + kParts;
+  static_assert(kBlocks + kNear <= kA, "room for the blocks");
   static constexpr int kTau = (D / 64) * 8 * 64 * 4;     // decays of 8 tokens
   static constexpr int kBytes = 1024 + kEnd + kTau + 4 * 64 * 4 + 256;
 };
 
-template <int D, bool PER_HEAD>
-__global__ void __launch_bounds__(kDcThreads, 2)
-delta_chunk_kernel(const __grid_constant__ DcParams DP) {
-  using T = __nv_bfloat16;
-  using R = DcRecord<D>;
+// a CTA's shared memory
+template <int D>
+struct DcLocal {
   using M = DcSmem<D>;
-  const DeltaParams& P = DP.d;
-  extern __shared__ __align__(1024) uint8_t dc_smem_raw[];
-  uint8_t* smem = dc_smem_raw + (-smem_u32(dc_smem_raw) & 1023u);       // (not through an integer: the compiler has to know that it is shared memory)
-  float* sA = reinterpret_cast<float*>(smem + M::kAAt);
-  float* sQs = reinterpret_cast<float*>(smem + M::kQsAt);
-  float* s_tau = reinterpret_cast<float*>(smem + M::kEnd);             // [D / 64][8][64]
-  float* s_beta = s_tau + (D / 64) * 8 * 64;
-  float *s_g = s_beta + 64, *s_p = s_g + 64, *s_e = s_p + 64;          // one decay per head: of a token, P, P_end / P
-  uint64_t *scored = reinterpret_cast<uint64_t*>(s_e + 64), *made = scored + 1, *drained = made + 1;
-  uint32_t* s_max = reinterpret_cast<uint32_t*>(drained + 1);          // largest magnitudes: k, q, v, and what must stay below two
-  uint32_t* tmem_slot = s_max + 4;
-  int *s_far = reinterpret_cast<int*>(tmem_slot + 1), *s_where = s_far + 1, *s_next = s_where + 2;
-  volatile int* gave_up = s_next + 1;
+  uint8_t* at;
+  __device__ __forceinline__ DcLocal() {
+    extern __shared__ __align__(1024) uint8_t dc_smem_raw[];
+    at = dc_smem_raw + (-smem_u32(dc_smem_raw) & 1023u);               // (not through an integer: the compiler has to know that it is shared memory)
+  }
+  __device__ __forceinline__ float* A() const { return reinterpret_cast<float*>(at + M::kAAt); }
+  __device__ __forceinline__ float* Qs() const { return reinterpret_cast<float*>(at + M::kQsAt); }
+  __device__ __forceinline__ float* parts() const { return reinterpret_cast<float*>(at + M::kPartsAt); }
+  __device__ __forceinline__ float* tau() const { return reinterpret_cast<float*>(at + M::kEnd); }             // [D / 64][8][64]
+  __device__ __forceinline__ float* beta() const { return tau() + (D / 64) * 8 * 64; }
+  __device__ __forceinline__ float* g() const { return beta() + 64; }  // one decay per head: of a token, P, P_end / P
+  __device__ __forceinline__ float* p() const { return beta() + 128; }
+  __device__ __forceinline__ float* e() const { return beta() + 192; }
+  __device__ __forceinline__ uint64_t* scored() const { return reinterpret_cast<uint64_t*>(beta() + 256); }
+  __device__ __forceinline__ uint64_t* made() const { return scored() + 1; }
+  __device__ __forceinline__ uint64_t* drained() const { return scored() + 2; }
+  __device__ __forceinline__ uint32_t* max() const { return reinterpret_cast<uint32_t*>(scored() + 3); }       // largest magnitudes: k, q, v, and what must stay below two
+  __device__ __forceinline__ uint32_t* tmem_slot() const { return max() + 4; }
+  __device__ __forceinline__ int* where() const { return reinterpret_cast<int*>(max() + 5); }                  // two
+  __device__ __forceinline__ int* next() const { return where() + 2; }
+  __device__ __forceinline__ volatile int* gave_up() const { return where() + 3; }
+};
+constexpr uint32_t kTmSC = 0, kTmX = 128;                // scores of 64 channels each, then [W; Y] and [U; O0], 128 columns; X 3 x 32
 
-  pdl_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.x % P.H, lin = DP.c.first + blockIdx.x / P.H;
-  if (warp == 0) {                                       // the sequence of chunk `lin`
-    int base = 0, found = -1, at = 0;
-    for (int s0 = 0; s0 < DP.num_seqs && found < 0; s0 += 32) {
-      const int n = s0 + lane < DP.num_seqs ? chunks_of(P.cu_q[s0 + lane + 1] - P.cu_q[s0 + lane]) : 0;
-      int to = n;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, to, o);
-        if (lane >= o) to += up;
-      }
-      const uint32_t hit = __ballot_sync(0xffffffffu, lin < base + to);
-      if (hit != 0) {
-        const int l = __ffs(hit) - 1;
-        found = s0 + l, at = lin - base - __shfl_sync(0xffffffffu, to - n, l);
-      }
-      base += __shfl_sync(0xffffffffu, to, 31);
-    }
-    if (lane == 0) s_where[0] = found, s_where[1] = at;
-  }
-  if (threadIdx.x == 32) {
-    mbar_init(scored, 1), mbar_init(made, 1), mbar_init(drained, 1);
-    mbar_fence_init();
-    for (int i = 0; i < 4; ++i) s_max[i] = 0;
-    *s_far = 0, *s_next = 0, *gave_up = 0;
-  }
-  __syncthreads();
-  const int s = s_where[0], chunk = s_where[1];
-  if (s < 0) return;                                     // the grid has room for sequences that all end in a chunk of their own
-  if (warp == 1) umma::tmem_alloc(tmem_slot, 256);
-  const int64_t tok0 = P.cu_q[s] + chunk * kDcL;
-  const int nt = min(kDcL, P.cu_q[s + 1] - (int)tok0);
-  const int grp = h / (P.H / P.groups);
-  const float* q = P.q + tok0 * P.q_stride + (int64_t)grp * D;
-  const float* k = P.k + tok0 * P.k_stride + (int64_t)grp * D;
-  const float* g = P.g + tok0 * ((int64_t)P.H * (PER_HEAD ? 1 : D)) + (int64_t)h * (PER_HEAD ? 1 : D);
-  const int64_t g_stride = (int64_t)P.H * (PER_HEAD ? 1 : D);
-  const T* v = (const T*)P.v + tok0 * P.v_stride + (int64_t)h * D;
-  uint8_t* record = DP.c.records + ((int64_t)(lin - DP.c.first) * P.H + h) * DP.c.bytes;
-  const bool issuer = warp == 0 && umma::elect_one();
-  auto wait = [&](uint64_t* bar, int parity) { return mbar_warp_wait(bar, parity & 1, DP.wait_tries, gave_up); };
-
-  if (threadIdx.x < kDcL) {
-    const int t = threadIdx.x;
-    const float b = t < nt ? P.beta[(tok0 + t) * P.H + h] : 0.f;
-    s_beta[t] = b;
-    uint32_t most = magnitude(b);
-    if (PER_HEAD) {
-      const float d = t < nt ? g[t * g_stride] : 1.f;
-      s_g[t] = d;
-      most = max(most, magnitude(d));
-    }
-    most = __reduce_max_sync(0xffffffffu, most);
-    if (lane == 0) atomicMax(&s_max[3], most);
-  }
-  umma::fence_before_sync();
-  __syncthreads();
-  umma::fence_after_sync();
-  const uint32_t tb = *tmem_slot;
-  constexpr uint32_t kTmSC = 0, kTmX = 128;              // scores of 64 channels each, then [W; Y] and [U; O0], 128 columns; X 3 x 32
-  if (PER_HEAD && threadIdx.x < kDcL) {
-    float p = 1.f, e = 1.f;
-    for (int i = 0; i <= (int)threadIdx.x; ++i) p *= s_g[i];
-    for (int i = kDcL - 1; i > (int)threadIdx.x; --i) e *= s_g[i];
-    s_p[threadIdx.x] = p, s_e[threadIdx.x] = e;
-  }
-
-  // 8 tokens of two channels; rows are found by 32-bit offsets from the chunk's first
-  const uint32_t k_step = (uint32_t)P.k_stride * 4, q_step = (uint32_t)P.q_stride * 4, g_step = (uint32_t)g_stride * 4;
-  auto fetch = [&](int t0, int ch, float2 (&kk)[8], float2 (&qq)[8], float2 (&gg)[8]) {
-    auto rows = [&](auto all) {
-      uint32_t ka = t0 * k_step + ch * 4, qa = t0 * q_step + ch * 4, ga = t0 * g_step + ch * 4;
-#pragma unroll
-      for (int x = 0; x < 8; ++x) {
-        const bool ok = decltype(all)::value || t0 + x < nt;
-        kk[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(k) + ka) : make_float2(0.f, 0.f);
-        qq[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(q) + qa) : make_float2(0.f, 0.f);
-        if (!PER_HEAD) gg[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(g) + ga) : make_float2(1.f, 1.f);
-        ka += k_step, qa += q_step, ga += g_step;
-      }
-    };
-    if (t0 + 8 <= nt) rows(std::true_type{});
-    else rows(std::false_type{});
-  };
-  bool alive = true;
-  // ------------------------------------------------ scores, 64 channels at a time; a thread has two channels and 8 tokens
-  float most_k = 0.f, most_q = 0.f, most_g = 0.f;
-  bool far = false;
-  const float2 one = make_float2(1.f, 1.f);
-#pragma unroll 1
-  for (int half = 0; half < D / 64; ++half) {
-    const int ch = half * 64 + 2 * lane;
-    float2 kk[8], qq[8], gg[8];
-    fetch(8 * warp, ch, kk, qq, gg);
+// ---- scores
+struct DcTokens {                                        // a chunk's rows of a head: found by 32-bit offsets from the first
+  const float *k, *q, *g;
+  uint32_t k_step, q_step, g_step;
+  int nt;
+};
+struct DcChunk {                                         // and what a CTA knows once its scores are on their way
+  DcTokens t;
+  const __nv_bfloat16* v;
+  int64_t v_stride;
+  uint8_t* record;
+  uint32_t tb;                                           // its columns
+  int issued, wait_tries;                                // commits to `scored`
+  bool alive;
+  int* wait_status;
+  __device__ __forceinline__ bool wait(uint64_t* bar, int parity, volatile int* gave_up) const { return mbar_warp_wait(bar, parity & 1, wait_tries, gave_up); }
+};
+// 8 tokens of two channels
+template <bool PER_HEAD>
+__device__ __forceinline__ void dc_fetch(const DcTokens& C, int t0, int ch, float2 (&kk)[8], float2 (&qq)[8], float2 (&gg)[8]) {
+  auto rows = [&](auto all) {
+    uint32_t ka = t0 * C.k_step + ch * 4, qa = t0 * C.q_step + ch * 4, ga = t0 * C.g_step + ch * 4;
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
-      most_k = largest(most_k, kk[x]), most_q = largest(most_q, qq[x]);
-      if (!PER_HEAD) most_g = largest(most_g, gg[x]);
+      const bool ok = decltype(all)::value || t0 + x < C.nt;
+      kk[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(C.k) + ka) : make_float2(0.f, 0.f);
+      qq[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(C.q) + qa) : make_float2(0.f, 0.f);
+      if (!PER_HEAD) gg[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(C.g) + ga) : make_float2(1.f, 1.f);
+      ka += C.k_step, qa += C.q_step, ga += C.g_step;
     }
-    // the decay between a token and the chunk's middle, between tokens 31 and 32: of this warp's nearest tokens `f`
-    float2 f = one;
-    if (!PER_HEAD) {
-      float2 all = gg[0];
+  };
+  if (t0 + 8 <= C.nt) rows(std::true_type{});
+  else rows(std::false_type{});
+}
+// two channels of a token into row x of a group of eight rows of the operands: of K~ and Q~, of K^
+__device__ __forceinline__ void dc_put_up(uint8_t* group, int lane, int x, float2 kk, float2 qq, float2 up) {
+  uint32_t a[3], b[3];
+  const float2 kx = mul2(kk, up), qx = mul2(qq, up);
+  split3cut(kx.x, kx.y, a);
+  split3cut(qx.x, qx.y, b);
+  const uint32_t at = x * 128 + (((lane >> 2) ^ x) << 4);
 #pragma unroll
-      for (int x = 1; x < 8; ++x) all = mul2(all, gg[x]);
-      float2* tau = reinterpret_cast<float2*>(s_tau + half * 512) + lane;      // [8][32] pairs
-      tau[warp * 32] = all;
-      __syncthreads();
-      for (int w = warp < 4 ? warp + 1 : 4; w < (warp < 4 ? 4 : warp); ++w) f = mul2(f, tau[w * 32]);
-    }
-    if (half > 0) {                                      // the products of the channels before have read their operands
-      alive = alive && wait(scored, half - 1);
+  for (int p = 0; p < 3; ++p) {
+    *reinterpret_cast<uint32_t*>(group + p * 16384 + at) = a[p];
+    *reinterpret_cast<uint32_t*>(group + p * 16384 + 8192 + at) = b[p];
+  }
+}
+__device__ __forceinline__ void dc_put_dn(uint8_t* group, int lane, int x, float2 kk, float2 dn) {
+  uint32_t c[3];
+  const float2 kx = mul2(kk, dn);
+  split3x2(kx.x, kx.y, c);
+  const uint32_t at = x * 128 + (((lane >> 2) ^ x) << 4);
+#pragma unroll
+  for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(group + 49152 + p * 8192 + at) = c[p];
+}
+template <int D>
+__device__ __forceinline__ void dc_issue_scores(uint8_t* smem, uint32_t to, uint64_t* scored) {
+  const uint32_t id = umma::make_idesc<__nv_bfloat16>(128, 64, 0, 0);
+  const uint32_t a0 = umma::desc_low(smem_u32(smem), 16), b0 = umma::desc_low(smem_u32(smem + 49152), 16);
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+      umma::mma_ss_low(to + (ks >> 1) * 64, a0 + ((term_a(i) * 16384 + ks * 32) >> 4), b0 + ((term_b(i) * 8192 + ks * 32) >> 4), id, i > 0 || (ks & 1) > 0);
+  umma::commit(scored);
+}
+
+// Scores of decays per channel of any size (delta_chunk_kernel's own go by a reciprocal, which has to stay within 2^90). Between tokens of one
+// block of 16 in fp32; between blocks on the tensor core, split at token 32 and inside either half at its middle: products of decays alone.
+// Accumulators as delta_chunk_kernel's, of which columns 0-31 are what rows of tokens 32 to 63 have of tokens 0 to 31, and columns 32-63 of tokens
+// 0 to 15 and 32 to 47, for tokens 16 to 31 in their rows, 48 to 63 in rows 0 to 15. What bounds a CTA here: phases behind one another, of 8 warps
+// (an instruction every 3.2 cycles; code that does not fit the instruction cache is the first of its stalls). us, token form / so / decays that need
+// it not: 16 prompts of 500-1300, 8 heads of 128 702 / 458 / 318, 1 x 1024 360 / 110 / 99, 4 x 256 93 / 61 / 49; 32 heads of 64 1 x 1024 299 / 145 / 121
+template <int D>
+__device__ __forceinline__ void dc_block_scores(DcChunk& W) {
+  const DcLocal<D> L;
+  uint8_t* const smem = L.at;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float2 one = make_float2(1.f, 1.f);
+  float most_k = 0.f, most_q = 0.f, most_g = 0.f;
+  uint8_t* to = smem + (lane & 3) * 4;
+  float2* raw_kq = reinterpret_cast<float2*>(smem);      // k, q and g as they are, 64 channels at a time: [64][64] pairs of k and q, [64][64] of g
+  float* raw_g = reinterpret_cast<float*>(smem + kDcL * 64 * 8);
+#pragma unroll 1
+  for (int half = 0; half < D / 64; ++half) {
+    float2* tau = reinterpret_cast<float2*>(L.tau() + half * 512) + lane;
+    if (W.issued > 0) {                                  // the products under way have read their operands
+      W.alive = W.alive && W.wait(L.scored(), W.issued - 1, L.gave_up());
       umma::fence_after_sync();
     }
-    uint8_t* sKQ = smem + (lane & 3) * 4 + warp * 1024;
-    auto put_up = [&](int x, float2 up) {
-      uint32_t a[3], b[3];
-      const float2 kx = mul2(kk[x], up), qx = mul2(qq[x], up);
-      split3cut(kx.x, kx.y, a);
-      split3cut(qx.x, qx.y, b);
-      const uint32_t at = x * 128 + (((lane >> 2) ^ x) << 4);
+    {
+      float2 kk[8], qq[8], gg[8], all = one;
+      dc_fetch<false>(W.t, 8 * warp, half * 64 + 2 * lane, kk, qq, gg);
+      __syncthreads();
 #pragma unroll
-      for (int p = 0; p < 3; ++p) {
-        *reinterpret_cast<uint32_t*>(sKQ + p * 16384 + at) = a[p];
-        *reinterpret_cast<uint32_t*>(sKQ + p * 16384 + 8192 + at) = b[p];
+      for (int x = 0; x < 8; ++x) {
+        most_k = largest(most_k, kk[x]), most_q = largest(most_q, qq[x]), most_g = largest(most_g, gg[x]);
+        all = mul2(all, gg[x]);
+        const int at = (8 * warp + x) * 64 + 2 * lane;
+        *reinterpret_cast<float4*>(raw_kq + at) = make_float4(kk[x].x, qq[x].x, kk[x].y, qq[x].y);
+        *reinterpret_cast<float2*>(raw_g + at) = gg[x];
       }
-    };
-    auto put_dn = [&](int x, float2 dn) {
-      uint32_t c[3];
-      const float2 kx = mul2(kk[x], dn);
-      split3x2(kx.x, kx.y, c);
-      const uint32_t at = x * 128 + (((lane >> 2) ^ x) << 4);
-#pragma unroll
-      for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(sKQ + 49152 + p * 8192 + at) = c[p];
-    };
-    if (PER_HEAD) {
-#pragma unroll
-      for (int x = 0; x < 8; ++x) put_up(x, one), put_dn(x, one);
-    } else {
-      // (a token's two factors are one and its reciprocal: between tokens that are near each other, no rounding but those of the decays in between)
-      float near = 1.f, most = 1.f;
-      auto inverse = [&](float2 x) {
-        near = fminf(near, fminf(fabsf(x.x), fabsf(x.y))), most = fmaxf(most, fmaxf(fabsf(x.x), fabsf(x.y)));
-        return make_float2(rcp_newton(x.x), rcp_newton(x.y));
-      };
-      if (warp < 4) {
-#pragma unroll
-        for (int x = 7; x >= 0; --x) {
-          put_dn(x, f);
-          put_up(x, inverse(f));
-          f = mul2(f, gg[x]);
-        }
-      } else {
-#pragma unroll
-        for (int x = 0; x < 8; ++x) {
-          f = mul2(f, gg[x]);
-          put_up(x, f);
-          put_dn(x, inverse(f));
-        }
-      }
-      far = far || !(near >= kNear && most <= kFar);
+      tau[warp * 32] = all;
     }
-    if (!PER_HEAD && __any_sync(0xffffffffu, far) && lane == 0) *s_far = 1;
+    __syncthreads();
+    // ---- blocks of 16 tokens: a warp has a quarter of the channels, a lane two tokens j of a block (in turn of two groups of four, 0 and 3 or 1 and 2) and
+    // a quarter of those, and walks the tokens i behind them
+    auto walk = [&](auto group) {
+      constexpr int J = 4 * decltype(group)::value, N = 16 - J;
+      const int slice = lane & 3, own = (lane >> 2) & 1, block = lane >> 3;
+      const int at = (16 * block + J) * 64 + (warp >> 1) * 16 + slice * 4;
+      float a[2][N], b[2][N], p[2][4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          const float4 y = *reinterpret_cast<const float4*>(raw_kq + at + (2 * own + x) * 64 + e);
+          p[x][e] = y.x, p[x][e + 1] = y.z;
+        }
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        if (i % 2 == 0) asm volatile("" ::: "memory");   // (loads of later tokens would take the sums' registers)
+        const float4 g4 = *reinterpret_cast<const float4*>(raw_g + at + i * 64);
+        const float4 y0 = *reinterpret_cast<const float4*>(raw_kq + at + i * 64), y1 = *reinterpret_cast<const float4*>(raw_kq + at + i * 64 + 2);
+        const float g_[4] = {g4.x, g4.y, g4.z, g4.w}, k_[4] = {y0.x, y0.z, y1.x, y1.z}, q_[4] = {y0.y, y0.w, y1.y, y1.w};
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          a[x][i] = b[x][i] = 0.f;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (i >= 4 || i > 2 * own + x) p[x][e] *= g_[e];
+            a[x][i] = fmaf(k_[e], p[x][e], a[x][i]);
+            b[x][i] = fmaf(q_[e], p[x][e], b[x][i]);
+          }
+        }
+      }
+      // the four slices: a lane keeps k or q of one of the two tokens j
+      float* part = L.parts() + (((warp >> 1) * 16 + J) * 4 + J / 4) * 32 + (lane & 1) * 16 + block * 4 + 2 * own + ((lane >> 1) & 1);
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const float keep = lane & 1 ? b[x][i] : a[x][i], give = lane & 1 ? a[x][i] : b[x][i];
+          a[x][i] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+        }
+        const float keep = lane & 2 ? a[1][i] : a[0][i], give = lane & 2 ? a[0][i] : a[1][i];
+        const float sum = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+        part[i * 128] = half > 0 ? part[i * 128] + sum : sum;
+      }
+    };
+    if (warp & 1) walk(std::integral_constant<int, 1>{}), walk(std::integral_constant<int, 2>{});
+    else walk(std::integral_constant<int, 0>{}), walk(std::integral_constant<int, 3>{});
+    // ---- across blocks: relative to token 32 (rows i of 32 and later, columns j before it) and inside either half to its middle (rows 0-15: tokens 48 to 63,
+    // rows 16-31: those; columns 32-63: tokens 0 to 15 and 32 to 47): products of decays alone
+    float2 kk[8], qq[8], gg[8], f = one, near = one;
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      const int at = (8 * warp + x) * 64 + 2 * lane;
+      const float4 y = *reinterpret_cast<const float4*>(raw_kq + at);
+      kk[x] = make_float2(y.x, y.z), qq[x] = make_float2(y.y, y.w), gg[x] = *reinterpret_cast<const float2*>(raw_g + at);
+    }
+    if (warp < 4) {
+      for (int w = warp + 1; w < 4; ++w) f = mul2(f, tau[w * 32]);
+    } else {
+      for (int w = 4; w < warp; ++w) f = mul2(f, tau[w * 32]);
+    }
+    const bool upper = (warp & 2) != 0;                  // half of its half
+    if (upper && (warp & 1)) near = tau[(warp - 1) * 32];
+    if (!upper && !(warp & 1)) near = tau[(warp + 1) * 32];
+    __syncthreads();                                     // k, q and g have been read
+    if (warp < 4) {
+#pragma unroll
+      for (int x = 7; x >= 0; --x) dc_put_dn(to + warp * 1024, lane, x, kk[x], f), f = mul2(f, gg[x]);
+    } else {
+#pragma unroll
+      for (int x = 0; x < 8; ++x) f = mul2(f, gg[x]), dc_put_up(to + warp * 1024, lane, x, kk[x], qq[x], f);
+    }
+    if (upper) {
+#pragma unroll
+      for (int x = 0; x < 8; ++x) near = mul2(near, gg[x]), dc_put_up(to + (warp < 4 ? warp : warp - 6) * 1024, lane, x, kk[x], qq[x], near);
+    } else {
+#pragma unroll
+      for (int x = 7; x >= 0; --x) dc_put_dn(to + (warp < 4 ? warp + 4 : warp + 2) * 1024, lane, x, kk[x], near), near = mul2(near, gg[x]);
+    }
     fence_proxy_async_smem();
     __syncthreads();
-    if (!PER_HEAD && *s_far && !*gave_up) {              // not for chunks (no product is under way)
-      if (threadIdx.x == 0) *reinterpret_cast<int*>(record + R::kFlagAt) = 1;
-      if (warp == 1) umma::tmem_dealloc(tb, 256);
-      return;
-    }
-    if (issuer && alive) {
-      const uint32_t id = umma::make_idesc<T>(128, 64, 0, 0);
-      const uint32_t a0 = umma::desc_low(smem_u32(smem), 16), b0 = umma::desc_low(smem_u32(smem + 49152), 16);
-#pragma unroll
-      for (int i = 0; i < 6; ++i)
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma::mma_ss_low(tb + kTmSC + half * 128 + (ks >> 1) * 64, a0 + ((term_a(i) * 16384 + ks * 32) >> 4), b0 + ((term_b(i) * 8192 + ks * 32) >> 4), id,
-                           i > 0 || (ks & 1) > 0);
-      umma::commit(scored);
-    }
+    if (warp == 0 && W.alive && umma::elect_one()) dc_issue_scores<D>(smem, W.tb + kTmSC + half * 128, L.scored());
     __syncwarp();
+    ++W.issued;
   }
   const uint32_t mk = __reduce_max_sync(0xffffffffu, magnitude(most_k)), mq = __reduce_max_sync(0xffffffffu, magnitude(most_q)),
                  mg = __reduce_max_sync(0xffffffffu, magnitude(most_g));
-  if (lane == 0) atomicMax(&s_max[0], mk), atomicMax(&s_max[1], mq), atomicMax(&s_max[3], mg);
-  alive = alive && wait(scored, D / 64 - 1);
+  if (lane == 0) atomicMax(&L.max()[0], mk), atomicMax(&L.max()[1], mq), atomicMax(&L.max()[3], mg);
+}
+
+// ---- behind the scores: X, [W; Y], [U; O0], the record. BLOCKS: from dc_block_scores
+template <int D, bool PER_HEAD, bool BLOCKS>
+__device__ __forceinline__ void dc_chunk_rest(const DcChunk& W) {
+  using T = __nv_bfloat16;
+  using R = DcRecord<D>;
+  using M = DcSmem<D>;
+  const DcLocal<D> L;
+  uint8_t* const smem = L.at;
+  float *const sA = L.A(), *const sQs = L.Qs(), *const s_tau = L.tau(), *const s_beta = L.beta(), *const s_g = L.g(), *const s_p = L.p(), *const s_e = L.e();
+  uint64_t *const scored = L.scored(), *const made = L.made(), *const drained = L.drained();
+  uint32_t* const s_max = L.max();
+  int* const s_next = L.next();
+  volatile int* const gave_up = L.gave_up();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nt = W.t.nt;
+  const uint32_t tb = W.tb;
+  const T* const v = W.v;
+  uint8_t* const record = W.record;
+  const bool issuer = warp == 0 && umma::elect_one();
+  const float2 one = make_float2(1.f, 1.f);
+  bool alive = W.alive;
+  auto wait = [&](uint64_t* bar, int parity) { return W.wait(bar, parity, gave_up); };
+  alive = alive && wait(scored, W.issued - 1);
   umma::fence_after_sync();
   __syncthreads();                                       // all that the scores were made of is free
+  if (BLOCKS) {                                          // the blocks' four parts, to where A will be (P q will be where they are)
+    static_assert(2 * kDcL * 16 == 8 * kDcThreads, "eight sums a thread");
+    const int of = threadIdx.x >> 1;                     // [k, q][block][i]
+    const float4* part = reinterpret_cast<const float4*>(L.parts()) + (of & 15) * 32 + (threadIdx.x & 1) * 16 + (of >> 6) * 4 + ((of >> 4) & 3);
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      float4 sum = part[y * 8];
+#pragma unroll
+      for (int z = 1; z < 4; ++z) {
+        const float4 more = part[z * 512 + y * 8];
+        sum.x += more.x, sum.y += more.y, sum.z += more.z, sum.w += more.w;
+      }
+      *reinterpret_cast<float4*>(sA + (threadIdx.x >> 1) * M::kBlockRow + (threadIdx.x & 1) * 8 + 4 * y) = sum;
+    }
+    __syncthreads();
+  }
 
   uint4 held[D / 16];                                    // values on their way to where A is
   float2 X[32];                                          // warps 0-3: a row of X
@@ -378,6 +437,25 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
       }
 #pragma unroll
       for (int c = 0; c < 16; ++c) X[16 * part + c] = make_float2(__uint_as_float(w[2 * c]), __uint_as_float(w[2 * c + 1]));
+    }
+    if (BLOCKS) {
+      // (see dc_block_scores) the columns of a row's own half: of its block, and of the block before, which rows 48 to 63 have had in rows 0 to 15
+      float* s_near = sA + M::kBlocks / 4 + (of_k ? 0 : 32 * M::kBlockRow);        // [k, q][tokens 16-31, 48-63][kBlockRow]
+      if (!(warp & 1)) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) *reinterpret_cast<float2*>(s_near + (lane ^ 16) * M::kBlockRow + 2 * c) = lane < 16 ? X[24 + c] : X[16 + c];
+      }
+      named_bar_sync(1, 128);
+      const float* own = sA + ((of_k ? 0 : kDcL) + i) * M::kBlockRow;
+      const float* other = lane < 16 ? own : s_near + (warp & 1 ? lane : lane - 16) * M::kBlockRow;
+      if (warp & 1) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) X[16 + c] = *reinterpret_cast<const float2*>(other + 2 * c), X[24 + c] = *reinterpret_cast<const float2*>(own + 2 * c);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) X[c] = *reinterpret_cast<const float2*>(other + 2 * c), X[8 + c] = *reinterpret_cast<const float2*>(own + 2 * c);
+      }
+      named_bar_sync(1, 128);                            // A takes their place
     }
     if (PER_HEAD) {                                      // the decay from j to i
       float d = 1.f;
@@ -439,7 +517,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
 #pragma unroll
     for (int i = 0; i < D / 16; ++i) {
       const int e = i * 128 + threadIdx.x - 128, row = e / (D / 8), c16 = e % (D / 8);
-      held[i] = row < nt ? ld_nc_v4(v + row * P.v_stride + c16 * 8) : make_uint4(0, 0, 0, 0);
+      held[i] = row < nt ? ld_nc_v4(v + row * W.v_stride + c16 * 8) : make_uint4(0, 0, 0, 0);
     }
     uint32_t most_v = 0;
 #pragma unroll
@@ -459,7 +537,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
     if (u >= 8 * (D / 64)) break;
     const int half = u >> 3, e = u & 7, ch = half * 64 + 2 * lane;
     float2 kk[8], qq[8], gg[8], to_end[8], p = one, post = one;
-    fetch(8 * e, ch, kk, qq, gg);
+    dc_fetch<PER_HEAD>(W.t, 8 * e, ch, kk, qq, gg);
     if (!PER_HEAD) {
       const float2* tau = reinterpret_cast<const float2*>(s_tau + half * 512) + lane;
       for (int w = 0; w < e; ++w) p = mul2(p, tau[w * 32]);
@@ -503,7 +581,7 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
   fence_proxy_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {
-    constexpr uint32_t big = PER_HEAD ? kBig : kBigUp, small = PER_HEAD ? kSmall : kSmallDn;
+    constexpr uint32_t big = PER_HEAD || BLOCKS ? kBig : kBigUp, small = PER_HEAD || BLOCKS ? kSmall : kSmallDn;
     const bool odd = s_max[0] >= big || s_max[1] >= big || s_max[2] >= kBig || s_max[3] >= kTwo || (s_max[0] > 0 && s_max[0] < small) ||
                      (s_max[1] > 0 && s_max[1] < small) || (s_max[2] > 0 && s_max[2] < kSmall);
     *reinterpret_cast<int*>(record + R::kFlagAt) = odd ? 1 : 0;
@@ -589,9 +667,179 @@ delta_chunk_kernel(const __grid_constant__ DcParams DP) {
   __syncthreads();
   if (warp == 1) umma::tmem_dealloc(tb, 256);
   if (threadIdx.x == 0 && *gave_up) {
-    *reinterpret_cast<volatile int*>(DP.wait_status) = 1;
+    *reinterpret_cast<volatile int*>(W.wait_status) = 1;
     __threadfence_system();
   }
+}
+
+// A chunk whose decays are too strong for the scores of delta_chunk_kernel, from there on. A call, as the last thing that CTA does: nothing
+// of the kernel's own way lives across it
+template <int D>
+__device__ __noinline__ void dc_block_chunk(DcChunk W) {
+  dc_block_scores<D>(W);
+  dc_chunk_rest<D, false, true>(W);
+}
+
+template <int D, bool PER_HEAD>
+__global__ void __launch_bounds__(kDcThreads, 2)
+delta_chunk_kernel(const __grid_constant__ DcParams DP) {
+  using T = __nv_bfloat16;
+  const DeltaParams& P = DP.d;
+  const DcLocal<D> L;
+  uint8_t* const smem = L.at;
+  float *const s_tau = L.tau(), *const s_beta = L.beta(), *const s_g = L.g(), *const s_p = L.p(), *const s_e = L.e();
+  uint64_t *const scored = L.scored(), *const made = L.made(), *const drained = L.drained();
+  uint32_t *const s_max = L.max(), *const tmem_slot = L.tmem_slot();
+  int *const s_where = L.where(), *const s_next = L.next();
+  volatile int* const gave_up = L.gave_up();
+
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = blockIdx.x % P.H, lin = DP.c.first + blockIdx.x / P.H;
+  if (warp == 0) {                                       // the sequence of chunk `lin`
+    int base = 0, found = -1, at = 0;
+    for (int s0 = 0; s0 < DP.num_seqs && found < 0; s0 += 32) {
+      const int n = s0 + lane < DP.num_seqs ? chunks_of(P.cu_q[s0 + lane + 1] - P.cu_q[s0 + lane]) : 0;
+      int to = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, to, o);
+        if (lane >= o) to += up;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, lin < base + to);
+      if (hit != 0) {
+        const int l = __ffs(hit) - 1;
+        found = s0 + l, at = lin - base - __shfl_sync(0xffffffffu, to - n, l);
+      }
+      base += __shfl_sync(0xffffffffu, to, 31);
+    }
+    if (lane == 0) s_where[0] = found, s_where[1] = at;
+  }
+  if (threadIdx.x == 32) {
+    mbar_init(scored, 1), mbar_init(made, 1), mbar_init(drained, 1);
+    mbar_fence_init();
+    for (int i = 0; i < 4; ++i) s_max[i] = 0;
+    *s_next = 0, *gave_up = 0;
+  }
+  __syncthreads();
+  const int s = s_where[0], chunk = s_where[1];
+  if (s < 0) return;                                     // the grid has room for sequences that all end in a chunk of their own
+  if (warp == 1) umma::tmem_alloc(tmem_slot, 256);
+  const int64_t tok0 = P.cu_q[s] + chunk * kDcL;
+  const int nt = min(kDcL, P.cu_q[s + 1] - (int)tok0);
+  const int grp = h / (P.H / P.groups);
+  const float* q = P.q + tok0 * P.q_stride + (int64_t)grp * D;
+  const float* k = P.k + tok0 * P.k_stride + (int64_t)grp * D;
+  const float* g = P.g + tok0 * ((int64_t)P.H * (PER_HEAD ? 1 : D)) + (int64_t)h * (PER_HEAD ? 1 : D);
+  const int64_t g_stride = (int64_t)P.H * (PER_HEAD ? 1 : D);
+  const T* v = (const T*)P.v + tok0 * P.v_stride + (int64_t)h * D;
+  uint8_t* record = DP.c.records + ((int64_t)(lin - DP.c.first) * P.H + h) * DP.c.bytes;
+  const bool issuer = warp == 0 && umma::elect_one();
+  auto wait = [&](uint64_t* bar, int parity) { return mbar_warp_wait(bar, parity & 1, DP.wait_tries, gave_up); };
+
+  if (threadIdx.x < kDcL) {
+    const int t = threadIdx.x;
+    const float b = t < nt ? P.beta[(tok0 + t) * P.H + h] : 0.f;
+    s_beta[t] = b;
+    uint32_t most = magnitude(b);
+    if (PER_HEAD) {
+      const float d = t < nt ? g[t * g_stride] : 1.f;
+      s_g[t] = d;
+      most = max(most, magnitude(d));
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) atomicMax(&s_max[3], most);
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tb = *tmem_slot;
+  if (PER_HEAD && threadIdx.x < kDcL) {
+    float p = 1.f, e = 1.f;
+    for (int i = 0; i <= (int)threadIdx.x; ++i) p *= s_g[i];
+    for (int i = kDcL - 1; i > (int)threadIdx.x; --i) e *= s_g[i];
+    s_p[threadIdx.x] = p, s_e[threadIdx.x] = e;
+  }
+
+  const DcTokens C{k, q, g, (uint32_t)P.k_stride * 4, (uint32_t)P.q_stride * 4, (uint32_t)g_stride * 4, nt};
+  bool alive = true;
+  // ------------------------------------------------ scores, 64 channels at a time; a thread has two channels and 8 tokens
+  float most_k = 0.f, most_q = 0.f, most_g = 0.f;
+  const float2 one = make_float2(1.f, 1.f);
+#pragma unroll 1
+  for (int half = 0; half < D / 64; ++half) {
+    const int ch = half * 64 + 2 * lane;
+    float2 kk[8], qq[8], gg[8];
+    dc_fetch<PER_HEAD>(C, 8 * warp, ch, kk, qq, gg);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      most_k = largest(most_k, kk[x]), most_q = largest(most_q, qq[x]);
+      if (!PER_HEAD) most_g = largest(most_g, gg[x]);
+    }
+    // the decay between a token and the chunk's middle, between tokens 31 and 32: of this warp's nearest tokens `f`. All warps have the same channels and
+    // look at all decays between eight tokens and the middle: one way or the other, they go it together
+    float2 f = one;
+    if (!PER_HEAD) {
+      float2 all = gg[0];
+#pragma unroll
+      for (int x = 1; x < 8; ++x) all = mul2(all, gg[x]);
+      float2* tau = reinterpret_cast<float2*>(s_tau + half * 512) + lane;      // [8][32] pairs
+      tau[warp * 32] = all;
+      __syncthreads();
+      float least = 1.f;
+#pragma unroll
+      for (int side = 0; side < 2; ++side) {
+        float2 r = one;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          if ((side ? 4 + w : 3 - w) == warp) f = r;
+          r = mul2(r, tau[(side ? 4 + w : 3 - w) * 32]);
+          least = fminf(least, fminf(fabsf(r.x), fabsf(r.y)));
+        }
+      }
+      if (__any_sync(0xffffffffu, !(least >= kNear))) {
+        dc_block_chunk<D>(DcChunk{C, v, P.v_stride, record, tb, half, DP.wait_tries, alive, DP.wait_status});
+        return;
+      }
+    }
+    if (half > 0) {                                      // the products of the channels before have read their operands
+      alive = alive && wait(scored, half - 1);
+      umma::fence_after_sync();
+    }
+    uint8_t* to = smem + (lane & 3) * 4 + warp * 1024;
+    auto put_up = [&](int x, float2 up) { dc_put_up(to, lane, x, kk[x], qq[x], up); };
+    auto put_dn = [&](int x, float2 dn) { dc_put_dn(to, lane, x, kk[x], dn); };
+    if (PER_HEAD) {
+#pragma unroll
+      for (int x = 0; x < 8; ++x) put_up(x, one), put_dn(x, one);
+    } else {
+      // (a token's two factors are one and its reciprocal: between tokens that are near each other, no rounding but those of the decays in between)
+      auto inverse = [](float2 x) { return make_float2(rcp_newton(x.x), rcp_newton(x.y)); };
+      if (warp < 4) {
+#pragma unroll
+        for (int x = 7; x >= 0; --x) {
+          put_dn(x, f);
+          put_up(x, inverse(f));
+          f = mul2(f, gg[x]);
+        }
+      } else {
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+          f = mul2(f, gg[x]);
+          put_up(x, f);
+          put_dn(x, inverse(f));
+        }
+      }
+    }
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (issuer && alive) dc_issue_scores<D>(smem, tb + kTmSC + half * 128, scored);
+    __syncwarp();
+  }
+  const uint32_t mk = __reduce_max_sync(0xffffffffu, magnitude(most_k)), mq = __reduce_max_sync(0xffffffffu, magnitude(most_q)),
+                 mg = __reduce_max_sync(0xffffffffu, magnitude(most_g));
+  if (lane == 0) atomicMax(&s_max[0], mk), atomicMax(&s_max[1], mq), atomicMax(&s_max[3], mg);
+  dc_chunk_rest<D, PER_HEAD, false>(DcChunk{C, v, P.v_stride, record, tb, D / 64, DP.wait_tries, alive, DP.wait_status});
 }
 
 

@@ -82,7 +82,7 @@ LENS = [[1, 63, 64, 65, 0, 130, 201], [300], [96, 128, 33]]
 @pytest.mark.parametrize("decay", ["mild", "none", "edge", "strong", "signed"])
 def test_against_64_bits(H, G, N, per_head, lens, decay):
     """No further from the result than 1.5 times the token form, or 2e-7 (a chunk sums in another order; both are 24-bit arithmetic). Strong decays
-    are down to e^-30 a token, some exactly zero: one per head goes on the scores, those per channel are not for chunks."""
+    are down to e^-30 a token, some exactly zero: one per head goes on the scores, those per channel take the blocks of 16 tokens."""
     from nanovllm import ops
     q, k, v, gate, beta, g = _inputs(lens, H, G, N, per_head, decay)
     past = [9 if i % 2 else 0 for i in range(len(lens))]
@@ -95,11 +95,7 @@ def test_against_64_bits(H, G, N, per_head, lens, decay):
     live = [i for i, n in enumerate(lens) if n]
     for got, token, exact in ((out, ref, want), (state.flip(0)[live], tokens.flip(0)[live], want_S[live])):
         assert _off(got, exact) <= max(1.5 * _off(token, exact), 2e-7), (_off(got, exact), _off(token, exact))
-    if not per_head and decay == "strong":                 # decays per channel beyond what chunks take: a head with half a chunk is left to tokens
-        out, ref = (torch.cat([o for o in x.split(lens) if len(o) >= 32]) for x in (out, ref))
-        assert torch.equal(out, ref)
-    else:
-        assert not torch.equal(out, ref)
+    assert not torch.equal(out, ref)                       # (no head is left to tokens)
     for i, n in enumerate(lens):
         if n == 0:
             assert torch.equal(state.flip(0)[i], first[i])
@@ -123,6 +119,36 @@ def test_no_precision_is_lost(H, G, N, per_head, decay, states):
         off.append([_off(out, want), _off(ref, want), _off(state, want_S), _off(tokens, want_S)])
     out, ref, state, tokens = (sum(x) / 2 for x in zip(*off))
     assert out <= 1.02 * ref and state <= states * tokens, (out / ref, state / tokens)
+
+
+@pytest.mark.parametrize("H,G,N", SIZES)
+@pytest.mark.parametrize("pattern", ["one channel", "second half of the channels", "one token of zeros", "each block", "2^-83"])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 150])
+def test_strong_decays_of_few_channels(H, G, N, pattern, n):
+    """Every pair of the blocks of 16 tokens in turn, beside a sequence that does not need them: outputs of each as near to 64 bits as the token form."""
+    from nanovllm import ops
+    lens = [n, 130]
+    q, k, v, gate, beta, g = _inputs(lens, H, G, N, False)
+    marks = gate.view(n + 130, H, N)
+    if pattern == "one channel":
+        marks[:, 0, 5] = 1e-4
+    elif pattern == "second half of the channels":
+        marks[:, 1, N // 2:] = 3e-3
+    elif pattern == "one token of zeros":
+        marks[n // 2, :, ::3] = 0.0
+    elif pattern == "each block":
+        marks[::16] = 1e-30
+    else:                                                  # around the line of a half chunk's decays
+        marks[:32, :, 3], marks[32:, :, 3] = 2.0 ** -2.59, 2.0 ** -2.60
+    first, slots = torch.randn(2, H, N, N, device="cuda", generator=g), torch.arange(2, dtype=torch.int32, device="cuda")
+    spans, state, tokens = _spans(lens, [4, 0]), first.clone(), first.clone()
+    want, want_S = _exact(lens, [4, 0], q, k, v, gate, beta, H, G, N, first)
+    out = ops.delta_rule(q, k, v, gate, beta, spans, H, G, N, N, state, slots)
+    ref = _call("tokens", q, k, v, gate, beta, spans, H, G, N, tokens, slots)
+    assert not torch.equal(out, ref)
+    for rows in (slice(0, n), slice(n, n + 130)):          # (a few rows alone: their errors spread by a quarter)
+        assert _off(out[rows], want[rows]) <= 1.3 * _off(ref[rows], want[rows])
+    assert _off(state, want_S) <= 1.6 * _off(tokens, want_S)
 
 
 @pytest.mark.parametrize("H,G,N", SIZES)
