@@ -1126,20 +1126,30 @@ constexpr int64_t kDcWorkspace = 512ll << 20;           // more than this and a 
 static int64_t dc_chunks(int num_seqs, int64_t total_q) { return total_q / kDcL + num_seqs; }      // no step has more
 static int64_t dc_record(int D) { return D == 128 ? DcRecord<128>::kBytes : DcRecord<64>::kBytes; }
 
-// Steps with a span of 96 tokens at least whose chunks are the faster way. Either way's time in ns, from prompts alone, of equal and of
-// ragged lengths and beside single tokens (us, tokens / chunks; a decay per channel, with one per head 2 to 10 % less on both sides):
-//   8 heads of 128:  1 x 96 37 / 36, x 256 93 / 45, x 1024 360 / 100;  16 x 96 61 / 54, x 256 153 / 103, x 1024 594 / 314;  64 x 128 304 / 192;
-//                    16 of 500-1300 699 / 306;  1024 beside 32 x 1 364 / 133, beside 64 x 16 396 / 173;  [64 x 32 83 / 112, kept to tokens]
-//   32 heads of 64:  1 x 96 31 / 31, x 256 77 / 42, x 1024 299 / 117;  4 x 256 77 / 67, x 1024 300 / 214;  1024 beside 64 x 16 389 / 262;
-//                    [16 x 128 68 / 115, x 1024 508 / 734, 16 of 500-1300 572 / 708, kept to tokens: a chunk of a head of 64 costs
-//                    delta_chunk_kernel 0.6 of one of 128, a token of it delta_rule_kernel a fifth]
+// Steps with a span of 96 tokens at least whose chunks are the faster way. Both ways' times in ns, fitted to the times of prompts of 96 to 1024 tokens,
+// 1 to 64 at a time: chunks by the waves of delta_chunk_kernel (a little CTA of a wave that finds SMs empty takes 0.6 of one) and the length that a
+// scan's CTA walks; all but two of the points within 11 %, where two CTAs' worth of waves lie between them. us, tokens / chunks (a decay per channel;
+// with strong decays):
+//   8 heads of 128:  1 x 128 48 / 37 (47), x 256 93 / 45 (56), x 1024 361 / 99 (110);  4 x 256 93 / 50 (61);  8 x 400 144 / 111 (151);  16 x 96 61 / 57 (76),
+//                    x 256 153 / 106 (153), x 400 236 / 174 (253), x 1024 594 / 325 (463);  64 x 128 305 / 198 (286);  16 of 500-1300 699 / 318 (463);
+//                    1024 beside 32 x 1 364 / 140 (177), beside 64 x 16 430 / 176 (233);  [1 x 96 37 / 37 (47), 8 x 96 38 / 41 (52): tokens]
+//   32 heads of 64:  1 x 128 40 / 32 (40), x 256 77 / 43 (51), x 1024 299 / 121 (146);  2 x 400 119 / 79 (94);  4 x 256 77 / 70 (92), x 1024 301 / 227 (291);
+//                    4 of 300-600 177 / 142 (185);  [4 x 400 119 / 128, 8 x 256 78 / 116, 16 x 1024 510 / 755: tokens]
+// A decay per head: tokens 0.86 to 0.93 of that, chunks the same.
 static bool dc_shape(int mode, int dtype, int num_seqs, int max_q, int64_t total_q, int H, int kdim, int vdim) {
   if (mode == kWkv || dtype != B200_DTYPE_BF16 || num_seqs <= 0 || num_seqs > 65535 || kdim != vdim || max_q < 96) return false;
   if (!(kdim == 128 || (kdim == 64 && H % 2 == 0)) || H > 65535 || (total_q / kDcL + num_seqs) * H > INT_MAX / 2) return false;
-  const int64_t chunks = (total_q / kDcL + num_seqs / 2) * H, more = std::max<int64_t>(chunks - 300, 0);       // 300 run at a time
-  const int64_t tokens_ns = kdim == 128 ? std::max<int64_t>(355ll * max_q, total_q * H * 44 / 10) : std::max<int64_t>(285ll * max_q, total_q * H * 97 / 100);
-  const int64_t chunks_ns = kdim == 128 ? 26000 + 72ll * max_q + 140 * more : 20000 + 85ll * max_q + 77 * more;
-  return chunks_ns < tokens_ns;
+  const bool wide = kdim == 128, even = total_q == (int64_t)num_seqs * max_q;
+  const int64_t sms = sm_count(), wave = 2 * sms;        // CTAs at a time
+  // waves in tenths: known where all spans are of one length, otherwise as many as half a chunk more per span comes to
+  const int64_t chunks = (even ? (int64_t)num_seqs * ((max_q + kDcL - 1) / kDcL) : total_q / kDcL + num_seqs / 2) * H, rest = chunks % wave;
+  const int64_t waves = even ? chunks / wave * 10 + (rest > sms ? 10 : rest > 0 ? 6 : 0) : chunks * 10 / wave + 5;
+  const int64_t scan = std::max<int64_t>(max_q, total_q * H * kdim / 128 / sms);
+  const int64_t chunks_ns = (wide ? 8000 : 11000) + 63 * scan + (wide ? 4050 : 2340) * waves;
+  const bool head = mode == kDecayPerHead;
+  const int64_t tokens_ns = wide ? 4000 + std::max<int64_t>((head ? 328ll : 350ll) * max_q, total_q * H * (head ? 390 : 445) / 100)
+                                 : 2500 + std::max<int64_t>((head ? 284ll : 290ll) * max_q, total_q * H * (head ? 92 : 97) / 100);
+  return chunks_ns < tokens_ns * 99 / 100;
 }
 
 int64_t delta_chunks_workspace(int mode, int dtype, int num_seqs, int max_q, int64_t total_q, int H, int groups, int kdim, int vdim) {
