@@ -216,9 +216,12 @@ def test_heads_left_to_tokens(H, G, N, what, passes):
         assert torch.equal(out[:150, cols], clean[:150, cols])
         if h in hit and not passes:
             assert same(out[150:, cols], ref[150:, cols]) and same(state[1, h], tokens[1, h])
-        elif h in hit:                                     # (earlier passes may have taken chunks)
-            assert torch.allclose(out[150:at, cols], ref[150:at, cols], rtol=1e-4, atol=1e-5) or what == "state inf"
-            assert torch.equal(out[150:, cols].isfinite(), ref[150:, cols].isfinite())
+        elif h in hit:                                     # (earlier passes may have taken chunks: another order of sums, then the same)
+            for got, want in ((out[150:, cols], ref[150:, cols]), (state[1, h], tokens[1, h])):
+                fine = want.isfinite()
+                assert torch.equal(got.isfinite(), fine)
+                size = want.where(fine, want.new_zeros(())).abs().amax(0, keepdim=True)      # (of a value column: one may be huge)
+                assert bool((((got - want).abs() <= 1e-4 * want.abs() + 1e-5 * size) | ~fine).all())
         else:
             assert torch.equal(out[150:, cols], clean[150:, cols]) and torch.equal(state[1, h], clean_state[1, h])
 
