@@ -617,17 +617,17 @@ static int decode_windowed(void* out, const void* q, const void* k_cache, const 
                      p.rows_box, hkv_cta * value_dim / 64, dtype, &mv);
   if (rc != B200_OK) return rc;
 
-  // num_ctas 0: the library's choice (few rows: decode_small.cu, above; us at 64 / 112 / 148 CTAs; contexts a third to all of the length named).
+  // num_ctas 0: the library's choice (us at 64 / 112 / 148 CTAs; contexts a third to all of the length named).
   // * A CTA's tiles of 8 heads of 128 (64 KB per stage) in batches of 16 and more: three quarters of the SMs, each with
   //   192 KB under way, keep HBM busier than all of them: 256 x 1074 tokens 152 / 114 / 119, 64 x 1074 46 / 37.6 / 38.7, 256 x
-  //   50 21 / 16.9 / 18.3, 16 x 1024 17 / 14.8 / 15.3. Smaller tiles need every SM: 8 heads of 64 105 / 73 / 68.
-  //   The line was drawn at 16 rows; 3 to 15 rows of 8 heads of 128 measure 0 to 6 % less with 112 as well (8 x 4000 21.5 / 22.4).
+  //   50 21 / 16.9 / 18.3. Smaller tiles need every SM: 8 heads of 64 105 / 73 / 68.
+  //   The line was drawn at 16 rows; 3 to 15 rows of 8 heads of 128 measure 0 to 6 % less with 112 as well.
   // * One or two (sequence, group of 8 kv heads) of up to 8192 tokens in all (by the width of the block table) whose query
-  //   heads have 2048 output columns and more: what counts is the partial results to merge, and there are as many as CTAs.
-  //   16 heads over 8 of 128: 1 x 300 7.0 / 7.5 / 8.1, 1 x 1000 8.4 / 8.7 / 9.2, 1 x 4000 11.2 / 11.6 / 12.5, 2 x 300 7.3 / 7.7 /
-  //   8.2, 2 x 1000 9.1 / 8.8 / 9.4, 2 x 4000 13.5 / 13.0 / 13.3; 32 over 8 of 64: 1 x 1000 8.2 / 9.6 / 10.7, 2 x 4000 11.5 / 12.1 /
-  //   13.6. Narrower ones and more groups want the SMs: 32 over 32 of 128 1 x 300 8.6 / 7.4 / 7.5, 2 x 4000 26.8 / 22.6 / 23.2; 16
-  //   over 16 of 64 1 x 4000 11.1 / 10.4 / 10.5; 8 over 2 of 128 2 x 4000 11.0 / 9.4 / 9.8; 4 over 4 of 128 2 x 4000 11.2 / 10.7 / 10.9.
+  //   heads have 2048 output columns and more: what counts is the partial results to merge, and there are as many as CTAs. Few rows without a
+  //   window went to decode_small.cu above, so that this is for windows and chunks, values of another size, and tables of 4097 to 8192 tokens of
+  //   heads of 128. Full contexts of the window named: 16 heads over 8 of 128: 1 x 300 7.3 / 7.8 / 8.4, 1 x 512 7.6 / 8.3 / 8.8, 1 x 1024 8.7 / 8.9 / 9.5, 2 x
+  //   512 9.0 / 8.4 / 8.9, 2 x 2048 10.1 / 10.9 / 10.7, without one 1 x 6000 12.6 / 12.5 / 12.9; 32 over 8 of 64: 1 x 512 7.7 / 9.0 / 10.2, 2 x 2048 9.5 /
+  //   11.4 / 11.8. Narrower ones want the SMs: 16 over 16 of 64 1 x 512 8.3 / 7.3 / 7.3, 2 x 2048 10.3 / 9.6 / 8.8; 8 over 2 of 128 2 x 2048 10.9 / 9.0 / 9.3.
   int grid = num_ctas > 0 ? num_ctas : num_sms();
   if (num_ctas <= 0) {
     if (batch * hg_count <= 2 && num_heads / hg_count * value_dim >= 2048 && (int64_t)batch * block_table_stride * block_size <= 8192)

@@ -118,13 +118,13 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
         }
     } else {
 #pragma unroll
-    for (int ks = 0; ks < KSTEPS; ++ks) {
-      const int c16 = ((ks & 3) << 1) + k_half;
-      uint32_t r0, r1, r2, r3;
-      ldsm_x4(kb + (ks >> 2) * 2048 + k_tok * 128 + ((c16 ^ (k_tok & 7)) << 4), r0, r1, r2, r3);
-      mma_16816<T>(s[0], qa[ks][0], 0u, qa[ks][1], 0u, r0, r1);
-      mma_16816<T>(s[1], qa[ks][0], 0u, qa[ks][1], 0u, r2, r3);
-    }
+      for (int ks = 0; ks < KSTEPS; ++ks) {
+        const int c16 = ((ks & 3) << 1) + k_half;
+        uint32_t r0, r1, r2, r3;
+        ldsm_x4(kb + (ks >> 2) * 2048 + k_tok * 128 + ((c16 ^ (k_tok & 7)) << 4), r0, r1, r2, r3);
+        mma_16816<T>(s[0], qa[ks][0], 0u, qa[ks][1], 0u, r0, r1);
+        mma_16816<T>(s[1], qa[ks][0], 0u, qa[ks][1], 0u, r2, r3);
+      }
     }
     const int valid = len - (first + n * step) * 16;
 #pragma unroll
@@ -161,30 +161,30 @@ decode_small_kernel(const __grid_constant__ DecodeSmallParams S) {
         mma_16816<__half>(o_acc[4 * jp + 3], pa0, 0u, pa2, 0u, e4m3x2_to_f16x2(o1 & 0xffffu), e4m3x2_to_f16x2(o1 >> 16));
       }
     } else {
-    // two 16-bit terms of the probabilities, the second in the rows of the tile that the group does not use
-    const uint32_t pa0 = pack2<T>(p00, p01), pa2 = pack2<T>(p10, p11);
-    const float2 h0 = unpack2<T>(pa0), h1 = unpack2<T>(pa2);
-    const uint32_t pa1 = pack2<T>(p00 - h0.x, p01 - h0.y), pa3 = pack2<T>(p10 - h1.x, p11 - h1.y);
+      // two 16-bit terms of the probabilities, the second in the rows of the tile that the group does not use
+      const uint32_t pa0 = pack2<T>(p00, p01), pa2 = pack2<T>(p10, p11);
+      const float2 h0 = unpack2<T>(pa0), h1 = unpack2<T>(pa2);
+      const uint32_t pa1 = pack2<T>(p00 - h0.x, p01 - h0.y), pa3 = pack2<T>(p10 - h1.x, p11 - h1.y);
 #pragma unroll
-    for (int jp = 0; jp < NT / 2; ++jp) {
-      const int dt = 2 * jp + v_dt;
-      uint32_t r0, r1, r2, r3;
-      ldsm_x4_trans(vb + (dt >> 3) * 2048 + v_tok * 128 + (((dt & 7) ^ (v_tok & 7)) << 4), r0, r1, r2, r3);
-      mma_16816<T>(o_acc[2 * jp], pa0, pa1, pa2, pa3, r0, r1);
-      mma_16816<T>(o_acc[2 * jp + 1], pa0, pa1, pa2, pa3, r2, r3);
-    }
+      for (int jp = 0; jp < NT / 2; ++jp) {
+        const int dt = 2 * jp + v_dt;
+        uint32_t r0, r1, r2, r3;
+        ldsm_x4_trans(vb + (dt >> 3) * 2048 + v_tok * 128 + (((dt & 7) ^ (v_tok & 7)) << 4), r0, r1, r2, r3);
+        mma_16816<T>(o_acc[2 * jp], pa0, pa1, pa2, pa3, r0, r1);
+        mma_16816<T>(o_acc[2 * jp + 1], pa0, pa1, pa2, pa3, r2, r3);
+      }
     }
     __syncwarp();
     load(n + kStages, stage);
   }
   cp_async_wait<0>();
   if constexpr (!FP8) {
-  // the second term is left out where an infinite value made it 0 x inf or inf - inf
+    // the second term is left out where an infinite value made it 0 x inf or inf - inf
 #pragma unroll
-  for (int n = 0; n < NT; ++n)
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-    for (int e = 0; e < 2; ++e)
-      if (fabsf(o_acc[n][2 + e]) < INFINITY) o_acc[n][e] += o_acc[n][2 + e];
+      for (int e = 0; e < 2; ++e)
+        if (fabsf(o_acc[n][2 + e]) < INFINITY) o_acc[n][e] += o_acc[n][2 + e];
   }
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
