@@ -248,8 +248,9 @@ __device__ __forceinline__ void dc_issue_scores(uint8_t* smem, uint32_t to, uint
 // block of 16 in fp32; between blocks on the tensor core, split at token 32 and inside either half at its middle: products of decays alone.
 // Accumulators as delta_chunk_kernel's, of which columns 0-31 are what rows of tokens 32 to 63 have of tokens 0 to 31, and columns 32-63 of tokens
 // 0 to 15 and 32 to 47, for tokens 16 to 31 in their rows, 48 to 63 in rows 0 to 15. What bounds a CTA here: phases behind one another, of 8 warps
-// (an instruction every 3.2 cycles; code that does not fit the instruction cache is the first of its stalls). us, token form / so / decays that need
-// it not: 16 prompts of 500-1300, 8 heads of 128 702 / 458 / 318, 1 x 1024 360 / 110 / 99, 4 x 256 93 / 61 / 49; 32 heads of 64 1 x 1024 299 / 145 / 121
+// (an instruction every 3.2 cycles; code that does not fit the instruction cache is the first of its stalls: with the four channels of a lane behind one
+// another instead of in a loop, the first figure is 461). us, token form / so / decays that need it not: 16 prompts of 500-1300, 8 heads of 128 700 / 414 /
+// 317, 1 x 1024 360 / 108 / 99, 4 x 256 93 / 59 / 49; 32 heads of 64 1 x 1024 299 / 144 / 121
 template <int D>
 __device__ __forceinline__ void dc_block_scores(DcChunk& W) {
   const DcLocal<D> L;
@@ -259,7 +260,7 @@ __device__ __forceinline__ void dc_block_scores(DcChunk& W) {
   float most_k = 0.f, most_q = 0.f, most_g = 0.f;
   uint8_t* to = smem + (lane & 3) * 4;
   float2* raw_kq = reinterpret_cast<float2*>(smem);      // k, q and g as they are, 64 channels at a time: [64][64] pairs of k and q, [64][64] of g
-  float* raw_g = reinterpret_cast<float*>(smem + kDcL * 64 * 8);
+  float* raw_g = reinterpret_cast<float*>(smem + (kDcL * 64 + 16) * 8);        // (rows of a block of 16 are 4 elements on: blocks in other banks)
 #pragma unroll 1
   for (int half = 0; half < D / 64; ++half) {
     float2* tau = reinterpret_cast<float2*>(L.tau() + half * 512) + lane;
@@ -275,7 +276,7 @@ __device__ __forceinline__ void dc_block_scores(DcChunk& W) {
       for (int x = 0; x < 8; ++x) {
         most_k = largest(most_k, kk[x]), most_q = largest(most_q, qq[x]), most_g = largest(most_g, gg[x]);
         all = mul2(all, gg[x]);
-        const int at = (8 * warp + x) * 64 + 2 * lane;
+        const int at = (8 * warp + x) * 64 + 2 * lane + (warp >> 1) * 4;
         *reinterpret_cast<float4*>(raw_kq + at) = make_float4(kk[x].x, qq[x].x, kk[x].y, qq[x].y);
         *reinterpret_cast<float2*>(raw_g + at) = gg[x];
       }
@@ -287,29 +288,23 @@ __device__ __forceinline__ void dc_block_scores(DcChunk& W) {
     auto walk = [&](auto group) {
       constexpr int J = 4 * decltype(group)::value, N = 16 - J;
       const int slice = lane & 3, own = (lane >> 2) & 1, block = lane >> 3;
-      const int at = (16 * block + J) * 64 + (warp >> 1) * 16 + slice * 4;
-      float a[2][N], b[2][N], p[2][4];
+      int at = (16 * block + J) * 64 + block * 4 + (warp >> 1) * 16 + slice;
+      float a[2][N], b[2][N], p[2];
 #pragma unroll
-      for (int x = 0; x < 2; ++x)
+      for (int i = 0; i < N; ++i) a[0][i] = a[1][i] = b[0][i] = b[1][i] = 0.f;
+#pragma unroll 1
+      for (int e = 0; e < 4; ++e, at += 4) {             // (a loop, and not its four rounds behind one another: less code to fetch)
 #pragma unroll
-        for (int e = 0; e < 4; e += 2) {
-          const float4 y = *reinterpret_cast<const float4*>(raw_kq + at + (2 * own + x) * 64 + e);
-          p[x][e] = y.x, p[x][e + 1] = y.z;
-        }
+        for (int x = 0; x < 2; ++x) p[x] = raw_kq[at + (2 * own + x) * 64].x;
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        if (i % 2 == 0) asm volatile("" ::: "memory");   // (loads of later tokens would take the sums' registers)
-        const float4 g4 = *reinterpret_cast<const float4*>(raw_g + at + i * 64);
-        const float4 y0 = *reinterpret_cast<const float4*>(raw_kq + at + i * 64), y1 = *reinterpret_cast<const float4*>(raw_kq + at + i * 64 + 2);
-        const float g_[4] = {g4.x, g4.y, g4.z, g4.w}, k_[4] = {y0.x, y0.z, y1.x, y1.z}, q_[4] = {y0.y, y0.w, y1.y, y1.w};
+        for (int i = 0; i < N; ++i) {
+          const float2 y = raw_kq[at + i * 64];
+          const float g = raw_g[at + i * 64];
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          a[x][i] = b[x][i] = 0.f;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (i >= 4 || i > 2 * own + x) p[x][e] *= g_[e];
-            a[x][i] = fmaf(k_[e], p[x][e], a[x][i]);
-            b[x][i] = fmaf(q_[e], p[x][e], b[x][i]);
+          for (int x = 0; x < 2; ++x) {
+            if (i >= 4 || i > 2 * own + x) p[x] *= g;
+            a[x][i] = fmaf(y.x, p[x], a[x][i]);
+            b[x][i] = fmaf(y.y, p[x], b[x][i]);
           }
         }
       }
@@ -334,7 +329,7 @@ __device__ __forceinline__ void dc_block_scores(DcChunk& W) {
     float2 kk[8], qq[8], gg[8], f = one, near = one;
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
-      const int at = (8 * warp + x) * 64 + 2 * lane;
+      const int at = (8 * warp + x) * 64 + 2 * lane + (warp >> 1) * 4;
       const float4 y = *reinterpret_cast<const float4*>(raw_kq + at);
       kk[x] = make_float2(y.x, y.z), qq[x] = make_float2(y.y, y.w), gg[x] = *reinterpret_cast<const float2*>(raw_g + at);
     }
@@ -1130,11 +1125,12 @@ static int64_t dc_record(int D) { return D == 128 ? DcRecord<128>::kBytes : DcRe
 // 1 to 64 at a time: chunks by the waves of delta_chunk_kernel (a little CTA of a wave that finds SMs empty takes 0.6 of one) and the length that a
 // scan's CTA walks; all but two of the points within 11 %, where two CTAs' worth of waves lie between them. us, tokens / chunks (a decay per channel;
 // with strong decays):
-//   8 heads of 128:  1 x 128 48 / 37 (47), x 256 93 / 45 (56), x 1024 361 / 99 (110);  4 x 256 93 / 50 (61);  8 x 400 144 / 111 (151);  16 x 96 61 / 57 (76),
-//                    x 256 153 / 106 (153), x 400 236 / 174 (253), x 1024 594 / 325 (463);  64 x 128 305 / 198 (286);  16 of 500-1300 699 / 318 (463);
-//                    1024 beside 32 x 1 364 / 140 (177), beside 64 x 16 430 / 176 (233);  [1 x 96 37 / 37 (47), 8 x 96 38 / 41 (52): tokens]
-//   32 heads of 64:  1 x 128 40 / 32 (40), x 256 77 / 43 (51), x 1024 299 / 121 (146);  2 x 400 119 / 79 (94);  4 x 256 77 / 70 (92), x 1024 301 / 227 (291);
-//                    4 of 300-600 177 / 142 (185);  [4 x 400 119 / 128, 8 x 256 78 / 116, 16 x 1024 510 / 755: tokens]
+//   8 heads of 128:  1 x 128 48 / 37 (46), x 256 93 / 45 (55), x 1024 361 / 99 (108);  4 x 256 93 / 50 (59);  8 x 400 144 / 111 (143);  16 x 96 61 / 57 (72),
+//                    x 192 116 / 96 (126), x 256 153 / 106 (144), x 400 236 / 174 (232), x 1024 594 / 325 (416);  64 x 96 231 / 200 (260), x 128 305 / 198 (261);
+//                    16 of 500-1300 699 / 317 (414);  1024 beside 32 x 1 364 / 140 (171), beside 64 x 16 430 / 176 (222);  [1 x 96 37 / 37 (47), 8 x 96 38 / 41 (52): tokens]
+//   32 heads of 64:  1 x 128 40 / 32 (39), x 256 77 / 43 (50), x 1024 299 / 121 (144);  2 x 400 119 / 79 (92);  4 x 256 77 / 70 (89), x 512 151 / 131 (174),
+//                    x 1024 301 / 227 (286);
+//                    4 of 300-600 177 / 142 (181);  [4 x 400 119 / 128, 8 x 256 78 / 116, 16 x 1024 510 / 755: tokens]
 // A decay per head: tokens 0.86 to 0.93 of that, chunks the same.
 static bool dc_shape(int mode, int dtype, int num_seqs, int max_q, int64_t total_q, int H, int kdim, int vdim) {
   if (mode == kWkv || dtype != B200_DTYPE_BF16 || num_seqs <= 0 || num_seqs > 65535 || kdim != vdim || max_q < 96) return false;
