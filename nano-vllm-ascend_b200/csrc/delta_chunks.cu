@@ -22,12 +22,12 @@
 //   w -> three terms; o out;  dS^T = w^T (P_end / P_j k_j)    M128 N = D K64;   S = P_end S + dS in registers.
 // Every fp32 operand is three bf16 terms (24 bits, exact), six products, small ones first; values are bf16 as they are. One operand of every
 // product is split by rounding: where both are by cutting off, the three products left out have one sign and lack 6e-8 on average.
-// Outputs are 0.8 to 0.98 times as far from 64 bits as the token form's, states 0.4 to 1.15 times, where the last token is nearly all of a
-// state 1.4 (test_no_precision_is_lost; the inputs of 16 prompts below: 2.0e-7 of either).
+// Outputs are 0.45 to 0.98 times as far from 64 bits as the token form's, states 0.34 to 1.15 times, where the last token is nearly all of a
+// state 1.3 to 1.5 (test_no_precision_is_lost).
 //
-// What bounds them, 16 prompts of 500-1300 tokens, 8 heads of 128 (delta_rule_kernel 650 us): delta_chunk_kernel 205, a CTA's phases behind
-// one another (loads, scores, substitution, products, 48000 cycles, of which 11000 are issue); delta_scan_kernel 106, the chain
-// E -> w -> dS -> S -> E of 8500 cycles a chunk, 6000 of them for 72 MMAs. The records that pass between them (216 KB per chunk and head
+// What bounds them, 16 prompts of 500-1250 tokens, 8 heads of 128 (delta_rule_kernel 700 us): delta_chunk_kernel 213, a CTA's phases behind
+// one another (loads, scores, substitution, products, 48000 cycles, of which 11000 are issue, and code that has to be fetched); delta_scan_kernel
+// 104, the chain E -> w -> dS -> S -> E of 8500 cycles a chunk, 6000 of them for 72 MMAs. The records that pass between them (216 KB per chunk and head
 // of 128, written and read once) would take 2 x 63 at HBM's rate.
 //
 // Decays per channel that come to less than 2^-83 over half a chunk (0.17 a token) would take the reciprocals, or low terms, out of the range: a CTA
@@ -1122,15 +1122,14 @@ static int64_t dc_chunks(int num_seqs, int64_t total_q) { return total_q / kDcL 
 static int64_t dc_record(int D) { return D == 128 ? DcRecord<128>::kBytes : DcRecord<64>::kBytes; }
 
 // Steps with a span of 96 tokens at least whose chunks are the faster way. Both ways' times in ns, fitted to the times of prompts of 96 to 1024 tokens,
-// 1 to 64 at a time: chunks by the waves of delta_chunk_kernel (a little CTA of a wave that finds SMs empty takes 0.6 of one) and the length that a
-// scan's CTA walks; all but two of the points within 11 %, where two CTAs' worth of waves lie between them. us, tokens / chunks (a decay per channel;
-// with strong decays):
+// 1 to 64 at a time: chunks by the waves of delta_chunk_kernel (one that leaves no SM a second CTA takes 0.6 of a full one) and the length that a
+// scan's CTA walks; 70 of 75 points are met within 11 %. Strong decays are not the host's to see: the line is for decays that need no blocks. us,
+// tokens / chunks (with strong decays), a decay per channel:
 //   8 heads of 128:  1 x 128 48 / 37 (46), x 256 93 / 45 (55), x 1024 361 / 99 (108);  4 x 256 93 / 50 (59);  8 x 400 144 / 111 (143);  16 x 96 61 / 57 (72),
 //                    x 192 116 / 96 (126), x 256 153 / 106 (144), x 400 236 / 174 (232), x 1024 594 / 325 (416);  64 x 96 231 / 200 (260), x 128 305 / 198 (261);
 //                    16 of 500-1300 699 / 317 (414);  1024 beside 32 x 1 364 / 140 (171), beside 64 x 16 430 / 176 (222);  [1 x 96 37 / 37 (47), 8 x 96 38 / 41 (52): tokens]
 //   32 heads of 64:  1 x 128 40 / 32 (39), x 256 77 / 43 (50), x 1024 299 / 121 (144);  2 x 400 119 / 79 (92);  4 x 256 77 / 70 (89), x 512 151 / 131 (174),
-//                    x 1024 301 / 227 (286);
-//                    4 of 300-600 177 / 142 (181);  [4 x 400 119 / 128, 8 x 256 78 / 116, 16 x 1024 510 / 755: tokens]
+//                    x 1024 301 / 227 (286);  4 of 300-600 177 / 142 (181);  [4 x 400 119 / 128, 8 x 256 78 / 116, 16 x 1024 510 / 755: tokens]
 // A decay per head: tokens 0.86 to 0.93 of that, chunks the same.
 static bool dc_shape(int mode, int dtype, int num_seqs, int max_q, int64_t total_q, int H, int kdim, int vdim) {
   if (mode == kWkv || dtype != B200_DTYPE_BF16 || num_seqs <= 0 || num_seqs > 65535 || kdim != vdim || max_q < 96) return false;
