@@ -1245,12 +1245,13 @@ def wkv(r, k, v, decay, bonus, spans: StepSpans, num_heads, kdim, vdim, state=No
 
 def _lent(need, device):
     """`need` bytes to work in, or what there is: a quarter, a sixteenth, .. (more passes), down to a MB. None: nothing is left."""
-    while need >= 1 << 20:
+    while True:
         try:
             return torch.empty(need, dtype=torch.uint8, device=device)
         except torch.OutOfMemoryError:
             need //= 4
-    return None
+            if need < 1 << 20:
+                return None
 
 
 def _fp32_state_rule(mode, q, k, v, g, beta, spans: StepSpans, num_heads, groups, kdim, vdim, state, state_slots):

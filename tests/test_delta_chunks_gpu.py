@@ -153,11 +153,12 @@ def test_strong_decays_of_few_channels(H, G, N, pattern, n):
 
 @pytest.mark.parametrize("H,G,N", SIZES)
 @pytest.mark.parametrize("with_state", [False, True])
-def test_any_workspace_gives_the_same(H, G, N, with_state):
+@pytest.mark.parametrize("decay", ["mild", "strong"])
+def test_any_workspace_gives_the_same(H, G, N, decay, with_state):
     """One chunk of every head at a time, a few, all: the same bits (a pass hands the state on in fp32)."""
     from nanovllm import _C
     lens = [200, 1, 130, 64, 333]
-    q, k, v, gate, beta, g = _inputs(lens, H, G, N, False)
+    q, k, v, gate, beta, g = _inputs(lens, H, G, N, False, decay)
     first = torch.randn(len(lens), H, N, N, device="cuda", generator=g)
     spans, slots = _spans(lens, [5, 0, 3, 0, 0] if with_state else [0] * 5), torch.arange(len(lens), dtype=torch.int32, device="cuda") if with_state else None
     whole = _C.load().b200_delta_rule_workspace_size(len(lens), max(lens), sum(lens), H, G, N, N, 0, 0)
@@ -326,3 +327,14 @@ def test_what_memory_there_is(monkeypatch, free):
         got = ops.delta_rule(q, k, v, gate, beta, spans, H, G, N, N)
     assert (len(asked) == 1) == (free > 1 << 30)
     assert torch.equal(got, want if free else _call("tokens", q, k, v, gate, beta, spans, H, G, N, None, None))
+
+
+def test_a_step_whose_workspace_is_small_takes_chunks():
+    """Less than a MB, which is where a step gives up asking for less: it is asked for all the same."""
+    from nanovllm import _C, ops
+    H, G, N, lens = 2, 2, 64, [130]
+    q, k, v, gate, beta, _ = _inputs(lens, H, G, N, False)
+    spans = _spans(lens, [0])
+    assert 0 < _C.load().b200_delta_rule_workspace_size(1, 130, 130, H, G, N, N, 0, 0) < 1 << 20
+    out = ops.delta_rule(q, k, v, gate, beta, spans, H, G, N, N)
+    assert not torch.equal(out, _call("tokens", q, k, v, gate, beta, spans, H, G, N, None, None))
