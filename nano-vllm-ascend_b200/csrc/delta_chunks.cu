@@ -293,7 +293,7 @@ __device__ __forceinline__ void dc_block_scores(DcChunk& W) {
 #pragma unroll
       for (int i = 0; i < N; ++i) a[0][i] = a[1][i] = b[0][i] = b[1][i] = 0.f;
 #pragma unroll 1
-      for (int e = 0; e < 4; ++e, at += 4) {             // (a loop, and not its four rounds behind one another: less code to fetch)
+      for (int e = 0; e < 4; ++e, at += 4) {             // (a loop, not unrolled: less code to fetch)
 #pragma unroll
         for (int x = 0; x < 2; ++x) p[x] = raw_kq[at + (2 * own + x) * 64].x;
 #pragma unroll
