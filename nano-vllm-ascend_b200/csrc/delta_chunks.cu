@@ -194,22 +194,18 @@ struct DcChunk {                                         // and what a CTA knows
   int* wait_status;
   __device__ __forceinline__ bool wait(uint64_t* bar, int parity, volatile int* gave_up) const { return mbar_warp_wait(bar, parity & 1, wait_tries, gave_up); }
 };
-// 8 tokens of two channels
+// 8 tokens of two channels. (Full chunks without the questions, in code of their own, were slower: 316 us for 314, strong decays 415 for 401)
 template <bool PER_HEAD>
 __device__ __forceinline__ void dc_fetch(const DcTokens& C, int t0, int ch, float2 (&kk)[8], float2 (&qq)[8], float2 (&gg)[8]) {
-  auto rows = [&](auto all) {
-    uint32_t ka = t0 * C.k_step + ch * 4, qa = t0 * C.q_step + ch * 4, ga = t0 * C.g_step + ch * 4;
+  uint32_t ka = t0 * C.k_step + ch * 4, qa = t0 * C.q_step + ch * 4, ga = t0 * C.g_step + ch * 4;
 #pragma unroll
-    for (int x = 0; x < 8; ++x) {
-      const bool ok = decltype(all)::value || t0 + x < C.nt;
-      kk[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(C.k) + ka) : make_float2(0.f, 0.f);
-      qq[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(C.q) + qa) : make_float2(0.f, 0.f);
-      if (!PER_HEAD) gg[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(C.g) + ga) : make_float2(1.f, 1.f);
-      ka += C.k_step, qa += C.q_step, ga += C.g_step;
-    }
-  };
-  if (t0 + 8 <= C.nt) rows(std::true_type{});
-  else rows(std::false_type{});
+  for (int x = 0; x < 8; ++x) {
+    const bool ok = t0 + x < C.nt;
+    kk[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(C.k) + ka) : make_float2(0.f, 0.f);
+    qq[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(C.q) + qa) : make_float2(0.f, 0.f);
+    if (!PER_HEAD) gg[x] = ok ? *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(C.g) + ga) : make_float2(1.f, 1.f);
+    ka += C.k_step, qa += C.q_step, ga += C.g_step;
+  }
 }
 // two channels of a token into row x of a group of eight rows of the operands: of K~ and Q~, of K^
 __device__ __forceinline__ void dc_put_up(uint8_t* group, int lane, int x, float2 kk, float2 qq, float2 up) {
@@ -249,8 +245,8 @@ __device__ __forceinline__ void dc_issue_scores(uint8_t* smem, uint32_t to, uint
 // Accumulators as delta_chunk_kernel's, of which columns 0-31 are what rows of tokens 32 to 63 have of tokens 0 to 31, and columns 32-63 of tokens
 // 0 to 15 and 32 to 47, for tokens 16 to 31 in their rows, 48 to 63 in rows 0 to 15. What bounds a CTA here: phases behind one another, of 8 warps
 // (an instruction every 3.2 cycles; code that does not fit the instruction cache is the first of its stalls: with the four channels of a lane behind one
-// another instead of in a loop, the first figure is 461). us, token form / so / decays that need it not: 16 prompts of 500-1300, 8 heads of 128 700 / 414 /
-// 317, 1 x 1024 360 / 108 / 99, 4 x 256 93 / 59 / 49; 32 heads of 64 1 x 1024 299 / 144 / 121
+// another instead of in a loop, the first figure is 461). us, token form / so / decays that need it not: 16 prompts of 500-1250, 8 heads of 128 700 / 401 /
+// 314, 1 x 1024 360 / 108 / 99, 4 x 256 93 / 59 / 49; 32 heads of 64 1 x 1024 299 / 144 / 121
 template <int D>
 __device__ __forceinline__ void dc_block_scores(DcChunk& W) {
   const DcLocal<D> L;
@@ -1127,7 +1123,7 @@ static int64_t dc_record(int D) { return D == 128 ? DcRecord<128>::kBytes : DcRe
 // tokens / chunks (with strong decays), a decay per channel:
 //   8 heads of 128:  1 x 128 48 / 37 (46), x 256 93 / 45 (55), x 1024 361 / 99 (108);  4 x 256 93 / 50 (59);  8 x 400 144 / 111 (143);  16 x 96 61 / 57 (72),
 //                    x 192 116 / 96 (126), x 256 153 / 106 (144), x 400 236 / 174 (232), x 1024 594 / 325 (416);  64 x 96 231 / 200 (260), x 128 305 / 198 (261);
-//                    16 of 500-1300 699 / 317 (414);  1024 beside 32 x 1 364 / 140 (171), beside 64 x 16 430 / 176 (222);  [1 x 96 37 / 37 (47), 8 x 96 38 / 41 (52): tokens]
+//                    16 of 500-1250 699 / 314 (401);  1024 beside 32 x 1 364 / 140 (171), beside 64 x 16 430 / 176 (222);  [1 x 96 37 / 37 (47), 8 x 96 38 / 41 (52): tokens]
 //   32 heads of 64:  1 x 128 40 / 32 (39), x 256 77 / 43 (50), x 1024 299 / 121 (144);  2 x 400 119 / 79 (92);  4 x 256 77 / 70 (89), x 512 151 / 131 (174),
 //                    x 1024 301 / 227 (286);  4 of 300-600 177 / 142 (181);  [4 x 400 119 / 128, 8 x 256 78 / 116, 16 x 1024 510 / 755: tokens]
 // A decay per head: tokens 0.86 to 0.93 of that, chunks the same.
